@@ -212,6 +212,7 @@ struct Plan {
     int64_t v0, v1;  // global vis range
     int t0, t1;      // global tile range
     int T, W, chunk; // tile, warps per sub-grid group (0: by support), records per item
+    bool reg;        // register-tile kernel
   };
   std::vector<ClassRange> classes;
   std::vector<JobDesc> hjobs;
@@ -350,6 +351,7 @@ static int resolve_mode(const gg_options *o, int S, int vals_f64) {
 // Launch configuration of one support class of the moving window
 struct ClassCfg {
   int T = 0, W = 0, chunk = 0;
+  bool reg = false;  // register-tile kernel (regtile_class)
 };
 using ClassCfgs = std::map<int, ClassCfg>;  // by support
 
@@ -420,11 +422,48 @@ static const TuneEntry *tune_lookup(const TuneKey &k) {
   return best;
 }
 
+// Whether the moving-window class of support S takes the register-tile kernel:
+// one-warp groups on 8-cell tiles (the defaults of supports 8 and 16) of FP32
+// values, binned by the library, with one GCF table for the whole class, whose
+// padded copy has to fit an SM's shared memory (oversampling up to 8).
+static bool regtile_class(const gg_options *o, const gg_job *jobs, int njobs, int S,
+                          const ClassCfg &cf) {
+  if ((S != 8 && S != 16) || cf.T != kRegTile || cf.W > 1 || o->input_sorted) return false;
+  if (regtile_smem_bytes(S, o->oversample) > 227 * 1024) return false;
+  const gg_job *one = nullptr;
+  for (int j = 0; j < njobs; ++j) {
+    if (jobs[j].gcf_dim != S) continue;
+    if (jobs[j].vals_type != GG_C64 || jobs[j].gcf_index) return false;
+    if (o->gcf_kind == GG_GCF_TABLE && one && jobs[j].gcf != one->gcf) return false;
+    one = &jobs[j];
+  }
+  return one != nullptr;
+}
+
+// Records per work item of a register-tile class when the caller leaves it
+// open: four items for every resident warp, between 64 records (a warp's item
+// is a serial chain, and small jobs leave most warps without one) and 512
+// (every item reduces its whole sub-grid once; 256 mixed jobs 5.53 ms, with
+// 256 records 5.74, with 128 6.37).
+static int regtile_chunk(int64_t vis, int sm_count) {
+  const int64_t c = vis / ((int64_t)sm_count * 16 * 4);
+  return (int)std::min<int64_t>(512, std::max<int64_t>(64, (c + 31) / 32 * 32));
+}
+
+// uv tiles along one axis of a job
+static int64_t tile_side(int64_t N, int S, const ClassCfg &cf) {
+  // main cells up to N + S/2 - 2 reach the grid
+  if (cf.reg) return ((N + S / 2 - 2 + kRegOff) / kRegTile) + 1;
+  return (N + cf.T - 1) / cf.T;
+}
+
 // Build the plan for a batch: validate, resolve, order jobs by support class,
 // lay out the workspace.  No device work.  `force` fixes the configuration of
-// support classes (autotuner trials).
+// support classes (autotuner trials); `bin_only`: the caller wants the tiles
+// of set_bookmarks (gg_bin), nothing is gridded.
 static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
-                      int njobs, Plan &pl, const ClassCfgs *force = nullptr) {
+                      int njobs, Plan &pl, const ClassCfgs *force = nullptr,
+                      bool bin_only = false) {
   int st = check_options(opt);
   if (st) return st;
   if (njobs < 1) return fail(GG_ERR_ARG, "no jobs");
@@ -444,14 +483,14 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
       if (cfgs.count(S)) continue;
       // automatic tile: the moving window keeps one (T+S-1)^2 sub-grid per
       // warp group, so supports up to 16 use 8-cell tiles (small sub-grids,
-      // many resident groups: measured fastest on every track workload);
+      // held in registers where regtile_class allows it);
       // gather needs 32; input declared tile-sorted: the caller's tiles are
       // the default 32
       ClassCfg cf;
       cf.T = opt->tile > 0 ? opt->tile
                            : (m0 == GG_MODE_WINDOW && S <= 16 && !opt->input_sorted ? 8 : 32);
       cf.W = opt->group_warps;
-      cf.chunk = opt->window_chunk > 0 ? opt->window_chunk : 2048;
+      cf.chunk = opt->window_chunk;  // 0: chosen below
       if (m0 == GG_MODE_WINDOW && tunable(opt)) {
         if (force && force->count(S)) {
           cf = force->at(S);
@@ -461,6 +500,14 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
           if (e) cf = e->cfg;
         }
       }
+      cf.reg = m0 == GG_MODE_WINDOW && !bin_only && regtile_class(opt, jobs, njobs, S, cf);
+      if (cf.reg && cf.chunk == 0) {
+        int64_t cvis = 0;
+        for (int i = 0; i < njobs; ++i)
+          if (jobs[i].gcf_dim == S) cvis += std::max<int64_t>(0, jobs[i].npts);
+        cf.chunk = regtile_chunk(cvis, c->sm_count);
+      }
+      if (cf.chunk == 0) cf.chunk = 2048;
       cfgs[S] = cf;
     }
     pl.T = cfgs.begin()->second.T;
@@ -537,7 +584,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     if (mode == GG_MODE_GATHER && J.gcf_index)
       return fail(GG_ERR_ARG, "job %d: gcf_index: use the scatter or moving-window method", j);
     vis += J.npts;
-    int ntx = (int)((J.img_dim + T - 1) / T);
+    const int64_t ntx = tile_side(J.img_dim, (int)J.gcf_dim, cfgs[(int)J.gcf_dim]);
     tiles += (int64_t)ntx * ntx * (J.gcf_index ? J.n_gcf : 1);
   }
   if (vis >= (1ll << 31) - 1024) return fail(GG_ERR_ARG, "batch has >= 2^31 visibilities");
@@ -546,6 +593,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
   if (mode == GG_MODE_WINDOW) {
     for (int j = 0; j < njobs; ++j) {
       const ClassCfg &cf = cfgs[(int)jobs[j].gcf_dim];
+      if (cf.reg) continue;
       const size_t need = window_smem_bytes((int)jobs[j].gcf_dim, opt->accum, vt == GG_C128,
                                             cf.T, cf.W, opt->gcf_kind == GG_GCF_GAUSSIAN);
       if (need > 227 * 1024)
@@ -610,6 +658,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     std::map<std::tuple<const void *, int, int>, size_t> seen;  // -> copy index
     for (int k = 0; k < njobs; ++k) {
       const gg_job &J = jobs[order[k]];
+      if (cfgs[(int)J.gcf_dim].reg) continue;  // reads the caller's table
       const int ntab = J.gcf_index ? (int)J.n_gcf : 1;
       const std::tuple<const void *, int, int> key(count ? nullptr : J.gcf, (int)J.gcf_dim, ntab);
       auto it = seen.find(key);
@@ -636,7 +685,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
       for (int j = 0; j < njobs; ++j)
         if (jobs[j].gcf_dim == S) {
           cvis += jobs[j].npts;
-          const int64_t ntx = (jobs[j].img_dim + kv.second.T - 1) / kv.second.T;
+          const int64_t ntx = tile_side(jobs[j].img_dim, S, kv.second);
           ctiles += ntx * ntx * (jobs[j].gcf_index ? jobs[j].n_gcf : 1);
           c64 |= jobs[j].out_type == GG_C64;
         }
@@ -672,11 +721,11 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
         pl.classes.back().t1 = tb;
       }
       const ClassCfg &cf = cfgs[S];
-      pl.classes.push_back({S, k, k, vb, vb, tb, tb, cf.T, cf.W, cf.chunk});
+      pl.classes.push_back({S, k, k, vb, vb, tb, tb, cf.T, cf.W, cf.chunk, cf.reg});
     }
     const int T = pl.classes.back().T;
     const int N = (int)J.img_dim;
-    const int ntx = (N + T - 1) / T;
+    const int ntx = (int)tile_side(N, S, cfgs[S]);
     JobDesc &D = pl.hjobs[k];
     memset(&D, 0, sizeof D);
     D.out = J.out;
@@ -693,6 +742,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     D.T = T;
     D.log2T = ilog2(T);
     D.ntx = ntx;
+    D.off = cfgs[S].reg ? kRegOff : 0;
     int layout = opt->layout;
     if (layout == GG_LAYOUT_REFERENCE)
       layout = mode == GG_MODE_WINDOW ? GG_LAYOUT_PLANAR : GG_LAYOUT_INTERLEAVED;
@@ -720,6 +770,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     B.ntx = ntx;
     B.P = pl.P;
     B.uv_f64 = D.uv_f64;
+    B.off = D.off;
     pl.hvis_base[k] = vb;
     pl.htile_base[k] = tb;
     pl.hclass[k] = (int)pl.classes.size() - 1;
@@ -932,7 +983,29 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
       g.item_next = flags + 12 + ci;
       g.max_items = pl.class_cap;
       g.merge = slots.m[ci];
-      GG_CUDA(launch_window(g, s));
+      if (cl.reg) {
+        RegTileLaunch r{};
+        r.jobs = djobs;
+        r.items = g.items;
+        r.nitems = g.nitems;
+        r.item_next = g.item_next;
+        r.idx = (const int2 *)(ws + pl.o_sidx);
+        r.vals = (const float2 *)(ws + pl.o_svals);
+        r.vstride = pl.vstride;
+        r.gcf = (const float2 *)pl.hjobs[cl.j0].gcf;
+        r.S = cl.S;
+        r.G = pl.G;
+        r.P = pl.P;
+        r.compensated = pl.accum == GG_ACC_COMPENSATED;
+        r.gauss = pl.gauss;
+        r.sigma = pl.sigma;
+        r.max_items = std::min<int64_t>(pl.class_cap, cl.v1 - cl.v0);
+        r.sm_count = sm_count;
+        r.merge = slots.m[ci];
+        GG_CUDA(launch_regtile(r, s));
+      } else {
+        GG_CUDA(launch_window(g, s));
+      }
       GG_CUDA(launch_merge_finalize(slots.m[ci], flags + 16 + ci, djobs, cl.S, cl.T, pl.P,
                                     sm_count, s));
     }
@@ -1511,7 +1584,7 @@ int gg_bin(gg_context *ctx, const gg_options *opt, int uv_type, const void *uv,
   j.out_type = GG_C64;
   if (o.tile != 32) o.mode = GG_MODE_WINDOW;
   Plan pl;
-  int st = plan_build(ctx, &o, &j, 1, pl);
+  int st = plan_build(ctx, &o, &j, 1, pl, nullptr, true);
   if (st) return st;
   pl.P = 1;
   if (pl.ws_bytes > ctx->ws.n) GG_CUDA(cudaEventSynchronize(ctx->exec_done));

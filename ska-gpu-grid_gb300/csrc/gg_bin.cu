@@ -140,8 +140,9 @@ __global__ void __launch_bounds__(256) bin_count_kernel(BinBuffers b) {
         pk = make_int2(mx * J.G + sx, my * J.G + sy);
         const int h = J.S >> 1;
         if (mx + h >= 0 && mx - h + 1 < J.N && my + h >= 0 && my - h + 1 < J.N) {
-          int cx = min(max(mx, 0), J.N - 1) >> J.log2T;
-          int cy = min(max(my, 0), J.N - 1) >> J.log2T;
+          // register tiles start before the grid and need no clamping
+          const int cx = (J.off ? mx + J.off : min(max(mx, 0), J.N - 1)) >> J.log2T;
+          const int cy = (J.off ? my + J.off : min(max(my, 0), J.N - 1)) >> J.log2T;
           key = J.tile_base + (cy * J.ntx + cx) * J.n_gcf + gi;
         }
       }
@@ -208,10 +209,13 @@ __global__ void __launch_bounds__(256) bin_scatter_kernel(BinBuffers b) {
       if (key >= 0) pos = start + __popc(peers & lanemask_lt());
     }
     if (pos >= 0) {
-      b.sorted_idx[pos] = b.window_records
-                              ? window_record(pk.x >> J->log2G, pk.x & (J->G - 1),
-                                              pk.y >> J->log2G, pk.y & (J->G - 1), J->G)
-                              : pk;
+      if (b.window_records) {
+        const int mx = pk.x >> J->log2G, sx = pk.x & (J->G - 1);
+        const int my = pk.y >> J->log2G, sy = pk.y & (J->G - 1);
+        pk = J->off ? regtile_record(mx & (kRegTile - 1), sx, my & (kRegTile - 1), sy, J->G, J->S)
+                    : window_record(mx, sx, my, sy, J->G);
+      }
+      b.sorted_idx[pos] = pk;
       if (b.vals_bytes == 8) {
         const float2 *v = (const float2 *)J->vals + n * b.P;
         float2 *o = (float2 *)b.sorted_vals;
@@ -425,14 +429,23 @@ __global__ void __launch_bounds__(256)
       if (kc) {
         WorkItem *dst = items + c * class_cap + start + (incl - kc);
         int local = t - tile_base[j];
+        int ox = 0, oy = 0;
+        if (jobs) {
+          const JobDesc &J = jobs[j];
+          const int tile = J.n_gcf > 1 ? local / J.n_gcf : local;
+          ox = (tile % J.ntx) * J.T - J.off - J.S / 2 + 1;
+          oy = (tile / J.ntx) * J.T - J.off - J.S / 2 + 1;
+        }
         for (int i = 0; i < kc; ++i) {
           WorkItem w;
+          w.ox = ox;
+          w.oy = oy;
           w.job = j;
           w.bin = local;
           w.start = s0 + i * chunk;
           w.end = min(e0, s0 + (i + 1) * chunk);
           w.slot = slot;
-          w.pad_[0] = w.pad_[1] = w.pad_[2] = 0;
+          w.pad_ = 0;
           dst[i] = w;
         }
       }
@@ -485,7 +498,7 @@ __global__ void __launch_bounds__(256)
     const int2 d = m.desc[sl];
     const JobDesc &J = jobs[d.x];
     const int tile = J.n_gcf > 1 ? d.y / J.n_gcf : d.y;
-    const int ox = (tile % J.ntx) * T - H + 1, oy = (tile / J.ntx) * T - H + 1;
+    const int ox = (tile % J.ntx) * T - J.off - H + 1, oy = (tile / J.ntx) * T - J.off - H + 1;
     const double2 *src = m.base + (size_t)sl * m.cells;
     for (int i = threadIdx.x; i < P * R * R; i += 256) {
       const double2 v = src[i];

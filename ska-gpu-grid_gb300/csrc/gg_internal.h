@@ -28,6 +28,7 @@ struct BinJob {
   int N, S, G, log2G, log2T, ntx, P;
   int uv_f64;
   int n_gcf;
+  int off;  // register-tile class: kRegOff (see regtile_record); else 0
 };
 
 struct BinBuffers {
@@ -66,6 +67,19 @@ constexpr int kWinMainBias = 64;
 __host__ __device__ inline int2 window_record(int mx, int sx, int my, int sy, int G) {
   return make_int2((int)(((unsigned)(my + kWinMainBias) << 16) | (unsigned)(mx + kWinMainBias)),
                    sy * G + sx);
+}
+
+// Sorted record of the register-tile kernel, for a main cell at (fx, fy) in
+// its 8-cell tile: the byte offset of the footprint's first tap, seen from
+// the sub-grid's first cell, in the table in shared memory, and the cell (fy
+// alone for support 8, fy | fx << 8 for 16).  Table rows are regtile_row bytes
+// long, their first tap at byte regtile_pad.
+__host__ __device__ constexpr int regtile_row(int S) { return S == 8 ? 80 : 96; }
+__host__ __device__ constexpr int regtile_pad(int S) { return S == 8 ? 32 : 0; }
+__host__ __device__ inline int2 regtile_record(int fx, int sx, int fy, int sy, int G, int S) {
+  const int row = regtile_row(S);
+  return make_int2((sy * G + sx) * S * row + regtile_pad(S) - 4 * fx - row * fy,
+                   S == 8 ? fy : fy | fx << 8);
 }
 
 // index step only (vis2ints)
@@ -193,6 +207,28 @@ cudaError_t launch_degrid(const DegridLaunch &d, cudaStream_t s);
 // first use); 0 on success, else a message in err.  Synchronises s.
 int image_inverse_fft(void *grid, int64_t N, int P, bool f64, int sm_count, cudaStream_t s,
                       std::string &err);
+
+// Register-tile moving window (gg_regtile.cu): FP32 values, support 8 or 16,
+// one GCF table per launch (its padded copy fills the CTA's shared memory).
+struct RegTileLaunch {
+  const JobDesc *jobs;
+  const WorkItem *items;
+  const int *nitems;
+  int *item_next;
+  const int2 *idx;         // sorted records (regtile_record)
+  const float2 *vals;      // sorted values, P planes of vstride
+  int64_t vstride;
+  const float2 *gcf;       // [G*G][S][S]
+  int S, G, P;
+  int compensated;
+  int gauss;               // factors computed from sigma instead of gcf
+  float sigma;
+  int64_t max_items;       // upper bound of *nitems
+  int sm_count;
+  MergeSlots merge;        // base null: none
+};
+cudaError_t launch_regtile(const RegTileLaunch &g, cudaStream_t s);
+size_t regtile_smem_bytes(int S, int G);
 
 cudaError_t launch_scatter(const GridLaunch &g, cudaStream_t s);
 cudaError_t launch_window(const GridLaunch &g, cudaStream_t s);

@@ -1,0 +1,503 @@
+// Moving-window gridding with the sub-grid of an 8-cell uv tile held in
+// registers (the reference's MOVING_WINDOW method, grid_kernel_window,
+// grid_gpu.cu:504-673, for FP32 values and supports 8 and 16).
+//
+// The visibilities of one 8x8 tile touch an R x R sub-grid, R = S + 7: 15x15
+// or 23x23 cells.  A warp takes a work item (a slice of a tile's sorted
+// records) and owns every cell of it: lane (lx, ly) of an LX x LY arrangement
+// holds the cells x = LX i + lx, y = LY j + ly, 8 cells for support 8 and 18
+// for support 16.  No cell ever moves, so a record costs its table loads and
+// its multiply-adds whether or not it moves the footprint: the shared-memory
+// sub-grid of window_kernel costs a read-modify-write of every tap at each
+// move, and on uv tracks most records move.
+//
+//  * Rows.  A footprint of S rows starting at fy in 0..7 covers, of the S + 8
+//    rows a lane owns, exactly S / LY: the rows j in [8/LY, S/LY) always, and
+//    of each pair (j, j + S/LY), j < 8/LY, the first when fy <= LY j + ly and
+//    the second otherwise.  The records of a block are therefore put in order
+//    of fy (a counting sort of up to kRtBlock records in shared memory): while
+//    fy stays the same a lane adds to one cell of each pair in a running sum,
+//    which goes to the right cell when fy changes.
+//  * Columns.  Support 8: table rows sit behind eight zeros in shared memory,
+//    so the four columns of a lane are read at fixed offsets and those outside
+//    the footprint read zero.  Support 16, whose table reads would bind: of
+//    its three columns the middle one is always inside and the outer two are
+//    complementary, so they share one load, and one of them gets the value
+//    replaced by zero.  The row length puts the LY rows that a warp reads in
+//    distinct banks.
+//  * Products by zero turn a value (or table entry) that is not finite into
+//    NaN in cells its footprint does not cover.  A sub-grid that is not finite
+//    at the end of its item is therefore summed again cell by cell, only
+//    inside footprints.
+//  * Compensated sums: a run of at most kRtRun records is summed plainly,
+//    then added into the cell's (hi, lo) pair by TwoSum.
+//  * The records of a block are fetched while the previous block (also of the
+//    previous plane or item) is summed.
+//  * Real and imaginary parts of the table are kept apart; an item of a table
+//    without imaginary parts never touches the second half.
+//
+// The whole table lives in each CTA's shared memory (2 x 98 KB for support 16
+// at oversampling 8), hence one CTA per SM and one table per launch.
+//
+// Bound by instruction issue (60-63 % of active cycles issue; 42 and 87 warp
+// instructions a record for supports 8 and 16 on the batched tracks, about
+// half of them sorting, TwoSum and flushes of small tiles).  Measured against
+// window_kernel on the same jobs: 4.19 M support-8 records of a 4096^2
+// observation 435 -> 253 us; 256 mixed jobs, 24.4 M support-8 records 1366 ->
+// 1337 us, 20.9 M support-16 records 3189 -> 2228 us; 100 k support-16 records
+// on 777^2 74 -> 47 us; 10 k support-8 records on 256^2 36 -> 13 us.
+#include <algorithm>
+
+#include "gg_kernels.cuh"
+
+namespace gg {
+
+namespace {
+
+constexpr int kRtRun = 16;
+// records sorted together: four per lane
+constexpr int kRtBlock = 128;
+// staged records: every fy's share is padded to an even number, and two more
+// are read ahead
+constexpr int kRtStage = kRtBlock + 8 + 2;
+
+template <int S> struct RtCfg {
+  static constexpr int LX = S == 8 ? 4 : 8, LY = 32 / LX;
+  static constexpr int NX = (S + 8) / LX, NY = (S + 8) / LY, R = S + kRegTile - 1;
+  static constexpr int Q = S / LY;      // rows of a footprint per lane
+  static constexpr int PAIRS = 8 / LY;  // rows j < PAIRS alternate with j + Q
+  // columns behind zeros (every column loaded), or shared loads of the
+  // outer columns (support 16: NX = 3, the first and last complementary)
+  static constexpr bool PADX = S == 8;
+  static constexpr int NL = PADX ? NX : 2;  // loads per row
+  static constexpr int WARPS = S == 8 ? 16 : 12;
+  static constexpr int ROW = regtile_row(S);  // bytes of a table row
+  static constexpr int PAD = regtile_pad(S);  // bytes before its first tap
+  static constexpr int SUB = S * ROW;
+};
+
+// floats of one table (a row behind the last: the zeros after its taps)
+__host__ __device__ constexpr int rt_table_floats(int S, int G) {
+  return (G * G * S + 1) * (regtile_row(S) / 4);
+}
+
+template <int OFF> __device__ __forceinline__ float lds(uint32_t a) {
+  float v;
+  asm("ld.shared.f32 %0, [%1+%2];" : "=f"(v) : "r"(a), "n"(OFF));
+  return v;
+}
+
+// compile-time loop
+template <int I, int N, class F> __device__ __forceinline__ void rt_for(F &&f) {
+  if constexpr (I < N) {
+    f(std::integral_constant<int, I>{});
+    rt_for<I + 1, N>(f);
+  }
+}
+
+// The sub-grid of an item whose packed sums are not finite, cell by cell and
+// only from the records whose footprints cover the cell.
+template <int S, bool COMP>
+__device__ __noinline__ void rt_redo(const RegTileLaunch &p, const WorkItem &w, int plane,
+                                     const float *tr, bool cplx, double2 *slot) {
+  using C = RtCfg<S>;
+  constexpr int R = C::R;
+  const JobDesc &J = p.jobs[w.job];
+  const float *const ti = tr + rt_table_floats(S, p.G);
+  for (int c = threadIdx.x & 31; c < R * R; c += 32) {
+    const int x = c % R, y = c / R;
+    const int gx = w.ox + x, gy = w.oy + y;
+    if ((unsigned)gx >= (unsigned)J.N || (unsigned)gy >= (unsigned)J.N) continue;
+    u64 run = 0ull, hi = 0ull, lo = 0ull;
+    int since = 0;
+    auto merge = [&]() {
+      u64 e;
+      hi = two_sum2(hi, run, e);
+      lo = add2(lo, e);
+      run = 0ull;
+      since = 0;
+    };
+    for (int k = w.start; k < w.end; ++k) {
+      const int2 q = __ldg(p.idx + k);
+      const int fy = q.y & 0xff;
+      const int fx = S == 8 ? (-(q.x + fy * C::ROW - C::PAD) & 31) >> 2 : q.y >> 8;
+      if ((unsigned)(x - fx) >= (unsigned)S || (unsigned)(y - fy) >= (unsigned)S) continue;
+      const float2 v = __ldg(p.vals + plane * p.vstride + k);
+      const int at = (q.x + y * C::ROW) / 4 + x;
+      run = fma2(pk2(v.x, v.y), pk2(tr[at], tr[at]), run);
+      if (cplx) run = fma2(pk2(-v.y, v.x), pk2(ti[at], ti[at]), run);
+      if (COMP && ++since == kRtRun) merge();
+    }
+    if (COMP) merge();
+    const float2 h = upk2(COMP ? hi : run), l = upk2(lo);
+    if (slot) {
+      red_add(&slot[c].x, (double)h.x + (double)l.x);
+      red_add(&slot[c].y, (double)h.y + (double)l.y);
+    } else if (J.out_f64) {
+      out_red(J, (size_t)gy * J.N + gx, plane, p.P, (double)h.x + (double)l.x,
+              (double)h.y + (double)l.y);
+    } else {
+      out_red(J, (size_t)gy * J.N + gx, plane, p.P, (double)__fadd_rn(h.x, l.x),
+              (double)__fadd_rn(h.y, l.y));
+    }
+  }
+}
+
+// A warp's share of the launch's items.
+template <int S, bool COMP>
+__device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr, float4 *stage,
+                                         bool cplx) {
+  using C = RtCfg<S>;
+  constexpr int LX = C::LX, LY = C::LY, NX = C::NX, NY = C::NY, R = C::R, Q = C::Q,
+                PAIRS = C::PAIRS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lx = lane % LX, ly = lane / LX;
+  const uint32_t tab = smem_addr(tr) + lx * 4 + ly * C::ROW;
+  const uint32_t im_off = 4u * rt_table_floats(S, p.G);
+  const int total = *p.nitems;
+  const int first = gridDim.x * C::WARPS;
+
+  // The first items are spread over the SMs; later ones are claimed ahead:
+  // while an item is summed, the range of the next is in registers and its
+  // first records, the range of the one after and a further claim are on
+  // their way.
+  int item = blockIdx.x + warp * gridDim.x;
+  auto claim_one = [&]() { return lane == 0 ? atomicAdd(p.item_next, 1) + first : 0; };
+  auto range = [&](int it) {
+    return it < total ? __ldg(reinterpret_cast<const int4 *>(p.items + it)) : make_int4(0, 0, 0, 0);
+  };
+  constexpr int PER = kRtBlock / 32;
+  int2 pk[PER];
+  float2 pv[PER];
+  auto fetch = [&](int k0, int end, int plane) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const int k = k0 + u * 32 + lane;
+      if (k < end) {
+        pk[u] = __ldg(p.idx + k);
+        pv[u] = __ldg(p.vals + plane * p.vstride + k);
+      }
+    }
+  };
+  if (item >= total) return;  // the whole warp; no barrier follows
+  int claim = claim_one();
+  int4 cur = range(item);  // {job, bin, start, end}
+  fetch(cur.z, cur.w, 0);
+  int next = __shfl_sync(0xffffffffu, claim, 0);
+  claim = claim_one();
+  int4 nxt = range(next);
+  while (true) {
+    const int next2 = __shfl_sync(0xffffffffu, claim, 0);
+    claim = claim_one();
+    const int4 nxt2 = range(next2);
+    const int4 tail = __ldg(reinterpret_cast<const int4 *>(p.items + item) + 1);  // {slot, ox, oy}
+    const JobDesc &J = p.jobs[cur.x];
+    const int N = J.N;
+    const bool other = J.out_f64 || J.planar;
+    float2 *const out = static_cast<float2 *>(J.out);
+    for (int plane = 0; plane < p.P; ++plane) {
+      // cells: (hi, lo) pairs, or plain sums in hi; run: the running sums of
+      // the rows that the current fy selects
+      u64 run[NX][Q], hi[NX][NY], lo[COMP ? NX : 1][COMP ? NY : 1];
+#pragma unroll
+      for (int i = 0; i < NX; ++i) {
+#pragma unroll
+        for (int j = 0; j < NY; ++j) {
+          hi[i][j] = 0ull;
+          if constexpr (COMP) lo[i][j] = 0ull;
+        }
+#pragma unroll
+        for (int j = 0; j < Q; ++j) run[i][j] = 0ull;
+      }
+      auto put = [&](int i, int j, u64 r) {
+        if constexpr (COMP) {
+          u64 e;
+          hi[i][j] = two_sum2(hi[i][j], r, e);
+          lo[i][j] = add2(lo[i][j], e);
+        } else {
+          hi[i][j] = add2(hi[i][j], r);
+        }
+      };
+      // the running sums of the alternating rows into the cells of fy = f
+      auto merge_pairs = [&](int f) {
+#pragma unroll
+        for (int j = 0; j < PAIRS; ++j) {
+          const bool low = f <= LY * j + ly;
+#pragma unroll
+          for (int i = 0; i < NX; ++i) {
+            put(i, j, low ? run[i][j] : 0ull);
+            put(i, j + Q, low ? 0ull : run[i][j]);
+            run[i][j] = 0ull;
+          }
+        }
+      };
+      // those of the rows that every footprint covers
+      auto merge_rest = [&]() {
+#pragma unroll
+        for (int j = PAIRS; j < Q; ++j)
+#pragma unroll
+          for (int i = 0; i < NX; ++i) {
+            put(i, j, run[i][j]);
+            run[i][j] = 0ull;
+          }
+      };
+      // one staged record: its table entries (h: imaginary parts) and value
+      struct Taps {
+        float g[Q][C::NL], h[Q][C::NL];
+        float vr, vi;
+        bool left;  // the first column, not the last, is in the footprint
+      };
+      auto load = [&](Taps &t, const float4 q, auto cx) {
+        const int at = __float_as_int(q.y);
+        const int fy = C::PADX ? at : at & 0xff;
+        t.vr = q.z;
+        t.vi = q.w;
+        t.left = at < (lx + 1) << 8;
+        const uint32_t b = tab + (uint32_t)__float_as_int(q.x);
+        const uint32_t side = C::PADX || t.left ? 0 : 64;
+        rt_for<0, Q>([&](auto JJ) {
+          constexpr int j = decltype(JJ)::value;
+          uint32_t a = b;
+          if (j < PAIRS && fy > ly + LY * j) a = b + C::SUB;
+          rt_for<0, C::NL>([&](auto II) {
+            constexpr int i = decltype(II)::value;
+            constexpr int OFF = j * LY * C::ROW + i * LX * 4;
+            const uint32_t ai = !C::PADX && i == 0 ? a + side : a;
+            t.g[j][i] = lds<OFF>(ai);
+            if constexpr (decltype(cx)::value) t.h[j][i] = lds<OFF>(ai + im_off);
+          });
+        });
+      };
+      auto add = [&](const Taps &t, auto cx) {
+        auto columns = [&](u64 v, const float(&g)[Q][C::NL]) {
+          const u64 v0 = C::PADX || t.left ? v : 0ull, v2 = t.left ? 0ull : v;
+          rt_for<0, Q>([&](auto JJ) {
+            constexpr int j = decltype(JJ)::value;
+            rt_for<0, NX>([&](auto II) {
+              constexpr int i = decltype(II)::value;
+              constexpr int l = C::PADX ? i : (i == 1 ? 1 : 0);
+              run[i][j] = fma2(C::PADX || i == 1 ? v : (i == 0 ? v0 : v2),
+                               pk2(g[j][l], g[j][l]), run[i][j]);
+            });
+          });
+        };
+        columns(pk2(t.vr, t.vi), t.g);
+        if constexpr (decltype(cx)::value) columns(pk2(-t.vi, t.vr), t.h);
+      };
+      // the staged records of a block in order of fy, cnt[f] of them (bytes;
+      // even numbers) for each, the table entries of one loaded while the
+      // previous one is added
+      auto add_block = [&](u64 cnt, auto cx) {
+        Taps a, b;
+        load(a, stage[0], cx);
+        float4 q = stage[1];
+        int since = 0;
+        const float4 *st = stage + 2;
+#pragma unroll 1
+        for (int f = 0; f < 8; ++f) {
+          int left = (int)(cnt >> (8 * f)) & 0xff;
+#pragma unroll 1
+          while (left > 0) {
+            const int m = min(left, kRtRun);
+            const float4 *const end = st + m;
+#pragma unroll 1
+            while (st != end) {
+              load(b, q, cx);
+              q = st[0];
+              add(a, cx);
+              load(a, q, cx);
+              q = st[1];
+              add(b, cx);
+              st += 2;
+            }
+            left -= m;
+            since += m;
+        merge_pairs(f);
+            if (PAIRS < Q && since >= kRtRun) {
+              merge_rest();
+              since = 0;
+            }
+          }
+        }
+        if (PAIRS < Q) merge_rest();
+      };
+      for (int k0 = cur.z; k0 < cur.w; k0 += kRtBlock) {
+        const int n = min(kRtBlock, cur.w - k0);
+        // counting sort by fy: counters of 8 bits, one 64-bit word for all
+        // eight (at most 128 records)
+        u64 mine = 0ull;
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+          if (u * 32 + lane < n) mine += 1ull << (8 * (pk[u].y & 7));
+        u64 incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const u64 y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
+        }
+        const u64 all = __shfl_sync(0xffffffffu, incl, 31);
+        const u64 even = (all + 0x0101010101010101ull) & 0xfefefefefefefefeull;
+        const u64 starts = even * 0x0101010101010100ull;  // sums of the lower bytes
+        u64 at = starts + (incl - mine);
+        __syncwarp();  // the previous block's records were all read
+        if (lane < 8) {  // the zero behind an odd share
+          const int c = (int)(all >> (8 * lane)) & 0xff;
+          if (c & 1)
+            stage[((int)(starts >> (8 * lane)) & 0xff) + c] =
+                make_float4(__int_as_float(C::PAD), 0.f, 0.f, 0.f);
+        } else if (lane < 10) {  // two zeros behind the last
+          const int e = ((int)(starts >> 56) & 0xff) + ((int)(even >> 56) & 0xff);
+          stage[e + lane - 8] = make_float4(__int_as_float(C::PAD), 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < PER; ++u)
+          if (u * 32 + lane < n) {
+            const int sh = 8 * (pk[u].y & 7);
+            stage[(int)(at >> sh) & 0xff] =
+                make_float4(__int_as_float(pk[u].x), __int_as_float(pk[u].y), pv[u].x, pv[u].y);
+            at += 1ull << sh;
+          }
+        if (k0 + kRtBlock < cur.w) fetch(k0 + kRtBlock, cur.w, plane);
+        else if (plane + 1 < p.P) fetch(cur.z, cur.w, plane + 1);
+        else fetch(nxt.z, nxt.w, 0);
+        __syncwarp();
+        if (cplx) add_block(even, std::true_type{});
+        else add_block(even, std::false_type{});
+      }
+      const int ox = tail.y, oy = tail.z;
+      double2 *const slot = COMP && p.merge.base && tail.x >= 0
+                                ? p.merge.base + (size_t)tail.x * p.merge.cells + plane * R * R
+                                : nullptr;
+      u64 z = 0ull;
+#pragma unroll
+      for (int i = 0; i < NX; ++i)
+#pragma unroll
+        for (int j = 0; j < NY; ++j) z = fma2(hi[i][j], 0ull, z);
+      const float2 zf = upk2(z);
+      if (__any_sync(0xffffffffu, !(zf.x == 0.f && zf.y == 0.f))) {
+        rt_redo<S, COMP>(p, p.items[item], plane, tr, cplx, slot);
+        continue;
+      }
+      if (!slot && !other) {
+        // complex64 interleaved grid: hi + lo rounded once
+        float2 *const row0 = out + (size_t)plane * N * N;
+        const bool inside = ox >= 0 && oy >= 0 && ox + R <= N && oy + R <= N;
+#pragma unroll
+        for (int j = 0; j < NY; ++j) {
+          const int gy = oy + LY * j + ly;
+          float2 *const row = row0 + ((ptrdiff_t)gy * N + ox + lx);
+          const bool yin = inside || (unsigned)gy < (unsigned)N;
+#pragma unroll
+          for (int i = 0; i < NX; ++i) {
+            float2 v;
+            if constexpr (COMP) v = upk2(add2(hi[i][j], lo[i][j]));
+            else v = upk2(hi[i][j]);
+            if ((v.x != 0.f || v.y != 0.f) && yin &&
+                (inside || (unsigned)(ox + lx + LX * i) < (unsigned)N))
+              red_add_v2(reinterpret_cast<float *>(row + LX * i), v.x, v.y);
+          }
+        }
+        continue;
+      }
+#pragma unroll
+      for (int j = 0; j < NY; ++j)
+#pragma unroll
+        for (int i = 0; i < NX; ++i) {
+          const int x = LX * i + lx, y = LY * j + ly;
+          const int gx = ox + x, gy = oy + y;
+          const float2 h = upk2(hi[i][j]);
+          float2 l = make_float2(0.f, 0.f);
+          if constexpr (COMP) l = upk2(lo[i][j]);
+          if (h.x == 0.f && h.y == 0.f && l.x == 0.f && l.y == 0.f) continue;
+          // merge slot and complex128 grid: hi + lo exactly
+          double dr = (double)h.x + (double)l.x, di = (double)h.y + (double)l.y;
+          if (slot) {
+            red_add(&slot[y * R + x].x, dr);
+            red_add(&slot[y * R + x].y, di);
+          } else if ((unsigned)gx < (unsigned)N && (unsigned)gy < (unsigned)N) {
+            if (!J.out_f64) {
+              dr = (double)__fadd_rn(h.x, l.x);
+              di = (double)__fadd_rn(h.y, l.y);
+            }
+            out_red(J, (size_t)gy * N + gx, plane, p.P, dr, di);
+          }
+        }
+    }
+    if (next >= total) return;
+    item = next;
+    cur = nxt;
+    next = next2;
+    nxt = nxt2;
+  }
+}
+
+template <int S, bool COMP>
+__global__ void __launch_bounds__(32 * RtCfg<S>::WARPS, 1)
+    regtile_kernel(const __grid_constant__ RegTileLaunch p) {
+  using C = RtCfg<S>;
+  constexpr int NT = 32 * C::WARPS, RF = C::ROW / 4, PF = C::PAD / 4;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int tid = threadIdx.x;
+  const int nf = rt_table_floats(S, p.G), rows = p.G * p.G * S;
+  float *const tr = reinterpret_cast<float *>(smem), *const ti = tr + nf;
+  float4 *const stage = reinterpret_cast<float4 *>(smem + 8 * (size_t)nf) + (tid >> 5) * kRtStage;
+
+  // tables: from the caller's [G*G][S][S], or the Gaussian's factors (expf as
+  // everywhere; their product rounds as the on-the-fly factor does)
+  int imag = 0;
+  if (p.gauss) {
+    float *g1 = reinterpret_cast<float *>(smem + 8 * (size_t)nf);
+    gauss_fill(g1, S, p.G, p.sigma, tid, NT);
+    __syncthreads();
+    for (int i = tid; i < nf; i += NT) {
+      const int row = i / RF, c = i - row * RF - PF;
+      float g = 0.f;
+      if ((unsigned)c < (unsigned)S && row < rows) {
+        const int sub = row / S, b = row % S, sy = sub / p.G, sx = sub - sy * p.G;
+        g = g1[sx * S + c] * g1[sy * S + b];
+      }
+      tr[i] = g;
+    }
+  } else {
+#pragma unroll 4
+    for (int i = tid; i < nf; i += NT) {
+      const int row = i / RF, c = i - row * RF - PF;
+      float2 v = make_float2(0.f, 0.f);
+      if ((unsigned)c < (unsigned)S && row < rows) v = __ldg(p.gcf + row * S + c);
+      tr[i] = v.x;
+      ti[i] = v.y;
+      imag |= v.y != 0.f;
+    }
+  }
+  rt_items<S, COMP>(p, tr, stage, __syncthreads_or(imag));
+}
+
+template <int S, bool COMP> cudaError_t rt_launch(const RegTileLaunch &g, cudaStream_t s) {
+  using C = RtCfg<S>;
+  const size_t smem = regtile_smem_bytes(S, g.G);
+  auto kern = regtile_kernel<S, COMP>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)smem);
+  if (e != cudaSuccess) return e;
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(g.sm_count, g.max_items));
+  kern<<<(unsigned)blocks, 32 * C::WARPS, smem, s>>>(g);
+  count_launch();
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+size_t regtile_smem_bytes(int S, int G) {
+  const int warps = S == 8 ? RtCfg<8>::WARPS : RtCfg<16>::WARPS;
+  return 8 * (size_t)rt_table_floats(S, G) + (size_t)warps * kRtStage * sizeof(float4);
+}
+
+cudaError_t launch_regtile(const RegTileLaunch &g, cudaStream_t s) {
+  switch (g.S) {
+    case 8: return g.compensated ? rt_launch<8, true>(g, s) : rt_launch<8, false>(g, s);
+    case 16: return g.compensated ? rt_launch<16, true>(g, s) : rt_launch<16, false>(g, s);
+  }
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace gg

@@ -13,6 +13,11 @@ enum { FLAG_INDEX = 0, FLAG_TIMEOUT = 1, FLAG_UNSORTED = 2, FLAG_BOUNDS = 3 };
 constexpr int kMaxPols = 8;
 constexpr int kBinThreads = 256;
 
+// Register-tile classes (gg_regtile.cu): uv tiles of 8 cells whose numbering
+// starts kRegOff cells before the grid, so that every visibility that can
+// reach the grid (supports up to 16) has its main cell inside its own tile.
+constexpr int kRegTile = 8, kRegOff = 8;
+
 // One gridding job as the kernels see it.  For the binned methods `idx` and
 // `vals` are the tile-sorted copies made by the binning pass: idx[k] is the
 // packed (main*G+sub) pair of sorted visibility k and vals holds P planes of
@@ -28,6 +33,7 @@ struct JobDesc {
   int64_t npts;          // visibilities (scatter) / kept (binned)
   int64_t vstride;       // plane stride of sorted vals
   int N, S, G, log2G, P, T, log2T, ntx;
+  int off;               // cells by which the uv tiles start before the grid
   int planar, out_f64, uv_f64;
   float sigma;
   // per-visibility GCF tables (1 = a single table); binned methods: the
@@ -51,7 +57,8 @@ struct __align__(16) WorkItem {
   int start;
   int end;
   int slot;
-  int pad_[3];
+  int ox, oy;  // grid cell of the sub-grid's first cell
+  int pad_;
 };
 
 // FP64 merge slots of one support class of a compensated moving-window
