@@ -194,6 +194,10 @@ static int check_options(const gg_options *o) {
 // ---------------------------------------------------------------------------
 // context and plan
 // ---------------------------------------------------------------------------
+// Kernel of a class: the method's own, the register-tile or the output-block
+// form of the moving window
+enum ClassKind { kOwn = 0, kReg, kSep };
+
 struct Plan {
   // resolved launch configuration
   int mode = GG_MODE_WINDOW;
@@ -212,7 +216,8 @@ struct Plan {
     int64_t v0, v1;  // global vis range
     int t0, t1;      // global tile range
     int T, W, chunk; // tile, warps per sub-grid group (0: by support), records per item
-    bool reg;        // register-tile kernel
+    ClassKind kind;
+    int blocks;      // kSep: output blocks
   };
   std::vector<ClassRange> classes;
   std::vector<JobDesc> hjobs;
@@ -351,7 +356,7 @@ static int resolve_mode(const gg_options *o, int S, int vals_f64) {
 // Launch configuration of one support class of the moving window
 struct ClassCfg {
   int T = 0, W = 0, chunk = 0;
-  bool reg = false;  // register-tile kernel (regtile_class)
+  ClassKind kind = kOwn;
 };
 using ClassCfgs = std::map<int, ClassCfg>;  // by support
 
@@ -450,10 +455,38 @@ static int regtile_chunk(int64_t vis, int sm_count) {
   return (int)std::min<int64_t>(512, std::max<int64_t>(64, (c + 31) / 32 * 32));
 }
 
+// Whether the moving-window class of support S is summed by output block:
+// support 32 with the on-the-fly Gaussian, FP32 values, binned by the library
+// at its own choice of tiles, factors of at most 16 sub-cells (20 KB).  Blocks
+// are stored, not added: jobs whose grids overlap keep the adding kernel.
+static bool septile_class(const gg_options *o, const gg_job *jobs, int njobs, int S) {
+  if (S != 32 || o->gcf_kind != GG_GCF_GAUSSIAN || o->input_sorted || !tunable(o) ||
+      o->oversample > 16)
+    return false;
+  std::vector<std::pair<uintptr_t, uintptr_t>> outs;
+  int64_t blocks = 0;
+  for (int j = 0; j < njobs; ++j) {
+    const gg_job &J = jobs[j];
+    if (J.img_dim < 1 || J.img_dim > 32768) return false;  // refused below
+    const uintptr_t n = (uintptr_t)J.img_dim * J.img_dim * o->polarizations *
+                        (J.out_type == GG_C128 ? 16 : 8);
+    outs.push_back({(uintptr_t)J.out, (uintptr_t)J.out + n});
+    if (J.gcf_dim != S) continue;
+    if (J.vals_type != GG_C64) return false;
+    blocks += septile_blocks(J.img_dim);
+  }
+  if (blocks >= (1ll << 30)) return false;
+  std::sort(outs.begin(), outs.end());
+  for (size_t i = 1; i < outs.size(); ++i)
+    if (outs[i].first < outs[i - 1].second) return false;
+  return true;
+}
+
 // uv tiles along one axis of a job
 static int64_t tile_side(int64_t N, int S, const ClassCfg &cf) {
   // main cells up to N + S/2 - 2 reach the grid
-  if (cf.reg) return ((N + S / 2 - 2 + kRegOff) / kRegTile) + 1;
+  if (cf.kind == kReg) return (N + S / 2 - 2 + kRegOff) / kRegTile + 1;
+  if (cf.kind == kSep) return (N + S / 2 - 2 + kSepOff) / kSepTile + 1;
   return (N + cf.T - 1) / cf.T;
 }
 
@@ -500,8 +533,16 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
           if (e) cf = e->cfg;
         }
       }
-      cf.reg = m0 == GG_MODE_WINDOW && !bin_only && regtile_class(opt, jobs, njobs, S, cf);
-      if (cf.reg && cf.chunk == 0) {
+      if (m0 == GG_MODE_WINDOW && !bin_only) {
+        if (septile_class(opt, jobs, njobs, S)) {
+          cf.kind = kSep;
+          cf.T = kSepTile;
+          cf.chunk = 2048;  // no work items
+        } else if (regtile_class(opt, jobs, njobs, S, cf)) {
+          cf.kind = kReg;
+        }
+      }
+      if (cf.kind == kReg && cf.chunk == 0) {
         int64_t cvis = 0;
         for (int i = 0; i < njobs; ++i)
           if (jobs[i].gcf_dim == S) cvis += std::max<int64_t>(0, jobs[i].npts);
@@ -593,7 +634,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
   if (mode == GG_MODE_WINDOW) {
     for (int j = 0; j < njobs; ++j) {
       const ClassCfg &cf = cfgs[(int)jobs[j].gcf_dim];
-      if (cf.reg) continue;
+      if (cf.kind != kOwn) continue;
       const size_t need = window_smem_bytes((int)jobs[j].gcf_dim, opt->accum, vt == GG_C128,
                                             cf.T, cf.W, opt->gcf_kind == GG_GCF_GAUSSIAN);
       if (need > 227 * 1024)
@@ -634,7 +675,8 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     pl.o_svals = take(vbytes * pl.P * pl.vstride + 64);
     pl.o_order = 0;
     pl.o_kept = pl.input_sorted ? take(sizeof(int) * (vis + 8)) : 0;
-    pl.o_items = mode == GG_MODE_WINDOW ? take(sizeof(WorkItem) * 4 * pl.class_cap) : 0;
+    const bool with_items = mode == GG_MODE_WINDOW && cfgs.begin()->second.kind != kSep;
+    pl.o_items = with_items ? take(sizeof(WorkItem) * 4 * pl.class_cap) : 0;
   }
   const bool count = opt->gcf_kind == GG_GCF_COUNT;
   pl.o_count_vals = count ? take(vbytes * pl.P * (vis + 1)) : 0;
@@ -658,7 +700,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     std::map<std::tuple<const void *, int, int>, size_t> seen;  // -> copy index
     for (int k = 0; k < njobs; ++k) {
       const gg_job &J = jobs[order[k]];
-      if (cfgs[(int)J.gcf_dim].reg) continue;  // reads the caller's table
+      if (cfgs[(int)J.gcf_dim].kind != kOwn) continue;  // reads the caller's table, or none
       const int ntab = J.gcf_index ? (int)J.n_gcf : 1;
       const std::tuple<const void *, int, int> key(count ? nullptr : J.gcf, (int)J.gcf_dim, ntab);
       auto it = seen.find(key);
@@ -689,7 +731,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
           ctiles += ntx * ntx * (jobs[j].gcf_index ? jobs[j].n_gcf : 1);
           c64 |= jobs[j].out_type == GG_C64;
         }
-      if (c64 && ci < kMaxClasses) {
+      if (c64 && kv.second.kind != kSep && ci < kMaxClasses) {
         const int R = kv.second.T + S - 1;
         pl.merge_cap[ci] = merge_slot_cap(cvis, kv.second.chunk, ctiles);
         pl.merge_cells[ci] = pl.P * R * R;
@@ -721,7 +763,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
         pl.classes.back().t1 = tb;
       }
       const ClassCfg &cf = cfgs[S];
-      pl.classes.push_back({S, k, k, vb, vb, tb, tb, cf.T, cf.W, cf.chunk, cf.reg});
+      pl.classes.push_back({S, k, k, vb, vb, tb, tb, cf.T, cf.W, cf.chunk, cf.kind, 0});
     }
     const int T = pl.classes.back().T;
     const int N = (int)J.img_dim;
@@ -742,7 +784,12 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     D.T = T;
     D.log2T = ilog2(T);
     D.ntx = ntx;
-    D.off = cfgs[S].reg ? kRegOff : 0;
+    const ClassKind kind = cfgs[S].kind;
+    D.off = kind == kReg ? kRegOff : (kind == kSep ? kSepOff : 0);
+    if (kind == kSep) {
+      D.blk0 = pl.classes.back().blocks;
+      pl.classes.back().blocks += (int)septile_blocks(N);
+    }
     int layout = opt->layout;
     if (layout == GG_LAYOUT_REFERENCE)
       layout = mode == GG_MODE_WINDOW ? GG_LAYOUT_PLANAR : GG_LAYOUT_INTERLEAVED;
@@ -771,13 +818,15 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     B.P = pl.P;
     B.uv_f64 = D.uv_f64;
     B.off = D.off;
+    B.reg = kind == kReg;
     pl.hvis_base[k] = vb;
     pl.htile_base[k] = tb;
     pl.hclass[k] = (int)pl.classes.size() - 1;
     const size_t out_bytes = (size_t)(D.out_f64 ? 16 : 8) * pl.P * N * N;
     // the binned scatter-type kernels add into the grid: cleared first unless
     // the caller accumulates into it (gather stores, or adds, every cell)
-    if (mode != GG_MODE_GATHER && !opt->accumulate) pl.zero_ranges.push_back({J.out, out_bytes});
+    if (mode != GG_MODE_GATHER && kind != kSep && !opt->accumulate)
+      pl.zero_ranges.push_back({J.out, out_bytes});
     if (pl.comp_lo && J.out_type == GG_C64) {
       // filled in once the workspace base is known (plan_bind)
       D.lo = reinterpret_cast<float *>(lo_off + 1);
@@ -964,9 +1013,12 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
         slots.m[ci].cells = pl.merge_cells[ci];
       }
     }
-    GG_CUDA(launch_make_items((const int *)(ws + pl.o_bm), dtileb, dclass, pl.njobs,
-                              pl.total_tiles, chunks, items, pl.class_cap, flags + 8, s,
-                              djobs, &slots, flags + 16, flags));
+    // output-block classes take no items (the Gaussian: one class per batch)
+    const bool items_needed = pl.classes[0].kind != kSep;
+    if (items_needed)
+      GG_CUDA(launch_make_items((const int *)(ws + pl.o_bm), dtileb, dclass, pl.njobs,
+                                pl.total_tiles, chunks, items, pl.class_cap, flags + 8, s,
+                                djobs, &slots, flags + 16, flags));
     for (int ci = 0; ci < kMaxClasses; ++ci)
       GG_CUDA(launch_merge_zero(slots.m[ci], flags + 16 + ci, sm_count, s));
     if (prof) GG_CUDA(cudaEventRecord(prof->ev[1], s));
@@ -983,7 +1035,23 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
       g.item_next = flags + 12 + ci;
       g.max_items = pl.class_cap;
       g.merge = slots.m[ci];
-      if (cl.reg) {
+      if (cl.kind == kSep) {
+        SepTileLaunch q{};
+        q.jobs = djobs + cl.j0;
+        q.njobs = cl.j1 - cl.j0;
+        q.total_blocks = cl.blocks;
+        q.next = g.item_next;
+        q.idx = (const int2 *)(ws + pl.o_sidx);
+        q.vals = (const float2 *)(ws + pl.o_svals);
+        q.vstride = pl.vstride;
+        q.G = pl.G;
+        q.P = pl.P;
+        q.compensated = pl.accum == GG_ACC_COMPENSATED;
+        q.accumulate = opt->accumulate;
+        q.sigma = pl.sigma;
+        q.sm_count = sm_count;
+        GG_CUDA(launch_septile(q, s));
+      } else if (cl.kind == kReg) {
         RegTileLaunch r{};
         r.jobs = djobs;
         r.items = g.items;
@@ -1091,6 +1159,7 @@ static int autotune_batch(gg_context *c, const gg_options *opt, const gg_job *jo
     if (std::find(supports.begin(), supports.end(), (int)jobs[j].gcf_dim) == supports.end())
       supports.push_back((int)jobs[j].gcf_dim);
   for (int S : supports) {
+    if (septile_class(opt, jobs, njobs, S)) continue;  // nothing to choose
     const TuneKey key = tune_key(opt, vf64, S, density_class(jobs, njobs, S));
     std::vector<gg_job> sub;
     double vis = 0;

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(256) bin_count_kernel(BinBuffers b) {
         pk = make_int2(mx * J.G + sx, my * J.G + sy);
         const int h = J.S >> 1;
         if (mx + h >= 0 && mx - h + 1 < J.N && my + h >= 0 && my - h + 1 < J.N) {
-          // register tiles start before the grid and need no clamping
+          // tiles that start before the grid need no clamping
           const int cx = (J.off ? mx + J.off : min(max(mx, 0), J.N - 1)) >> J.log2T;
           const int cy = (J.off ? my + J.off : min(max(my, 0), J.N - 1)) >> J.log2T;
           key = J.tile_base + (cy * J.ntx + cx) * J.n_gcf + gi;
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(256) bin_scatter_kernel(BinBuffers b) {
       if (b.window_records) {
         const int mx = pk.x >> J->log2G, sx = pk.x & (J->G - 1);
         const int my = pk.y >> J->log2G, sy = pk.y & (J->G - 1);
-        pk = J->off ? regtile_record(mx & (kRegTile - 1), sx, my & (kRegTile - 1), sy, J->G, J->S)
+        pk = J->reg ? regtile_record(mx & (kRegTile - 1), sx, my & (kRegTile - 1), sy, J->G, J->S)
                     : window_record(mx, sx, my, sy, J->G);
       }
       b.sorted_idx[pos] = pk;

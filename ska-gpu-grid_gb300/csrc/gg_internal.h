@@ -28,7 +28,8 @@ struct BinJob {
   int N, S, G, log2G, log2T, ntx, P;
   int uv_f64;
   int n_gcf;
-  int off;  // register-tile class: kRegOff (see regtile_record); else 0
+  int off;  // cells by which the uv tiles start before the grid (0: clamped)
+  int reg;  // register-tile class: records of regtile_record
 };
 
 struct BinBuffers {
@@ -228,6 +229,27 @@ struct RegTileLaunch {
   MergeSlots merge;        // base null: none
 };
 cudaError_t launch_regtile(const RegTileLaunch &g, cudaStream_t s);
+// Support 32 with the on-the-fly Gaussian, FP32 values (gg_septile.cu): one
+// launch over the 16x16 output blocks of all jobs of a class.
+struct SepTileLaunch {
+  const JobDesc *jobs;     // the class's jobs, blk0 set
+  int njobs;
+  int total_blocks;
+  int *next;               // zeroed counter of claimed blocks
+  const int2 *idx;         // sorted records (window_record)
+  const float2 *vals;      // sorted values, P planes of vstride
+  int64_t vstride;
+  int G, P;
+  int compensated;
+  int accumulate;          // add into the grid instead of storing
+  float sigma;
+  int sm_count;
+};
+cudaError_t launch_septile(const SepTileLaunch &g, cudaStream_t s);
+inline int64_t septile_blocks(int64_t N) {
+  const int64_t b = (N + kSepBlock - 1) / kSepBlock;
+  return b * b;
+}
 size_t regtile_smem_bytes(int S, int G);
 
 cudaError_t launch_scatter(const GridLaunch &g, cudaStream_t s);

@@ -1,0 +1,392 @@
+// Gridding with the on-the-fly Gaussian at support 32, FP32 values: every
+// 16x16 block of output cells is summed in the registers of one warp.
+//
+// The factor of a tap is the product of two 1-D factors, so a record costs a
+// block two vectors instead of a 32x32 table, and a support-32 footprint
+// covers a large share of any block it touches.  Lane (c, h) of a warp holds
+// the columns 2c, 2c+1 and the rows 4h .. 4h+3 of its block.  The visibilities that
+// reach a block have their main cells in a 48x48 neighbourhood: 6x6 uv tiles
+// of 8 cells, which are 6 contiguous ranges of the sorted records.  Each of
+// them costs
+//   * v * gx for two columns: one 8-byte load of column factors, padded with
+//     zeros so that columns outside the footprint get zero;
+//   * 8 packed multiply-adds by four row factors, one 16-byte load.
+// Both loads read a copy of the padded factors shifted to the alignment of the
+// footprint (four copies).  Shared memory returns 8 bytes a lane and cycle
+// also for broadcasts, so the shape of a lane's cells decides: 2 x 4 takes 5
+// cycles for 10 packed operations, 1 x 8 took 7 for 9.
+// Nothing moves, no cell is shared, every cell is stored once: no atomics, no
+// cleared grid.  9 blocks visit a record, 45 % of their multiply-adds are
+// inside its footprint; the moving window's shared-memory sub-grid cost a
+// read-modify-write of each of the 1024 taps of (nearly) every record.
+//
+// A value that is not finite would reach cells outside its footprint through
+// the zeros: a block whose sums are not finite is summed again cell by cell.
+//
+// Compensated sums: runs of 16 records are summed plainly (about half of them
+// cover a given cell), then added into (hi, lo) by TwoSum.
+//
+// Few blocks (small grids), compensated sums: the warps of a CTA share a
+// block, every warp takes every WARPS-th group of 32 records, and the partial
+// (hi, lo) sums are added by TwoSum in shared memory.  Plain sums stay one
+// sequence of additions.
+//
+// Bound by the FMA pipe (69 % of its cycles, 18 of 30 warp instructions a
+// visit).  Measured on 16.8 M visibilities of a uniform disk on 8192^2: the
+// moving window's shared-memory sub-grid 24.7 ms, this kernel 5.3 ms (runs of
+// 32 records 4.7 ms, with 1.3 times the error against 64 bits: not taken).
+#include <algorithm>
+
+#include "gg_kernels.cuh"
+
+namespace gg {
+
+namespace {
+
+constexpr int kSepS = 32, kSepB = kSepBlock;  // support, block side
+constexpr int kSepWarps = 8;
+constexpr int kSepRow = 64;  // floats of a padded factor row: tap 0 at 16
+
+constexpr int kSepRun = 16;  // at least 16: a group is added in halves
+// staged records of a warp: a group of 32 and zeros for the read-ahead
+constexpr int kSepStage = 36;
+
+// shared memory: factors [G][4][64] (copy c holds the row from its entry c
+// on), a staging block per warp, and the partial sums of a shared block
+__host__ __device__ constexpr size_t sep_factor_floats(int G) { return (size_t)G * 4 * kSepRow; }
+
+__device__ __forceinline__ float2 lds64(uint32_t a) {
+  float2 v;
+  asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float4 lds128(uint32_t a) {
+  float4 v;
+  asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(a));
+  return v;
+}
+
+// (hi, lo) into a cell of the grid
+template <bool COMP>
+__device__ __forceinline__ void sep_store(const JobDesc &J, int gx, int gy, int plane, int P,
+                                          bool accumulate, const float2 h, const float2 l) {
+  if (gx >= J.N || gy >= J.N) return;
+  const size_t cell = (size_t)gy * J.N + gx, NN = (size_t)J.N * J.N;
+  const double dr = (double)h.x + (double)l.x, di = (double)h.y + (double)l.y;
+  const float fr = __fadd_rn(h.x, l.x), fi = __fadd_rn(h.y, l.y);
+  if (accumulate) {
+    if (J.out_f64) out_red(J, cell, plane, P, dr, di);
+    else out_red(J, cell, plane, P, (double)fr, (double)fi);
+  } else if (J.out_f64) {
+    grid_store<double>((double *)J.out, cell, plane, P, NN, J.planar, dr, di);
+  } else if (J.planar) {
+    grid_store<float>((float *)J.out, cell, plane, P, NN, true, fr, fi);
+  } else {
+    reinterpret_cast<float2 *>(J.out)[plane * NN + cell] = make_float2(fr, fi);
+  }
+}
+
+// main cells and sub-kernel of a sorted record (window_record)
+__device__ __forceinline__ void sep_decode(const int2 q, int log2G, int &mx, int &my, int &sx,
+                                           int &sy) {
+  mx = (int)((unsigned)q.x & 0xffffu) - kWinMainBias;
+  my = (int)((unsigned)q.x >> 16) - kWinMainBias;
+  sx = q.y & ((1 << log2G) - 1);
+  sy = q.y >> log2G;
+}
+
+// A block whose packed sums are not finite: its cells from the records whose
+// footprints cover them.
+template <bool COMP>
+__device__ __noinline__ void sep_redo(const SepTileLaunch &p, const JobDesc &J, int x0, int y0,
+                                      int plane, const float *gt, int tid, int nt) {
+  constexpr int H = kSepS / 2;
+  const float2 *const vals = p.vals + plane * p.vstride;
+  for (int c = tid; c < kSepB * kSepB; c += nt) {
+    const int x = x0 + c % kSepB, y = y0 + c / kSepB;
+    u64 run = 0ull, hi = 0ull, lo = 0ull;
+    int since = 0;
+    auto merge = [&]() {
+      u64 e;
+      hi = two_sum2(hi, run, e);
+      lo = add2(lo, e);
+      run = 0ull;
+      since = 0;
+    };
+    const int bx = x0 / kSepTile, by = y0 / kSepTile;
+    for (int r = 0; r < 6; ++r) {
+      if (by + r >= J.ntx) break;
+      const int *const bm = J.bookmarks + (by + r) * J.ntx;
+      for (int k = bm[bx]; k < bm[min(bx + 6, J.ntx)]; ++k) {
+        int mx, my, sx, sy;
+        sep_decode(__ldg(p.idx + k), J.log2G, mx, my, sx, sy);
+        const int a = x - (mx - H + 1), b = y - (my - H + 1);
+        if ((unsigned)a >= (unsigned)kSepS || (unsigned)b >= (unsigned)kSepS) continue;
+        const float2 v = __ldg(vals + k);
+        const float gx = gt[sx * 4 * kSepRow + 16 + a], gy = gt[sy * 4 * kSepRow + 16 + b];
+        run = fma2(mul2(pk2(v.x, v.y), pk2(gx, gx)), pk2(gy, gy), run);
+        if (COMP && ++since == kSepRun) merge();
+      }
+    }
+    if (COMP) merge();
+    sep_store<COMP>(J, x, y, plane, p.P, p.accumulate, upk2(COMP ? hi : run), upk2(lo));
+  }
+}
+
+template <bool COMP, bool SHARE>
+__global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
+    septile_kernel(const __grid_constant__ SepTileLaunch p) {
+  constexpr int H = kSepS / 2, NT = 32 * kSepWarps;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float *const gt = reinterpret_cast<float *>(smem);
+  // factor offsets and values of a group, and the zeros behind it
+  int2 *const off = reinterpret_cast<int2 *>(gt + sep_factor_floats(p.G)) + warp * kSepStage;
+  float2 *const val = reinterpret_cast<float2 *>(off) + kSepWarps * kSepStage;
+  float4 *const part = reinterpret_cast<float4 *>(gt + sep_factor_floats(p.G)) +
+                       kSepWarps * kSepStage;
+  if (lane < kSepStage - 32) {
+    off[32 + lane] = make_int2(0, 0);
+    val[32 + lane] = make_float2(0.f, 0.f);
+  }
+
+  // padded factors: entry i of a row is tap i - 16, zero outside
+  const float inv = 1.0f / (2.0f * p.sigma * p.sigma);
+  for (int i = tid; i < p.G * 4 * kSepRow; i += NT) {
+    const int s = i / (4 * kSepRow), ap = i % kSepRow + i / kSepRow % 4 - 16;
+    const float x = (float)(ap - H + 1) - (float)s / (float)p.G;
+    gt[i] = (unsigned)ap < (unsigned)kSepS ? expf(-(x * x) * inv) : 0.f;
+  }
+  __syncthreads();
+
+  const int c = lane & 7, h = lane >> 3;
+  const uint32_t ax = smem_addr(gt) + 8 * c, ay = smem_addr(gt) + 16 * h;
+  // blocks are spread over the SMs first, then claimed
+  const int workers = SHARE ? (int)gridDim.x : (int)gridDim.x * kSepWarps;
+  int blk = SHARE ? (int)blockIdx.x : (int)(blockIdx.x + warp * gridDim.x);
+  __shared__ int s_next;
+  while (blk < p.total_blocks) {
+    int next = 0;
+    if (SHARE ? tid == 0 : lane == 0) next = atomicAdd(p.next, 1) + workers;
+    int j = 0;
+    {
+      int e = p.njobs - 1;
+      while (j < e) {
+        const int mid = (j + e + 1) >> 1;
+        if (p.jobs[mid].blk0 <= blk) j = mid; else e = mid - 1;
+      }
+    }
+    const JobDesc &J = p.jobs[j];
+    const int nb = (J.N + kSepB - 1) / kSepB, b = blk - J.blk0;
+    const int x0 = (b % nb) * kSepB, y0 = (b / nb) * kSepB;
+    const int bx = x0 / kSepTile, by = y0 / kSepTile;  // tiles start kSepOff before the grid
+    const int log2G = J.log2G;
+    // lane r < 6: the r-th row of tiles
+    int beg = 0, end = 0;
+    if (lane < 6 && by + lane < J.ntx) {
+      const int *const bm = J.bookmarks + (by + lane) * J.ntx;
+      beg = __ldg(bm + bx);
+      end = __ldg(bm + min(bx + 6, J.ntx));
+    }
+    // first: groups of the ranges before it
+    int first = (end - beg + 31) / 32, groups = first;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, groups, o);
+      if (lane >= o) groups += y;
+    }
+    first = groups - first;
+    groups = __shfl_sync(0xffffffffu, groups, 5);
+    for (int plane = 0; plane < p.P; ++plane) {
+      // cell k: column 2c + (k & 1), row 4h + k / 2
+      u64 run[8], hi[COMP ? 8 : 1], lo[COMP ? 8 : 1];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        run[k] = 0ull;
+        if constexpr (COMP) hi[k] = lo[k] = 0ull;
+      }
+      int since = 0;  // records in the running sums
+      auto merge = [&]() {
+        if constexpr (COMP) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            u64 e;
+            hi[k] = two_sum2(hi[k], run[k], e);
+            lo[k] = add2(lo[k], e);
+            run[k] = 0ull;
+          }
+        }
+        since = 0;
+      };
+      const float2 *const vals = p.vals + plane * p.vstride;
+      // the groups of 32 records of the six ranges as one stream: group g lies
+      // in the last range r whose first group is at most g
+      int2 q = make_int2(0, 0);
+      float2 v = make_float2(0.f, 0.f);
+      int n = 0;
+      auto fetch = [&](int g) {
+        n = 0;
+        if (g >= groups) return;
+        const int r = __popc(__ballot_sync(0xffffffffu, lane < 6 && first <= g)) - 1;
+        const int k = __shfl_sync(0xffffffffu, beg, r) +
+                      32 * (g - __shfl_sync(0xffffffffu, first, r));
+        n = min(32, __shfl_sync(0xffffffffu, end, r) - k);
+        if (lane < n) {
+          q = __ldg(p.idx + k + lane);
+          v = __ldg(vals + k + lane);
+        }
+      };
+      int g = SHARE ? warp : 0;
+      fetch(g);
+      while (n > 0) {
+        const int m = n;
+        __syncwarp();  // the previous group was read
+        int2 at = make_int2(0, 0);
+        if (lane < m) {
+          int mx, my, sx, sy;
+          sep_decode(q, log2G, mx, my, sx, sy);
+          // entries of the padded rows at the block's first column and row
+          const int ix = x0 - (mx - H + 1) + 16, iy = y0 - (my - H + 1) + 16;
+          at = make_int2(((sx * 4 + (ix & 3)) * kSepRow + (ix & ~3)) * 4,
+                         ((sy * 4 + (iy & 3)) * kSepRow + (iy & ~3)) * 4);
+        } else {
+          v = make_float2(0.f, 0.f);
+        }
+        off[lane] = at;
+        val[lane] = v;
+        g += SHARE ? kSepWarps : 1;
+        fetch(g);
+        __syncwarp();
+        // the factors of a record are loaded while the previous one is added
+        struct Taps {
+          float2 v, gx;
+          float4 gy;
+        } a, b;
+        auto load = [&](Taps &t, const int2 o, int i) {
+          t.gx = lds64(ax + (uint32_t)o.x);
+          t.gy = lds128(ay + (uint32_t)o.y);
+          t.v = val[i];
+        };
+        auto add = [&](const Taps &t) {
+          const u64 vv = pk2(t.v.x, t.v.y);
+          const u64 w0 = mul2(vv, pk2(t.gx.x, t.gx.x)), w1 = mul2(vv, pk2(t.gx.y, t.gx.y));
+          run[0] = fma2(w0, pk2(t.gy.x, t.gy.x), run[0]);
+          run[1] = fma2(w1, pk2(t.gy.x, t.gy.x), run[1]);
+          run[2] = fma2(w0, pk2(t.gy.y, t.gy.y), run[2]);
+          run[3] = fma2(w1, pk2(t.gy.y, t.gy.y), run[3]);
+          run[4] = fma2(w0, pk2(t.gy.z, t.gy.z), run[4]);
+          run[5] = fma2(w1, pk2(t.gy.z, t.gy.z), run[5]);
+          run[6] = fma2(w0, pk2(t.gy.w, t.gy.w), run[6]);
+          run[7] = fma2(w1, pk2(t.gy.w, t.gy.w), run[7]);
+        };
+        load(a, off[0], 0);
+        int2 o = off[1];
+        for (int i0 = 0; i0 < m; i0 += 16) {
+          const int i1 = min(m, i0 + 16);
+#pragma unroll 1
+          for (int i = i0; i < i1; i += 2) {
+            load(b, o, i + 1);
+            o = off[i + 2];
+            add(a);
+            load(a, o, i + 2);
+            o = off[i + 3];
+            add(b);
+          }
+          since += i1 - i0;
+          if (COMP && since > kSepRun - 16) merge();
+        }
+      }
+      merge();
+      bool bad = false;
+      if constexpr (SHARE) {
+        // cell (x, y) of warp w at part[w][16 y + x]
+        __syncthreads();  // the previous block's partial sums were read
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float2 a = upk2(COMP ? hi[k] : run[k]);
+          float2 l = make_float2(0.f, 0.f);
+          if constexpr (COMP) l = upk2(lo[k]);
+          part[warp * 256 + (4 * h + k / 2) * 16 + 2 * c + (k & 1)] = make_float4(a.x, a.y, l.x, l.y);
+        }
+        __syncthreads();
+        u64 sh = 0ull, sl = 0ull;
+        for (int w = 0; w < kSepWarps; ++w) {
+          const float4 t = part[w * 256 + tid];
+          if constexpr (COMP) {
+            u64 e;
+            sh = two_sum2(sh, pk2(t.x, t.y), e);
+            sl = add2(sl, add2(e, pk2(t.z, t.w)));
+          } else {
+            sh = add2(sh, pk2(t.x, t.y));
+          }
+        }
+        const float2 z = upk2(fma2(sh, 0ull, 0ull));
+        bad = __syncthreads_or(!(z.x == 0.f && z.y == 0.f));
+        if (!bad)
+          sep_store<COMP>(J, x0 + (tid & 15), y0 + (tid >> 4), plane, p.P, p.accumulate, upk2(sh),
+                          upk2(sl));
+        else sep_redo<COMP>(p, J, x0, y0, plane, gt, tid, NT);
+      } else {
+        u64 z = 0ull;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          if constexpr (COMP) z = fma2(hi[k], 0ull, z);
+          else z = fma2(run[k], 0ull, z);
+        }
+        const float2 zf = upk2(z);
+        bad = __any_sync(0xffffffffu, !(zf.x == 0.f && zf.y == 0.f));
+        if (!bad) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            float2 l = make_float2(0.f, 0.f);
+            if constexpr (COMP) l = upk2(lo[k]);
+            sep_store<COMP>(J, x0 + 2 * c + (k & 1), y0 + 4 * h + k / 2, plane, p.P, p.accumulate,
+                            upk2(COMP ? hi[k] : run[k]), l);
+          }
+        } else {
+          sep_redo<COMP>(p, J, x0, y0, plane, gt, lane, 32);
+        }
+      }
+    }
+    if constexpr (SHARE) {
+      if (tid == 0) s_next = next;
+      __syncthreads();
+      blk = s_next;
+      __syncthreads();
+    } else {
+      blk = __shfl_sync(0xffffffffu, next, 0);
+    }
+  }
+}
+
+template <bool COMP, bool SHARE>
+cudaError_t sep_launch(const SepTileLaunch &g, cudaStream_t s) {
+  const size_t smem = sep_factor_floats(g.G) * 4 + kSepWarps * kSepStage * sizeof(float4) +
+                      (SHARE ? kSepWarps * 256 * sizeof(float4) : 0);
+  auto kern = septile_kernel<COMP, SHARE>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)smem);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kSepWarps, smem);
+  if (e != cudaSuccess) return e;
+  if (per_sm < 1) return cudaErrorInvalidConfiguration;
+  const int64_t blocks = std::min<int64_t>((int64_t)g.sm_count * per_sm, g.total_blocks);
+  if (blocks < 1) return cudaSuccess;
+  kern<<<(unsigned)blocks, 32 * kSepWarps, smem, s>>>(g);
+  count_launch();
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_septile(const SepTileLaunch &g, cudaStream_t s) {
+  // a block a warp while that gives every resident warp a few blocks
+  const bool share = g.total_blocks < (int64_t)g.sm_count * 24 * 4;
+  if (!g.compensated) return sep_launch<false, false>(g, s);
+  return share ? sep_launch<true, true>(g, s) : sep_launch<true, false>(g, s);
+}
+
+}  // namespace gg
