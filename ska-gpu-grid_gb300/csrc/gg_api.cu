@@ -211,13 +211,14 @@ struct Plan {
   int total_tiles = 0;
   int input_sorted = 0;
   int comp_lo = 0;  // compensated scatter with complex64 output
+  int aos = 0;      // sorted {record, value} pairs (BinBuffers::aos)
   struct ClassRange {
     int S, j0, j1;
     int64_t v0, v1;  // global vis range
     int t0, t1;      // global tile range
     int T, W, chunk; // tile, warps per sub-grid group (0: by support), records per item
     ClassKind kind;
-    int blocks;      // kSep: output blocks
+    int blocks;      // output blocks (kSep) or pieces to clear, see JobDesc::blk0
   };
   std::vector<ClassRange> classes;
   std::vector<JobDesc> hjobs;
@@ -247,8 +248,7 @@ struct Plan {
   size_t o_merge[kMaxClasses] = {}, o_mdesc[kMaxClasses] = {};
   int merge_cap[kMaxClasses] = {}, merge_cells[kMaxClasses] = {};
   // workspace carve (offsets into the device workspace)
-  size_t o_jobs, o_bin, o_visb, o_tileb, o_class, o_packed, o_key, o_bm,
-      o_cursor, o_scan, o_sidx, o_svals, o_order, o_items, o_kept, o_lo,
+  size_t o_jobs, o_bin, o_visb, o_tileb, o_class, o_kr, o_cnt, o_bm, o_scan, o_sidx, o_svals, o_order, o_items, o_kept, o_lo,
       o_count_vals, o_count_gcf, ws_bytes;
   int64_t vstride = 0, class_cap = 0;
   size_t table_bytes = 0;  // bytes uploaded from staging (jobs..class)
@@ -666,13 +666,15 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
   pl.vstride = vis + 8;
   pl.class_cap = tiles + vis / pl.chunk + njobs + 1;
   if (binned) {
-    pl.o_packed = take(sizeof(int2) * (vis + 1));
-    pl.o_key = take(sizeof(int) * (vis + 1));
+    pl.aos = mode == GG_MODE_WINDOW && pl.P == 1 && !bin_only;
+    for (const auto &kv : cfgs) pl.aos = pl.aos && kv.second.kind != kOwn;
+    pl.o_kr = take(sizeof(int2) * (vis + 1));
+    pl.o_cnt = take(sizeof(int) * (tiles + 8));
     pl.o_bm = take(sizeof(int) * (tiles + 8));
-    pl.o_cursor = take(sizeof(int) * (tiles + 8));
-    pl.o_scan = take(sizeof(int) * scan_tmp_ints(std::max<int64_t>(tiles + 1, vis + 1)));
-    pl.o_sidx = take(sizeof(int2) * (vis + 8));
-    pl.o_svals = take(vbytes * pl.P * pl.vstride + 64);
+    pl.o_scan = take(sizeof(int) * (scan_tmp_ints(tiles + 1) +
+                                    (pl.input_sorted ? scan_tmp_ints(vis + 1) : 0)));
+    pl.o_sidx = take((pl.aos ? 16 : sizeof(int2)) * (vis + 8));
+    pl.o_svals = pl.aos ? 0 : take(vbytes * pl.P * pl.vstride + 64);
     pl.o_order = 0;
     pl.o_kept = pl.input_sorted ? take(sizeof(int) * (vis + 8)) : 0;
     const bool with_items = mode == GG_MODE_WINDOW && cfgs.begin()->second.kind != kSep;
@@ -736,7 +738,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
         pl.merge_cap[ci] = merge_slot_cap(cvis, kv.second.chunk, ctiles);
         pl.merge_cells[ci] = pl.P * R * R;
         pl.o_merge[ci] = take(sizeof(double2) * (size_t)pl.merge_cap[ci] * pl.merge_cells[ci]);
-        pl.o_mdesc[ci] = take(sizeof(int2) * (size_t)pl.merge_cap[ci]);
+        pl.o_mdesc[ci] = take(sizeof(int4) * (size_t)pl.merge_cap[ci]);
       }
       ++ci;
     }
@@ -825,8 +827,11 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     const size_t out_bytes = (size_t)(D.out_f64 ? 16 : 8) * pl.P * N * N;
     // the binned scatter-type kernels add into the grid: cleared first unless
     // the caller accumulates into it (gather stores, or adds, every cell)
-    if (mode != GG_MODE_GATHER && kind != kSep && !opt->accumulate)
+    if (mode != GG_MODE_GATHER && kind != kSep && !opt->accumulate) {
       pl.zero_ranges.push_back({J.out, out_bytes});
+      D.blk0 = pl.classes.back().blocks;
+      pl.classes.back().blocks += (int)((out_bytes + kZeroChunk - 1) / kZeroChunk);
+    }
     if (pl.comp_lo && J.out_type == GG_C64) {
       // filled in once the workspace base is known (plan_bind)
       D.lo = reinterpret_cast<float *>(lo_off + 1);
@@ -888,6 +893,22 @@ static void plan_bind(const gg_options *opt, Plan &pl, char *ws, char *host) {
   pl.ws = ws;
 }
 
+// The workspace arrays of a plan's binning.
+static void plan_bin_buffers(const Plan &pl, BinBuffers &b) {
+  char *ws = pl.ws;
+  b.key_rank = (int2 *)(ws + pl.o_kr);
+  b.counts = (int *)(ws + pl.o_cnt);
+  b.scan_tmp = (int *)(ws + pl.o_scan);
+  b.block_off = b.scan_tmp + kScanHead;
+  b.bookmarks = (int *)(ws + pl.o_bm);
+  b.sorted_idx = (int2 *)(ws + pl.o_sidx);
+  b.sorted_vals = ws + pl.o_svals;
+  b.vstride = pl.vstride;
+  b.aos = pl.aos;
+  b.input_sorted = pl.input_sorted;
+  b.kept_pos = pl.input_sorted ? (int *)(ws + pl.o_kept) : nullptr;
+}
+
 // Profiling events of one enqueue (null: none)
 struct ProfEvents {
   cudaEvent_t ev[4];
@@ -895,7 +916,7 @@ struct ProfEvents {
 
 // Enqueue the whole computation on stream s: zeroing, binning, work queue,
 // gridding kernels.  `upload` (host tables) is sent into the workspace first
-// when given, through kernel parameters (launch_upload): a copy-engine
+// when given, through kernel parameters (launch_setup): a copy-engine
 // transfer would queue behind other streams' input and output copies (one
 // to two milliseconds per batch on a server moving host data), a launch does
 // not, and the staging buffer is free again when the call returns
@@ -907,31 +928,49 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
                         const ProfEvents *prof, const AuxStream *aux) {
   char *ws = pl.ws;
   if (prof) GG_CUDA(cudaEventRecord(prof->ev[0], s));
-  if (upload) {
-    GG_CUDA(launch_upload(ws, upload, pl.table_bytes, s));
-    if (upload_ev) GG_CUDA(cudaEventRecord(upload_ev, s));
-  }
   const JobDesc *djobs = (const JobDesc *)(ws + pl.o_jobs);
   const int64_t *dvisb = (const int64_t *)(ws + pl.o_visb);
   const int *dtileb = (const int *)(ws + pl.o_tileb);
   const int *dclass = (const int *)(ws + pl.o_class);
   const size_t vbytes = pl.vals_f64 ? 16 : 8;
+  const bool binned = pl.mode != GG_MODE_SCATTER;
+
+  // One launch writes the tables and clears what starts at zero: the binning's
+  // counters and, of a single job, an output small enough (4 MB: 2 us) not to
+  // be worth a stream of its own.
+  ZeroRanges zero{};
+  if (binned) {
+    zero.add(ws + pl.o_cnt, ((size_t)(pl.total_tiles + 1) * sizeof(int) + 15) & ~(size_t)15);
+    zero.add(ws + pl.o_scan, kScanHead * sizeof(int));
+    zero.add(ws + pl.o_bm + sizeof(int) * ((size_t)pl.total_tiles + 1), sizeof(int));
+  }
+  // item counters [8, 12), item claims [12, 16), merge slots taken [16, 20)
+  if (pl.mode == GG_MODE_WINDOW) zero.add(flags + 8, 12 * sizeof(int));
+  if (!pl.gcf_copies.empty()) zero.add(ws + pl.o_gcf_flags, sizeof(int) * pl.gcf_copies.size());
+  const bool small_out = pl.zero_ranges.size() == 1 && pl.zero_ranges[0].second <= (4u << 20);
+  if (small_out) zero.add(pl.zero_ranges[0].first, pl.zero_ranges[0].second);
+  GG_CUDA(launch_setup(ws, upload, upload ? pl.table_bytes : 0, zero, s));
+  if (upload && upload_ev) GG_CUDA(cudaEventRecord(upload_ev, s));
 
   // output zeroing: on the side stream, class by class, for the moving
-  // window (jobs are in class order, one zero range each); else here
-  const bool side = aux && aux->s && pl.mode == GG_MODE_WINDOW &&
-                    pl.zero_ranges.size() == (size_t)pl.njobs &&
+  // window; else here
+  const bool clear = !small_out && !pl.zero_ranges.empty();
+  const bool side = clear && aux && aux->s && pl.mode == GG_MODE_WINDOW &&
                     pl.classes.size() <= (size_t)kMaxClasses;
-  if (side) {
-    GG_CUDA(cudaEventRecord(aux->fork, s));
-    GG_CUDA(cudaStreamWaitEvent(aux->s, aux->fork, 0));
-    for (size_t ci = 0; ci < pl.classes.size(); ++ci) {
-      for (int j = pl.classes[ci].j0; j < pl.classes[ci].j1; ++j)
-        GG_CUDA(cudaMemsetAsync(pl.zero_ranges[j].first, 0, pl.zero_ranges[j].second, aux->s));
-      GG_CUDA(cudaEventRecord(aux->done[ci], aux->s));
+  if (clear) {
+    cudaStream_t zs = side ? aux->s : s;
+    if (side) {
+      GG_CUDA(cudaEventRecord(aux->fork, s));
+      GG_CUDA(cudaStreamWaitEvent(aux->s, aux->fork, 0));
     }
-  } else {
-    for (auto &z : pl.zero_ranges) GG_CUDA(cudaMemsetAsync(z.first, 0, z.second, s));
+    for (size_t ci = 0; ci < pl.classes.size(); ++ci) {
+      const auto &cl = pl.classes[ci];
+      if (pl.njobs == 1)
+        GG_CUDA(cudaMemsetAsync(pl.zero_ranges[0].first, 0, pl.zero_ranges[0].second, zs));
+      else
+        GG_CUDA(launch_zero_jobs(djobs + cl.j0, cl.j1 - cl.j0, cl.blocks, sm_count, zs));
+      if (side) GG_CUDA(cudaEventRecord(aux->done[ci], aux->s));
+    }
   }
   if (pl.comp_lo) {
     size_t lo_bytes = pl.ws_bytes - pl.o_lo;
@@ -947,8 +986,6 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
                                   k == 0 ? (int64_t)pl.G * pl.G * maxS * maxS : 0, s));
     }
   }
-  if (!pl.gcf_copies.empty())
-    GG_CUDA(cudaMemsetAsync(ws + pl.o_gcf_flags, 0, sizeof(int) * pl.gcf_copies.size(), s));
   for (size_t ci = 0; ci < pl.gcf_copies.size(); ++ci) {
     const auto &c = pl.gcf_copies[ci];
     GG_CUDA(launch_gcf_double_rows(c.src ? c.src : ws + pl.o_count_gcf, ws + c.off, c.S, pl.G,
@@ -971,7 +1008,8 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
   g.flags = flags;
   g.sm_count = sm_count;
 
-  if (pl.mode != GG_MODE_SCATTER) {
+  ItemBuffers it{};
+  if (binned) {
     BinBuffers b{};
     b.jobs = (const BinJob *)(ws + pl.o_bin);
     b.vis_base = dvisb;
@@ -981,46 +1019,35 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
     b.total_tiles = pl.total_tiles;
     b.vals_bytes = (int)vbytes;
     b.P = pl.P;
-    b.packed = (int2 *)(ws + pl.o_packed);
-    b.key = (int *)(ws + pl.o_key);
-    b.bookmarks = (int *)(ws + pl.o_bm);
-    b.cursor = (int *)(ws + pl.o_cursor);
-    b.scan_tmp = (int *)(ws + pl.o_scan);
-    b.sorted_idx = (int2 *)(ws + pl.o_sidx);
-    b.sorted_vals = ws + pl.o_svals;
-    b.vstride = pl.vstride;
+    plan_bin_buffers(pl, b);
     b.order = nullptr;
     b.flags = flags;
-    b.input_sorted = pl.input_sorted;
-    b.kept_pos = pl.input_sorted ? (int *)(ws + pl.o_kept) : nullptr;
     b.window_records = pl.mode == GG_MODE_WINDOW;
-    GG_CUDA(run_binning(b, s));
+    // output-block classes take no items (the Gaussian: one class per batch)
+    const bool with_items = pl.mode == GG_MODE_WINDOW && pl.classes[0].kind != kSep;
+    if (with_items) {
+      it.items = (WorkItem *)(ws + pl.o_items);
+      it.jobs = djobs;
+      it.job_class = dclass;
+      it.nclasses = (int)pl.classes.size();
+      it.class_cap = pl.class_cap;
+      it.counters = flags + 8;
+      it.heavy_counters = flags + 16;
+      for (int ci = 0; ci < kMaxClasses; ++ci) {
+        it.chunks.c[ci] = ci < (int)pl.classes.size() ? pl.classes[ci].chunk : pl.chunk;
+        if (pl.merge_cap[ci] > 0) {
+          it.slots.m[ci].base = (double2 *)(ws + pl.o_merge[ci]);
+          it.slots.m[ci].desc = (int4 *)(ws + pl.o_mdesc[ci]);
+          it.slots.m[ci].cap = pl.merge_cap[ci];
+          it.slots.m[ci].cells = pl.merge_cells[ci];
+        }
+      }
+    }
+    GG_CUDA(run_binning(b, with_items ? &it : nullptr, s));
     g.holes = b.bookmarks + pl.total_tiles + 1;
   }
 
   if (pl.mode == GG_MODE_WINDOW) {
-    // item counters [8, 12), item claims [12, 16), merge slots taken [16, 20)
-    GG_CUDA(cudaMemsetAsync(flags + 8, 0, 12 * sizeof(int), s));
-    WorkItem *items = (WorkItem *)(ws + pl.o_items);
-    ClassChunks chunks;
-    ClassSlots slots{};
-    for (int ci = 0; ci < kMaxClasses; ++ci) {
-      chunks.c[ci] = ci < (int)pl.classes.size() ? pl.classes[ci].chunk : pl.chunk;
-      if (pl.merge_cap[ci] > 0) {
-        slots.m[ci].base = (double2 *)(ws + pl.o_merge[ci]);
-        slots.m[ci].desc = (int2 *)(ws + pl.o_mdesc[ci]);
-        slots.m[ci].cap = pl.merge_cap[ci];
-        slots.m[ci].cells = pl.merge_cells[ci];
-      }
-    }
-    // output-block classes take no items (the Gaussian: one class per batch)
-    const bool items_needed = pl.classes[0].kind != kSep;
-    if (items_needed)
-      GG_CUDA(launch_make_items((const int *)(ws + pl.o_bm), dtileb, dclass, pl.njobs,
-                                pl.total_tiles, chunks, items, pl.class_cap, flags + 8, s,
-                                djobs, &slots, flags + 16, flags));
-    for (int ci = 0; ci < kMaxClasses; ++ci)
-      GG_CUDA(launch_merge_zero(slots.m[ci], flags + 16 + ci, sm_count, s));
     if (prof) GG_CUDA(cudaEventRecord(prof->ev[1], s));
     for (size_t ci = 0; ci < pl.classes.size(); ++ci) {
       const auto &cl = pl.classes[ci];
@@ -1029,12 +1056,12 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
       g.S = cl.S;
       g.tile = cl.T;
       g.group_warps = cl.W;
-      g.items = items + ci * pl.class_cap;
+      g.items = it.items + ci * pl.class_cap;
       g.nitems = flags + 8 + ci;
       if (side) GG_CUDA(cudaStreamWaitEvent(s, aux->done[ci], 0));
       g.item_next = flags + 12 + ci;
       g.max_items = pl.class_cap;
-      g.merge = slots.m[ci];
+      g.merge = it.slots.m[ci];
       if (cl.kind == kSep) {
         SepTileLaunch q{};
         q.jobs = djobs + cl.j0;
@@ -1042,7 +1069,7 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
         q.total_blocks = cl.blocks;
         q.next = g.item_next;
         q.idx = (const int2 *)(ws + pl.o_sidx);
-        q.vals = (const float2 *)(ws + pl.o_svals);
+        q.vals = pl.aos ? nullptr : (const float2 *)(ws + pl.o_svals);
         q.vstride = pl.vstride;
         q.G = pl.G;
         q.P = pl.P;
@@ -1058,7 +1085,7 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
         r.nitems = g.nitems;
         r.item_next = g.item_next;
         r.idx = (const int2 *)(ws + pl.o_sidx);
-        r.vals = (const float2 *)(ws + pl.o_svals);
+        r.vals = pl.aos ? nullptr : (const float2 *)(ws + pl.o_svals);
         r.vstride = pl.vstride;
         r.gcf = (const float2 *)pl.hjobs[cl.j0].gcf;
         r.S = cl.S;
@@ -1069,13 +1096,13 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
         r.sigma = pl.sigma;
         r.max_items = std::min<int64_t>(pl.class_cap, cl.v1 - cl.v0);
         r.sm_count = sm_count;
-        r.merge = slots.m[ci];
+        r.merge = it.slots.m[ci];
         GG_CUDA(launch_regtile(r, s));
       } else {
         GG_CUDA(launch_window(g, s));
+        GG_CUDA(launch_merge_finalize(it.slots.m[ci], flags + 16 + ci, djobs, cl.S, cl.T, pl.P,
+                                      sm_count, s));
       }
-      GG_CUDA(launch_merge_finalize(slots.m[ci], flags + 16 + ci, djobs, cl.S, cl.T, pl.P,
-                                    sm_count, s));
     }
     if (prof) GG_CUDA(cudaEventRecord(prof->ev[2], s));
   } else if (pl.mode == GG_MODE_GATHER) {
@@ -1666,8 +1693,6 @@ int gg_bin(gg_context *ctx, const gg_options *opt, int uv_type, const void *uv,
   char *ws = (char *)ctx->ws.p;
   cudaStream_t s = (cudaStream_t)stream;
   GG_CUDA(cudaStreamWaitEvent(s, ctx->exec_done, 0));
-  GG_CUDA(launch_upload(ws, ctx->staging.p, pl.table_bytes, s));
-  GG_CUDA(cudaEventRecord(ctx->upload_done, s));
   BinBuffers b{};
   b.jobs = (const BinJob *)(ws + pl.o_bin);
   b.vis_base = (const int64_t *)(ws + pl.o_visb);
@@ -1677,19 +1702,16 @@ int gg_bin(gg_context *ctx, const gg_options *opt, int uv_type, const void *uv,
   b.total_tiles = pl.total_tiles;
   b.vals_bytes = 8;
   b.P = 1;
-  b.packed = (int2 *)(ws + pl.o_packed);
-  b.key = (int *)(ws + pl.o_key);
-  b.bookmarks = (int *)(ws + pl.o_bm);
-  b.cursor = (int *)(ws + pl.o_cursor);
-  b.scan_tmp = (int *)(ws + pl.o_scan);
-  b.sorted_idx = (int2 *)(ws + pl.o_sidx);
-  b.sorted_vals = ws + pl.o_svals;
-  b.vstride = pl.vstride;
+  plan_bin_buffers(pl, b);
   b.order = (int *)(ws + order_off);
   b.flags = (int *)ctx->flags.p;
-  b.input_sorted = pl.input_sorted;
-  b.kept_pos = pl.input_sorted ? (int *)(ws + pl.o_kept) : nullptr;
-  GG_CUDA(run_binning(b, s));
+  ZeroRanges zero{};
+  zero.add(b.counts, ((size_t)(pl.total_tiles + 1) * sizeof(int) + 15) & ~(size_t)15);
+  zero.add(b.scan_tmp, kScanHead * sizeof(int));
+  zero.add(b.bookmarks + pl.total_tiles + 1, sizeof(int));
+  GG_CUDA(launch_setup(ws, ctx->staging.p, pl.table_bytes, zero, s));
+  GG_CUDA(cudaEventRecord(ctx->upload_done, s));
+  GG_CUDA(run_binning(b, nullptr, s));
   GG_CUDA(cudaMemcpyAsync(bookmarks, b.bookmarks, sizeof(int) * (pl.total_tiles + 1),
                           cudaMemcpyDeviceToDevice, s));
   if (order)

@@ -5,11 +5,14 @@
 // (grid_gpu.cu:352-365) and set_bookmarks (grid_gpu.cu:366-390):
 //
 //   bin_count    index step per visibility (bit-exact with grid.cu:159-163),
-//                packed main*G+sub pair, global uv-tile key, tile histogram
-//   scan         exclusive prefix sum of the histogram = bookmarks
-//   bin_scatter  places every kept visibility at its sorted position and
-//                copies its packed indices and values there (SoA planes), so
-//                the gridding kernels stream each tile contiguously
+//                global uv-tile key, tile histogram, rank in the tile
+//   scan         exclusive prefix sum of the histogram
+//   bin_finish   places every kept visibility's record and values at its
+//                sorted position, so the gridding kernels stream each tile
+//                contiguously; writes the bookmarks; makes the work items
+//
+// Four launches with the set-up; they had been up to ten, a quarter of the time
+// of a 10 k visibility call.
 //
 // All kernels work on a batch of jobs sharing one global visibility index
 // space and one global tile space; a single job is a batch of one.
@@ -54,9 +57,10 @@ __device__ __forceinline__ int find_job32(const int *base, int njobs, int g) {
 // the job table (dependent loads) on every step.
 struct WarpSlice {
   int64_t w0, w1;
-  __device__ WarpSlice(int64_t total) {
-    const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const int64_t wid = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  __device__ WarpSlice(int64_t total) : WarpSlice(total, blockIdx.x, gridDim.x) {}
+  __device__ WarpSlice(int64_t total, int64_t block, int64_t nblocks) {
+    const int64_t nwarps = nblocks * (blockDim.x >> 5);
+    const int64_t wid = block * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int64_t per = ((total + nwarps - 1) / nwarps + 31) & ~(int64_t)31;
     w0 = min(total, wid * per);
     w1 = min(total, w0 + per);
@@ -67,11 +71,8 @@ __device__ __forceinline__ int advance_job(const int64_t *base, int njobs, int j
   return j;
 }
 
-__device__ __forceinline__ unsigned lanemask_lt() {
-  unsigned m;
-  asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-  return m;
-}
+// entries of a scan block, and of one of its threads
+constexpr int kScanPer = 8, kScanBlock = 2048;
 
 // index step of visibility n of a uv array of either precision
 __device__ __forceinline__ bool uv_index(const void *uv, int uv_f64, int64_t n,
@@ -104,152 +105,145 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Pass 1.  Every visibility of every job: index step, drop rules, tile key,
-// warp-aggregated histogram increment.
+// resident CTAs per SM of the two passes over the visibilities: both wait on
+// loads and atomics, and 42 registers a thread hold a visibility without
+// spills (4.19 M visibilities, both passes and the tiles: 6 CTAs 384 us of the
+// whole call, 8 CTAs 396; two or four visibilities a lane at once 396-409)
+constexpr int kBinCtas = 6;
+
+// Pass 1.  Every visibility of every job: index step, drop rules, tile key, and
+// its rank among the visibilities of its tile.
 //  * a visibility whose oversample index falls outside [0,G) would address
 //    outside the GCF table in the reference; it is dropped and counted
 //  * a visibility whose footprint misses the grid contributes nothing and is
 //    dropped silently (the reference skips all of its taps, grid.cu:174-176)
-//  * mains left/right of the grid are clamped into the edge tile: all of
-//    their on-grid taps still lie inside that tile's window region
-__global__ void __launch_bounds__(256) bin_count_kernel(BinBuffers b) {
+//  * mains left/right of the grid are clamped into the edge tile (all of their
+//    on-grid taps still lie inside that tile's window region), unless the
+//    tiles start before the grid
+// The rank comes from the histogram's own atomics, one for each run of equal
+// keys in a warp's 32 visibilities (tracks stay in a tile for many samples):
+// the scattering pass then needs no second round of claims.
+__global__ void __launch_bounds__(256, kBinCtas)
+    bin_count_kernel(const __grid_constant__ BinBuffers b) {
   const int lane = threadIdx.x & 31;
   const WarpSlice ws(b.total_vis);
   int jw = b.njobs == 1 || ws.w0 >= ws.w1 ? 0 : find_job64(b.vis_base, b.njobs, ws.w0);
   for (int64_t base = ws.w0; base < ws.w1; base += 32) {
-    int64_t g = base + lane;
-    bool valid = g < ws.w1;
+    const int64_t g = base + lane;
     int key = -1;
     bool bad = false;
     if (b.njobs > 1) jw = advance_job(b.vis_base, b.njobs, jw, base);
-    if (valid) {
-      int j = b.njobs == 1 ? 0 : job_from(b.vis_base, b.njobs, jw, g);
-      const BinJob &J = b.jobs[j];
+    if (g < ws.w1) {
+      const BinJob &J = b.jobs[b.njobs == 1 ? 0 : job_from(b.vis_base, b.njobs, jw, g)];
       int mx, sx, my, sy;
-      int2 pk = make_int2(INT_MIN, INT_MIN);
-      bool ok = uv_index(J.uv, J.uv_f64, g - J.vis_base, J.G, mx, sx, my, sy);
-      if (ok && ((unsigned)sx >= (unsigned)J.G || (unsigned)sy >= (unsigned)J.G))
-        ok = false;
+      bool ok = uv_index(J.uv, J.uv_f64, g - J.vis_base, J.G, mx, sx, my, sy) &&
+                (unsigned)sx < (unsigned)J.G && (unsigned)sy < (unsigned)J.G;
       int gi = 0;
       if (ok && J.gcf_index) {
         gi = __ldg(J.gcf_index + (g - J.vis_base));
-        if ((unsigned)gi >= (unsigned)J.n_gcf) ok = false;
+        ok = (unsigned)gi < (unsigned)J.n_gcf;
       }
       bad = !ok;
-      if (ok) {
-        pk = make_int2(mx * J.G + sx, my * J.G + sy);
-        const int h = J.S >> 1;
-        if (mx + h >= 0 && mx - h + 1 < J.N && my + h >= 0 && my - h + 1 < J.N) {
-          // tiles that start before the grid need no clamping
-          const int cx = (J.off ? mx + J.off : min(max(mx, 0), J.N - 1)) >> J.log2T;
-          const int cy = (J.off ? my + J.off : min(max(my, 0), J.N - 1)) >> J.log2T;
-          key = J.tile_base + (cy * J.ntx + cx) * J.n_gcf + gi;
-        }
+      const int h = J.S >> 1;
+      if (ok && mx + h >= 0 && mx - h + 1 < J.N && my + h >= 0 && my - h + 1 < J.N) {
+        // tiles that start before the grid need no clamping
+        const int cx = (J.off ? mx + J.off : min(max(mx, 0), J.N - 1)) >> J.log2T;
+        const int cy = (J.off ? my + J.off : min(max(my, 0), J.N - 1)) >> J.log2T;
+        key = J.tile_base + (cy * J.ntx + cx) * J.n_gcf + gi;
       }
-      b.packed[g] = pk;
-      b.key[g] = key;
+    }
+    const unsigned badm = __ballot_sync(0xffffffffu, bad);
+    if (badm && lane == 0) atomicAdd(&b.flags[FLAG_INDEX], __popc(badm));
+    // runs of equal keys: the first lane of each claims for all
+    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
+    const bool head = lane == 0 || key != prev;
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+    const unsigned after = lane == 31 ? 0u : heads >> (lane + 1);
+    int start = 0;
+    if (head && key >= 0) start = atomicAdd(&b.counts[key], after ? __ffs(after) : 32 - lane);
+    start = __shfl_sync(0xffffffffu, start, first);
+    if (g < ws.w1) {
+      b.key_rank[g] = make_int2(key, start + lane - first);
       if (b.kept_pos) b.kept_pos[g] = key >= 0 ? 1 : 0;
     }
-    unsigned badm = __ballot_sync(0xffffffffu, bad);
-    if (badm && lane == 0) atomicAdd(&b.flags[FLAG_INDEX], __popc(badm));
-    unsigned peers = __match_any_sync(0xffffffffu, key);
-    if (key >= 0 && lane == __ffs(peers) - 1)
-      atomicAdd(&b.bookmarks[key], __popc(peers));
   }
 }
 
-// Pass 3.  Sorted position of every kept visibility; copy of its packed
-// indices (and of its values, one plane per polarisation).
-//   generic:       position = bookmarks[key] + claim on cursor[key]
-//                  (one atomic per run of equal keys within a warp)
-//   input_sorted:  position = number of kept visibilities before it, which
-//                  keeps input order; a visibility landing outside its own
-//                  tile's range proves the input was not tile-sorted
-__global__ void __launch_bounds__(256) bin_scatter_kernel(BinBuffers b) {
+// first sorted position of tile t: the scan's block-local sum and its block's
+// offset
+__device__ __forceinline__ int tile_first(const BinBuffers &b, int t) {
+  return b.counts[t] + b.block_off[t / kScanBlock];
+}
+
+// Pass 3, one part.  Sorted record of every kept visibility at the first
+// position of its tile + its rank (input_sorted: the number of kept
+// visibilities before it, which keeps input order; a visibility landing
+// outside its own tile's range proves the input was not tile-sorted), and its
+// values (one plane per polarisation; with `aos` the one value beside the
+// record, one 16-byte store instead of two of 8).
+__device__ __forceinline__ void bin_scatter_part(const BinBuffers &b, int64_t block,
+                                                 int64_t nblocks) {
   const int lane = threadIdx.x & 31;
-  const WarpSlice ws(b.total_vis);
+  const WarpSlice ws(b.total_vis, block, nblocks);
   int jw = b.njobs == 1 || ws.w0 >= ws.w1 ? 0 : find_job64(b.vis_base, b.njobs, ws.w0);
   for (int64_t base = ws.w0; base < ws.w1; base += 32) {
-    int64_t g = base + lane;
-    bool valid = g < ws.w1;
-    int key = valid ? b.key[g] : -1;
-    // What is copied does not depend on the sorted position: its loads (the
-    // packed indices and the first value plane) are issued before the
-    // position's atomic, so that their latency overlaps it.
+    const int64_t g = base + lane;
+    const int2 kr = g < ws.w1 ? __ldg(b.key_rank + g) : make_int2(-1, 0);
     if (b.njobs > 1) jw = advance_job(b.vis_base, b.njobs, jw, base);
-    const BinJob *J = nullptr;
-    int64_t n = 0;
-    int2 pk = make_int2(0, 0);
+    if (kr.x < 0) continue;
+    const BinJob &J = b.jobs[b.njobs == 1 ? 0 : job_from(b.vis_base, b.njobs, jw, g)];
+    const int64_t n = g - J.vis_base;
+    // the value and the position do not depend on each other: both loads first
     float2 v8 = make_float2(0.f, 0.f);
-    double2 v16 = make_double2(0.0, 0.0);
-    if (key >= 0) {
-      J = b.jobs + (b.njobs == 1 ? 0 : job_from(b.vis_base, b.njobs, jw, g));
-      n = g - J->vis_base;
-      pk = b.packed[g];
-      if (b.vals_bytes == 8) v8 = __ldg((const float2 *)J->vals + n * b.P);
-      else v16 = __ldg((const double2 *)J->vals + n * b.P);
-    }
-    int pos = -1;
+    if (b.vals_bytes == 8) v8 = __ldg((const float2 *)J.vals + n * b.P);
+    int pos;
     if (b.input_sorted) {
-      if (key >= 0) {
-        pos = b.kept_pos[g];
-        if (pos < b.bookmarks[key] || pos >= b.bookmarks[key + 1]) {
-          atomicOr(&b.flags[FLAG_UNSORTED], 1);
-          b.bookmarks[b.total_tiles + 1] = 1;  // this call's records have holes
-          pos = -1;
-        }
+      pos = b.kept_pos[g];
+      if (pos < tile_first(b, kr.x) || pos >= tile_first(b, kr.x + 1)) {
+        atomicOr(&b.flags[FLAG_UNSORTED], 1);
+        b.bookmarks[b.total_tiles + 1] = 1;  // this call's records have holes
+        continue;
       }
     } else {
-      unsigned peers = __match_any_sync(0xffffffffu, key);
-      int leader = __ffs(peers) - 1;
-      int start = 0;
-      if (key >= 0 && lane == leader)
-        start = atomicAdd(&b.cursor[key], __popc(peers));
-      start = __shfl_sync(0xffffffffu, start, leader);
-      if (key >= 0) pos = start + __popc(peers & lanemask_lt());
+      pos = tile_first(b, kr.x) + kr.y;
     }
-    if (pos >= 0) {
-      if (b.window_records) {
-        const int mx = pk.x >> J->log2G, sx = pk.x & (J->G - 1);
-        const int my = pk.y >> J->log2G, sy = pk.y & (J->G - 1);
-        pk = J->reg ? regtile_record(mx & (kRegTile - 1), sx, my & (kRegTile - 1), sy, J->G, J->S)
-                    : window_record(mx, sx, my, sy, J->G);
-      }
-      b.sorted_idx[pos] = pk;
+    int mx, sx, my, sy;
+    uv_index(J.uv, J.uv_f64, n, J.G, mx, sx, my, sy);
+    int2 rec;
+    if (!b.window_records) rec = make_int2(mx * J.G + sx, my * J.G + sy);
+    else if (J.reg)
+      rec = regtile_record(mx & (kRegTile - 1), sx, my & (kRegTile - 1), sy, J.G, J.S);
+    else rec = window_record(mx, sx, my, sy, J.G);
+    if (b.aos) {
+      reinterpret_cast<float4 *>(b.sorted_idx)[pos] =
+          make_float4(__int_as_float(rec.x), __int_as_float(rec.y), v8.x, v8.y);
+    } else {
+      b.sorted_idx[pos] = rec;
       if (b.vals_bytes == 8) {
-        const float2 *v = (const float2 *)J->vals + n * b.P;
+        const float2 *v = (const float2 *)J.vals + n * b.P;
         float2 *o = (float2 *)b.sorted_vals;
         o[pos] = v8;
         for (int p = 1; p < b.P; ++p) o[p * b.vstride + pos] = __ldg(v + p);
       } else {
-        const double2 *v = (const double2 *)J->vals + n * b.P;
+        const double2 *v = (const double2 *)J.vals + n * b.P;
         double2 *o = (double2 *)b.sorted_vals;
-        o[pos] = v16;
-        for (int p = 1; p < b.P; ++p) o[p * b.vstride + pos] = __ldg(v + p);
+        for (int p = 0; p < b.P; ++p) o[p * b.vstride + pos] = __ldg(v + p);
       }
-      if (b.order) b.order[pos] = (int)g;
     }
+    if (b.order) b.order[pos] = (int)g;
   }
 }
 
 // ---- exclusive scan ---------------------------------------------------------
-constexpr int kScanThreads = 256, kScanPer = 8,
-              kScanBlock = kScanThreads * kScanPer;
+constexpr int kScanThreads = kScanBlock / kScanPer;
 
-__global__ void __launch_bounds__(kScanThreads)
-    scan_block_kernel(int *d, int64_t n, int *bsum) {
+// Exclusive prefix of a block's kScanBlock entries (v: this thread's kScanPer,
+// replaced by their prefixes); returns the block's total.
+__device__ __forceinline__ int scan_in_block(int (&v)[kScanPer]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int64_t base = blockIdx.x * (int64_t)kScanBlock + threadIdx.x * kScanPer;
-  int v[kScanPer];
-  if (base + kScanPer <= n) {
-    int4 a = *reinterpret_cast<const int4 *>(d + base);
-    int4 c = *reinterpret_cast<const int4 *>(d + base + 4);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
-  } else {
-#pragma unroll
-    for (int i = 0; i < kScanPer; ++i) v[i] = base + i < n ? d[base + i] : 0;
-  }
+  __shared__ int wsum[kScanThreads / 32];
+  __shared__ int total;
   int s = 0;
 #pragma unroll
   for (int i = 0; i < kScanPer; ++i) {
@@ -263,8 +257,7 @@ __global__ void __launch_bounds__(kScanThreads)
     int y = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += y;
   }
-  __shared__ int wsum[kScanThreads / 32];
-  __shared__ int total;
+  __syncthreads();  // an earlier call's sums were read
   if (lane == 31) wsum[warp] = incl;
   __syncthreads();
   if (warp == 0) {
@@ -279,20 +272,71 @@ __global__ void __launch_bounds__(kScanThreads)
     if (lane == 31) total = xi;
   }
   __syncthreads();
-  int off = wsum[warp] + incl - s;
+  const int off = wsum[warp] + incl - s;
+#pragma unroll
+  for (int i = 0; i < kScanPer; ++i) v[i] += off;
+  return total;
+}
+
+__device__ __forceinline__ void scan_load(const int *d, int64_t n, int64_t base,
+                                          int (&v)[kScanPer]) {
   if (base + kScanPer <= n) {
-    int4 a = make_int4(v[0] + off, v[1] + off, v[2] + off, v[3] + off);
-    int4 c = make_int4(v[4] + off, v[5] + off, v[6] + off, v[7] + off);
-    *reinterpret_cast<int4 *>(d + base) = a;
-    *reinterpret_cast<int4 *>(d + base + 4) = c;
+    const int4 a = *reinterpret_cast<const int4 *>(d + base);
+    const int4 c = *reinterpret_cast<const int4 *>(d + base + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < kScanPer; ++i) v[i] = base + i < n ? d[base + i] : 0;
+  }
+}
+__device__ __forceinline__ void scan_store(int *d, int64_t n, int64_t base,
+                                           const int (&v)[kScanPer]) {
+  if (base + kScanPer <= n) {
+    *reinterpret_cast<int4 *>(d + base) = make_int4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<int4 *>(d + base + 4) = make_int4(v[4], v[5], v[6], v[7]);
   } else {
 #pragma unroll
     for (int i = 0; i < kScanPer; ++i)
-      if (base + i < n) d[base + i] = v[i] + off;
+      if (base + i < n) d[base + i] = v[i];
   }
-  if (bsum && threadIdx.x == 0) bsum[blockIdx.x] = total;
 }
 
+// Block-local exclusive prefixes of d in place; block_off[b] = the sum of the
+// blocks before b, worked out by the block that finishes last (ticket, zeroed
+// by the caller, counts them): one launch, and nothing waits.  The readers add
+// d[i] and block_off[i / kScanBlock].
+__global__ void __launch_bounds__(kScanThreads)
+    scan_kernel(int *d, int64_t n, int *block_off, int *ticket) {
+  __shared__ bool last;
+  const int64_t base = blockIdx.x * (int64_t)kScanBlock + threadIdx.x * kScanPer;
+  int v[kScanPer];
+  scan_load(d, n, base, v);
+  const int total = scan_in_block(v);
+  scan_store(d, n, base, v);
+  if (threadIdx.x == 0) {
+    block_off[blockIdx.x] = total;
+    __threadfence();
+    last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  int carry = 0;
+  for (int64_t b0 = 0; b0 < gridDim.x; b0 += kScanBlock) {
+    const int64_t at = b0 + threadIdx.x * kScanPer;
+#pragma unroll
+    for (int i = 0; i < kScanPer; ++i)
+      v[i] = at + i < gridDim.x ? __ldcg(block_off + at + i) : 0;
+    const int sum = scan_in_block(v);
+#pragma unroll
+    for (int i = 0; i < kScanPer; ++i)
+      if (at + i < gridDim.x) block_off[at + i] = v[i] + carry;
+    carry += sum;
+  }
+}
+
+// the block offsets added in place
 __global__ void __launch_bounds__(kScanThreads)
     scan_add_kernel(int *d, int64_t n, const int *boff) {
   int add = boff[blockIdx.x];
@@ -304,25 +348,14 @@ __global__ void __launch_bounds__(kScanThreads)
 static int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 size_t scan_tmp_ints(int64_t n) {
-  size_t t = 0;
-  while (n > kScanBlock) {
-    n = cdiv(n, kScanBlock);
-    t += (size_t)((n + 7) & ~7ll) + 8;
-  }
-  return t + 8;
+  return (size_t)cdiv(n, kScanBlock) + kScanHead;
 }
 
-cudaError_t scan_exclusive(int *d, int64_t n, int *tmp, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  int64_t nb = cdiv(n, kScanBlock);
-  scan_block_kernel<<<(unsigned)nb, kScanThreads, 0, s>>>(d, n, nb > 1 ? tmp : nullptr);
+// tmp: the ticket (zeroed by the caller) in its first word, block offsets from
+// kScanHead on
+static cudaError_t scan_local(int *d, int64_t n, int *tmp, cudaStream_t s) {
+  scan_kernel<<<(unsigned)cdiv(n, kScanBlock), kScanThreads, 0, s>>>(d, n, tmp + kScanHead, tmp);
   count_launch();
-  if (nb > 1) {
-    cudaError_t e = scan_exclusive(tmp, nb, tmp + ((nb + 7) & ~7ll) + 8, s);
-    if (e != cudaSuccess) return e;
-    scan_add_kernel<<<(unsigned)nb, kScanThreads, 0, s>>>(d, n, tmp);
-    count_launch();
-  }
   return cudaGetLastError();
 }
 
@@ -341,32 +374,6 @@ cudaError_t launch_vis2ints(int uv_f64, const void *uv, int64_t npts, int G,
   return cudaGetLastError();
 }
 
-cudaError_t run_binning(const BinBuffers &b, cudaStream_t s) {
-  cudaError_t e;
-  e = cudaMemsetAsync(b.bookmarks, 0, sizeof(int) * (size_t)(b.total_tiles + 2), s);
-  if (e != cudaSuccess) return e;
-  if (b.total_vis > 0) {
-    bin_count_kernel<<<grid_for(b.total_vis), 256, 0, s>>>(b);
-    count_launch();
-  }
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = scan_exclusive(b.bookmarks, b.total_tiles + 1, b.scan_tmp, s)) != cudaSuccess)
-    return e;
-  if (b.input_sorted) {
-    if ((e = scan_exclusive(b.kept_pos, b.total_vis, b.scan_tmp, s)) != cudaSuccess)
-      return e;
-  } else {
-    e = cudaMemcpyAsync(b.cursor, b.bookmarks, sizeof(int) * (size_t)b.total_tiles,
-                        cudaMemcpyDeviceToDevice, s);
-    if (e != cudaSuccess) return e;
-  }
-  if (b.total_vis > 0) {
-    bin_scatter_kernel<<<grid_for(b.total_vis), 256, 0, s>>>(b);
-    count_launch();
-  }
-  return cudaGetLastError();
-}
-
 // ---- work items ---------------------------------------------------------------
 
 // inclusive warp prefix sum
@@ -379,73 +386,79 @@ __device__ __forceinline__ int warp_incl_sum(int v, int lane) {
   return v;
 }
 
-__global__ void __launch_bounds__(256)
-    make_items_kernel(const int *bm, const int *tile_base, const int *job_class,
-                      int njobs, int total_tiles, ClassChunks chunks, WorkItem *items,
-                      int64_t class_cap, int *counters, const JobDesc *jobs, ClassSlots slots,
-                      int *heavy_counters, int *flags) {
+// Pass 3, the other part.  The final bookmarks, and the work items of the
+// moving window: every non-empty tile cut into slices of at most its class's
+// records.  A tile cut into several items gets a merge slot, cleared here.
+__device__ __forceinline__ void bin_tiles_part(const BinBuffers &b, const ItemBuffers &it,
+                                               int block, int nblocks) {
   const int lane = threadIdx.x & 31;
-  for (int base = blockIdx.x * 256 + (threadIdx.x & ~31); base < total_tiles;
-       base += gridDim.x * 256) {
-    int t = base + lane;
-    int k = 0, s0 = 0, e0 = 0, j = 0, cls = 0, chunk = 1;
-    if (t < total_tiles) {
-      s0 = bm[t];
-      e0 = bm[t + 1];
-      j = njobs == 1 ? 0 : find_job32(tile_base, njobs, t);
-      cls = job_class ? job_class[j] : 0;
-      chunk = chunks.c[cls];
+  for (int64_t base = (int64_t)block * 256 + (threadIdx.x & ~31); base <= b.total_tiles;
+       base += (int64_t)nblocks * 256) {
+    const int t = (int)(base + lane);
+    int s0 = 0, e0 = 0;
+    if (t <= b.total_tiles) {
+      s0 = tile_first(b, t);
+      b.bookmarks[t] = s0;
+      if (t < b.total_tiles) e0 = tile_first(b, t + 1);
+    }
+    const bool full = t < b.total_tiles && e0 > s0;
+    if (!it.items || !__any_sync(0xffffffffu, full)) continue;  // most tiles are empty
+    int k = 0, j = 0, cls = 0, chunk = 1;
+    if (full) {
+      j = b.njobs == 1 ? 0 : find_job32(b.tile_base, b.njobs, t);
+      cls = it.job_class[j];
+      chunk = it.chunks.c[cls];
       k = (e0 - s0 + chunk - 1) / chunk;
     }
-#pragma unroll
-    for (int c = 0; c < kMaxClasses; ++c) {
-      int kc = (cls == c) ? k : 0;
-      int incl = warp_incl_sum(kc, lane);
-      int tot = __shfl_sync(0xffffffffu, incl, 31);
+    for (int c = 0; c < it.nclasses; ++c) {
+      const int kc = cls == c ? k : 0;
+      if (!__any_sync(0xffffffffu, kc > 0)) continue;
+      const int incl = warp_incl_sum(kc, lane);
       int start = 0;
-      if (lane == 0 && tot) start = atomicAdd(&counters[c], tot);
-      start = __shfl_sync(0xffffffffu, start, 0);
+      if (lane == 31) start = atomicAdd(&it.counters[c], incl);
+      start = __shfl_sync(0xffffffffu, start, 31);
       // a merge slot for a tile cut into several items (complex64 grids of
       // classes with slots)
-      const MergeSlots &ms = slots.m[c];
+      const MergeSlots &ms = it.slots.m[c];
       int slot = -1;
       if (ms.base != nullptr) {  // uniform over the warp
-        const int need = kc > 1 && !jobs[j].out_f64 ? 1 : 0;
-        const int hin = warp_incl_sum(need, lane);
-        const int htot = __shfl_sync(0xffffffffu, hin, 31);
-        int h0 = 0;
-        if (lane == 0 && htot) h0 = atomicAdd(&heavy_counters[c], htot);
-        h0 = __shfl_sync(0xffffffffu, h0, 0);
-        if (need) {
-          slot = h0 + hin - 1;
-          if (slot >= ms.cap) {
-            atomicOr(&flags[FLAG_BOUNDS], 1);
-            slot = -1;
-          } else {
-            ms.desc[slot] = make_int2(j, t - tile_base[j]);
+        const int need = kc > 1 && !it.jobs[j].out_f64 ? 1 : 0;
+        const unsigned needs = __ballot_sync(0xffffffffu, need);
+        if (needs) {
+          int h0 = 0;
+          if (lane == 0) h0 = atomicAdd(&it.heavy_counters[c], __popc(needs));
+          h0 = __shfl_sync(0xffffffffu, h0, 0);
+          if (need) {
+            slot = h0 + __popc(needs & ((1u << lane) - 1));
+            if (slot >= ms.cap) {
+              atomicOr(&b.flags[FLAG_BOUNDS], 1);
+              slot = -1;
+            } else {
+              ms.desc[slot] = make_int4(j, t - b.tile_base[j], kc, 0);
+            }
+          }
+          for (unsigned left = needs; left; left &= left - 1) {
+            const int sl = __shfl_sync(0xffffffffu, slot, __ffs(left) - 1);
+            if (sl < 0) continue;
+            double2 *const cells = ms.base + (size_t)sl * ms.cells;
+            for (int i = lane; i < ms.cells; i += 32) cells[i] = make_double2(0.0, 0.0);
           }
         }
       }
       if (kc) {
-        WorkItem *dst = items + c * class_cap + start + (incl - kc);
-        int local = t - tile_base[j];
-        int ox = 0, oy = 0;
-        if (jobs) {
-          const JobDesc &J = jobs[j];
-          const int tile = J.n_gcf > 1 ? local / J.n_gcf : local;
-          ox = (tile % J.ntx) * J.T - J.off - J.S / 2 + 1;
-          oy = (tile / J.ntx) * J.T - J.off - J.S / 2 + 1;
-        }
+        WorkItem *dst = it.items + c * it.class_cap + start + (incl - kc);
+        const JobDesc &J = it.jobs[j];
+        const int local = t - b.tile_base[j], tile = J.n_gcf > 1 ? local / J.n_gcf : local;
+        WorkItem w;
+        w.job = j;
+        w.bin = local;
+        w.slot = slot;
+        w.ox = (tile % J.ntx) * J.T - J.off - J.S / 2 + 1;
+        w.oy = (tile / J.ntx) * J.T - J.off - J.S / 2 + 1;
+        w.pad_ = 0;
         for (int i = 0; i < kc; ++i) {
-          WorkItem w;
-          w.ox = ox;
-          w.oy = oy;
-          w.job = j;
-          w.bin = local;
           w.start = s0 + i * chunk;
           w.end = min(e0, s0 + (i + 1) * chunk);
-          w.slot = slot;
-          w.pad_ = 0;
           dst[i] = w;
         }
       }
@@ -453,39 +466,44 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-cudaError_t launch_make_items(const int *bookmarks, const int *tile_base,
-                              const int *job_class, int njobs, int total_tiles,
-                              ClassChunks chunk, WorkItem *items, int64_t class_cap,
-                              int *counters, cudaStream_t s, const JobDesc *jobs,
-                              const ClassSlots *slots, int *heavy_counters, int *flags) {
-  if (total_tiles <= 0) return cudaSuccess;
-  ClassSlots cs{};
-  if (slots && jobs && heavy_counters && flags) cs = *slots;
+// Pass 3: both parts side by side, the tiles' blocks first.
+__global__ void __launch_bounds__(256, kBinCtas)
+    bin_finish_kernel(const __grid_constant__ BinBuffers b, const __grid_constant__ ItemBuffers it,
+                      int tile_blocks) {
+  if ((int)blockIdx.x < tile_blocks) bin_tiles_part(b, it, blockIdx.x, tile_blocks);
+  else bin_scatter_part(b, (int64_t)blockIdx.x - tile_blocks, (int64_t)gridDim.x - tile_blocks);
+}
+
+cudaError_t run_binning(const BinBuffers &b, const ItemBuffers *items, cudaStream_t s) {
+  cudaError_t e;
+  if (b.total_vis > 0) {
+    bin_count_kernel<<<grid_for(b.total_vis), 256, 0, s>>>(b);
+    count_launch();
+  }
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if ((e = scan_local(b.counts, (int64_t)b.total_tiles + 1, b.scan_tmp, s)) != cudaSuccess)
+    return e;
+  if (b.input_sorted && b.total_vis > 0) {
+    // the ticket once more; the tiles' block offsets lie before this scan's
+    int *const tmp = b.scan_tmp + scan_tmp_ints((int64_t)b.total_tiles + 1);
+    if ((e = cudaMemsetAsync(tmp, 0, sizeof(int), s)) != cudaSuccess) return e;
+    if ((e = scan_local(b.kept_pos, b.total_vis, tmp, s)) != cudaSuccess) return e;
+    scan_add_kernel<<<(unsigned)cdiv(b.total_vis, kScanBlock), kScanThreads, 0, s>>>(
+        b.kept_pos, b.total_vis, tmp + kScanHead);
+    count_launch();
+  }
+  ItemBuffers it{};
+  if (items) it = *items;
   for (int c = 0; c < kMaxClasses; ++c)
-    if (cs.m[c].cap <= 0) cs.m[c].base = nullptr;
-  make_items_kernel<<<grid_for(total_tiles), 256, 0, s>>>(
-      bookmarks, tile_base, job_class, njobs, total_tiles, chunk, items,
-      class_cap, counters, jobs, cs, heavy_counters, flags);
+    if (it.slots.m[c].cap <= 0) it.slots.m[c].base = nullptr;
+  const unsigned tiles = grid_for(cdiv((int64_t)b.total_tiles + 1, 4));
+  const unsigned vis = b.total_vis > 0 ? grid_for(b.total_vis) : 0;
+  bin_finish_kernel<<<tiles + vis, 256, 0, s>>>(b, it, (int)tiles);
   count_launch();
   return cudaGetLastError();
 }
 
 // ---- FP64 merge slots of tiles cut into several work items ---------------------
-
-__global__ void __launch_bounds__(256)
-    merge_zero_kernel(double2 *base, int cells, int cap, const int *count) {
-  const int64_t n = (int64_t)min(*count, cap) * cells;
-  for (int64_t i = blockIdx.x * 256ll + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256)
-    base[i] = make_double2(0.0, 0.0);
-}
-
-cudaError_t launch_merge_zero(const MergeSlots &m, const int *heavy_counter, int sm_count,
-                              cudaStream_t s) {
-  if (!m.base || m.cap <= 0) return cudaSuccess;
-  merge_zero_kernel<<<sm_count * 4, 256, 0, s>>>(m.base, m.cells, m.cap, heavy_counter);
-  count_launch();
-  return cudaGetLastError();
-}
 
 // one CTA per slot (grid-stride over slots): cells of the slot's R x R
 // sub-grid (P planes), origin at the tile's corner minus the halo
@@ -495,7 +513,7 @@ __global__ void __launch_bounds__(256)
   const int n = min(*count, m.cap);
   const int R = T + S - 1, H = S / 2;
   for (int sl = blockIdx.x; sl < n; sl += gridDim.x) {
-    const int2 d = m.desc[sl];
+    const int4 d = m.desc[sl];
     const JobDesc &J = jobs[d.x];
     const int tile = J.n_gcf > 1 ? d.y / J.n_gcf : d.y;
     const int ox = (tile % J.ntx) * T - J.off - H + 1, oy = (tile / J.ntx) * T - J.off - H + 1;
@@ -531,33 +549,90 @@ cudaError_t launch_inject_flags(int *flags, int bits, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// ---- table upload through kernel parameters -------------------------------------
+// ---- set-up: table upload through kernel parameters, and clearing ----------------
 // A launch carries its parameters with it (copied by the driver at the call),
 // so tables sent this way never wait on a copy engine behind the bulk
 // transfers of other streams, and the host buffer is free once the call
 // returns.
 constexpr int kUploadChunk = 16384;  // bytes per launch (parameters: up to 32 KB)
-struct UploadChunk {
+struct SetupParams {
   uint4 *dst;
   int n16;  // 16-byte words in this chunk
+  ZeroRanges zero;
   uint4 data[kUploadChunk / 16];
 };
 
-__global__ void __launch_bounds__(256) upload_kernel(const __grid_constant__ UploadChunk p) {
-  for (int i = threadIdx.x; i < p.n16; i += 256) p.dst[i] = p.data[i];
+__device__ __forceinline__ void zero_range(void *p, size_t bytes, size_t i, size_t stride) {
+  if ((reinterpret_cast<uintptr_t>(p) | bytes) % 16 == 0) {
+    uint4 *const q = static_cast<uint4 *>(p);
+    for (; i < bytes / 16; i += stride) q[i] = make_uint4(0, 0, 0, 0);
+  } else {
+    int *const q = static_cast<int *>(p);
+    for (; i < bytes / 4; i += stride) q[i] = 0;
+  }
 }
 
-cudaError_t launch_upload(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+__global__ void __launch_bounds__(256) setup_kernel(const __grid_constant__ SetupParams p) {
+  const size_t i = blockIdx.x * 256 + threadIdx.x, stride = (size_t)gridDim.x * 256;
+  for (int k = (int)i; k < p.n16; k += (int)stride) p.dst[k] = p.data[k];
+  for (int r = 0; r < p.zero.n; ++r) zero_range(p.zero.p[r], p.zero.bytes[r], i, stride);
+}
+// the same without a table: its launch carries no 16 KB of parameters
+__global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ ZeroRanges z) {
+  const size_t i = blockIdx.x * 256 + threadIdx.x, stride = (size_t)gridDim.x * 256;
+  for (int r = 0; r < z.n; ++r) zero_range(z.p[r], z.bytes[r], i, stride);
+}
+
+cudaError_t launch_setup(void *dst, const void *src, size_t bytes, const ZeroRanges &zero,
+                         cudaStream_t s) {
   if (bytes % 16 || (uintptr_t)dst % 16) return cudaErrorInvalidValue;
-  static thread_local UploadChunk p;  // 16 KB: off the stack
+  size_t clear = 0;
+  for (int r = 0; r < zero.n; ++r) clear += zero.bytes[r];
+  // 4 KB a block, up to eight blocks on each of 152 SMs
+  const unsigned blocks = (unsigned)std::min<size_t>(152 * 8, 1 + clear / 4096);
+  if (bytes == 0) {
+    if (zero.n > 0) {
+      clear_kernel<<<blocks, 256, 0, s>>>(zero);
+      count_launch();
+    }
+    return cudaGetLastError();
+  }
+  static thread_local SetupParams p;  // 16 KB: off the stack
   for (size_t o = 0; o < bytes; o += kUploadChunk) {
     const size_t n = std::min<size_t>(kUploadChunk, bytes - o);
     p.dst = reinterpret_cast<uint4 *>(static_cast<char *>(dst) + o);
     p.n16 = (int)(n / 16);
+    p.zero = o == 0 ? zero : ZeroRanges{};
     memcpy(p.data, static_cast<const char *>(src) + o, n);
-    upload_kernel<<<1, 256, 0, s>>>(p);
+    setup_kernel<<<o == 0 ? blocks : 1, 256, 0, s>>>(p);
     count_launch();
   }
+  return cudaGetLastError();
+}
+
+// The output grids of a batch's jobs [j0, j1), kZeroChunk bytes at a time
+// (JobDesc::blk0 numbers the chunks of the jobs of a class): one launch where
+// a memset for each of 256 jobs took twice the time.
+__global__ void __launch_bounds__(256)
+    zero_jobs_kernel(const JobDesc *jobs, int njobs, int chunks) {
+  for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
+    int j = 0, e = njobs - 1;
+    while (j < e) {
+      const int mid = (j + e + 1) >> 1;
+      if (__ldg(&jobs[mid].blk0) <= c) j = mid; else e = mid - 1;
+    }
+    const JobDesc &J = jobs[j];
+    const size_t bytes = (size_t)(J.out_f64 ? 16 : 8) * J.P * J.N * J.N;
+    const size_t o = (size_t)(c - J.blk0) * kZeroChunk;
+    zero_range(static_cast<char *>(J.out) + o, min(kZeroChunk, bytes - o), threadIdx.x, 256);
+  }
+}
+
+cudaError_t launch_zero_jobs(const JobDesc *jobs, int njobs, int chunks, int sm_count,
+                             cudaStream_t s) {
+  if (chunks <= 0) return cudaSuccess;
+  zero_jobs_kernel<<<std::min(chunks, sm_count * 8), 256, 0, s>>>(jobs, njobs, chunks);
+  count_launch();
   return cudaGetLastError();
 }
 

@@ -41,13 +41,16 @@ struct BinBuffers {
   int total_tiles;         // sum of ntiles
   int vals_bytes;          // 8 (complex64) or 16 (complex128)
   int P;                   // polarisations (uniform over the batch)
-  int2 *packed;            // [total_vis]
-  int *key;                // [total_vis] global tile id or -1 (dropped)
-  int *bookmarks;          // [total_tiles+1]: counts, then exclusive offsets;
-                           // [total_tiles+1]: set when input declared sorted
-                           // is not (records left unwritten)
-  int *cursor;             // [total_tiles]
-  int *scan_tmp;           // scratch for the multi-level scan
+  int2 *key_rank;          // [total_vis] global tile id (-1: dropped), rank in
+                           // the tile
+  int *counts;             // [total_tiles+1], zeroed by the caller: histogram,
+                           // then block-local offsets
+  int *scan_tmp;           // scan_tmp_ints; the first word zeroed by the caller
+  int *block_off;          // scan_tmp + kScanHead: offsets of the scan's blocks
+  int *bookmarks;          // [total_tiles+2]: exclusive offsets; the word at
+                           // total_tiles+1 (zeroed by the caller) is set when
+                           // input declared sorted is not (records left
+                           // unwritten)
   int2 *sorted_idx;        // [total_vis + pad]
   void *sorted_vals;       // [P][vstride]
   int64_t vstride;
@@ -59,6 +62,8 @@ struct BinBuffers {
   // 1 = moving window: {main cells (my+64)<<16 | (mx+64), sub-kernel
   //     sy*G+sx} -- see window_record()
   int window_records;
+  // one value per visibility, complex64: {record, value} in sorted_idx
+  int aos;
 };
 
 // Sorted record of the moving-window kernel: both main cells in one word
@@ -86,11 +91,10 @@ __host__ __device__ inline int2 regtile_record(int fx, int sx, int fy, int sy, i
 // index step only (vis2ints)
 cudaError_t launch_vis2ints(int uv_f64, const void *uv, int64_t npts, int G,
                             int2 *packed, int *flags, cudaStream_t s);
-// count, scan, scatter; leaves bookmarks = exclusive offsets [total_tiles+1]
-cudaError_t run_binning(const BinBuffers &b, cudaStream_t s);
-// exclusive scan of n ints in place; tmp needs scan_tmp_ints(n) ints
+// words before the block offsets in a scan's scratch
+constexpr int kScanHead = 8;
+// ints of scratch for a scan of n entries
 size_t scan_tmp_ints(int64_t n);
-cudaError_t scan_exclusive(int *data, int64_t n, int *tmp, cudaStream_t s);
 
 // Work items for the moving-window kernel: every non-empty tile of job j
 // (global tiles tile_base..) is cut into slices of at most `chunk` sorted
@@ -110,12 +114,20 @@ struct ClassChunks {
 struct ClassSlots {
   MergeSlots m[kMaxClasses];
 };
-cudaError_t launch_make_items(const int *bookmarks, const int *tile_base,
-                              const int *job_class, int njobs, int total_tiles,
-                              ClassChunks chunk, WorkItem *items, int64_t class_cap,
-                              int *counters, cudaStream_t s,
-                              const JobDesc *jobs = nullptr, const ClassSlots *slots = nullptr,
-                              int *heavy_counters = nullptr, int *flags = nullptr);
+struct ItemBuffers {
+  WorkItem *items;         // null: no items
+  const JobDesc *jobs;
+  const int *job_class;
+  int nclasses;
+  ClassChunks chunks;
+  int64_t class_cap;
+  int *counters;           // [kMaxClasses], zeroed by the caller
+  int *heavy_counters;     // [kMaxClasses], zeroed by the caller
+  ClassSlots slots;
+};
+// count, scan, scatter; leaves bookmarks = exclusive offsets [total_tiles+1],
+// and makes the work items when given
+cudaError_t run_binning(const BinBuffers &b, const ItemBuffers *items, cudaStream_t s);
 // Number of merge slots a class needs at most: tiles with more than `chunk`
 // records, at most vis / (chunk + 1) of them.
 inline int merge_slot_cap(int64_t vis, int chunk, int64_t tiles) {
@@ -123,10 +135,6 @@ inline int merge_slot_cap(int64_t vis, int chunk, int64_t tiles) {
   if (c > tiles) c = tiles;
   return (int)c;
 }
-// Clears the slots a class took (heavy_counter on the device) before its
-// window kernel adds into them.
-cudaError_t launch_merge_zero(const MergeSlots &m, const int *heavy_counter, int sm_count,
-                              cudaStream_t s);
 // Rounds every slot of the class once into its job's grid (after the
 // class's window kernel): cell values that are nonzero are reduced into the
 // output with the grid's layout, cells outside the grid skipped.
@@ -136,10 +144,27 @@ cudaError_t launch_merge_finalize(const MergeSlots &m, const int *heavy_counter,
 // ORs `bits` (1 << FLAG_*) into flags[FLAG_*] on the stream: the host-side
 // injection behind gg_debug_inject_device_flags.
 cudaError_t launch_inject_flags(int *flags, int bits, cudaStream_t s);
-// Copies `bytes` (a multiple of 16, dst 16-byte aligned) from host memory to
-// dst on the stream through kernel parameters, 16 KB per launch: nothing
-// waits on a copy engine, and src may be rewritten once the call returns.
-cudaError_t launch_upload(void *dst, const void *src, size_t bytes, cudaStream_t s);
+// Up to kMaxZero ranges of device memory (4-byte aligned) to clear.
+constexpr int kMaxZero = 7;
+struct ZeroRanges {
+  void *p[kMaxZero];
+  size_t bytes[kMaxZero];
+  int n;
+  void add(void *q, size_t b) {
+    p[n] = q;
+    bytes[n++] = b;
+  }
+};
+// Copies `bytes` (a multiple of 16, dst 16-byte aligned; 0: none) from host
+// memory to dst on the stream through kernel parameters, 16 KB per launch
+// (nothing waits on a copy engine, and src may be rewritten once the call
+// returns), and clears the ranges.
+cudaError_t launch_setup(void *dst, const void *src, size_t bytes, const ZeroRanges &zero,
+                         cudaStream_t s);
+// clears the output grids of `njobs` jobs in `chunks` pieces of kZeroChunk
+constexpr size_t kZeroChunk = 64 << 10;
+cudaError_t launch_zero_jobs(const JobDesc *jobs, int njobs, int chunks, int sm_count,
+                             cudaStream_t s);
 // flags of a context (device int32[64], see gg_read_flags)
 int *context_flags(gg_context *c);
 // Makes the batched calls of a context use `flags` (device int32[64], the
@@ -216,7 +241,8 @@ struct RegTileLaunch {
   const WorkItem *items;
   const int *nitems;
   int *item_next;
-  const int2 *idx;         // sorted records (regtile_record)
+  const int2 *idx;         // sorted records (regtile_record); {record, value}
+                           // pairs of 16 bytes when vals is null
   const float2 *vals;      // sorted values, P planes of vstride
   int64_t vstride;
   const float2 *gcf;       // [G*G][S][S]
@@ -236,7 +262,8 @@ struct SepTileLaunch {
   int njobs;
   int total_blocks;
   int *next;               // zeroed counter of claimed blocks
-  const int2 *idx;         // sorted records (window_record)
+  const int2 *idx;         // sorted records (window_record); {record, value}
+                           // pairs of 16 bytes when vals is null
   const float2 *vals;      // sorted values, P planes of vstride
   int64_t vstride;
   int G, P;

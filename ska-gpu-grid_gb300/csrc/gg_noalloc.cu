@@ -13,7 +13,7 @@
 // Limits: at most kNoAllocMaxVis visibilities, img_dim up to 4096 with the
 // default 32-cell tile (kNoAllocMaxTiles uv tiles), one polarisation,
 // complex64 values, a GCF table of at most 65536 taps (G*G*S*S).  The array
-// (kScratchBytes = 12206336 bytes, 11.6 MiB) is held by every GPU that loads
+// (kScratchBytes = 11165696 bytes, 10.6 MiB) is held by every GPU that loads
 // this library until the process exits.
 //
 // Set-up: the first call on a device looks up the device address of the
@@ -54,13 +54,13 @@ constexpr size_t kOffClass = kOffTileBase + al(2 * sizeof(int));
 // taken [16, 20)
 constexpr int kFlagInts = 32;
 constexpr size_t kOffFlags = kOffClass + al(sizeof(int));
-constexpr size_t kOffPacked = kOffFlags + al(kFlagInts * sizeof(int));
-constexpr size_t kOffKey = kOffPacked + al(sizeof(int2) * (kNoAllocMaxVis + 1));
-constexpr size_t kOffBm = kOffKey + al(sizeof(int) * (kNoAllocMaxVis + 1));
-constexpr size_t kOffCursor = kOffBm + al(sizeof(int) * (kNoAllocMaxTiles + 8));
-constexpr size_t kOffScan = kOffCursor + al(sizeof(int) * (kNoAllocMaxTiles + 8));
-// scan scratch for up to max(tiles, vis)+1 entries: 2048-entry blocks
-constexpr size_t kScanInts = (kNoAllocMaxVis + 1) / 2048 + 64;
+constexpr size_t kOffKr = kOffFlags + al(kFlagInts * sizeof(int));
+constexpr size_t kOffBm = kOffKr + al(sizeof(int2) * (kNoAllocMaxVis + 1));
+constexpr size_t kOffCnt = kOffBm + al(sizeof(int) * (kNoAllocMaxTiles + 8));
+constexpr size_t kOffScan = kOffCnt + al(sizeof(int) * (kNoAllocMaxTiles + 8));
+// scratch of the scans over tiles and (input_sorted) visibilities: 2048-entry
+// blocks
+constexpr size_t kScanInts = (kNoAllocMaxVis + kNoAllocMaxTiles + 2) / 2048 + 2 + 2 * kScanHead;
 constexpr size_t kOffKept = kOffScan + al(sizeof(int) * kScanInts);
 constexpr size_t kOffSidx = kOffKept + al(sizeof(int) * (kNoAllocMaxVis + 8));
 constexpr size_t kOffSvals = kOffSidx + al(sizeof(int2) * (kNoAllocMaxVis + 8));
@@ -77,10 +77,10 @@ constexpr size_t kMergeBytes = size_t(2) << 20;
 constexpr int kMergeMaxSlots = 1024;
 constexpr size_t kOffMerge = kOffGcf + al(sizeof(float2) * 2 * kNoAllocMaxGcf);
 constexpr size_t kOffMergeDesc = kOffMerge + al(kMergeBytes);
-constexpr size_t kScratchBytes = kOffMergeDesc + al(sizeof(int2) * kMergeMaxSlots);
+constexpr size_t kScratchBytes = kOffMergeDesc + al(sizeof(int4) * kMergeMaxSlots);
 
 // the size the header and the documentation state
-static_assert(kScratchBytes == 12206336, "update the stated size of the allocation-free array");
+static_assert(kScratchBytes == 11165696, "update the stated size of the allocation-free array");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -281,11 +281,11 @@ extern "C" int gg_grid_device_noalloc(const gg_options *opt, const gg_job *job,
   b.total_tiles = (int)(ntx * ntx);
   b.vals_bytes = 8;
   b.P = 1;
-  b.packed = (int2 *)(ws + kOffPacked);
-  b.key = (int *)(ws + kOffKey);
+  b.key_rank = (int2 *)(ws + kOffKr);
+  b.counts = (int *)(ws + kOffCnt);
   b.bookmarks = (int *)(ws + kOffBm);
-  b.cursor = (int *)(ws + kOffCursor);
   b.scan_tmp = (int *)(ws + kOffScan);
+  b.block_off = b.scan_tmp + kScanHead;
   b.sorted_idx = (int2 *)(ws + kOffSidx);
   b.sorted_vals = ws + kOffSvals;
   b.vstride = kNoAllocMaxVis + 8;
@@ -294,21 +294,27 @@ extern "C" int gg_grid_device_noalloc(const gg_options *opt, const gg_job *job,
   b.input_sorted = opt->input_sorted ? 1 : 0;
   b.window_records = 1;
   b.kept_pos = b.input_sorted ? (int *)(ws + kOffKept) : nullptr;
-  GG_NA(run_binning(b, s));
-
-  WorkItem *items = (WorkItem *)(ws + kOffItems);
-  ClassChunks chunks = {{chunk, chunk, chunk, chunk}};
-  ClassSlots slots{};
+  ZeroRanges zero{};
+  zero.add(b.counts, ((size_t)(b.total_tiles + 1) * sizeof(int) + 15) & ~(size_t)15);
+  zero.add(b.scan_tmp, kScanHead * sizeof(int));
+  zero.add(b.bookmarks + b.total_tiles + 1, sizeof(int));
+  GG_NA(launch_setup(nullptr, nullptr, 0, zero, s));
+  ItemBuffers it{};
+  it.items = (WorkItem *)(ws + kOffItems);
+  it.jobs = (const JobDesc *)(ws + kOffJobs);
+  it.job_class = (const int *)(ws + kOffClass);
+  it.nclasses = 1;
+  it.chunks.c[0] = chunk;
+  it.class_cap = kClassCap;
+  it.counters = flags + 8;
+  it.heavy_counters = flags + 16;
   if (merge_cap > 0) {
-    slots.m[0].base = (double2 *)(ws + kOffMerge);
-    slots.m[0].desc = (int2 *)(ws + kOffMergeDesc);
-    slots.m[0].cap = merge_cap;
-    slots.m[0].cells = merge_cells;
+    it.slots.m[0].base = (double2 *)(ws + kOffMerge);
+    it.slots.m[0].desc = (int4 *)(ws + kOffMergeDesc);
+    it.slots.m[0].cap = merge_cap;
+    it.slots.m[0].cells = merge_cells;
   }
-  GG_NA(launch_make_items(b.bookmarks, b.tile_base, (const int *)(ws + kOffClass), 1,
-                          b.total_tiles, chunks, items, kClassCap, flags + 8, s,
-                          (const JobDesc *)(ws + kOffJobs), &slots, flags + 16, flags));
-  GG_NA(launch_merge_zero(slots.m[0], flags + 16, sms, s));
+  GG_NA(run_binning(b, &it, s));
   GridLaunch g{};
   g.jobs = (const JobDesc *)(ws + kOffJobs);
   g.njobs = 1;
@@ -323,13 +329,13 @@ extern "C" int gg_grid_device_noalloc(const gg_options *opt, const gg_job *job,
   g.flags = flags;
   g.holes = b.bookmarks + b.total_tiles + 1;
   g.sm_count = sms;
-  g.items = items;
+  g.items = it.items;
   g.nitems = flags + 8;
   g.item_next = flags + 12;
   g.max_items = kClassCap;
-  g.merge = slots.m[0];
+  g.merge = it.slots.m[0];
   GG_NA(launch_window(g, s));
-  GG_NA(launch_merge_finalize(slots.m[0], flags + 16, (const JobDesc *)(ws + kOffJobs), (int)S, T,
+  GG_NA(launch_merge_finalize(it.slots.m[0], flags + 16, (const JobDesc *)(ws + kOffJobs), (int)S, T,
                               1, sms, s));
   if (const int bits = injected_device_flags()) GG_NA(launch_inject_flags(flags, bits, s));
 #undef GG_NA

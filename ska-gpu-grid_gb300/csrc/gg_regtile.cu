@@ -95,6 +95,19 @@ template <int I, int N, class F> __device__ __forceinline__ void rt_for(F &&f) {
   }
 }
 
+// sorted record k and its value in a plane
+__device__ __forceinline__ void rt_record(const RegTileLaunch &p, int k, int plane, int2 &q,
+                                          float2 &v) {
+  if (p.vals) {
+    q = __ldg(p.idx + k);
+    v = __ldg(p.vals + plane * p.vstride + k);
+  } else {
+    const float4 t = __ldg(reinterpret_cast<const float4 *>(p.idx) + k);
+    q = make_int2(__float_as_int(t.x), __float_as_int(t.y));
+    v = make_float2(t.z, t.w);
+  }
+}
+
 // The sub-grid of an item whose packed sums are not finite, cell by cell and
 // only from the records whose footprints cover the cell.
 template <int S, bool COMP>
@@ -118,11 +131,12 @@ __device__ __noinline__ void rt_redo(const RegTileLaunch &p, const WorkItem &w, 
       since = 0;
     };
     for (int k = w.start; k < w.end; ++k) {
-      const int2 q = __ldg(p.idx + k);
+      int2 q;
+      float2 v;
+      rt_record(p, k, plane, q, v);
       const int fy = q.y & 0xff;
       const int fx = S == 8 ? (-(q.x + fy * C::ROW - C::PAD) & 31) >> 2 : q.y >> 8;
       if ((unsigned)(x - fx) >= (unsigned)S || (unsigned)(y - fy) >= (unsigned)S) continue;
-      const float2 v = __ldg(p.vals + plane * p.vstride + k);
       const int at = (q.x + y * C::ROW) / 4 + x;
       run = fma2(pk2(v.x, v.y), pk2(tr[at], tr[at]), run);
       if (cplx) run = fma2(pk2(-v.y, v.x), pk2(ti[at], ti[at]), run);
@@ -173,10 +187,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
       const int k = k0 + u * 32 + lane;
-      if (k < end) {
-        pk[u] = __ldg(p.idx + k);
-        pv[u] = __ldg(p.vals + plane * p.vstride + k);
-      }
+      if (k < end) rt_record(p, k, plane, pk[u], pv[u]);
     }
   };
   if (item >= total) return;  // the whole warp; no barrier follows
@@ -422,6 +433,26 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
             out_red(J, (size_t)gy * N + gx, plane, p.P, dr, di);
           }
         }
+    }
+    // the last item of a cut tile rounds the merged sums into the grid
+    if (COMP && p.merge.base && tail.x >= 0) {
+      __threadfence();
+      __syncwarp();
+      int4 *const d = p.merge.desc + tail.x;
+      int done = 0;
+      if (lane == 0) done = atomicAdd(&d->w, 1) + 1;
+      if (__shfl_sync(0xffffffffu, done == d->z, 0)) {
+        __threadfence();
+        const double2 *const src = p.merge.base + (size_t)tail.x * p.merge.cells;
+        for (int i = lane; i < p.P * R * R; i += 32) {
+          const double2 v = __ldcg(src + i);
+          if (v.x == 0.0 && v.y == 0.0) continue;
+          const int plane = i / (R * R), c = i - plane * R * R;
+          const int gx = tail.y + c % R, gy = tail.z + c / R;
+          if ((unsigned)gx < (unsigned)N && (unsigned)gy < (unsigned)N)
+            out_red(J, (size_t)gy * N + gx, plane, p.P, v.x, v.y);
+        }
+      }
     }
     if (next >= total) return;
     item = next;

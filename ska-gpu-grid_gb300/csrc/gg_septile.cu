@@ -88,6 +88,19 @@ __device__ __forceinline__ void sep_store(const JobDesc &J, int gx, int gy, int 
   }
 }
 
+// sorted record k and its value in a plane
+__device__ __forceinline__ void sep_record(const SepTileLaunch &p, int k, int plane, int2 &q,
+                                           float2 &v) {
+  if (p.vals) {
+    q = __ldg(p.idx + k);
+    v = __ldg(p.vals + plane * p.vstride + k);
+  } else {
+    const float4 t = __ldg(reinterpret_cast<const float4 *>(p.idx) + k);
+    q = make_int2(__float_as_int(t.x), __float_as_int(t.y));
+    v = make_float2(t.z, t.w);
+  }
+}
+
 // main cells and sub-kernel of a sorted record (window_record)
 __device__ __forceinline__ void sep_decode(const int2 q, int log2G, int &mx, int &my, int &sx,
                                            int &sy) {
@@ -103,7 +116,6 @@ template <bool COMP>
 __device__ __noinline__ void sep_redo(const SepTileLaunch &p, const JobDesc &J, int x0, int y0,
                                       int plane, const float *gt, int tid, int nt) {
   constexpr int H = kSepS / 2;
-  const float2 *const vals = p.vals + plane * p.vstride;
   for (int c = tid; c < kSepB * kSepB; c += nt) {
     const int x = x0 + c % kSepB, y = y0 + c / kSepB;
     u64 run = 0ull, hi = 0ull, lo = 0ull;
@@ -120,11 +132,13 @@ __device__ __noinline__ void sep_redo(const SepTileLaunch &p, const JobDesc &J, 
       if (by + r >= J.ntx) break;
       const int *const bm = J.bookmarks + (by + r) * J.ntx;
       for (int k = bm[bx]; k < bm[min(bx + 6, J.ntx)]; ++k) {
+        int2 q;
+        float2 v;
+        sep_record(p, k, plane, q, v);
         int mx, my, sx, sy;
-        sep_decode(__ldg(p.idx + k), J.log2G, mx, my, sx, sy);
+        sep_decode(q, J.log2G, mx, my, sx, sy);
         const int a = x - (mx - H + 1), b = y - (my - H + 1);
         if ((unsigned)a >= (unsigned)kSepS || (unsigned)b >= (unsigned)kSepS) continue;
-        const float2 v = __ldg(vals + k);
         const float gx = gt[sx * 4 * kSepRow + 16 + a], gy = gt[sy * 4 * kSepRow + 16 + b];
         run = fma2(mul2(pk2(v.x, v.y), pk2(gx, gx)), pk2(gy, gy), run);
         if (COMP && ++since == kSepRun) merge();
@@ -220,7 +234,6 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
         }
         since = 0;
       };
-      const float2 *const vals = p.vals + plane * p.vstride;
       // the groups of 32 records of the six ranges as one stream: group g lies
       // in the last range r whose first group is at most g
       int2 q = make_int2(0, 0);
@@ -234,8 +247,7 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
                       32 * (g - __shfl_sync(0xffffffffu, first, r));
         n = min(32, __shfl_sync(0xffffffffu, end, r) - k);
         if (lane < n) {
-          q = __ldg(p.idx + k + lane);
-          v = __ldg(vals + k + lane);
+          sep_record(p, k + lane, plane, q, v);
         }
       };
       int g = SHARE ? warp : 0;

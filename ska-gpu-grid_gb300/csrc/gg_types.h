@@ -37,7 +37,8 @@ struct JobDesc {
   int64_t vstride;       // plane stride of sorted vals
   int N, S, G, log2G, P, T, log2T, ntx;
   int off;               // cells by which the uv tiles start before the grid
-  int blk0;              // output blocks of the class's jobs before this one
+  int blk0;              // output blocks (kSep), or pieces of kZeroChunk bytes
+                         // of output, of the class's jobs before this one
   int planar, out_f64, uv_f64;
   float sigma;
   // per-visibility GCF tables (1 = a single table); binned methods: the
@@ -76,7 +77,8 @@ struct __align__(16) WorkItem {
 // FP64 reduction directly).
 struct MergeSlots {
   double2 *base;  // [cap][cells], null: no slots in this class
-  int2 *desc;     // [cap]: {job, bin} of the tile owning each slot
+  int4 *desc;     // [cap]: {job, bin, items, items done} of the tile owning
+                  // each slot
   int cap;        // slots available
   int cells;      // double2 values per slot
 };
