@@ -9,10 +9,18 @@
 // is a data race and has no counterpart here.
 //
 // A CTA takes 256 consecutive visibilities: every thread loads one (u,v) as a
-// 128-bit vector, performs the FP64 index step once, and parks the packed
-// indices and values in shared memory; each warp then walks the visibilities
-// with its lanes spread over the S*S taps, so a warp's reductions hit
-// consecutive cells of a footprint row.
+// 128-bit vector, performs the FP64 index step once, and parks the footprint's
+// place, the sub-kernel and the values in shared memory; each warp then walks
+// the visibilities with its lanes spread over the S*S taps, so a warp's
+// reductions hit consecutive cells of a footprint row.
+//
+// What binds: FP32 values, the L2's reductions by 32-byte sector (1 M
+// visibilities of support 8 on 2048^2: 22 sectors each, 172 G/s of the 190 G/s
+// that coalesced reductions reach; 190 -> 134 us once a visibility cost 83
+// warp instructions instead of 156).  FP64 values, the FP64 pipe: 16
+// multiplications a visibility of support 16 and lane when the table has no
+// imaginary parts (32 operations before), one reduction per component with
+// every sector touched once (262,144 visibilities on 1024^2: 594 -> 415 us).
 //
 // Compensated mode (complex64 output): the hi grid is updated with
 // atom.global.v2.f32.add, which returns the previous value; two_sum of
@@ -35,6 +43,11 @@ __device__ __forceinline__ int find_job_v(const int64_t *base, int njobs,
   return lo;
 }
 
+// neither infinite nor NaN, without the FP64 pipe
+__device__ __forceinline__ bool finite_bits(double x) {
+  return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
+}
+
 template <int S, class ACC, int GK>
 __global__ void __launch_bounds__(kScatterThreads)
     scatter_kernel(KParams kp) {
@@ -43,7 +56,10 @@ __global__ void __launch_bounds__(kScatterThreads)
   using VT2 = typename vec2_of<VT>::type;
   constexpr int NT = kScatterThreads, H = S / 2;
   extern __shared__ __align__(16) unsigned char smem[];
-  int4 *rec = reinterpret_cast<int4 *>(smem);                   // mx, my, sx|sy<<8, job (-1 = skip)
+  // grid cell of the footprint's first tap, sub-kernel (of all tables), the
+  // tap's column and row + 64 (16 bits each), job * 2 + inside the grid (-1:
+  // skip)
+  int4 *rec = reinterpret_cast<int4 *>(smem);
   VT2 *sval = reinterpret_cast<VT2 *>(smem + NT * sizeof(int4));  // [NT][P]
   float *g1 = reinterpret_cast<float *>(smem + NT * sizeof(int4) +
                                         (size_t)NT * kp.P * sizeof(VT2));
@@ -54,6 +70,17 @@ __global__ void __launch_bounds__(kScatterThreads)
   const int P = kp.P;
   if constexpr (GAUSS) gauss_fill(g1, S, kp.G, kp.sigma, tid, NT);
   const int64_t vb0 = kp.njobs > 1 ? __ldg(kp.vis_base) : 0;
+  constexpr bool F64 = std::is_same<VT, double>::value;
+  constexpr int TAPS = (S * S + 31) / 32;    // of a lane
+  constexpr int ROWS = S < 32 ? 32 / S : 1;  // rows between them
+  const int lx = lane % S, ly = lane / S;
+  // the current job
+  int job = -1, N = 0, lane_cell = 0, step = 0;
+  bool planar = false, f64 = false, native = false;
+  size_t NN = 0;
+  char *out = nullptr;
+  float *lo = nullptr;
+  const VT2 *gcf = nullptr;
 
   for (int64_t c0 = (int64_t)blockIdx.x * NT; c0 < kp.total_vis;
        c0 += (int64_t)gridDim.x * NT) {
@@ -94,8 +121,10 @@ __global__ void __launch_bounds__(kScatterThreads)
           }
         }
         if (ok && mx + H >= 0 && mx - H + 1 < J.N && my + H >= 0 && my - H + 1 < J.N) {
-          // sx, sy < 64 (8 bits each), table index < 32768
-          r = make_int4(mx, my, sx | (sy << 8) | (tab << 16), j);
+          const int fx = mx - H + 1, fy = my - H + 1;
+          const bool inside = fx >= 0 && fy >= 0 && fx + S <= J.N && fy + S <= J.N;
+          r = make_int4(fy * J.N + fx, tab * J.G * J.G + sy * J.G + sx,
+                        (fx + 64) | ((fy + 64) << 16), 2 * j + inside);
           const VT2 *v = reinterpret_cast<const VT2 *>(J.vals) + n * P;
           for (int p = 0; p < P; ++p) sval[tid * P + p] = __ldg(v + p);
           if constexpr (WPHASE) {
@@ -118,69 +147,146 @@ __global__ void __launch_bounds__(kScatterThreads)
       rec[tid] = r;
     }
     __syncthreads();
+    // Lane l takes the taps l, l + 32, ... of a visibility: their places in
+    // the footprint are the same for all, and so are the table offsets.  The
+    // job's fields stay in registers while the job does.
     for (int q = warp; q < NT; q += NT / 32) {
       const int4 r = rec[q];
       if (r.w < 0) continue;
-      const JobDesc &J = kp.jobs[r.w];
-      const int N = J.N;
-      const size_t NN = (size_t)N * N;
-      const int sx = r.z & 0xff, sy = (r.z >> 8) & 0xff, tab = r.z >> 16;
-      GcfSrc<S, GK, VT> gsrc;
-      if constexpr (GAUSS) {
-        gsrc.g1 = g1;
-      } else if constexpr (WPHASE) {
-        gsrc.fr = sfac[q].x;
-        gsrc.fi = sfac[q].y;
-      } else {
-        gsrc.tab = reinterpret_cast<const VT2 *>(J.gcf) + (size_t)tab * J.G * J.G * S * S;
-        gsrc.G = J.G;
+      if (r.w >> 1 != job) {
+        job = r.w >> 1;
+        const JobDesc &J = kp.jobs[job];
+        N = J.N;
+        planar = J.planar;
+        f64 = J.out_f64;
+        out = static_cast<char *>(J.out);
+        gcf = reinterpret_cast<const VT2 *>(J.gcf);
+        lo = J.lo;
+        lane_cell = ly * N + lx;
+        step = ROWS * N;
+        NN = (size_t)N * N;
+        native = !planar && f64 == std::is_same<VT, double>::value &&
+                 !std::is_same<ACC, AccComp>::value;
       }
-      for (int tap = lane; tap < S * S; tap += 32) {
-        const int ap = tap % S, bp = tap / S;
-        const int gx = r.x - H + 1 + ap, gy = r.y - H + 1 + bp;
-        if ((unsigned)gx >= (unsigned)N || (unsigned)gy >= (unsigned)N) continue;
-        const size_t cell = (size_t)gy * N + gx;
-        VT gr, gi;
-        gsrc.value(sx, sy, ap, bp, gr, gi);
-        for (int p = 0; p < P; ++p) {
-          const VT2 v = sval[q * P + p];
-          VT tr, ti;
-          if constexpr (GAUSS) {
-            tr = v.x * gr;
-            ti = v.y * gr;
-          } else {
-            cmul<VT>(v.x, v.y, gr, gi, tr, ti);
-          }
-          if constexpr (std::is_same<ACC, AccComp>::value) {
-            if (J.out_f64) {
-              grid_red<double>((double *)J.out, cell, p, P, NN, J.planar, (double)tr,
-                               (double)ti);
+      const bool inside = r.w & 1;
+      const VT2 *const g0 = gcf + (int64_t)r.y * (S * S);
+      const int cell0 = r.x + lane_cell;
+      // factor of the tap at column x, row y; false: off the grid
+      auto factor_at = [&](int x, int y, auto &g) {
+        if (!inside) {
+          const int fx = (r.z & 0xffff) - 64, fy = (int)((unsigned)r.z >> 16) - 64;
+          if ((unsigned)(fx + x) >= (unsigned)N || (unsigned)(fy + y) >= (unsigned)N) return false;
+        }
+        if constexpr (GAUSS) {
+          const int sub = r.y & (kp.G * kp.G - 1), sy = sub / kp.G, sx = sub - sy * kp.G;
+          g.x = (VT)(g1[sx * S + x] * g1[sy * S + y]);
+          g.y = (VT)0;
+        } else if constexpr (WPHASE) {
+          g.x = (VT)sfac[q].x;
+          g.y = (VT)sfac[q].y;
+        } else {
+          g = __ldg(g0 + y * S + x);
+        }
+        return true;
+      };
+      // of this lane's tap k; false also: no such tap
+      auto factor = [&](int k, VT &gr, VT &gi) {
+        if (S * S % 32 != 0 && lane + 32 * k >= S * S) return false;
+        VT2 g;
+        if (!factor_at(lx, ly + k * ROWS, g)) return false;
+        gr = g.x;
+        gi = g.y;
+        return true;
+      };
+      // from a lane's first part to its part k, in doubles
+      auto part_step = [&](int k) -> int64_t {
+        if constexpr (S == 32) return 2 * ((int64_t)(k >> 1) * N + 16 * (k & 1));
+        return 2 * (int64_t)k * (S < 16 ? 16 / S : 1) * N;
+      };
+      for (int p = 0; p < P; ++p) {
+        const VT2 v = sval[q * P + p];
+        if constexpr (F64) if (native) {
+          // Complex128 grid: a lane takes one component of a tap, so that a
+          // warp's reductions cover whole sectors (a reduction of the real
+          // parts and one of the imaginary parts touched every sector twice).
+          // FP64 products bind: a tap without an imaginary part takes one per
+          // component instead of two (unless 0 * v matters), decided for the
+          // whole warp, as a choice per tap would compute both.
+          constexpr int PARTS = (S * S * 2 + 31) / 32, U = PARTS < 8 ? PARTS : 8;
+          constexpr int PROWS = S < 16 ? 16 / S : 1;  // rows between a lane's parts
+          const int px = (lane >> 1) % S, py = (lane >> 1) / S, im = lane & 1;
+          // component = a * re(g) + b * im(g)
+          const double va = im ? v.y : v.x, vb = im ? v.x : -v.y;
+          double *const cell = reinterpret_cast<double *>(out) +
+                               2 * (p * NN + (size_t)(r.x + py * N + px)) + im;
+#pragma unroll 1
+          for (int k0 = 0; k0 < PARTS; k0 += U) {
+            double2 g[U];
+            bool on[U];
+            bool full = !finite_bits(va) || !finite_bits(vb);
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+              // S = 32: two parts per row
+              const int x = S == 32 ? px + 16 * ((k0 + k) & 1) : px;
+              const int y = S == 32 ? (k0 + k) >> 1 : py + (k0 + k) * PROWS;
+              g[k] = make_double2(0.0, 0.0);
+              on[k] = factor_at(x, y, g[k]);
+              full = full || (((unsigned)__double2hiint(g[k].y) << 1) | __double2loint(g[k].y)) != 0;
+            }
+            if (__any_sync(0xffffffffu, full)) {
+#pragma unroll
+              for (int k = 0; k < U; ++k)
+                if (on[k]) red_add(cell + part_step(k0 + k), va * g[k].x + vb * g[k].y);
             } else {
-              float *hi = (float *)J.out;
-              const size_t c = (size_t)p * NN + cell;
+#pragma unroll
+              for (int k = 0; k < U; ++k)
+                if (on[k]) red_add(cell + part_step(k0 + k), va * g[k].x);
+            }
+          }
+          continue;
+        }
+        if (!F64 && native) {
+          // complex64 grid
+          float *const cell = reinterpret_cast<float *>(out) + 2 * (p * NN + (size_t)cell0);
+#pragma unroll 4
+          for (int k = 0; k < TAPS; ++k) {
+            VT gr, gi, tr, ti;
+            if (!factor(k, gr, gi)) continue;
+            cmul<VT>(v.x, v.y, gr, gi, tr, ti);
+            red_add_v2(cell + 2 * (int64_t)(k * step), (float)tr, (float)ti);
+          }
+          continue;
+        }
+#pragma unroll 2
+        for (int k = 0; k < TAPS; ++k) {
+          VT gr, gi, tr, ti;
+          if (!factor(k, gr, gi)) continue;
+          cmul<VT>(v.x, v.y, gr, gi, tr, ti);
+          const size_t c = p * NN + (size_t)(cell0 + k * step);
+          if constexpr (std::is_same<ACC, AccComp>::value) {
+            if (!f64) {
+              float *const hi = reinterpret_cast<float *>(out);
               float er, ei, s;
-              if (J.planar) {
+              if (planar) {
                 float o = atomicAdd(hi + c, (float)tr);
                 two_sum(o, (float)tr, s, er);
                 o = atomicAdd(hi + (size_t)P * NN + c, (float)ti);
                 two_sum(o, (float)ti, s, ei);
-                if (er != 0.f) red_add(J.lo + c, er);
-                if (ei != 0.f) red_add(J.lo + (size_t)P * NN + c, ei);
+                if (er != 0.f) red_add(lo + c, er);
+                if (ei != 0.f) red_add(lo + (size_t)P * NN + c, ei);
               } else {
                 float2 o = atom_add_v2(hi + 2 * c, (float)tr, (float)ti);
                 two_sum(o.x, (float)tr, s, er);
                 two_sum(o.y, (float)ti, s, ei);
-                if (er != 0.f || ei != 0.f) red_add_v2(J.lo + 2 * c, er, ei);
+                if (er != 0.f || ei != 0.f) red_add_v2(lo + 2 * c, er, ei);
               }
+              continue;
             }
-          } else {
-            if (J.out_f64)
-              grid_red<double>((double *)J.out, cell, p, P, NN, J.planar, (double)tr,
-                               (double)ti);
-            else
-              grid_red<float>((float *)J.out, cell, p, P, NN, J.planar, (double)tr,
-                              (double)ti);
           }
+          if (f64)
+            grid_red<double>((double *)out, c, 0, P, NN, planar, (double)tr, (double)ti);
+          else
+            grid_red<float>((float *)out, c, 0, P, NN, planar, (double)tr, (double)ti);
         }
       }
     }
