@@ -194,9 +194,9 @@ static int check_options(const gg_options *o) {
 // ---------------------------------------------------------------------------
 // context and plan
 // ---------------------------------------------------------------------------
-// Kernel of a class: the method's own, the register-tile or the output-block
-// form of the moving window
-enum ClassKind { kOwn = 0, kReg, kSep };
+// Kernel of a class: the method's own; the register-tile form of the moving
+// window; the output-block forms of support 32 with the Gaussian and of gather
+enum ClassKind { kOwn = 0, kReg, kSep, kGat };
 
 struct Plan {
   // resolved launch configuration
@@ -455,6 +455,27 @@ static int regtile_chunk(int64_t vis, int sm_count) {
   return (int)std::min<int64_t>(512, std::max<int64_t>(64, (c + 31) / 32 * 32));
 }
 
+// Whether the gather class of support S is summed by output block: supports 8
+// and 16 of FP32 values, binned by the library, with one GCF table for the
+// class whose copy (and the partial sums of a shared block) fit an SM's shared
+// memory.
+static bool gathertile_class(const gg_options *o, const gg_job *jobs, int njobs, int S) {
+  if ((S != 8 && S != 16) || o->input_sorted || (o->tile != 0 && o->tile != 32)) return false;
+  if (gathertile_smem_bytes(S, o->oversample) > 227 * 1024) return false;
+  const gg_job *one = nullptr;
+  int64_t blocks = 0;
+  for (int j = 0; j < njobs; ++j) {
+    if (jobs[j].gcf_dim != S) continue;
+    if (jobs[j].vals_type != GG_C64 || jobs[j].gcf_index) return false;
+    if (o->gcf_kind == GG_GCF_TABLE && one && jobs[j].gcf != one->gcf) return false;
+    one = &jobs[j];
+    if (one->img_dim < 1 || one->img_dim > 32768) return false;  // refused below
+    const int64_t b = (one->img_dim + kGatBlock - 1) / kGatBlock;
+    blocks += b * b;
+  }
+  return one != nullptr && blocks < (1ll << 30);
+}
+
 // Whether the moving-window class of support S is summed by output block:
 // support 32 with the on-the-fly Gaussian, FP32 values, binned by the library
 // at its own choice of tiles, factors of at most 16 sub-cells (20 KB).  Blocks
@@ -485,7 +506,7 @@ static bool septile_class(const gg_options *o, const gg_job *jobs, int njobs, in
 // uv tiles along one axis of a job
 static int64_t tile_side(int64_t N, int S, const ClassCfg &cf) {
   // main cells up to N + S/2 - 2 reach the grid
-  if (cf.kind == kReg) return (N + S / 2 - 2 + kRegOff) / kRegTile + 1;
+  if (cf.kind == kReg || cf.kind == kGat) return (N + S / 2 - 2 + kRegOff) / kRegTile + 1;
   if (cf.kind == kSep) return (N + S / 2 - 2 + kSepOff) / kSepTile + 1;
   return (N + cf.T - 1) / cf.T;
 }
@@ -533,7 +554,10 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
           if (e) cf = e->cfg;
         }
       }
-      if (m0 == GG_MODE_WINDOW && !bin_only) {
+      if (m0 == GG_MODE_GATHER && !bin_only && gathertile_class(opt, jobs, njobs, S)) {
+        cf.kind = kGat;
+        cf.T = kRegTile;
+      } else if (m0 == GG_MODE_WINDOW && !bin_only) {
         if (septile_class(opt, jobs, njobs, S)) {
           cf.kind = kSep;
           cf.T = kSepTile;
@@ -620,7 +644,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
         return fail(GG_ERR_ARG, "on-the-fly GCF needs one support per batch");
     }
     const int T = cfgs[(int)J.gcf_dim].T;
-    if (mode == GG_MODE_GATHER && T != 32)
+    if (mode == GG_MODE_GATHER && cfgs[(int)J.gcf_dim].kind == kOwn && T != 32)
       return fail(GG_ERR_ARG, "gather needs tile 32");
     if (mode == GG_MODE_GATHER && J.gcf_index)
       return fail(GG_ERR_ARG, "job %d: gcf_index: use the scatter or moving-window method", j);
@@ -666,7 +690,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
   pl.vstride = vis + 8;
   pl.class_cap = tiles + vis / pl.chunk + njobs + 1;
   if (binned) {
-    pl.aos = mode == GG_MODE_WINDOW && pl.P == 1 && !bin_only;
+    pl.aos = pl.P == 1 && !bin_only;
     for (const auto &kv : cfgs) pl.aos = pl.aos && kv.second.kind != kOwn;
     pl.o_kr = take(sizeof(int2) * (vis + 1));
     pl.o_cnt = take(sizeof(int) * (tiles + 8));
@@ -787,9 +811,10 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     D.log2T = ilog2(T);
     D.ntx = ntx;
     const ClassKind kind = cfgs[S].kind;
-    D.off = kind == kReg ? kRegOff : (kind == kSep ? kSepOff : 0);
-    if (kind == kSep) {
+    D.off = kind == kOwn ? 0 : (kind == kSep ? kSepOff : kRegOff);
+    if (kind == kSep || kind == kGat) {
       D.blk0 = pl.classes.back().blocks;
+      // both kinds' blocks are 16 cells wide
       pl.classes.back().blocks += (int)septile_blocks(N);
     }
     int layout = opt->layout;
@@ -820,7 +845,9 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     B.P = pl.P;
     B.uv_f64 = D.uv_f64;
     B.off = D.off;
-    B.reg = kind == kReg;
+    B.rec = kind == kReg ? kRecRegtile
+                         : (mode == GG_MODE_WINDOW || kind != kOwn) && !bin_only ? kRecWindow
+                                                                                 : kRecPacked;
     pl.hvis_base[k] = vb;
     pl.htile_base[k] = tb;
     pl.hclass[k] = (int)pl.classes.size() - 1;
@@ -944,8 +971,9 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
     zero.add(ws + pl.o_scan, kScanHead * sizeof(int));
     zero.add(ws + pl.o_bm + sizeof(int) * ((size_t)pl.total_tiles + 1), sizeof(int));
   }
-  // item counters [8, 12), item claims [12, 16), merge slots taken [16, 20)
-  if (pl.mode == GG_MODE_WINDOW) zero.add(flags + 8, 12 * sizeof(int));
+  // item counters [8, 12), item or block claims [12, 16), merge slots taken
+  // [16, 20)
+  if (binned) zero.add(flags + 8, 12 * sizeof(int));
   if (!pl.gcf_copies.empty()) zero.add(ws + pl.o_gcf_flags, sizeof(int) * pl.gcf_copies.size());
   const bool small_out = pl.zero_ranges.size() == 1 && pl.zero_ranges[0].second <= (4u << 20);
   if (small_out) zero.add(pl.zero_ranges[0].first, pl.zero_ranges[0].second);
@@ -1022,7 +1050,6 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
     plan_bin_buffers(pl, b);
     b.order = nullptr;
     b.flags = flags;
-    b.window_records = pl.mode == GG_MODE_WINDOW;
     // output-block classes take no items (the Gaussian: one class per batch)
     const bool with_items = pl.mode == GG_MODE_WINDOW && pl.classes[0].kind != kSep;
     if (with_items) {
@@ -1107,10 +1134,33 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
     if (prof) GG_CUDA(cudaEventRecord(prof->ev[2], s));
   } else if (pl.mode == GG_MODE_GATHER) {
     if (prof) GG_CUDA(cudaEventRecord(prof->ev[1], s));
-    for (const auto &cl : pl.classes) {
+    for (size_t ci = 0; ci < pl.classes.size(); ++ci) {
+      const auto &cl = pl.classes[ci];
+      if (cl.kind == kGat) {
+        GatherTileLaunch q{};
+        q.jobs = djobs + cl.j0;
+        q.njobs = cl.j1 - cl.j0;
+        q.total_blocks = cl.blocks;
+        q.next = flags + 12 + ci;
+        q.idx = (const int2 *)(ws + pl.o_sidx);
+        q.vals = pl.aos ? nullptr : (const float2 *)(ws + pl.o_svals);
+        q.vstride = pl.vstride;
+        q.gcf = (const float2 *)pl.hjobs[cl.j0].gcf;
+        q.S = cl.S;
+        q.G = pl.G;
+        q.P = pl.P;
+        q.compensated = pl.accum == GG_ACC_COMPENSATED;
+        q.accumulate = opt->accumulate;
+        q.gauss = pl.gauss;
+        q.sigma = pl.sigma;
+        q.sm_count = sm_count;
+        GG_CUDA(launch_gathertile(q, s));
+        continue;
+      }
       g.jobs = djobs + cl.j0;
       g.njobs = cl.j1 - cl.j0;
       g.S = cl.S;
+      g.tile = cl.T;
       g.tile_base = dtileb + cl.j0;
       g.total_tiles = cl.t1 - cl.t0;
       GG_CUDA(launch_gather(g, s));

@@ -211,8 +211,8 @@ __device__ __forceinline__ void bin_scatter_part(const BinBuffers &b, int64_t bl
     int mx, sx, my, sy;
     uv_index(J.uv, J.uv_f64, n, J.G, mx, sx, my, sy);
     int2 rec;
-    if (!b.window_records) rec = make_int2(mx * J.G + sx, my * J.G + sy);
-    else if (J.reg)
+    if (J.rec == kRecPacked) rec = make_int2(mx * J.G + sx, my * J.G + sy);
+    else if (J.rec == kRecRegtile)
       rec = regtile_record(mx & (kRegTile - 1), sx, my & (kRegTile - 1), sy, J.G, J.S);
     else rec = window_record(mx, sx, my, sy, J.G);
     if (b.aos) {

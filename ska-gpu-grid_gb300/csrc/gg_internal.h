@@ -29,8 +29,12 @@ struct BinJob {
   int uv_f64;
   int n_gcf;
   int off;  // cells by which the uv tiles start before the grid (0: clamped)
-  int reg;  // register-tile class: records of regtile_record
+  int rec;  // format of its sorted records, kRec*
 };
+
+// Sorted records: packed (main*G+sub) pairs (gather, gg_bin), window_record or
+// regtile_record.
+enum { kRecPacked = 0, kRecWindow = 1, kRecRegtile = 2 };
 
 struct BinBuffers {
   const BinJob *jobs;      // device [njobs]
@@ -58,10 +62,6 @@ struct BinBuffers {
   int *flags;
   int input_sorted;
   int *kept_pos;           // [total_vis+1] (input_sorted only)
-  // sorted record format: 0 = packed (main*G+sub) pairs (gather, gg_bin);
-  // 1 = moving window: {main cells (my+64)<<16 | (mx+64), sub-kernel
-  //     sy*G+sx} -- see window_record()
-  int window_records;
   // one value per visibility, complex64: {record, value} in sorted_idx
   int aos;
 };
@@ -273,6 +273,27 @@ struct SepTileLaunch {
   int sm_count;
 };
 cudaError_t launch_septile(const SepTileLaunch &g, cudaStream_t s);
+// Gather by output block (gg_gathertile.cu): FP32 values, support 8 or 16, one
+// GCF table per launch.
+struct GatherTileLaunch {
+  const JobDesc *jobs;     // the class's jobs, blk0 set
+  int njobs;
+  int total_blocks;
+  int *next;               // zeroed counter of claimed blocks
+  const int2 *idx;         // sorted records (window_record); {record, value}
+                           // pairs of 16 bytes when vals is null
+  const float2 *vals;      // sorted values, P planes of vstride
+  int64_t vstride;
+  const float2 *gcf;       // [G*G][S][S]
+  int S, G, P;
+  int compensated;
+  int accumulate;          // add each finished cell into the grid
+  int gauss;               // factors computed from sigma instead of gcf
+  float sigma;
+  int sm_count;
+};
+cudaError_t launch_gathertile(const GatherTileLaunch &g, cudaStream_t s);
+size_t gathertile_smem_bytes(int S, int G);
 inline int64_t septile_blocks(int64_t N) {
   const int64_t b = (N + kSepBlock - 1) / kSepBlock;
   return b * b;

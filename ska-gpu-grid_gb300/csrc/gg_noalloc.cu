@@ -250,6 +250,7 @@ extern "C" int gg_grid_device_noalloc(const gg_options *opt, const gg_job *job,
   B.tile_base = 0;
   B.ntiles = (int)(ntx * ntx);
   B.n_gcf = 1;
+  B.rec = kRecWindow;
   B.N = (int)N;
   B.S = (int)S;
   B.G = G;
@@ -292,7 +293,6 @@ extern "C" int gg_grid_device_noalloc(const gg_options *opt, const gg_job *job,
   b.order = nullptr;
   b.flags = flags;
   b.input_sorted = opt->input_sorted ? 1 : 0;
-  b.window_records = 1;
   b.kept_pos = b.input_sorted ? (int *)(ws + kOffKept) : nullptr;
   ZeroRanges zero{};
   zero.add(b.counts, ((size_t)(b.total_tiles + 1) * sizeof(int) + 15) & ~(size_t)15);

@@ -20,6 +20,9 @@ constexpr int kRegTile = 8, kRegOff = 8;
 // Classes summed by output block (gg_septile.cu, support 32): the same tiles,
 // starting 16 cells before the grid; block side in cells.
 constexpr int kSepTile = 8, kSepOff = 16, kSepBlock = 16;
+// Gather by output block (gg_gathertile.cu, supports 8 and 16): tiles as for the
+// register tiles; block side in cells.
+constexpr int kGatBlock = 16;
 
 // One gridding job as the kernels see it.  For the binned methods `idx` and
 // `vals` are the tile-sorted copies made by the binning pass: idx[k] is the
@@ -37,7 +40,7 @@ struct JobDesc {
   int64_t vstride;       // plane stride of sorted vals
   int N, S, G, log2G, P, T, log2T, ntx;
   int off;               // cells by which the uv tiles start before the grid
-  int blk0;              // output blocks (kSep), or pieces of kZeroChunk bytes
+  int blk0;              // output blocks (kSep, kGat), or pieces of kZeroChunk bytes
                          // of output, of the class's jobs before this one
   int planar, out_f64, uv_f64;
   float sigma;
