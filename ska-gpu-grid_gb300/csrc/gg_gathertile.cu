@@ -70,17 +70,28 @@ template <int I, int N, class F> __device__ __forceinline__ void gt_for(F &&f) {
   }
 }
 
+__device__ __noinline__ void gt_store_f64(const JobDesc &J, size_t cell, int plane, int P,
+                                          bool accumulate, const float2 h, const float2 l) {
+  const size_t NN = (size_t)J.N * J.N;
+  const double dr = (double)h.x + (double)l.x, di = (double)h.y + (double)l.y;
+  if (!accumulate)
+    grid_store<double>((double *)J.out, cell, plane, P, NN, J.planar, dr, di);
+  else if (J.out_f64)  // into the present value, rounded once
+    grid_add<double>((double *)J.out, cell, plane, P, NN, J.planar, dr, di);
+  else
+    grid_add<float>((float *)J.out, cell, plane, P, NN, J.planar, dr, di);
+}
+
 // (hi, lo) into a cell of the grid
 __device__ __forceinline__ void gt_store(const JobDesc &J, int gx, int gy, int plane, int P,
                                          bool accumulate, const float2 h, const float2 l) {
   if (gx >= J.N || gy >= J.N) return;
   const size_t cell = (size_t)gy * J.N + gx, NN = (size_t)J.N * J.N;
-  const double dr = (double)h.x + (double)l.x, di = (double)h.y + (double)l.y;
-  if (accumulate) {  // into the present value, rounded once
-    if (J.out_f64) grid_add<double>((double *)J.out, cell, plane, P, NN, J.planar, dr, di);
-    else grid_add<float>((float *)J.out, cell, plane, P, NN, J.planar, dr, di);
-  } else if (J.out_f64) {
-    grid_store<double>((double *)J.out, cell, plane, P, NN, J.planar, dr, di);
+  // FP64 sums only where the grid or its present value needs them: the FP64
+  // pipe is so narrow that adding every cell in it took half of the kernel's
+  // time (284 -> 212 us with the ranges joined into one list)
+  if (accumulate || J.out_f64) {
+    gt_store_f64(J, cell, plane, P, accumulate, h, l);
   } else {
     const float2 v = make_float2(__fadd_rn(h.x, l.x), __fadd_rn(h.y, l.y));
     if (J.planar) grid_store<float>((float *)J.out, cell, plane, P, NN, true, v.x, v.y);
@@ -188,15 +199,21 @@ __device__ __forceinline__ void gt_blocks(const GatherTileLaunch &p, unsigned ch
       beg = __ldg(bm + bx);
       end = __ldg(bm + min(bx + 4, J.ntx));
     }
-    // first: groups of the ranges before it
-    int first = (end - beg + 31) / 32, groups = first;
+    // the ranges as one list: record t of it is record t + shift[r] of the
+    // sorted ones, r the last range with start[r] <= t
+    int sum = end - beg;
 #pragma unroll
     for (int o = 1; o < 4; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, groups, o);
-      if (lane >= o) groups += y;
+      const int y = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += y;
     }
-    first = groups - first;
-    groups = __shfl_sync(0xffffffffu, groups, 3);
+    int start[4], shift[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      start[r] = __shfl_sync(0xffffffffu, sum - (end - beg), r);
+      shift[r] = __shfl_sync(0xffffffffu, beg, r) - start[r];
+    }
+    const int records = __shfl_sync(0xffffffffu, sum, 3), groups = (records + 31) / 32;
     for (int plane = 0; plane < p.P; ++plane) {
       // cell (u, k): column c + 8u, row 4h + k
       u64 run[2][4], hi[COMP ? 2 : 1][4], lo[COMP ? 2 : 1][4];
@@ -227,11 +244,12 @@ __device__ __forceinline__ void gt_blocks(const GatherTileLaunch &p, unsigned ch
       bool have = false;
       auto fetch = [&](int g) {
         have = false;
-        if (g >= groups) return;
-        const int r = __popc(__ballot_sync(0xffffffffu, lane < 4 && first <= g)) - 1;
-        const int k = __shfl_sync(0xffffffffu, beg, r) +
-                      32 * (g - __shfl_sync(0xffffffffu, first, r)) + lane;
-        have = k < __shfl_sync(0xffffffffu, end, r);
+        const int t = 32 * g + lane;
+        have = t < records;
+        int k = t + shift[0];
+#pragma unroll
+        for (int r = 1; r < 4; ++r)
+          if (t >= start[r]) k = t + shift[r];
         if (have) gt_record(p, k, plane, q, v);
       };
       for (int g = SHARE ? warp : 0; g < groups; g += SHARE ? kGtWarps : 1) {

@@ -33,8 +33,8 @@
 //
 // Bound by the FMA pipe (69 % of its cycles, 18 of 30 warp instructions a
 // visit).  Measured on 16.8 M visibilities of a uniform disk on 8192^2: the
-// moving window's shared-memory sub-grid 24.7 ms, this kernel 5.3 ms (runs of
-// 32 records 4.7 ms, with 1.3 times the error against 64 bits: not taken).
+// moving window's shared-memory sub-grid 24.7 ms, this kernel 5.1 ms (5.3 with a group of 32 cut at every range; runs of
+// 32 records another 0.6 less, with 1.3 times the error against 64 bits: not taken).
 #include <algorithm>
 
 #include "gg_kernels.cuh"
@@ -68,19 +68,34 @@ __device__ __forceinline__ float4 lds128(uint32_t a) {
   return v;
 }
 
+__device__ __noinline__ void sep_store_f64(const JobDesc &J, size_t cell, int plane, int P,
+                                           bool accumulate, const float2 h, const float2 l) {
+  const double dr = (double)h.x + (double)l.x, di = (double)h.y + (double)l.y;
+  if (accumulate)
+    out_red(J, cell, plane, P, dr, di);
+  else
+    grid_store<double>((double *)J.out, cell, plane, P, (size_t)J.N * J.N, J.planar, dr, di);
+}
+
 // (hi, lo) into a cell of the grid
 template <bool COMP>
 __device__ __forceinline__ void sep_store(const JobDesc &J, int gx, int gy, int plane, int P,
                                           bool accumulate, const float2 h, const float2 l) {
   if (gx >= J.N || gy >= J.N) return;
   const size_t cell = (size_t)gy * J.N + gx, NN = (size_t)J.N * J.N;
-  const double dr = (double)h.x + (double)l.x, di = (double)h.y + (double)l.y;
+  // FP64 sums only for a complex128 grid: the FP64 pipe is narrow
+  if (J.out_f64) {
+    sep_store_f64(J, cell, plane, P, accumulate, h, l);
+    return;
+  }
   const float fr = __fadd_rn(h.x, l.x), fi = __fadd_rn(h.y, l.y);
   if (accumulate) {
-    if (J.out_f64) out_red(J, cell, plane, P, dr, di);
-    else out_red(J, cell, plane, P, (double)fr, (double)fi);
-  } else if (J.out_f64) {
-    grid_store<double>((double *)J.out, cell, plane, P, NN, J.planar, dr, di);
+    if (J.planar) {
+      red_add((float *)J.out + plane * NN + cell, fr);
+      red_add((float *)J.out + ((size_t)P + plane) * NN + cell, fi);
+    } else {
+      red_add_v2((float *)J.out + 2 * (plane * NN + cell), fr, fi);
+    }
   } else if (J.planar) {
     grid_store<float>((float *)J.out, cell, plane, P, NN, true, fr, fi);
   } else {
@@ -204,15 +219,16 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
       beg = __ldg(bm + bx);
       end = __ldg(bm + min(bx + 6, J.ntx));
     }
-    // first: groups of the ranges before it
-    int first = (end - beg + 31) / 32, groups = first;
+    // the ranges as one list: record t of it is record t + shift[r] of the
+    // sorted ones, r the last range with start[r] <= t
+    int sum = end - beg;
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, groups, o);
-      if (lane >= o) groups += y;
+      const int y = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += y;
     }
-    first = groups - first;
-    groups = __shfl_sync(0xffffffffu, groups, 5);
+    const int start = sum - (end - beg), shift = beg - start;  // of range `lane`
+    const int records = __shfl_sync(0xffffffffu, sum, 5);
     for (int plane = 0; plane < p.P; ++plane) {
       // cell k: column 2c + (k & 1), row 4h + k / 2
       u64 run[8], hi[COMP ? 8 : 1], lo[COMP ? 8 : 1];
@@ -234,21 +250,22 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
         }
         since = 0;
       };
-      // the groups of 32 records of the six ranges as one stream: group g lies
-      // in the last range r whose first group is at most g
+      // the list in groups of 32
       int2 q = make_int2(0, 0);
       float2 v = make_float2(0.f, 0.f);
       int n = 0;
       auto fetch = [&](int g) {
-        n = 0;
-        if (g >= groups) return;
-        const int r = __popc(__ballot_sync(0xffffffffu, lane < 6 && first <= g)) - 1;
-        const int k = __shfl_sync(0xffffffffu, beg, r) +
-                      32 * (g - __shfl_sync(0xffffffffu, first, r));
-        n = min(32, __shfl_sync(0xffffffffu, end, r) - k);
-        if (lane < n) {
-          sep_record(p, k + lane, plane, q, v);
+        const int t = 32 * g + lane;
+        n = min(32, records - 32 * g);
+        if (n <= 0) return;
+        int k = t + __shfl_sync(0xffffffffu, shift, 0);
+#pragma unroll
+        for (int r = 1; r < 6; ++r) {
+          const int s0 = __shfl_sync(0xffffffffu, start, r);
+          const int sh = __shfl_sync(0xffffffffu, shift, r);
+          if (t >= s0) k = t + sh;
         }
+        if (lane < n) sep_record(p, k, plane, q, v);
       };
       int g = SHARE ? warp : 0;
       fetch(g);
