@@ -195,8 +195,8 @@ static int check_options(const gg_options *o) {
 // context and plan
 // ---------------------------------------------------------------------------
 // Kernel of a class: the method's own; the register-tile form of the moving
-// window; the output-block forms of support 32 with the Gaussian and of gather
-enum ClassKind { kOwn = 0, kReg, kSep, kGat };
+// window with one table in shared memory, or with tables in global memory; the output-block forms of support 32 with the Gaussian and of gather
+enum ClassKind { kOwn = 0, kReg, kTab, kSep, kGat };
 
 struct Plan {
   // resolved launch configuration
@@ -356,6 +356,7 @@ static int resolve_mode(const gg_options *o, int S, int vals_f64) {
 // Launch configuration of one support class of the moving window
 struct ClassCfg {
   int T = 0, W = 0, chunk = 0;
+  bool auto_chunk = false;  // by regtile_chunk
   ClassKind kind = kOwn;
 };
 using ClassCfgs = std::map<int, ClassCfg>;  // by support
@@ -427,32 +428,49 @@ static const TuneEntry *tune_lookup(const TuneKey &k) {
   return best;
 }
 
-// Whether the moving-window class of support S takes the register-tile kernel:
-// one-warp groups on 8-cell tiles (the defaults of supports 8 and 16) of FP32
-// values, binned by the library, with one GCF table for the whole class, whose
-// padded copy has to fit an SM's shared memory (oversampling up to 8).
-static bool regtile_class(const gg_options *o, const gg_job *jobs, int njobs, int S,
-                          const ClassCfg &cf) {
-  if ((S != 8 && S != 16) || cf.T != kRegTile || cf.W > 1 || o->input_sorted) return false;
-  if (regtile_smem_bytes(S, o->oversample) > 227 * 1024) return false;
+// The register-tile kernel that a moving-window class of support S takes: one-warp
+// groups on 8-cell tiles (the defaults of supports 8 and 16) of FP32 values,
+// binned by the library.  With one GCF table for the whole class, whose copy
+// fits an SM's shared memory (oversampling up to 8), it is read from there;
+// several tables (also per-visibility ones) are read from global memory.
+static ClassKind regtile_class(const gg_options *o, const gg_job *jobs, int njobs, int S,
+                               const ClassCfg &cf) {
+  if ((S != 8 && S != 16) || cf.T != kRegTile || cf.W > 1 || o->input_sorted) return kOwn;
+  const bool fits = regtile_smem_bytes(S, o->oversample) <= 227 * 1024;
+  if (!fits && o->gcf_kind != GG_GCF_TABLE) return kOwn;
+  bool several = !fits;
   const gg_job *one = nullptr;
   for (int j = 0; j < njobs; ++j) {
     if (jobs[j].gcf_dim != S) continue;
-    if (jobs[j].vals_type != GG_C64 || jobs[j].gcf_index) return false;
-    if (o->gcf_kind == GG_GCF_TABLE && one && jobs[j].gcf != one->gcf) return false;
+    if (jobs[j].vals_type != GG_C64) return kOwn;
+    several = several || jobs[j].gcf_index ||
+              (o->gcf_kind == GG_GCF_TABLE && one && jobs[j].gcf != one->gcf);
     one = &jobs[j];
   }
-  return one != nullptr;
+  return several ? kTab : kReg;
 }
 
 // Records per work item of a register-tile class when the caller leaves it
-// open: four items for every resident warp, between 64 records (a warp's item
-// is a serial chain, and small jobs leave most warps without one) and 512
-// (every item reduces its whole sub-grid once; 256 mixed jobs 5.53 ms, with
-// 256 records 5.74, with 128 6.37).
-static int regtile_chunk(int64_t vis, int sm_count) {
-  const int64_t c = vis / ((int64_t)sm_count * 16 * 4);
-  return (int)std::min<int64_t>(512, std::max<int64_t>(64, (c + 31) / 32 * 32));
+// open: four items for every resident warp, at most 512 records (256 mixed jobs
+// 5.53 ms, with 256 records 5.74, with 128 6.37).  At least 64 for support 8
+// (a warp's item is a serial chain, and small jobs leave most warps without
+// one: 10 k records on 256^2 41.2 us, with 128 42.6) and 128 for support 16
+// (every item of a cut tile adds 529 cells into its merge slot: 100 k records
+// on 777^2 72 us, with 64 97).
+constexpr int kRegChunkMax = 512, kRegItemsPerSm = 16 * 4;
+static int regtile_chunk_min(int S) { return S == 8 ? 64 : 128; }
+static int regtile_chunk(int64_t vis, int S, int sm_count) {
+  const int64_t c = vis / ((int64_t)sm_count * kRegItemsPerSm);
+  return (int)std::min<int64_t>(kRegChunkMax,
+                                std::max<int64_t>(regtile_chunk_min(S), (c + 31) / 32 * 32));
+}
+// The most full items that a class of `vis` records, or any smaller one, is
+// cut into by the rule above.  Room is taken for this many, not for those of
+// the class itself, so that a workspace reserved for a larger job holds a
+// smaller one with shorter items.
+static int64_t regtile_items_cap(int64_t vis, int S, int sm_count) {
+  const int64_t middle = (int64_t)sm_count * (kRegItemsPerSm + 1);
+  return std::min(vis / regtile_chunk_min(S), std::max(middle, vis / kRegChunkMax)) + 1;
 }
 
 // Whether the gather class of support S is summed by output block: supports 8
@@ -506,7 +524,7 @@ static bool septile_class(const gg_options *o, const gg_job *jobs, int njobs, in
 // uv tiles along one axis of a job
 static int64_t tile_side(int64_t N, int S, const ClassCfg &cf) {
   // main cells up to N + S/2 - 2 reach the grid
-  if (cf.kind == kReg || cf.kind == kGat) return (N + S / 2 - 2 + kRegOff) / kRegTile + 1;
+  if (cf.kind == kReg || cf.kind == kTab || cf.kind == kGat) return (N + S / 2 - 2 + kRegOff) / kRegTile + 1;
   if (cf.kind == kSep) return (N + S / 2 - 2 + kSepOff) / kSepTile + 1;
   return (N + cf.T - 1) / cf.T;
 }
@@ -562,15 +580,16 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
           cf.kind = kSep;
           cf.T = kSepTile;
           cf.chunk = 2048;  // no work items
-        } else if (regtile_class(opt, jobs, njobs, S, cf)) {
-          cf.kind = kReg;
+        } else {
+          cf.kind = regtile_class(opt, jobs, njobs, S, cf);
         }
       }
-      if (cf.kind == kReg && cf.chunk == 0) {
+      if ((cf.kind == kReg || cf.kind == kTab) && cf.chunk == 0) {
         int64_t cvis = 0;
         for (int i = 0; i < njobs; ++i)
           if (jobs[i].gcf_dim == S) cvis += std::max<int64_t>(0, jobs[i].npts);
-        cf.chunk = regtile_chunk(cvis, c->sm_count);
+        cf.chunk = regtile_chunk(cvis, S, c->sm_count);
+        cf.auto_chunk = true;
       }
       if (cf.chunk == 0) cf.chunk = 2048;
       cfgs[S] = cf;
@@ -688,7 +707,11 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
   pl.o_class = take(sizeof(int) * njobs);
   pl.table_bytes = off;
   pl.vstride = vis + 8;
-  pl.class_cap = tiles + vis / pl.chunk + njobs + 1;
+  int64_t full_items = vis / pl.chunk;
+  for (const auto &kv : cfgs)
+    if (kv.second.auto_chunk)
+      full_items = std::max(full_items, regtile_items_cap(vis, kv.first, c->sm_count));
+  pl.class_cap = tiles + full_items + njobs + 1;
   if (binned) {
     pl.aos = pl.P == 1 && !bin_only;
     for (const auto &kv : cfgs) pl.aos = pl.aos && kv.second.kind != kOwn;
@@ -759,7 +782,10 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
         }
       if (c64 && kv.second.kind != kSep && ci < kMaxClasses) {
         const int R = kv.second.T + S - 1;
-        pl.merge_cap[ci] = merge_slot_cap(cvis, kv.second.chunk, ctiles);
+        pl.merge_cap[ci] =
+            kv.second.auto_chunk
+                ? (int)std::min(ctiles, regtile_items_cap(cvis, S, c->sm_count))
+                : merge_slot_cap(cvis, kv.second.chunk, ctiles);
         pl.merge_cells[ci] = pl.P * R * R;
         pl.o_merge[ci] = take(sizeof(double2) * (size_t)pl.merge_cap[ci] * pl.merge_cells[ci]);
         pl.o_mdesc[ci] = take(sizeof(int4) * (size_t)pl.merge_cap[ci]);
@@ -845,9 +871,10 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     B.P = pl.P;
     B.uv_f64 = D.uv_f64;
     B.off = D.off;
-    B.rec = kind == kReg ? kRecRegtile
-                         : (mode == GG_MODE_WINDOW || kind != kOwn) && !bin_only ? kRecWindow
-                                                                                 : kRecPacked;
+    B.rec = kind == kReg   ? kRecRegtile
+            : kind == kTab ? kRecTables
+            : (mode == GG_MODE_WINDOW || kind != kOwn) && !bin_only ? kRecWindow
+                                                                    : kRecPacked;
     pl.hvis_base[k] = vb;
     pl.htile_base[k] = tb;
     pl.hclass[k] = (int)pl.classes.size() - 1;
@@ -1105,8 +1132,9 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
         q.sigma = pl.sigma;
         q.sm_count = sm_count;
         GG_CUDA(launch_septile(q, s));
-      } else if (cl.kind == kReg) {
+      } else if (cl.kind == kReg || cl.kind == kTab) {
         RegTileLaunch r{};
+        r.tables = cl.kind == kTab;
         r.jobs = djobs;
         r.items = g.items;
         r.nitems = g.nitems;
@@ -1271,7 +1299,7 @@ static int autotune_batch(gg_context *c, const gg_options *opt, const gg_job *jo
     ClassCfg base;
     base.T = S <= 16 && !opt->input_sorted ? 8 : 32;
     base.W = 0;
-    base.chunk = 2048;
+    base.chunk = 0;  // the default of the kernel it goes to
     const double t_default = timeit(base);
     if (t_default >= 1e30) {
       st = fail(GG_ERR_CUDA, "autotune: the default configuration failed for support %d", S);
@@ -1461,10 +1489,21 @@ int gg_reserve(gg_context *ctx, const gg_options *opt, int64_t max_npts,
   Plan pl;
   int st = plan_build(ctx, opt, &j, 1, pl);
   if (st) return st;
+  size_t ws = pl.ws_bytes, tables = pl.table_bytes;
+  // smaller supports can take another kernel with more workspace
+  for (const int S : {4, 8, 16}) {
+    if (S >= max_gcf_dim) break;
+    Plan small;
+    j.gcf_dim = S;
+    if (plan_build(ctx, opt, &j, 1, small)) continue;
+    ws = std::max(ws, small.ws_bytes);
+    tables = std::max(tables, small.table_bytes);
+  }
+  g_last_error.clear();
   GG_CUDA(cudaEventSynchronize(ctx->exec_done));
-  st = ctx->ws.ensure(pl.ws_bytes);
+  st = ctx->ws.ensure(ws);
   if (st) return st;
-  return ctx->staging.ensure(pl.table_bytes + 4096);
+  return ctx->staging.ensure(tables + 4096);
 }
 
 int gg_workspace_bytes(gg_context *ctx, size_t *bytes) {

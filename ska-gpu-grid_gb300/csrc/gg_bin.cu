@@ -214,6 +214,8 @@ __device__ __forceinline__ void bin_scatter_part(const BinBuffers &b, int64_t bl
     if (J.rec == kRecPacked) rec = make_int2(mx * J.G + sx, my * J.G + sy);
     else if (J.rec == kRecRegtile)
       rec = regtile_record(mx & (kRegTile - 1), sx, my & (kRegTile - 1), sy, J.G, J.S);
+    else if (J.rec == kRecTables)
+      rec = regtile_table_record(mx & (kRegTile - 1), sx, my & (kRegTile - 1), sy, J.G, J.S);
     else rec = window_record(mx, sx, my, sy, J.G);
     if (b.aos) {
       reinterpret_cast<float4 *>(b.sorted_idx)[pos] =

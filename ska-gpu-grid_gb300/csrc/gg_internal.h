@@ -32,9 +32,9 @@ struct BinJob {
   int rec;  // format of its sorted records, kRec*
 };
 
-// Sorted records: packed (main*G+sub) pairs (gather, gg_bin), window_record or
-// regtile_record.
-enum { kRecPacked = 0, kRecWindow = 1, kRecRegtile = 2 };
+// Sorted records: packed (main*G+sub) pairs (gather, gg_bin), window_record,
+// regtile_record or regtile_table_record.
+enum { kRecPacked = 0, kRecWindow = 1, kRecRegtile = 2, kRecTables = 3 };
 
 struct BinBuffers {
   const BinJob *jobs;      // device [njobs]
@@ -86,6 +86,11 @@ __host__ __device__ inline int2 regtile_record(int fx, int sx, int fy, int sy, i
   const int row = regtile_row(S);
   return make_int2((sy * G + sx) * S * row + regtile_pad(S) - 4 * fx - row * fy,
                    S == 8 ? fy : fy | fx << 8);
+}
+
+// The same for tables in global memory ([G*G][S][S] complex entries).
+__host__ __device__ inline int2 regtile_table_record(int fx, int sx, int fy, int sy, int G, int S) {
+  return make_int2((((sy * G + sx) * S - fy) * S - fx) * 8, fy | fx << 8);
 }
 
 // index step only (vis2ints)
@@ -234,8 +239,9 @@ cudaError_t launch_degrid(const DegridLaunch &d, cudaStream_t s);
 int image_inverse_fft(void *grid, int64_t N, int P, bool f64, int sm_count, cudaStream_t s,
                       std::string &err);
 
-// Register-tile moving window (gg_regtile.cu): FP32 values, support 8 or 16,
-// one GCF table per launch (its padded copy fills the CTA's shared memory).
+// Register-tile moving window (gg_regtile.cu): FP32 values, support 8 or 16;
+// one GCF table per launch (its copy fills the CTA's shared memory), or any
+// number of them in global memory.
 struct RegTileLaunch {
   const JobDesc *jobs;
   const WorkItem *items;
@@ -245,6 +251,7 @@ struct RegTileLaunch {
                            // pairs of 16 bytes when vals is null
   const float2 *vals;      // sorted values, P planes of vstride
   int64_t vstride;
+  int tables;              // tables read per item from the jobs' (gcf ignored)
   const float2 *gcf;       // [G*G][S][S]
   int S, G, P;
   int compensated;

@@ -37,15 +37,23 @@
 //    without imaginary parts never touches the second half.
 //
 // The whole table lives in each CTA's shared memory (2 x 98 KB for support 16
-// at oversampling 8), hence one CTA per SM and one table per launch.
+// at oversampling 8), hence one CTA per SM and one table per launch.  Several
+// tables, or one that does not fit, are read from global memory by
+// regtile_tables_kernel, complex entries as the caller keeps them.  There the
+// planes of an item are units of their own, next to each other, so that the
+// warps of a CTA read the same sub-kernels at about the same time.  Bound by
+// those reads (2 KB a record and plane for support 16, 42 % of them found in
+// L1): 524 k records of 4 planes and 32 tables of support 16 on 2048^2
+// 880 us for the whole call with window_kernel, 808 now.
 //
 // Bound by instruction issue (60-63 % of active cycles issue; 42 and 87 warp
 // instructions a record for supports 8 and 16 on the batched tracks, about
 // half of them sorting, TwoSum and flushes of small tiles).  Measured against
 // window_kernel on the same jobs: 4.19 M support-8 records of a 4096^2
 // observation 435 -> 253 us; 256 mixed jobs, 24.4 M support-8 records 1366 ->
-// 1337 us, 20.9 M support-16 records 3189 -> 2228 us; 100 k support-16 records
-// on 777^2 74 -> 47 us; 10 k support-8 records on 256^2 36 -> 13 us.
+// 1337 us, 20.9 M support-16 records 3189 -> 2228 us; 10 k support-8 records
+// on 256^2 36 -> 13 us; 100 k support-16 records on 777^2, whole call, 135 ->
+// 73 us.
 #include <algorithm>
 
 #include "gg_kernels.cuh"
@@ -61,18 +69,20 @@ constexpr int kRtBlock = 128;
 // are read ahead
 constexpr int kRtStage = kRtBlock + 8 + 2;
 
-template <int S> struct RtCfg {
-  static constexpr int LX = S == 8 ? 4 : 8, LY = 32 / LX;
+// GT: tables read from global memory (complex entries as the caller has them)
+template <int S, bool GT> struct RtCfg {
+  static constexpr int LX = S == 8 && !GT ? 4 : 8, LY = 32 / LX;
   static constexpr int NX = (S + 8) / LX, NY = (S + 8) / LY, R = S + kRegTile - 1;
   static constexpr int Q = S / LY;      // rows of a footprint per lane
   static constexpr int PAIRS = 8 / LY;  // rows j < PAIRS alternate with j + Q
-  // columns behind zeros (every column loaded), or shared loads of the
-  // outer columns (support 16: NX = 3, the first and last complementary)
-  static constexpr bool PADX = S == 8;
-  static constexpr int NL = PADX ? NX : 2;  // loads per row
+  // columns behind zeros (every column loaded), or a shared load of the first
+  // and last column, which are complementary
+  static constexpr bool PADX = S == 8 && !GT;
+  static constexpr int NL = PADX ? NX : NX - 1;  // loads per row
   static constexpr int WARPS = S == 8 ? 16 : 12;
-  static constexpr int ROW = regtile_row(S);  // bytes of a table row
-  static constexpr int PAD = regtile_pad(S);  // bytes before its first tap
+  static constexpr int ENTRY = GT ? 8 : 4;    // bytes of a table entry
+  static constexpr int ROW = GT ? 8 * S : regtile_row(S);  // of a table row
+  static constexpr int PAD = GT ? 0 : regtile_pad(S);      // before its first tap
   static constexpr int SUB = S * ROW;
 };
 
@@ -108,15 +118,22 @@ __device__ __forceinline__ void rt_record(const RegTileLaunch &p, int k, int pla
   }
 }
 
+// the table of a bin (uv tile * n_gcf + table)
+template <int S> __device__ __forceinline__ const float2 *rt_table(const JobDesc &J, int bin) {
+  return reinterpret_cast<const float2 *>(J.gcf) +
+         (size_t)(J.n_gcf > 1 ? bin % J.n_gcf : 0) * J.G * J.G * S * S;
+}
+
 // The sub-grid of an item whose packed sums are not finite, cell by cell and
 // only from the records whose footprints cover the cell.
-template <int S, bool COMP>
+template <int S, bool COMP, bool GT>
 __device__ __noinline__ void rt_redo(const RegTileLaunch &p, const WorkItem &w, int plane,
                                      const float *tr, bool cplx, double2 *slot) {
-  using C = RtCfg<S>;
+  using C = RtCfg<S, GT>;
   constexpr int R = C::R;
   const JobDesc &J = p.jobs[w.job];
   const float *const ti = tr + rt_table_floats(S, p.G);
+  const float2 *const gt = rt_table<S>(J, w.bin);
   for (int c = threadIdx.x & 31; c < R * R; c += 32) {
     const int x = c % R, y = c / R;
     const int gx = w.ox + x, gy = w.oy + y;
@@ -135,11 +152,14 @@ __device__ __noinline__ void rt_redo(const RegTileLaunch &p, const WorkItem &w, 
       float2 v;
       rt_record(p, k, plane, q, v);
       const int fy = q.y & 0xff;
-      const int fx = S == 8 ? (-(q.x + fy * C::ROW - C::PAD) & 31) >> 2 : q.y >> 8;
+      const int fx = C::PADX ? (-(q.x + fy * C::ROW - C::PAD) & 31) >> 2 : q.y >> 8;
       if ((unsigned)(x - fx) >= (unsigned)S || (unsigned)(y - fy) >= (unsigned)S) continue;
-      const int at = (q.x + y * C::ROW) / 4 + x;
-      run = fma2(pk2(v.x, v.y), pk2(tr[at], tr[at]), run);
-      if (cplx) run = fma2(pk2(-v.y, v.x), pk2(ti[at], ti[at]), run);
+      const int at = (q.x + y * C::ROW) / C::ENTRY + x;
+      float2 g;
+      if constexpr (GT) g = __ldg(gt + at);
+      else g = make_float2(tr[at], cplx ? ti[at] : 0.f);
+      run = fma2(pk2(v.x, v.y), pk2(g.x, g.x), run);
+      if (cplx) run = fma2(pk2(-v.y, v.x), pk2(g.y, g.y), run);
       if (COMP && ++since == kRtRun) merge();
     }
     if (COMP) merge();
@@ -157,28 +177,30 @@ __device__ __noinline__ void rt_redo(const RegTileLaunch &p, const WorkItem &w, 
   }
 }
 
-// A warp's share of the launch's items.
-template <int S, bool COMP>
+// A warp's share of the launch's units: one plane of an item each, the planes
+// of an item next to each other (they read the same records and table rows).
+template <int S, bool COMP, bool GT>
 __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr, float4 *stage,
                                          bool cplx) {
-  using C = RtCfg<S>;
+  using C = RtCfg<S, GT>;
   constexpr int LX = C::LX, LY = C::LY, NX = C::NX, NY = C::NY, R = C::R, Q = C::Q,
                 PAIRS = C::PAIRS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lx = lane % LX, ly = lane / LX;
   const uint32_t tab = smem_addr(tr) + lx * 4 + ly * C::ROW;
   const uint32_t im_off = 4u * rt_table_floats(S, p.G);
-  const int total = *p.nitems;
+  const int P = p.P, total = *p.nitems * P;
   const int first = gridDim.x * C::WARPS;
 
-  // The first items are spread over the SMs; later ones are claimed ahead:
-  // while an item is summed, the range of the next is in registers and its
-  // first records, the range of the one after and a further claim are on
-  // their way.
-  int item = blockIdx.x + warp * gridDim.x;
+  // The first units are spread over the SMs (the planes of an item stay
+  // together); later ones are claimed ahead: while a unit is summed, the range
+  // of the next is in registers and its first records, the range of the one
+  // after and a further claim are on their way.
+  int unit = P == 1 ? blockIdx.x + warp * gridDim.x : blockIdx.x * C::WARPS + warp;
   auto claim_one = [&]() { return lane == 0 ? atomicAdd(p.item_next, 1) + first : 0; };
   auto range = [&](int it) {
-    return it < total ? __ldg(reinterpret_cast<const int4 *>(p.items + it)) : make_int4(0, 0, 0, 0);
+    return it < total ? __ldg(reinterpret_cast<const int4 *>(p.items + (P == 1 ? it : it / P)))
+                      : make_int4(0, 0, 0, 0);
   };
   constexpr int PER = kRtBlock / 32;
   int2 pk[PER];
@@ -190,10 +212,10 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
       if (k < end) rt_record(p, k, plane, pk[u], pv[u]);
     }
   };
-  if (item >= total) return;  // the whole warp; no barrier follows
+  if (unit >= total) return;  // the whole warp; no barrier follows
   int claim = claim_one();
-  int4 cur = range(item);  // {job, bin, start, end}
-  fetch(cur.z, cur.w, 0);
+  int4 cur = range(unit);  // {job, bin, start, end}
+  fetch(cur.z, cur.w, P == 1 ? 0 : unit % P);
   int next = __shfl_sync(0xffffffffu, claim, 0);
   claim = claim_one();
   int4 nxt = range(next);
@@ -201,12 +223,16 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
     const int next2 = __shfl_sync(0xffffffffu, claim, 0);
     claim = claim_one();
     const int4 nxt2 = range(next2);
+    const int item = P == 1 ? unit : unit / P, plane = unit - item * P;
     const int4 tail = __ldg(reinterpret_cast<const int4 *>(p.items + item) + 1);  // {slot, ox, oy}
     const JobDesc &J = p.jobs[cur.x];
     const int N = J.N;
     const bool other = J.out_f64 || J.planar;
     float2 *const out = static_cast<float2 *>(J.out);
-    for (int plane = 0; plane < p.P; ++plane) {
+    const char *gt = nullptr;  // this lane's entry under the sub-grid's first cell
+    if constexpr (GT)
+      gt = reinterpret_cast<const char *>(rt_table<S>(J, cur.y)) + lx * 8 + ly * C::ROW;
+    do {  // once; `break` ends the unit
       // cells: (hi, lo) pairs, or plain sums in hi; run: the running sums of
       // the rows that the current fy selects
       u64 run[NX][Q], hi[NX][NY], lo[COMP ? NX : 1][COMP ? NY : 1];
@@ -264,6 +290,23 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
         t.vr = q.z;
         t.vi = q.w;
         t.left = at < (lx + 1) << 8;
+        if constexpr (GT) {
+          const char *const b = gt + __float_as_int(q.x);
+          const int side = t.left ? 0 : C::ROW;
+          rt_for<0, Q>([&](auto JJ) {
+            constexpr int j = decltype(JJ)::value;
+            const char *a = b;
+            if (j < PAIRS && fy > ly + LY * j) a = b + C::SUB;
+            rt_for<0, C::NL>([&](auto II) {
+              constexpr int i = decltype(II)::value;
+              const float2 w = __ldg(reinterpret_cast<const float2 *>(
+                  (i == 0 ? a + side : a) + (j * LY * C::ROW + i * LX * 8)));
+              t.g[j][i] = w.x;
+              t.h[j][i] = w.y;
+            });
+          });
+          return;
+        }
         const uint32_t b = tab + (uint32_t)__float_as_int(q.x);
         const uint32_t side = C::PADX || t.left ? 0 : 64;
         rt_for<0, Q>([&](auto JJ) {
@@ -286,9 +329,9 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
             constexpr int j = decltype(JJ)::value;
             rt_for<0, NX>([&](auto II) {
               constexpr int i = decltype(II)::value;
-              constexpr int l = C::PADX ? i : (i == 1 ? 1 : 0);
-              run[i][j] = fma2(C::PADX || i == 1 ? v : (i == 0 ? v0 : v2),
-                               pk2(g[j][l], g[j][l]), run[i][j]);
+              constexpr bool outer = !C::PADX && (i == 0 || i == NX - 1);
+              constexpr int l = outer ? 0 : i;
+              run[i][j] = fma2(!outer ? v : (i == 0 ? v0 : v2), pk2(g[j][l], g[j][l]), run[i][j]);
             });
           });
         };
@@ -323,7 +366,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
             }
             left -= m;
             since += m;
-        merge_pairs(f);
+            merge_pairs(f);
             if (PAIRS < Q && since >= kRtRun) {
               merge_rest();
               since = 0;
@@ -369,10 +412,9 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
             at += 1ull << sh;
           }
         if (k0 + kRtBlock < cur.w) fetch(k0 + kRtBlock, cur.w, plane);
-        else if (plane + 1 < p.P) fetch(cur.z, cur.w, plane + 1);
-        else fetch(nxt.z, nxt.w, 0);
+        else fetch(nxt.z, nxt.w, P == 1 ? 0 : next % P);
         __syncwarp();
-        if (cplx) add_block(even, std::true_type{});
+        if (GT || cplx) add_block(even, std::true_type{});
         else add_block(even, std::false_type{});
       }
       const int ox = tail.y, oy = tail.z;
@@ -386,8 +428,8 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
         for (int j = 0; j < NY; ++j) z = fma2(hi[i][j], 0ull, z);
       const float2 zf = upk2(z);
       if (__any_sync(0xffffffffu, !(zf.x == 0.f && zf.y == 0.f))) {
-        rt_redo<S, COMP>(p, p.items[item], plane, tr, cplx, slot);
-        continue;
+        rt_redo<S, COMP, GT>(p, p.items[item], plane, tr, GT || cplx, slot);
+        break;
       }
       if (!slot && !other) {
         // complex64 interleaved grid: hi + lo rounded once
@@ -408,7 +450,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
               red_add_v2(reinterpret_cast<float *>(row + LX * i), v.x, v.y);
           }
         }
-        continue;
+        break;
       }
 #pragma unroll
       for (int j = 0; j < NY; ++j)
@@ -433,17 +475,18 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
             out_red(J, (size_t)gy * N + gx, plane, p.P, dr, di);
           }
         }
-    }
-    // the last item of a cut tile rounds the merged sums into the grid
+    } while (false);
+    // the last unit of a cut tile rounds the merged sums into the grid
     if (COMP && p.merge.base && tail.x >= 0) {
       __threadfence();
       __syncwarp();
       int4 *const d = p.merge.desc + tail.x;
       int done = 0;
       if (lane == 0) done = atomicAdd(&d->w, 1) + 1;
-      if (__shfl_sync(0xffffffffu, done == d->z, 0)) {
+      if (__shfl_sync(0xffffffffu, done == d->z * P, 0)) {
         __threadfence();
         const double2 *const src = p.merge.base + (size_t)tail.x * p.merge.cells;
+#pragma unroll 4
         for (int i = lane; i < p.P * R * R; i += 32) {
           const double2 v = __ldcg(src + i);
           if (v.x == 0.0 && v.y == 0.0) continue;
@@ -455,17 +498,26 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
       }
     }
     if (next >= total) return;
-    item = next;
+    unit = next;
     cur = nxt;
     next = next2;
     nxt = nxt2;
   }
 }
 
+// tables read from global memory: any number of them, complex or not
 template <int S, bool COMP>
-__global__ void __launch_bounds__(32 * RtCfg<S>::WARPS, 1)
+__global__ void __launch_bounds__(32 * RtCfg<S, true>::WARPS, 1)
+    regtile_tables_kernel(const __grid_constant__ RegTileLaunch p) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  rt_items<S, COMP, true>(p, nullptr,
+                          reinterpret_cast<float4 *>(smem) + (threadIdx.x >> 5) * kRtStage, true);
+}
+
+template <int S, bool COMP>
+__global__ void __launch_bounds__(32 * RtCfg<S, false>::WARPS, 1)
     regtile_kernel(const __grid_constant__ RegTileLaunch p) {
-  using C = RtCfg<S>;
+  using C = RtCfg<S, false>;
   constexpr int NT = 32 * C::WARPS, RF = C::ROW / 4, PF = C::PAD / 4;
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x;
@@ -500,17 +552,19 @@ __global__ void __launch_bounds__(32 * RtCfg<S>::WARPS, 1)
       imag |= v.y != 0.f;
     }
   }
-  rt_items<S, COMP>(p, tr, stage, __syncthreads_or(imag));
+  rt_items<S, COMP, false>(p, tr, stage, __syncthreads_or(imag));
 }
 
 template <int S, bool COMP> cudaError_t rt_launch(const RegTileLaunch &g, cudaStream_t s) {
-  using C = RtCfg<S>;
-  const size_t smem = regtile_smem_bytes(S, g.G);
-  auto kern = regtile_kernel<S, COMP>;
+  using C = RtCfg<S, false>;
+  static_assert(C::WARPS == RtCfg<S, true>::WARPS, "one launch shape");
+  const size_t smem =
+      g.tables ? C::WARPS * kRtStage * sizeof(float4) : regtile_smem_bytes(S, g.G);
+  auto kern = g.tables ? regtile_tables_kernel<S, COMP> : regtile_kernel<S, COMP>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
-  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(g.sm_count, g.max_items));
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(g.sm_count, g.max_items * g.P));
   kern<<<(unsigned)blocks, 32 * C::WARPS, smem, s>>>(g);
   count_launch();
   return cudaGetLastError();
@@ -519,7 +573,7 @@ template <int S, bool COMP> cudaError_t rt_launch(const RegTileLaunch &g, cudaSt
 }  // namespace
 
 size_t regtile_smem_bytes(int S, int G) {
-  const int warps = S == 8 ? RtCfg<8>::WARPS : RtCfg<16>::WARPS;
+  const int warps = S == 8 ? RtCfg<8, false>::WARPS : RtCfg<16, false>::WARPS;
   return 8 * (size_t)rt_table_floats(S, G) + (size_t)warps * kRtStage * sizeof(float4);
 }
 

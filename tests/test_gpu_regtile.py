@@ -96,6 +96,75 @@ def test_edges_layouts_and_items(ctx, N, G, P, layout, out, S, chunk):
     check(grid(ctx, o, uv, vals, gcf, N, S, out), uv, vals, gcf, N, S, P, G, True)
 
 
+@pytest.mark.parametrize("kind", ["real", "complex"])
+@pytest.mark.parametrize("S,G,P,ntab,n", [(8, 8, 1, 3, 4000), (16, 8, 2, 5, 3000),
+                                          (16, 16, 1, 1, 900), (8, 16, 3, 2, 2000)])
+def test_tables_in_global_memory(ctx, S, G, P, ntab, n, kind):
+    """per-visibility tables, one too large for shared memory, and (below) a
+    table for each job of a batch"""
+    N, rng = 90, np.random.default_rng(S + G)
+    uv = synth.fr(rng.uniform(-S, N + S, size=(n, 2)))
+    vals = synth.normal_vals(rng, n * P)
+    tabs = np.concatenate([table(S, G, kind, rng) * np.float32(1 + t) for t in range(ntab)])
+    idx = rng.integers(0, ntab, n).astype(np.int32)
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (uv, vals, tabs.reshape(-1), idx)]
+    out = torch.full((P * N * N,), float("nan"), dtype=torch.complex64, device="cuda")
+    o = gg.Options(mode=gg.MODE_WINDOW, accum=gg.ACC_COMPENSATED, layout=gg.LAYOUT_INTERLEAVED,
+                   oversample=G, polarizations=P)
+    ctx.grid_job(o, gg.Context.make_job(out, d[0], d[1], d[2], N, S,
+                                        gcf_index=d[3] if ntab > 1 else None, n_gcf=ntab))
+    torch.cuda.synchronize()
+    assert ctx.read_flags() == [0, 0, 0, 0]
+    got = planar_from_grid(torch.view_as_real(out).reshape(-1).cpu().numpy(), P, N, False)
+    for p in range(P):
+        v = vals.reshape(n, P)[:, p].copy()
+        ref = O.grid_pz_gcfinx(uv, v, idx, tabs.reshape(-1), N, S, gcf_grid=G, nthreads=8)
+        mag = O.grid_mag(uv, pairs(v), pairs(tabs), N, S, gcf_grid=G, gcfinx=idx, nthreads=8)
+        assert rel_err(got[:, p:p + 1], ref) <= 1e-6
+        assert cell_err(got[:, p:p + 1], ref, mag)[0] <= 1e-6
+
+
+def test_a_table_for_each_job(ctx):
+    S, n, rng = 16, 2500, np.random.default_rng(2)
+    o = gg.Options(mode=gg.MODE_WINDOW, accum=gg.ACC_COMPENSATED, layout=gg.LAYOUT_INTERLEAVED)
+    sets, jobs = [], []
+    for N in (40, 77, 120):
+        uv = synth.fr(rng.uniform(0, N, size=(n, 2)))
+        vals, gcf = synth.normal_vals(rng, n), table(S, 8, "complex", rng)
+        d = [torch.from_numpy(a).cuda() for a in (uv, vals, gcf.reshape(-1))]
+        g = torch.full((N * N,), float("nan"), dtype=torch.complex64, device="cuda")
+        sets.append((uv, vals, gcf, N, d, g))
+        jobs.append(gg.Context.make_job(g, *d, N, S))
+    ctx.grid_batch(o, jobs)
+    torch.cuda.synchronize()
+    for uv, vals, gcf, N, d, g in sets:
+        host = torch.view_as_real(g).reshape(-1).cpu().numpy()
+        check(planar_from_grid(host, 1, N, False), uv, vals, gcf, N, S, 1, 8, True)
+
+
+@pytest.mark.parametrize("kind", [gg.GCF_TABLE, gg.GCF_GAUSSIAN])
+def test_reserved_workspace_holds_smaller_jobs(kind):
+    """items get shorter with the job, so a smaller job has more of them for
+    its records: none of these may outgrow the workspace reserved for the largest"""
+    N, nmax = 2048, 3_000_000
+    o = gg.Options(mode=gg.MODE_WINDOW, accum=gg.ACC_COMPENSATED, gcf_kind=kind,
+                   layout=gg.LAYOUT_INTERLEAVED)
+    uv = torch.zeros(2 * nmax, dtype=torch.float32, device="cuda")   # inside: tile 0 only
+    vals = torch.zeros(nmax, dtype=torch.complex64, device="cuda")
+    gcf = torch.zeros(64 * 256, dtype=torch.complex64, device="cuda")
+    out = torch.empty(N * N, dtype=torch.complex64, device="cuda")
+    with gg.Context(0) as c:
+        c.reserve(o, nmax, N, 32 if kind == gg.GCF_GAUSSIAN else 16)
+        held = c.workspace_bytes()
+        for S in (16, 8, 4):
+            for n in (nmax, 2_000_000, 1_245_185, 700_001, 622_593, 400_000, 50_000, 777, 1):
+                kw = {"gcf_sigma": S / 6.0} if kind == gg.GCF_GAUSSIAN else {}
+                c.grid_job(o, gg.Context.make_job(out, uv[:2 * n], vals[:n],
+                                                  None if kw else gcf, N, S, **kw))
+                assert c.workspace_bytes() == held, (S, n)
+        torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("S", [8, 16])
 def test_gaussian(ctx, S):
     N, rng = 200, np.random.default_rng(S)
