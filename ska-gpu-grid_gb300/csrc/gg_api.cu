@@ -486,6 +486,8 @@ static bool gathertile_class(const gg_options *o, const gg_job *jobs, int njobs,
     if (jobs[j].gcf_dim != S) continue;
     if (jobs[j].vals_type != GG_C64 || jobs[j].gcf_index) return false;
     if (o->gcf_kind == GG_GCF_TABLE && one && jobs[j].gcf != one->gcf) return false;
+    // interleaved complex64 cells are stored whole, gather_kernel's by halves
+    if (o->layout == GG_LAYOUT_INTERLEAVED && (uintptr_t)jobs[j].out % 8) return false;
     one = &jobs[j];
     if (one->img_dim < 1 || one->img_dim > 32768) return false;  // refused below
     const int64_t b = (one->img_dim + kGatBlock - 1) / kGatBlock;

@@ -100,6 +100,20 @@ def test_dense_tile_empty_blocks_and_gaussian(ctx, N):
     check(d[3], o, uv, vals, synth.gcf_table(synth.gaussian_gcf_1d(S)), N, S)
 
 
+@pytest.mark.parametrize("layout", [gg.LAYOUT_INTERLEAVED, gg.LAYOUT_PLANAR])
+def test_grid_aligned_to_one_float(ctx, layout):
+    N, n, S, rng = 60, 3000, 8, np.random.default_rng(12)
+    uv, vals = synth.fr(rng.uniform(0, N, size=(n, 2))), synth.normal_vals(rng, n)
+    gcf, o = table(S, 8, "complex", rng), opts(layout=layout)
+    d_uv, d_vals, d_gcf, g = device(uv, vals, gcf, N * N + 1)
+    job = gg.Context.make_job(g, d_uv, d_vals, d_gcf, N, S)
+    job.out += 4
+    ctx.grid_job(o, job)
+    torch.cuda.synchronize()
+    cells = torch.view_as_real(g).reshape(-1)[1:-1].clone()
+    check(torch.view_as_complex(cells.reshape(-1, 2)), o, uv, vals, gcf, N, S)
+
+
 def test_accumulate_and_mixed_batch(ctx):
     """twice into the same grids; support 32 keeps the 32-cell tiles"""
     rng, n = np.random.default_rng(8), 2000
