@@ -1154,6 +1154,9 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
         r.max_items = std::min<int64_t>(pl.class_cap, cl.v1 - cl.v0);
         r.sm_count = sm_count;
         r.merge = it.slots.m[ci];
+        // its predecessor in the stream is then a kernel of this call, and the
+        // table the caller's
+        r.overlap = !side && !prof && opt->gcf_kind != GG_GCF_COUNT;
         GG_CUDA(launch_regtile(r, s));
       } else {
         GG_CUDA(launch_window(g, s));
@@ -1182,6 +1185,7 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
         q.compensated = pl.accum == GG_ACC_COMPENSATED;
         q.accumulate = opt->accumulate;
         q.gauss = pl.gauss;
+        q.overlap = !prof && opt->gcf_kind != GG_GCF_COUNT;
         q.sigma = pl.sigma;
         q.sm_count = sm_count;
         GG_CUDA(launch_gathertile(q, s));

@@ -125,6 +125,7 @@ constexpr int kBinCtas = 6;
 // the scattering pass then needs no second round of claims.
 __global__ void __launch_bounds__(256, kBinCtas)
     bin_count_kernel(const __grid_constant__ BinBuffers b) {
+  after_predecessor();
   const int lane = threadIdx.x & 31;
   const WarpSlice ws(b.total_vis);
   int jw = b.njobs == 1 || ws.w0 >= ws.w1 ? 0 : find_job64(b.vis_base, b.njobs, ws.w0);
@@ -311,6 +312,7 @@ __device__ __forceinline__ void scan_store(int *d, int64_t n, int64_t base,
 __global__ void __launch_bounds__(kScanThreads)
     scan_kernel(int *d, int64_t n, int *block_off, int *ticket) {
   __shared__ bool last;
+  after_predecessor();
   const int64_t base = blockIdx.x * (int64_t)kScanBlock + threadIdx.x * kScanPer;
   int v[kScanPer];
   scan_load(d, n, base, v);
@@ -356,9 +358,9 @@ size_t scan_tmp_ints(int64_t n) {
 // tmp: the ticket (zeroed by the caller) in its first word, block offsets from
 // kScanHead on
 static cudaError_t scan_local(int *d, int64_t n, int *tmp, cudaStream_t s) {
-  scan_kernel<<<(unsigned)cdiv(n, kScanBlock), kScanThreads, 0, s>>>(d, n, tmp + kScanHead, tmp);
   count_launch();
-  return cudaGetLastError();
+  return launch_overlapped(scan_kernel, (unsigned)cdiv(n, kScanBlock), kScanThreads, 0, s, true,
+                           d, n, tmp + kScanHead, tmp);
 }
 
 // ---- driver -----------------------------------------------------------------
@@ -472,6 +474,7 @@ __device__ __forceinline__ void bin_tiles_part(const BinBuffers &b, const ItemBu
 __global__ void __launch_bounds__(256, kBinCtas)
     bin_finish_kernel(const __grid_constant__ BinBuffers b, const __grid_constant__ ItemBuffers it,
                       int tile_blocks) {
+  after_predecessor();
   if ((int)blockIdx.x < tile_blocks) bin_tiles_part(b, it, blockIdx.x, tile_blocks);
   else bin_scatter_part(b, (int64_t)blockIdx.x - tile_blocks, (int64_t)gridDim.x - tile_blocks);
 }
@@ -479,10 +482,11 @@ __global__ void __launch_bounds__(256, kBinCtas)
 cudaError_t run_binning(const BinBuffers &b, const ItemBuffers *items, cudaStream_t s) {
   cudaError_t e;
   if (b.total_vis > 0) {
-    bin_count_kernel<<<grid_for(b.total_vis), 256, 0, s>>>(b);
     count_launch();
+    if ((e = launch_overlapped(bin_count_kernel, grid_for(b.total_vis), 256, 0, s, true, b)) !=
+        cudaSuccess)
+      return e;
   }
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if ((e = scan_local(b.counts, (int64_t)b.total_tiles + 1, b.scan_tmp, s)) != cudaSuccess)
     return e;
   if (b.input_sorted && b.total_vis > 0) {
@@ -500,9 +504,8 @@ cudaError_t run_binning(const BinBuffers &b, const ItemBuffers *items, cudaStrea
     if (it.slots.m[c].cap <= 0) it.slots.m[c].base = nullptr;
   const unsigned tiles = grid_for(cdiv((int64_t)b.total_tiles + 1, 4));
   const unsigned vis = b.total_vis > 0 ? grid_for(b.total_vis) : 0;
-  bin_finish_kernel<<<tiles + vis, 256, 0, s>>>(b, it, (int)tiles);
   count_launch();
-  return cudaGetLastError();
+  return launch_overlapped(bin_finish_kernel, tiles + vis, 256, 0, s, true, b, it, (int)tiles);
 }
 
 // ---- FP64 merge slots of tiles cut into several work items ---------------------
@@ -557,11 +560,12 @@ cudaError_t launch_inject_flags(int *flags, int bits, cudaStream_t s) {
 // transfers of other streams, and the host buffer is free once the call
 // returns.
 constexpr int kUploadChunk = 16384;  // bytes per launch (parameters: up to 32 KB)
-struct SetupParams {
+constexpr int kUploadSmall = 1024;   // a job or two: no 16 KB of parameters
+template <int BYTES> struct SetupParams {
   uint4 *dst;
   int n16;  // 16-byte words in this chunk
   ZeroRanges zero;
-  uint4 data[kUploadChunk / 16];
+  uint4 data[BYTES / 16];
 };
 
 __device__ __forceinline__ void zero_range(void *p, size_t bytes, size_t i, size_t stride) {
@@ -574,15 +578,30 @@ __device__ __forceinline__ void zero_range(void *p, size_t bytes, size_t i, size
   }
 }
 
-__global__ void __launch_bounds__(256) setup_kernel(const __grid_constant__ SetupParams p) {
+template <int BYTES>
+__global__ void __launch_bounds__(256) setup_kernel(const __grid_constant__ SetupParams<BYTES> p) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const size_t i = blockIdx.x * 256 + threadIdx.x, stride = (size_t)gridDim.x * 256;
   for (int k = (int)i; k < p.n16; k += (int)stride) p.dst[k] = p.data[k];
   for (int r = 0; r < p.zero.n; ++r) zero_range(p.zero.p[r], p.zero.bytes[r], i, stride);
 }
 // the same without a table: its launch carries no 16 KB of parameters
 __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ ZeroRanges z) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const size_t i = blockIdx.x * 256 + threadIdx.x, stride = (size_t)gridDim.x * 256;
   for (int r = 0; r < z.n; ++r) zero_range(z.p[r], z.bytes[r], i, stride);
+}
+
+template <int BYTES>
+static void upload_chunk(char *dst, const char *src, size_t n, const ZeroRanges &zero,
+                         unsigned blocks, cudaStream_t s) {
+  static thread_local SetupParams<BYTES> p;  // 16 KB: off the stack
+  p.dst = reinterpret_cast<uint4 *>(dst);
+  p.n16 = (int)(n / 16);
+  p.zero = zero;
+  memcpy(p.data, src, n);
+  setup_kernel<BYTES><<<blocks, 256, 0, s>>>(p);
+  count_launch();
 }
 
 cudaError_t launch_setup(void *dst, const void *src, size_t bytes, const ZeroRanges &zero,
@@ -599,16 +618,15 @@ cudaError_t launch_setup(void *dst, const void *src, size_t bytes, const ZeroRan
     }
     return cudaGetLastError();
   }
-  static thread_local SetupParams p;  // 16 KB: off the stack
-  for (size_t o = 0; o < bytes; o += kUploadChunk) {
-    const size_t n = std::min<size_t>(kUploadChunk, bytes - o);
-    p.dst = reinterpret_cast<uint4 *>(static_cast<char *>(dst) + o);
-    p.n16 = (int)(n / 16);
-    p.zero = o == 0 ? zero : ZeroRanges{};
-    memcpy(p.data, static_cast<const char *>(src) + o, n);
-    setup_kernel<<<o == 0 ? blocks : 1, 256, 0, s>>>(p);
-    count_launch();
+  char *const d = static_cast<char *>(dst);
+  const char *const h = static_cast<const char *>(src);
+  if (bytes <= kUploadSmall) {
+    upload_chunk<kUploadSmall>(d, h, bytes, zero, blocks, s);
+    return cudaGetLastError();
   }
+  for (size_t o = 0; o < bytes; o += kUploadChunk)
+    upload_chunk<kUploadChunk>(d + o, h + o, std::min<size_t>(kUploadChunk, bytes - o),
+                               o == 0 ? zero : ZeroRanges{}, o == 0 ? blocks : 1, s);
   return cudaGetLastError();
 }
 

@@ -287,6 +287,41 @@ __device__ __forceinline__ void grid_store(OT *out, size_t cell, int p, int P,
 }
 
 // ---------------------------------------------------------------------------
+// Launches that overlap the end of the kernel before them
+// ---------------------------------------------------------------------------
+// The small kernels of one call follow each other in a stream, and for small
+// jobs the gaps between them are a good part of the whole.  A kernel launched
+// by launch_overlapped may start while its predecessor still runs, and calls
+// after_predecessor() before it touches anything that the call has written or
+// that it writes itself; only then does it let its own successor start.  So
+// when a kernel starts, the one before its predecessor has ended: what that
+// one and the earlier ones wrote, and the caller's inputs, may be read even
+// before after_predecessor().  The first kernel of a call is launched plainly.
+// Whole calls: 10 k visibilities on 256^2 41.2 -> 32.5 us (four gaps and the
+// register tiles' table fill), 100 k on 777^2 with support 16 73 -> 65.7,
+// gather of 1.05 M on 4096^2 235 -> 227; from a millisecond on no difference.
+__device__ __forceinline__ void after_predecessor() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... P, class... A>
+cudaError_t launch_overlapped(void (*kern)(P...), unsigned blocks, unsigned threads, size_t smem,
+                              cudaStream_t s, bool overlap, const A &...args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
+// ---------------------------------------------------------------------------
 // 1-D bulk copies (TMA engine) with mbarrier completion
 // ---------------------------------------------------------------------------
 

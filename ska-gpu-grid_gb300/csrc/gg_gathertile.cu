@@ -414,6 +414,7 @@ __global__ void __launch_bounds__(32 * kGtWarps, 1)
   const int tid = threadIdx.x, n = p.G * p.G * S * S;
   float *const re = reinterpret_cast<float *>(smem);
   int imag = 0;
+  if (!p.overlap) after_predecessor();
   float *const g1 = reinterpret_cast<float *>(smem + gt_table_bytes(S, p.G));
   if (p.gauss) {
     gauss_fill(g1, S, p.G, p.sigma, tid, NT);
@@ -441,6 +442,7 @@ __global__ void __launch_bounds__(32 * kGtWarps, 1)
       re[i] = g;
     }
   }
+  if (p.overlap) after_predecessor();
   __syncthreads();
   // zeros behind the staged groups are written with each group
   if (cplx) gt_blocks<S, COMP, SHARE, true>(p, smem);
@@ -460,9 +462,8 @@ cudaError_t gt_launch(const GatherTileLaunch &g, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   const int blocks = std::min(g.sm_count, g.total_blocks);
   if (blocks < 1) return cudaSuccess;
-  kern<<<blocks, 32 * kGtWarps, smem, s>>>(g);
   count_launch();
-  return cudaGetLastError();
+  return launch_overlapped(kern, (unsigned)blocks, 32 * kGtWarps, smem, s, g.overlap, g);
 }
 
 }  // namespace

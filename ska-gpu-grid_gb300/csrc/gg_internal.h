@@ -260,6 +260,7 @@ struct RegTileLaunch {
   int64_t max_items;       // upper bound of *nitems
   int sm_count;
   MergeSlots merge;        // base null: none
+  int overlap;             // table fill while the binning ends (launch_overlapped)
 };
 cudaError_t launch_regtile(const RegTileLaunch &g, cudaStream_t s);
 // Support 32 with the on-the-fly Gaussian, FP32 values (gg_septile.cu): one
@@ -298,6 +299,7 @@ struct GatherTileLaunch {
   int gauss;               // factors computed from sigma instead of gcf
   float sigma;
   int sm_count;
+  int overlap;             // table fill while the binning ends (launch_overlapped)
 };
 cudaError_t launch_gathertile(const GatherTileLaunch &g, cudaStream_t s);
 size_t gathertile_smem_bytes(int S, int G);

@@ -510,6 +510,7 @@ template <int S, bool COMP>
 __global__ void __launch_bounds__(32 * RtCfg<S, true>::WARPS, 1)
     regtile_tables_kernel(const __grid_constant__ RegTileLaunch p) {
   extern __shared__ __align__(16) unsigned char smem[];
+  after_predecessor();
   rt_items<S, COMP, true>(p, nullptr,
                           reinterpret_cast<float4 *>(smem) + (threadIdx.x >> 5) * kRtStage, true);
 }
@@ -528,6 +529,7 @@ __global__ void __launch_bounds__(32 * RtCfg<S, false>::WARPS, 1)
   // tables: from the caller's [G*G][S][S], or the Gaussian's factors (expf as
   // everywhere; their product rounds as the on-the-fly factor does)
   int imag = 0;
+  if (!p.overlap) after_predecessor();
   if (p.gauss) {
     float *g1 = reinterpret_cast<float *>(smem + 8 * (size_t)nf);
     gauss_fill(g1, S, p.G, p.sigma, tid, NT);
@@ -552,6 +554,7 @@ __global__ void __launch_bounds__(32 * RtCfg<S, false>::WARPS, 1)
       imag |= v.y != 0.f;
     }
   }
+  if (p.overlap) after_predecessor();
   rt_items<S, COMP, false>(p, tr, stage, __syncthreads_or(imag));
 }
 
@@ -565,9 +568,8 @@ template <int S, bool COMP> cudaError_t rt_launch(const RegTileLaunch &g, cudaSt
                                        (int)smem);
   if (e != cudaSuccess) return e;
   const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(g.sm_count, g.max_items * g.P));
-  kern<<<(unsigned)blocks, 32 * C::WARPS, smem, s>>>(g);
   count_launch();
-  return cudaGetLastError();
+  return launch_overlapped(kern, (unsigned)blocks, 32 * C::WARPS, smem, s, g.overlap, g);
 }
 
 }  // namespace
