@@ -713,7 +713,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
   for (const auto &kv : cfgs)
     if (kv.second.auto_chunk)
       full_items = std::max(full_items, regtile_items_cap(vis, kv.first, c->sm_count));
-  pl.class_cap = tiles + full_items + njobs + 1;
+  pl.class_cap = std::min(tiles, vis) + full_items + njobs + 1;
   if (binned) {
     pl.aos = pl.P == 1 && !bin_only;
     for (const auto &kv : cfgs) pl.aos = pl.aos && kv.second.kind != kOwn;
@@ -727,7 +727,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     pl.o_order = 0;
     pl.o_kept = pl.input_sorted ? take(sizeof(int) * (vis + 8)) : 0;
     const bool with_items = mode == GG_MODE_WINDOW && cfgs.begin()->second.kind != kSep;
-    pl.o_items = with_items ? take(sizeof(WorkItem) * 4 * pl.class_cap) : 0;
+    pl.o_items = with_items ? take(sizeof(WorkItem) * cfgs.size() * pl.class_cap) : 0;
   }
   const bool count = opt->gcf_kind == GG_GCF_COUNT;
   pl.o_count_vals = count ? take(vbytes * pl.P * (vis + 1)) : 0;
