@@ -498,7 +498,7 @@ static bool gathertile_class(const gg_options *o, const gg_job *jobs, int njobs,
 
 // Whether the moving-window class of support S is summed by output block:
 // support 32 with the on-the-fly Gaussian, FP32 values, binned by the library
-// at its own choice of tiles, factors of at most 16 sub-cells (20 KB).  Blocks
+// at its own choice of tiles, factors of at most 16 sub-cells (8 KB).  Blocks
 // are stored, not added: jobs whose grids overlap keep the adding kernel.
 static bool septile_class(const gg_options *o, const gg_job *jobs, int njobs, int S) {
   if (S != 32 || o->gcf_kind != GG_GCF_GAUSSIAN || o->input_sorted || !tunable(o) ||

@@ -560,7 +560,7 @@ cudaError_t launch_inject_flags(int *flags, int bits, cudaStream_t s) {
 // transfers of other streams, and the host buffer is free once the call
 // returns.
 constexpr int kUploadChunk = 16384;  // bytes per launch (parameters: up to 32 KB)
-constexpr int kUploadSmall = 1024;   // a job or two: no 16 KB of parameters
+constexpr int kUploadSmall = 2048;   // a job or two: no 16 KB of parameters
 template <int BYTES> struct SetupParams {
   uint4 *dst;
   int n16;  // 16-byte words in this chunk
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(256) setup_kernel(const __grid_constant__ Setu
   for (int k = (int)i; k < p.n16; k += (int)stride) p.dst[k] = p.data[k];
   for (int r = 0; r < p.zero.n; ++r) zero_range(p.zero.p[r], p.zero.bytes[r], i, stride);
 }
-// the same without a table: its launch carries no 16 KB of parameters
+// the same without a table: its launch carries no table
 __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ ZeroRanges z) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const size_t i = blockIdx.x * 256 + threadIdx.x, stride = (size_t)gridDim.x * 256;

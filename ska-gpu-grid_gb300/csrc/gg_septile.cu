@@ -4,15 +4,17 @@
 // The factor of a tap is the product of two 1-D factors, so a record costs a
 // block two vectors instead of a 32x32 table, and a support-32 footprint
 // covers a large share of any block it touches.  Lane (c, h) of a warp holds
-// the columns 2c, 2c+1 and the rows 4h .. 4h+3 of its block.  The visibilities that
-// reach a block have their main cells in a 48x48 neighbourhood: 6x6 uv tiles
-// of 8 cells, which are 6 contiguous ranges of the sorted records.  Each of
-// them costs
+// the columns 2c, 2c+1 and the rows 2h, 2h+1, 8+2h, 9+2h of its block.  The
+// visibilities that reach a block have their main cells in a 48x48
+// neighbourhood: 6x6 uv tiles of 8 cells, which are 6 contiguous ranges of the
+// sorted records, one for each row of tiles.  Each of them costs
 //   * v * gx for two columns: one 8-byte load of column factors, padded with
 //     zeros so that columns outside the footprint get zero;
-//   * 8 packed multiply-adds by four row factors, one 16-byte load.
+//   * 8 packed multiply-adds by four row factors, two 8-byte loads.  The
+//     first range reaches only the rows 0..7 and the last only 8..15: groups
+//     of records that lie in one of them take one load and 4 multiply-adds.
 // Both loads read a copy of the padded factors shifted to the alignment of the
-// footprint (four copies).  Shared memory returns 8 bytes a lane and cycle
+// footprint (two copies).  Shared memory returns 8 bytes a lane and cycle
 // also for broadcasts, so the shape of a lane's cells decides: 2 x 4 takes 5
 // cycles for 10 packed operations, 1 x 8 took 7 for 9.
 // Nothing moves, no cell is shared, every cell is stored once: no atomics, no
@@ -31,11 +33,15 @@
 // (hi, lo) sums are added by TwoSum in shared memory.  Plain sums stay one
 // sequence of additions.
 //
-// Bound by the FMA pipe (69 % of its cycles, 18 of 30 warp instructions a
-// visit).  Measured on 16.8 M visibilities of a uniform disk on 8192^2: the
-// moving window's shared-memory sub-grid 24.7 ms, this kernel 5.1 ms (5.3 with a group of 32 cut at every range; runs of
-// 32 records another 0.6 less, with 1.3 times the error against 64 bits: not taken).
+// Bound by the FMA pipe (about 70 % of its cycles).  Measured on 16.8 M
+// visibilities of a uniform disk on 8192^2, whole call: the moving window's
+// shared-memory sub-grid 25.3 ms; this kernel 6.25 ms with all 8 multiply-adds
+// for every record, 5.52 with 4 where a range reaches half the rows, 4.95 with
+// half groups unrolled (two CTAs per SM: with three, which spill, 5.31).  Runs
+// of 32 records take another 0.6 off, with 1.3 times the error against 64
+// bits: not taken.
 #include <algorithm>
+#include <type_traits>
 
 #include "gg_kernels.cuh"
 
@@ -47,24 +53,17 @@ constexpr int kSepS = 32, kSepB = kSepBlock;  // support, block side
 constexpr int kSepWarps = 8;
 constexpr int kSepRow = 64;  // floats of a padded factor row: tap 0 at 16
 
-constexpr int kSepRun = 16;  // at least 16: a group is added in halves
+constexpr int kSepRun = 16;  // records summed plainly: half a group
 // staged records of a warp: a group of 32 and zeros for the read-ahead
 constexpr int kSepStage = 36;
 
-// shared memory: factors [G][4][64] (copy c holds the row from its entry c
+// shared memory: factors [G][2][64] (copy c holds the row from its entry c
 // on), a staging block per warp, and the partial sums of a shared block
-__host__ __device__ constexpr size_t sep_factor_floats(int G) { return (size_t)G * 4 * kSepRow; }
+__host__ __device__ constexpr size_t sep_factor_floats(int G) { return (size_t)G * 2 * kSepRow; }
 
 __device__ __forceinline__ float2 lds64(uint32_t a) {
   float2 v;
   asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ float4 lds128(uint32_t a) {
-  float4 v;
-  asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "r"(a));
   return v;
 }
 
@@ -154,7 +153,7 @@ __device__ __noinline__ void sep_redo(const SepTileLaunch &p, const JobDesc &J, 
         sep_decode(q, J.log2G, mx, my, sx, sy);
         const int a = x - (mx - H + 1), b = y - (my - H + 1);
         if ((unsigned)a >= (unsigned)kSepS || (unsigned)b >= (unsigned)kSepS) continue;
-        const float gx = gt[sx * 4 * kSepRow + 16 + a], gy = gt[sy * 4 * kSepRow + 16 + b];
+        const float gx = gt[sx * 2 * kSepRow + 16 + a], gy = gt[sy * 2 * kSepRow + 16 + b];
         run = fma2(mul2(pk2(v.x, v.y), pk2(gx, gx)), pk2(gy, gy), run);
         if (COMP && ++since == kSepRun) merge();
       }
@@ -165,33 +164,32 @@ __device__ __noinline__ void sep_redo(const SepTileLaunch &p, const JobDesc &J, 
 }
 
 template <bool COMP, bool SHARE>
-__global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
+__global__ void __launch_bounds__(32 * kSepWarps, COMP ? 2 : 4)
     septile_kernel(const __grid_constant__ SepTileLaunch p) {
   constexpr int H = kSepS / 2, NT = 32 * kSepWarps;
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float *const gt = reinterpret_cast<float *>(smem);
   // factor offsets and values of a group, and the zeros behind it
-  int2 *const off = reinterpret_cast<int2 *>(gt + sep_factor_floats(p.G)) + warp * kSepStage;
-  float2 *const val = reinterpret_cast<float2 *>(off) + kSepWarps * kSepStage;
+  float4 *const rec = reinterpret_cast<float4 *>(gt + sep_factor_floats(p.G)) + warp * kSepStage;
   float4 *const part = reinterpret_cast<float4 *>(gt + sep_factor_floats(p.G)) +
                        kSepWarps * kSepStage;
   if (lane < kSepStage - 32) {
-    off[32 + lane] = make_int2(0, 0);
-    val[32 + lane] = make_float2(0.f, 0.f);
+    rec[32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
 
   // padded factors: entry i of a row is tap i - 16, zero outside
   const float inv = 1.0f / (2.0f * p.sigma * p.sigma);
-  for (int i = tid; i < p.G * 4 * kSepRow; i += NT) {
-    const int s = i / (4 * kSepRow), ap = i % kSepRow + i / kSepRow % 4 - 16;
+  for (int i = tid; i < p.G * 2 * kSepRow; i += NT) {
+    const int s = i / (2 * kSepRow), ap = i % kSepRow + i / kSepRow % 2 - 16;
     const float x = (float)(ap - H + 1) - (float)s / (float)p.G;
     gt[i] = (unsigned)ap < (unsigned)kSepS ? expf(-(x * x) * inv) : 0.f;
   }
   __syncthreads();
 
   const int c = lane & 7, h = lane >> 3;
-  const uint32_t ax = smem_addr(gt) + 8 * c, ay = smem_addr(gt) + 16 * h;
+  const uint32_t ax = smem_addr(gt) + 8 * c, ay = smem_addr(gt) + 8 * h;
+  auto row = [&](int k) { return 2 * h + (k >> 1 & 1) + 8 * (k >> 2); };
   // blocks are spread over the SMs first, then claimed
   const int workers = SHARE ? (int)gridDim.x : (int)gridDim.x * kSepWarps;
   int blk = SHARE ? (int)blockIdx.x : (int)(blockIdx.x + warp * gridDim.x);
@@ -229,26 +227,26 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
     }
     const int start = sum - (end - beg), shift = beg - start;  // of range `lane`
     const int records = __shfl_sync(0xffffffffu, sum, 5);
+    const int first_end = __shfl_sync(0xffffffffu, sum, 0);
+    const int last_beg = __shfl_sync(0xffffffffu, start, 5);
     for (int plane = 0; plane < p.P; ++plane) {
-      // cell k: column 2c + (k & 1), row 4h + k / 2
+      // cell k: column 2c + (k & 1), row 2h + (k >> 1 & 1) + 8 (k >> 2)
       u64 run[8], hi[COMP ? 8 : 1], lo[COMP ? 8 : 1];
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         run[k] = 0ull;
         if constexpr (COMP) hi[k] = lo[k] = 0ull;
       }
-      int since = 0;  // records in the running sums
-      auto merge = [&]() {
+      // the records of a half group, into the cells [K0, K1)
+      auto merge = [&](auto k0, auto k1) {
         if constexpr (COMP) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
+          for (int k = decltype(k0)::value; k < decltype(k1)::value; ++k) {
             u64 e;
             hi[k] = two_sum2(hi[k], run[k], e);
             lo[k] = add2(lo[k], e);
-            run[k] = 0ull;
           }
         }
-        since = 0;
       };
       // the list in groups of 32
       int2 q = make_int2(0, 0);
@@ -270,7 +268,7 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
       int g = SHARE ? warp : 0;
       fetch(g);
       while (n > 0) {
-        const int m = n;
+        const int m = n, at_group = 32 * g;
         __syncwarp();  // the previous group was read
         int2 at = make_int2(0, 0);
         if (lane < m) {
@@ -278,56 +276,85 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
           sep_decode(q, log2G, mx, my, sx, sy);
           // entries of the padded rows at the block's first column and row
           const int ix = x0 - (mx - H + 1) + 16, iy = y0 - (my - H + 1) + 16;
-          at = make_int2(((sx * 4 + (ix & 3)) * kSepRow + (ix & ~3)) * 4,
-                         ((sy * 4 + (iy & 3)) * kSepRow + (iy & ~3)) * 4);
+          at = make_int2(((sx * 2 + (ix & 1)) * kSepRow + (ix & ~1)) * 4,
+                         ((sy * 2 + (iy & 1)) * kSepRow + (iy & ~1)) * 4);
         } else {
           v = make_float2(0.f, 0.f);
         }
-        off[lane] = at;
-        val[lane] = v;
+        rec[lane] = make_float4(__int_as_float(at.x), __int_as_float(at.y), v.x, v.y);
         g += SHARE ? kSepWarps : 1;
         fetch(g);
         __syncwarp();
         // the factors of a record are loaded while the previous one is added
-        struct Taps {
-          float2 v, gx;
-          float4 gy;
-        } a, b;
-        auto load = [&](Taps &t, const int2 o, int i) {
-          t.gx = lds64(ax + (uint32_t)o.x);
-          t.gy = lds128(ay + (uint32_t)o.y);
-          t.v = val[i];
-        };
-        auto add = [&](const Taps &t) {
-          const u64 vv = pk2(t.v.x, t.v.y);
-          const u64 w0 = mul2(vv, pk2(t.gx.x, t.gx.x)), w1 = mul2(vv, pk2(t.gx.y, t.gx.y));
-          run[0] = fma2(w0, pk2(t.gy.x, t.gy.x), run[0]);
-          run[1] = fma2(w1, pk2(t.gy.x, t.gy.x), run[1]);
-          run[2] = fma2(w0, pk2(t.gy.y, t.gy.y), run[2]);
-          run[3] = fma2(w1, pk2(t.gy.y, t.gy.y), run[3]);
-          run[4] = fma2(w0, pk2(t.gy.z, t.gy.z), run[4]);
-          run[5] = fma2(w1, pk2(t.gy.z, t.gy.z), run[5]);
-          run[6] = fma2(w0, pk2(t.gy.w, t.gy.w), run[6]);
-          run[7] = fma2(w1, pk2(t.gy.w, t.gy.w), run[7]);
-        };
-        load(a, off[0], 0);
-        int2 o = off[1];
-        for (int i0 = 0; i0 < m; i0 += 16) {
-          const int i1 = min(m, i0 + 16);
+        auto group = [&](auto k0, auto k1) {
+          constexpr bool LOW = decltype(k0)::value == 0, HIGH = decltype(k1)::value == 8;
+          struct Taps {
+            float2 v, gx, g0, g1;
+          } a, b;
+          auto load = [&](Taps &t, const float4 o) {
+            t.gx = lds64(ax + __float_as_uint(o.x));
+            if constexpr (LOW) t.g0 = lds64(ay + __float_as_uint(o.y));
+            if constexpr (HIGH) t.g1 = lds64(ay + __float_as_uint(o.y) + 32);
+            t.v = make_float2(o.z, o.w);
+          };
+          // fresh: the first of a run, whose sums are zero
+          auto add = [&](const Taps &t, bool fresh) {
+            const u64 vv = pk2(t.v.x, t.v.y);
+            const u64 w0 = mul2(vv, pk2(t.gx.x, t.gx.x)), w1 = mul2(vv, pk2(t.gx.y, t.gx.y));
+            auto cell = [&](int k, u64 w, float g) {
+              run[k] = fresh ? mul2(w, pk2(g, g)) : fma2(w, pk2(g, g), run[k]);
+            };
+            if constexpr (LOW) {
+              cell(0, w0, t.g0.x);
+              cell(1, w1, t.g0.x);
+              cell(2, w0, t.g0.y);
+              cell(3, w1, t.g0.y);
+            }
+            if constexpr (HIGH) {
+              cell(4, w0, t.g1.x);
+              cell(5, w1, t.g1.x);
+              cell(6, w0, t.g1.y);
+              cell(7, w1, t.g1.y);
+            }
+          };
+          load(a, rec[0]);
+          float4 o = rec[1];
+          for (int i0 = 0; i0 < m; i0 += kSepRun) {
+            if (m - i0 >= kSepRun) {
+#pragma unroll
+              for (int i = 0; i < kSepRun; i += 2) {
+                load(b, o);
+                o = rec[i0 + i + 2];
+                add(a, COMP && i == 0);
+                load(a, o);
+                o = rec[i0 + i + 3];
+                add(b, false);
+              }
+            } else {
+              if constexpr (COMP)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) run[k] = 0ull;
 #pragma unroll 1
-          for (int i = i0; i < i1; i += 2) {
-            load(b, o, i + 1);
-            o = off[i + 2];
-            add(a);
-            load(a, o, i + 2);
-            o = off[i + 3];
-            add(b);
+              for (int i = i0; i < m; i += 2) {
+                load(b, o);
+                o = rec[i + 2];
+                add(a, false);
+                load(a, o);
+                o = rec[i + 3];
+                add(b, false);
+              }
+            }
+            merge(k0, k1);
           }
-          since += i1 - i0;
-          if (COMP && since > kSepRun - 16) merge();
-        }
+        };
+        using std::integral_constant;
+        if (at_group + m <= first_end)
+          group(integral_constant<int, 0>(), integral_constant<int, 4>());
+        else if (at_group >= last_beg)
+          group(integral_constant<int, 4>(), integral_constant<int, 8>());
+        else
+          group(integral_constant<int, 0>(), integral_constant<int, 8>());
       }
-      merge();
       bool bad = false;
       if constexpr (SHARE) {
         // cell (x, y) of warp w at part[w][16 y + x]
@@ -337,7 +364,7 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
           const float2 a = upk2(COMP ? hi[k] : run[k]);
           float2 l = make_float2(0.f, 0.f);
           if constexpr (COMP) l = upk2(lo[k]);
-          part[warp * 256 + (4 * h + k / 2) * 16 + 2 * c + (k & 1)] = make_float4(a.x, a.y, l.x, l.y);
+          part[warp * 256 + row(k) * 16 + 2 * c + (k & 1)] = make_float4(a.x, a.y, l.x, l.y);
         }
         __syncthreads();
         u64 sh = 0ull, sl = 0ull;
@@ -371,7 +398,7 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 3 : 4)
           for (int k = 0; k < 8; ++k) {
             float2 l = make_float2(0.f, 0.f);
             if constexpr (COMP) l = upk2(lo[k]);
-            sep_store<COMP>(J, x0 + 2 * c + (k & 1), y0 + 4 * h + k / 2, plane, p.P, p.accumulate,
+            sep_store<COMP>(J, x0 + 2 * c + (k & 1), y0 + row(k), plane, p.P, p.accumulate,
                             upk2(COMP ? hi[k] : run[k]), l);
           }
         } else {
