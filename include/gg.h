@@ -423,7 +423,7 @@ int gg_server_destroy(gg_server *srv);
  * power of two in 16..256; oversample a power of two in 1..64; one
  * polarisation; complex64 values; GCF TABLE of at most 65536 taps (G*G*S*S,
  * e.g. G 8 with S 32) or GAUSSIAN; no per-visibility tables (gcf_index).  The
- * array (11165696 bytes, 10.6 MiB) stays resident on every GPU that loads
+ * array (10117120 bytes, 9.6 MiB) stays resident on every GPU that loads
  * libgg.so until the process exits.
  * The first call on a device looks up the array's device address
  * (cudaGetSymbolAddress) with that device current: make that first call

@@ -248,7 +248,7 @@ struct Plan {
   size_t o_merge[kMaxClasses] = {}, o_mdesc[kMaxClasses] = {};
   int merge_cap[kMaxClasses] = {}, merge_cells[kMaxClasses] = {};
   // workspace carve (offsets into the device workspace)
-  size_t o_jobs, o_bin, o_visb, o_tileb, o_class, o_kr, o_cnt, o_bm, o_scan, o_sidx, o_svals, o_order, o_items, o_kept, o_lo,
+  size_t o_jobs, o_bin, o_visb, o_tileb, o_class, o_rank, o_cnt, o_bm, o_scan, o_sidx, o_svals, o_order, o_items, o_kept, o_lo,
       o_count_vals, o_count_gcf, ws_bytes;
   int64_t vstride = 0, class_cap = 0;
   size_t table_bytes = 0;  // bytes uploaded from staging (jobs..class)
@@ -717,7 +717,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
   if (binned) {
     pl.aos = pl.P == 1 && !bin_only;
     for (const auto &kv : cfgs) pl.aos = pl.aos && kv.second.kind != kOwn;
-    pl.o_kr = take(sizeof(int2) * (vis + 1));
+    pl.o_rank = take(sizeof(int) * (vis + 1));
     pl.o_cnt = take(sizeof(int) * (tiles + 8));
     pl.o_bm = take(sizeof(int) * (tiles + 8));
     pl.o_scan = take(sizeof(int) * (scan_tmp_ints(tiles + 1) +
@@ -952,7 +952,7 @@ static void plan_bind(const gg_options *opt, Plan &pl, char *ws, char *host) {
 // The workspace arrays of a plan's binning.
 static void plan_bin_buffers(const Plan &pl, BinBuffers &b) {
   char *ws = pl.ws;
-  b.key_rank = (int2 *)(ws + pl.o_kr);
+  b.rank = (int *)(ws + pl.o_rank);
   b.counts = (int *)(ws + pl.o_cnt);
   b.scan_tmp = (int *)(ws + pl.o_scan);
   b.block_off = b.scan_tmp + kScanHead;
@@ -1069,6 +1069,7 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
   if (binned) {
     BinBuffers b{};
     b.jobs = (const BinJob *)(ws + pl.o_bin);
+    if (pl.njobs == 1) b.one = pl.hbin[0];
     b.vis_base = dvisb;
     b.tile_base = dtileb;
     b.njobs = pl.njobs;
@@ -1790,6 +1791,7 @@ int gg_bin(gg_context *ctx, const gg_options *opt, int uv_type, const void *uv,
   GG_CUDA(cudaStreamWaitEvent(s, ctx->exec_done, 0));
   BinBuffers b{};
   b.jobs = (const BinJob *)(ws + pl.o_bin);
+  b.one = pl.hbin[0];
   b.vis_base = (const int64_t *)(ws + pl.o_visb);
   b.tile_base = (const int *)(ws + pl.o_tileb);
   b.njobs = 1;

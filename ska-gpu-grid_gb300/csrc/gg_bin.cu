@@ -33,15 +33,6 @@ __device__ __forceinline__ int find_job64(const int64_t *base, int njobs,
   }
   return lo;
 }
-// Job of visibility g when the warp's first visibility g0 (<= g) belongs to
-// job j0: jobs are contiguous in g, so the search is done once per warp with
-// uniform loads and each lane only steps forward past job ends.
-__device__ __forceinline__ int job_from(const int64_t *base, int njobs, int j0, int64_t g) {
-  int j = j0;
-  while (j + 1 < njobs && __ldg(base + j + 1) <= g) ++j;
-  return j;
-}
-
 __device__ __forceinline__ int find_job32(const int *base, int njobs, int g) {
   int lo = 0, hi = njobs - 1;
   while (lo < hi) {
@@ -53,8 +44,8 @@ __device__ __forceinline__ int find_job32(const int *base, int njobs, int g) {
 
 // Contiguous slice [w0, w1) of the visibilities for this warp (multiples of
 // 32 apart), walked 32 at a time: the job of the slice's first visibility is
-// found once and then only advanced, where a grid-stride walk would search
-// the job table (dependent loads) on every step.
+// found once, where a grid-stride walk would search the job table (dependent
+// loads) on every step.
 struct WarpSlice {
   int64_t w0, w1;
   __device__ WarpSlice(int64_t total) : WarpSlice(total, blockIdx.x, gridDim.x) {}
@@ -66,9 +57,27 @@ struct WarpSlice {
     w1 = min(total, w0 + per);
   }
 };
-__device__ __forceinline__ int advance_job(const int64_t *base, int njobs, int j, int64_t g) {
-  while (j + 1 < njobs && __ldg(base + j + 1) <= g) ++j;
-  return j;
+// What a binning pass is compiled for: one job, described by the kernel's
+// parameters, with float or double coordinates, or any jobs.
+enum { kBinMany = 0, kBinOneF32 = 1, kBinOneF64 = 2 };
+
+// f(job, s, e) for the visibilities [s, e) of each job in the slice: what a job
+// has in common is loaded once, not for every visibility
+template <int KIND, class F>
+__device__ __forceinline__ void for_jobs(const BinBuffers &b, const WarpSlice &ws, F f) {
+  if (ws.w0 >= ws.w1) return;
+  if constexpr (KIND != kBinMany) {
+    f(b.one, ws.w0, ws.w1);
+    return;
+  }
+  int j = find_job64(b.vis_base, b.njobs, ws.w0);
+  for (int64_t s = ws.w0; s < ws.w1; ++j) {
+    const int64_t e = min(ws.w1, __ldg(b.vis_base + j + 1));
+    if (e <= s) continue;  // an empty job
+    const BinJob J = b.jobs[j];
+    f(J, s, e);
+    s = e;
+  }
 }
 
 // entries of a scan block, and of one of its threads
@@ -105,54 +114,67 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// resident CTAs per SM of the two passes over the visibilities: both wait on
-// loads and atomics, and 42 registers a thread hold a visibility without
-// spills (4.19 M visibilities, both passes and the tiles: 6 CTAs 384 us of the
-// whole call, 8 CTAs 396; two or four visibilities a lane at once 396-409)
+// resident CTAs per SM of the two passes over the visibilities of one job:
+// both wait on loads and atomics, and 42 registers a thread hold a visibility
+// and the next one's loads without spills (4.19 M visibilities, both passes
+// and the tiles: 6 CTAs 384 us of the whole call, 8 CTAs 396; two or four
+// visibilities a lane at once 396-409; the next one's loads ahead 387 -> 362).
+// The passes over many jobs hold the job's fields too and spill at 42: 5 CTAs
+// for the first and 4 for the other (256 jobs, whole call, 4.50 ms; 6 and 6
+// 4.66, 6 and 5 4.63, 5 and 5 4.64, 6 and 3 4.55).
 constexpr int kBinCtas = 6;
 
-// Pass 1.  Every visibility of every job: index step, drop rules, tile key, and
-// its rank among the visibilities of its tile.
+// Index step and tile of visibility n of a job at (u, v) = c.
 //  * a visibility whose oversample index falls outside [0,G) would address
-//    outside the GCF table in the reference; it is dropped and counted
+//    outside the GCF table in the reference; it is dropped and counted (bad)
 //  * a visibility whose footprint misses the grid contributes nothing and is
 //    dropped silently (the reference skips all of its taps, grid.cu:174-176)
 //  * mains left/right of the grid are clamped into the edge tile (all of their
 //    on-grid taps still lie inside that tile's window region), unless the
 //    tiles start before the grid
-// The rank comes from the histogram's own atomics, one for each run of equal
-// keys in a warp's 32 visibilities (tracks stay in a tile for many samples):
-// the scattering pass then needs no second round of claims.
-__global__ void __launch_bounds__(256, kBinCtas)
-    bin_count_kernel(const __grid_constant__ BinBuffers b) {
-  after_predecessor();
+// Returns the global tile, -1 when dropped.
+template <class T2>
+__device__ __forceinline__ int vis_tile(const BinJob &J, T2 c, int64_t n, int &mx, int &sx,
+                                        int &my, int &sy, bool &bad) {
+  const bool okx = index_step(c.x, J.G, mx, sx), oky = index_step(c.y, J.G, my, sy);
+  bool ok = okx && oky && (unsigned)sx < (unsigned)J.G && (unsigned)sy < (unsigned)J.G;
+  int gi = 0;
+  if (ok && J.gcf_index) {
+    gi = __ldg(J.gcf_index + n);
+    ok = (unsigned)gi < (unsigned)J.n_gcf;
+  }
+  bad = !ok;
+  const int h = J.S >> 1;
+  if (!ok || mx + h < 0 || mx - h + 1 >= J.N || my + h < 0 || my - h + 1 >= J.N) return -1;
+  const int cx = (J.off ? mx + J.off : min(max(mx, 0), J.N - 1)) >> J.log2T;
+  const int cy = (J.off ? my + J.off : min(max(my, 0), J.N - 1)) >> J.log2T;
+  return J.tile_base + (cy * J.ntx + cx) * J.n_gcf + gi;
+}
+
+template <class T> __device__ __forceinline__ T load_or_zero(const T *p, bool on) {
+  T v{};
+  if (on) v = __ldg(p);
+  return v;
+}
+
+// Pass 1.  Every visibility of every job: its tile, and its rank among the
+// visibilities of its tile (-1: dropped).  The rank comes from the histogram's
+// own atomics, one for each run of equal tiles in a warp's 32 visibilities
+// (tracks stay in a tile for many samples): the scattering pass then needs no
+// second round of claims.  The tile itself is not kept: working it out again
+// costs less than 8 bytes of traffic a visibility.
+template <class T2>
+__device__ __forceinline__ void bin_count_job(const BinBuffers &b, const BinJob &J, int64_t s,
+                                              int64_t e) {
   const int lane = threadIdx.x & 31;
-  const WarpSlice ws(b.total_vis);
-  int jw = b.njobs == 1 || ws.w0 >= ws.w1 ? 0 : find_job64(b.vis_base, b.njobs, ws.w0);
-  for (int64_t base = ws.w0; base < ws.w1; base += 32) {
-    const int64_t g = base + lane;
-    int key = -1;
+  const T2 *uv = static_cast<const T2 *>(J.uv) - J.vis_base;
+  T2 c = load_or_zero(uv + s + lane, s + lane < e);
+  for (int64_t g = s + lane; g - lane < e; g += 32) {
+    const T2 next = load_or_zero(uv + g + 32, g + 32 < e);
+    int key = -1, mx, sx, my, sy;
     bool bad = false;
-    if (b.njobs > 1) jw = advance_job(b.vis_base, b.njobs, jw, base);
-    if (g < ws.w1) {
-      const BinJob &J = b.jobs[b.njobs == 1 ? 0 : job_from(b.vis_base, b.njobs, jw, g)];
-      int mx, sx, my, sy;
-      bool ok = uv_index(J.uv, J.uv_f64, g - J.vis_base, J.G, mx, sx, my, sy) &&
-                (unsigned)sx < (unsigned)J.G && (unsigned)sy < (unsigned)J.G;
-      int gi = 0;
-      if (ok && J.gcf_index) {
-        gi = __ldg(J.gcf_index + (g - J.vis_base));
-        ok = (unsigned)gi < (unsigned)J.n_gcf;
-      }
-      bad = !ok;
-      const int h = J.S >> 1;
-      if (ok && mx + h >= 0 && mx - h + 1 < J.N && my + h >= 0 && my - h + 1 < J.N) {
-        // tiles that start before the grid need no clamping
-        const int cx = (J.off ? mx + J.off : min(max(mx, 0), J.N - 1)) >> J.log2T;
-        const int cy = (J.off ? my + J.off : min(max(my, 0), J.N - 1)) >> J.log2T;
-        key = J.tile_base + (cy * J.ntx + cx) * J.n_gcf + gi;
-      }
-    }
+    if (g < e) key = vis_tile(J, c, g - J.vis_base, mx, sx, my, sy, bad);
+    c = next;
     const unsigned badm = __ballot_sync(0xffffffffu, bad);
     if (badm && lane == 0) atomicAdd(&b.flags[FLAG_INDEX], __popc(badm));
     // runs of equal keys: the first lane of each claims for all
@@ -164,11 +186,21 @@ __global__ void __launch_bounds__(256, kBinCtas)
     int start = 0;
     if (head && key >= 0) start = atomicAdd(&b.counts[key], after ? __ffs(after) : 32 - lane);
     start = __shfl_sync(0xffffffffu, start, first);
-    if (g < ws.w1) {
-      b.key_rank[g] = make_int2(key, start + lane - first);
+    if (g < e) {
+      b.rank[g] = key >= 0 ? start + lane - first : -1;
       if (b.kept_pos) b.kept_pos[g] = key >= 0 ? 1 : 0;
     }
   }
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(256, KIND == kBinMany ? 5 : kBinCtas)
+    bin_count_kernel(const __grid_constant__ BinBuffers b) {
+  after_predecessor();
+  for_jobs<KIND>(b, WarpSlice(b.total_vis), [&](const BinJob &J, int64_t s, int64_t e) {
+    if (KIND == kBinOneF64 || (KIND == kBinMany && J.uv_f64)) bin_count_job<double2>(b, J, s, e);
+    else bin_count_job<float2>(b, J, s, e);
+  });
 }
 
 // first sorted position of tile t: the scan's block-local sum and its block's
@@ -183,34 +215,42 @@ __device__ __forceinline__ int tile_first(const BinBuffers &b, int t) {
 // outside its own tile's range proves the input was not tile-sorted), and its
 // values (one plane per polarisation; with `aos` the one value beside the
 // record, one 16-byte store instead of two of 8).
-__device__ __forceinline__ void bin_scatter_part(const BinBuffers &b, int64_t block,
-                                                 int64_t nblocks) {
+template <class T2>
+__device__ __forceinline__ void bin_scatter_job(const BinBuffers &b, const BinJob &J, int64_t s,
+                                                int64_t e) {
   const int lane = threadIdx.x & 31;
-  const WarpSlice ws(b.total_vis, block, nblocks);
-  int jw = b.njobs == 1 || ws.w0 >= ws.w1 ? 0 : find_job64(b.vis_base, b.njobs, ws.w0);
-  for (int64_t base = ws.w0; base < ws.w1; base += 32) {
-    const int64_t g = base + lane;
-    const int2 kr = g < ws.w1 ? __ldg(b.key_rank + g) : make_int2(-1, 0);
-    if (b.njobs > 1) jw = advance_job(b.vis_base, b.njobs, jw, base);
-    if (kr.x < 0) continue;
-    const BinJob &J = b.jobs[b.njobs == 1 ? 0 : job_from(b.vis_base, b.njobs, jw, g)];
+  const T2 *uv = static_cast<const T2 *>(J.uv) - J.vis_base;
+  const bool v32 = b.vals_bytes == 8;
+  const float2 *vals = static_cast<const float2 *>(J.vals) - J.vis_base * b.P;  // if v32
+  // the next visibility's coordinates, rank and value are loaded meanwhile
+  const bool on = s + lane < e;
+  T2 c = load_or_zero(uv + s + lane, on);
+  int rank = on ? __ldg(b.rank + s + lane) : -1;
+  float2 v8 = load_or_zero(vals + (s + lane) * b.P, on && v32);
+  for (int64_t g = s + lane; g < e; g += 32) {
+    const bool more = g + 32 < e;
+    const T2 c0 = c;
+    const int rank0 = rank;
+    const float2 v0 = v8;
+    c = load_or_zero(uv + g + 32, more);
+    rank = more ? __ldg(b.rank + g + 32) : -1;
+    v8 = load_or_zero(vals + (g + 32) * b.P, more && v32);
+    if (rank0 < 0) continue;
+    int mx, sx, my, sy;
+    bool bad;
     const int64_t n = g - J.vis_base;
-    // the value and the position do not depend on each other: both loads first
-    float2 v8 = make_float2(0.f, 0.f);
-    if (b.vals_bytes == 8) v8 = __ldg((const float2 *)J.vals + n * b.P);
+    const int key = vis_tile(J, c0, n, mx, sx, my, sy, bad);
     int pos;
     if (b.input_sorted) {
       pos = b.kept_pos[g];
-      if (pos < tile_first(b, kr.x) || pos >= tile_first(b, kr.x + 1)) {
+      if (pos < tile_first(b, key) || pos >= tile_first(b, key + 1)) {
         atomicOr(&b.flags[FLAG_UNSORTED], 1);
         b.bookmarks[b.total_tiles + 1] = 1;  // this call's records have holes
         continue;
       }
     } else {
-      pos = tile_first(b, kr.x) + kr.y;
+      pos = tile_first(b, key) + rank0;
     }
-    int mx, sx, my, sy;
-    uv_index(J.uv, J.uv_f64, n, J.G, mx, sx, my, sy);
     int2 rec;
     if (J.rec == kRecPacked) rec = make_int2(mx * J.G + sx, my * J.G + sy);
     else if (J.rec == kRecRegtile)
@@ -220,14 +260,13 @@ __device__ __forceinline__ void bin_scatter_part(const BinBuffers &b, int64_t bl
     else rec = window_record(mx, sx, my, sy, J.G);
     if (b.aos) {
       reinterpret_cast<float4 *>(b.sorted_idx)[pos] =
-          make_float4(__int_as_float(rec.x), __int_as_float(rec.y), v8.x, v8.y);
+          make_float4(__int_as_float(rec.x), __int_as_float(rec.y), v0.x, v0.y);
     } else {
       b.sorted_idx[pos] = rec;
-      if (b.vals_bytes == 8) {
-        const float2 *v = (const float2 *)J.vals + n * b.P;
+      if (v32) {
         float2 *o = (float2 *)b.sorted_vals;
-        o[pos] = v8;
-        for (int p = 1; p < b.P; ++p) o[p * b.vstride + pos] = __ldg(v + p);
+        o[pos] = v0;
+        for (int p = 1; p < b.P; ++p) o[p * b.vstride + pos] = __ldg(vals + g * b.P + p);
       } else {
         const double2 *v = (const double2 *)J.vals + n * b.P;
         double2 *o = (double2 *)b.sorted_vals;
@@ -236,6 +275,15 @@ __device__ __forceinline__ void bin_scatter_part(const BinBuffers &b, int64_t bl
     }
     if (b.order) b.order[pos] = (int)g;
   }
+}
+template <int KIND>
+__device__ __forceinline__ void bin_scatter_part(const BinBuffers &b, int64_t block,
+                                                 int64_t nblocks) {
+  const WarpSlice ws(b.total_vis, block, nblocks);
+  for_jobs<KIND>(b, ws, [&](const BinJob &J, int64_t s, int64_t e) {
+    if (KIND == kBinOneF64 || (KIND == kBinMany && J.uv_f64)) bin_scatter_job<double2>(b, J, s, e);
+    else bin_scatter_job<float2>(b, J, s, e);
+  });
 }
 
 // ---- exclusive scan ---------------------------------------------------------
@@ -471,19 +519,27 @@ __device__ __forceinline__ void bin_tiles_part(const BinBuffers &b, const ItemBu
 }
 
 // Pass 3: both parts side by side, the tiles' blocks first.
-__global__ void __launch_bounds__(256, kBinCtas)
+template <int KIND>
+__global__ void __launch_bounds__(256, KIND == kBinMany ? 4 : kBinCtas)
     bin_finish_kernel(const __grid_constant__ BinBuffers b, const __grid_constant__ ItemBuffers it,
                       int tile_blocks) {
   after_predecessor();
   if ((int)blockIdx.x < tile_blocks) bin_tiles_part(b, it, blockIdx.x, tile_blocks);
-  else bin_scatter_part(b, (int64_t)blockIdx.x - tile_blocks, (int64_t)gridDim.x - tile_blocks);
+  else bin_scatter_part<KIND>(b, (int64_t)blockIdx.x - tile_blocks, (int64_t)gridDim.x - tile_blocks);
 }
 
 cudaError_t run_binning(const BinBuffers &b, const ItemBuffers *items, cudaStream_t s) {
   cudaError_t e;
+  const int kind = b.njobs > 1 ? kBinMany : b.one.uv_f64 ? kBinOneF64 : kBinOneF32;
+  auto count = kind == kBinMany     ? bin_count_kernel<kBinMany>
+               : kind == kBinOneF64 ? bin_count_kernel<kBinOneF64>
+                                    : bin_count_kernel<kBinOneF32>;
+  auto finish = kind == kBinMany     ? bin_finish_kernel<kBinMany>
+                : kind == kBinOneF64 ? bin_finish_kernel<kBinOneF64>
+                                     : bin_finish_kernel<kBinOneF32>;
   if (b.total_vis > 0) {
     count_launch();
-    if ((e = launch_overlapped(bin_count_kernel, grid_for(b.total_vis), 256, 0, s, true, b)) !=
+    if ((e = launch_overlapped(count, grid_for(b.total_vis), 256, 0, s, true, b)) !=
         cudaSuccess)
       return e;
   }
@@ -505,7 +561,7 @@ cudaError_t run_binning(const BinBuffers &b, const ItemBuffers *items, cudaStrea
   const unsigned tiles = grid_for(cdiv((int64_t)b.total_tiles + 1, 4));
   const unsigned vis = b.total_vis > 0 ? grid_for(b.total_vis) : 0;
   count_launch();
-  return launch_overlapped(bin_finish_kernel, tiles + vis, 256, 0, s, true, b, it, (int)tiles);
+  return launch_overlapped(finish, tiles + vis, 256, 0, s, true, b, it, (int)tiles);
 }
 
 // ---- FP64 merge slots of tiles cut into several work items ---------------------

@@ -38,6 +38,7 @@ enum { kRecPacked = 0, kRecWindow = 1, kRecRegtile = 2, kRecTables = 3 };
 
 struct BinBuffers {
   const BinJob *jobs;      // device [njobs]
+  BinJob one;              // the job, if it is the only one
   const int64_t *vis_base; // device [njobs+1]
   const int *tile_base;    // device [njobs+1]
   int njobs;
@@ -45,8 +46,7 @@ struct BinBuffers {
   int total_tiles;         // sum of ntiles
   int vals_bytes;          // 8 (complex64) or 16 (complex128)
   int P;                   // polarisations (uniform over the batch)
-  int2 *key_rank;          // [total_vis] global tile id (-1: dropped), rank in
-                           // the tile
+  int *rank;               // [total_vis] rank in the tile (-1: dropped)
   int *counts;             // [total_tiles+1], zeroed by the caller: histogram,
                            // then block-local offsets
   int *scan_tmp;           // scan_tmp_ints; the first word zeroed by the caller

@@ -13,7 +13,7 @@
 // Limits: at most kNoAllocMaxVis visibilities, img_dim up to 4096 with the
 // default 32-cell tile (kNoAllocMaxTiles uv tiles), one polarisation,
 // complex64 values, a GCF table of at most 65536 taps (G*G*S*S).  The array
-// (kScratchBytes = 11165696 bytes, 10.6 MiB) is held by every GPU that loads
+// (kScratchBytes = 10117120 bytes, 9.6 MiB) is held by every GPU that loads
 // this library until the process exits.
 //
 // Set-up: the first call on a device looks up the device address of the
@@ -54,8 +54,8 @@ constexpr size_t kOffClass = kOffTileBase + al(2 * sizeof(int));
 // taken [16, 20)
 constexpr int kFlagInts = 32;
 constexpr size_t kOffFlags = kOffClass + al(sizeof(int));
-constexpr size_t kOffKr = kOffFlags + al(kFlagInts * sizeof(int));
-constexpr size_t kOffBm = kOffKr + al(sizeof(int2) * (kNoAllocMaxVis + 1));
+constexpr size_t kOffRank = kOffFlags + al(kFlagInts * sizeof(int));
+constexpr size_t kOffBm = kOffRank + al(sizeof(int) * (kNoAllocMaxVis + 1));
 constexpr size_t kOffCnt = kOffBm + al(sizeof(int) * (kNoAllocMaxTiles + 8));
 constexpr size_t kOffScan = kOffCnt + al(sizeof(int) * (kNoAllocMaxTiles + 8));
 // scratch of the scans over tiles and (input_sorted) visibilities: 2048-entry
@@ -80,7 +80,7 @@ constexpr size_t kOffMergeDesc = kOffMerge + al(kMergeBytes);
 constexpr size_t kScratchBytes = kOffMergeDesc + al(sizeof(int4) * kMergeMaxSlots);
 
 // the size the header and the documentation state
-static_assert(kScratchBytes == 11165696, "update the stated size of the allocation-free array");
+static_assert(kScratchBytes == 10117120, "update the stated size of the allocation-free array");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -275,6 +275,7 @@ extern "C" int gg_grid_device_noalloc(const gg_options *opt, const gg_job *job,
 
   BinBuffers b{};
   b.jobs = (const BinJob *)(ws + kOffBin);
+  b.one = B;
   b.vis_base = (const int64_t *)(ws + kOffVisBase);
   b.tile_base = (const int *)(ws + kOffTileBase);
   b.njobs = 1;
@@ -282,7 +283,7 @@ extern "C" int gg_grid_device_noalloc(const gg_options *opt, const gg_job *job,
   b.total_tiles = (int)(ntx * ntx);
   b.vals_bytes = 8;
   b.P = 1;
-  b.key_rank = (int2 *)(ws + kOffKr);
+  b.rank = (int *)(ws + kOffRank);
   b.counts = (int *)(ws + kOffCnt);
   b.bookmarks = (int *)(ws + kOffBm);
   b.scan_tmp = (int *)(ws + kOffScan);
