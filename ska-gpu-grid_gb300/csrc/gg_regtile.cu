@@ -40,11 +40,14 @@
 // at oversampling 8), hence one CTA per SM and one table per launch.  Several
 // tables, or one that does not fit, are read from global memory by
 // regtile_tables_kernel, complex entries as the caller keeps them.  There the
-// planes of an item are units of their own, next to each other, so that the
-// warps of a CTA read the same sub-kernels at about the same time.  Bound by
-// those reads (2 KB a record and plane for support 16, 42 % of them found in
-// L1): 524 k records of 4 planes and 32 tables of support 16 on 2048^2
-// 880 us for the whole call with window_kernel, 808 now.
+// planes of an item are units of their own, next to each other, and the warps
+// that sum them keep in step (where their number divides the CTA's warps), so
+// that all but the first find a record's sub-kernel (2 KB for support 16) in
+// L1: 80 % of the sectors, 42 % without.  Bound by the latency of the rest,
+// which one record of lookahead does not cover (48 % of cycles issue; fetching
+// the lines of the next 8 to 32 records into L1 cost more than it hid).  524 k
+// records of 4 planes and 32 tables of support 16 on 2048^2, whole call:
+// window_kernel 880 us, planes out of step 808, in step 746.
 //
 // Bound by instruction issue (60-63 % of active cycles issue; 42 and 87 warp
 // instructions a record for supports 8 and 16 on the batched tracks, about
@@ -191,13 +194,33 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
   const uint32_t im_off = 4u * rt_table_floats(S, p.G);
   const int P = p.P, total = *p.nitems * P;
   const int first = gridDim.x * C::WARPS;
+  // GT: the warps that sum the planes of an item keep in step (a barrier every
+  // few records), so that one of them finds in L1 what another has loaded
+  const bool grouped = GT && P > 1 && C::WARPS % P == 0;
+  const int group = grouped ? warp / P : 0, member = grouped ? warp - group * P : 0;
+  auto in_step = [&]() {
+    if (grouped) asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(32 * P) : "memory");
+  };
 
   // The first units are spread over the SMs (the planes of an item stay
   // together); later ones are claimed ahead: while a unit is summed, the range
   // of the next is in registers and its first records, the range of the one
   // after and a further claim are on their way.
   int unit = P == 1 ? blockIdx.x + warp * gridDim.x : blockIdx.x * C::WARPS + warp;
-  auto claim_one = [&]() { return lane == 0 ? atomicAdd(p.item_next, 1) + first : 0; };
+  // of a group, the first warp claims an item
+  __shared__ int s_claim[GT ? C::WARPS : 1];
+  auto claim_one = [&]() {
+    if (grouped) return lane == 0 && member == 0 ? (atomicAdd(p.item_next, 1) * P + first) : 0;
+    return lane == 0 ? atomicAdd(p.item_next, 1) + first : 0;
+  };
+  auto claimed = [&](int c) {
+    if (!grouped) return __shfl_sync(0xffffffffu, c, 0);
+    if (lane == 0 && member == 0) s_claim[group] = c;
+    in_step();
+    c = s_claim[group] + member;
+    in_step();  // all have read it
+    return c;
+  };
   auto range = [&](int it) {
     return it < total ? __ldg(reinterpret_cast<const int4 *>(p.items + (P == 1 ? it : it / P)))
                       : make_int4(0, 0, 0, 0);
@@ -216,11 +239,11 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
   int claim = claim_one();
   int4 cur = range(unit);  // {job, bin, start, end}
   fetch(cur.z, cur.w, P == 1 ? 0 : unit % P);
-  int next = __shfl_sync(0xffffffffu, claim, 0);
+  int next = claimed(claim);
   claim = claim_one();
   int4 nxt = range(next);
   while (true) {
-    const int next2 = __shfl_sync(0xffffffffu, claim, 0);
+    const int next2 = claimed(claim);
     claim = claim_one();
     const int4 nxt2 = range(next2);
     const int item = P == 1 ? unit : unit / P, plane = unit - item * P;
@@ -354,6 +377,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
           while (left > 0) {
             const int m = min(left, kRtRun);
             const float4 *const end = st + m;
+            in_step();
 #pragma unroll 1
             while (st != end) {
               load(b, q, cx);

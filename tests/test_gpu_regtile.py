@@ -98,7 +98,9 @@ def test_edges_layouts_and_items(ctx, N, G, P, layout, out, S, chunk):
 
 @pytest.mark.parametrize("kind", ["real", "complex"])
 @pytest.mark.parametrize("S,G,P,ntab,n", [(8, 8, 1, 3, 4000), (16, 8, 2, 5, 3000),
-                                          (16, 16, 1, 1, 900), (8, 16, 3, 2, 2000)])
+                                          (16, 16, 1, 1, 900), (8, 16, 3, 2, 2000),
+                                          (16, 8, 4, 2, 40000), (16, 4, 3, 7, 5000),
+                                          (8, 8, 4, 4, 30000), (16, 8, 5, 2, 1500)])
 def test_tables_in_global_memory(ctx, S, G, P, ntab, n, kind):
     """per-visibility tables, one too large for shared memory, and (below) a
     table for each job of a batch"""
