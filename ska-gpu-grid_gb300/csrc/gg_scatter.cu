@@ -8,19 +8,23 @@
 // loop).  The small-support kernel's unsynchronised += (grid_gpu.cu:309-310)
 // is a data race and has no counterpart here.
 //
-// A CTA takes 256 consecutive visibilities: every thread loads one (u,v) as a
-// 128-bit vector, performs the FP64 index step once, and parks the footprint's
-// place, the sub-kernel and the values in shared memory; each warp then walks
-// the visibilities with its lanes spread over the S*S taps, so a warp's
-// reductions hit consecutive cells of a footprint row.
+// A warp takes an equal share of the visibilities, 32 consecutive ones at a
+// time: every lane loads one (u,v) as a 128-bit vector, performs the FP64 index
+// step once, and parks the footprint's place, the sub-kernel and the values in
+// shared memory; then the warp walks the visibilities with its lanes spread
+// over the S*S taps, so its reductions hit consecutive cells of a footprint
+// row.  Nothing waits for the other warps (256 visibilities a CTA, between
+// barriers, left its last round three quarters empty).
 //
 // What binds: FP32 values, the L2's reductions by 32-byte sector (1 M
-// visibilities of support 8 on 2048^2: 22 sectors each, 172 G/s of the 190 G/s
+// visibilities of support 8 on 2048^2: 22 sectors each, 190 G/s of the 190 G/s
 // that coalesced reductions reach; 190 -> 134 us once a visibility cost 83
-// warp instructions instead of 156).  FP64 values, the FP64 pipe: 16
-// multiplications a visibility of support 16 and lane when the table has no
-// imaginary parts (32 operations before), one reduction per component with
-// every sector touched once (262,144 visibilities on 1024^2: 594 -> 415 us).
+// warp instructions instead of 156, 121 with equal shares).  FP64 values, the
+// FP64 pipe: 16 multiplications a visibility of support 16 and lane when the
+// table has no imaginary parts (32 operations before), one reduction per
+// component with every sector touched once (262,144 visibilities on 1024^2,
+// whole call: 605 -> 414 us, equal shares 362, four factors instead of eight
+// ahead and twice the warps 305; the multiplications alone 215).
 //
 // Compensated mode (complex64 output): the hi grid is updated with
 // atom.global.v2.f32.add, which returns the previous value; two_sum of
@@ -32,6 +36,9 @@
 namespace gg {
 
 constexpr int kScatterThreads = 256;
+// resident on an SM (FP64 values, support 16, the case below: 2 CTAs 362 us of
+// the whole call, 3 324, 4 305, 5 310)
+constexpr int kScatterCtas = 4;
 
 __device__ __forceinline__ int find_job_v(const int64_t *base, int njobs,
                                           int64_t g) {
@@ -49,7 +56,7 @@ __device__ __forceinline__ bool finite_bits(double x) {
 }
 
 template <int S, class ACC, int GK>
-__global__ void __launch_bounds__(kScatterThreads)
+__global__ void __launch_bounds__(kScatterThreads, kScatterCtas)
     scatter_kernel(KParams kp) {
   constexpr bool GAUSS = GK == 1, WPHASE = GK == 2;
   using VT = typename ACC::VT;
@@ -82,13 +89,15 @@ __global__ void __launch_bounds__(kScatterThreads)
   float *lo = nullptr;
   const VT2 *gcf = nullptr;
 
-  for (int64_t c0 = (int64_t)blockIdx.x * NT; c0 < kp.total_vis;
-       c0 += (int64_t)gridDim.x * NT) {
-    __syncthreads();  // previous chunk fully consumed
+  if constexpr (GAUSS) __syncthreads();
+  const int64_t nwarps = (int64_t)gridDim.x * (NT / 32), wid = blockIdx.x * (NT / 32) + warp;
+  const int64_t end = kp.total_vis * (wid + 1) / nwarps;
+  for (int64_t c0 = kp.total_vis * wid / nwarps; c0 < end; c0 += 32) {
+    __syncwarp();  // the previous 32 fully consumed
     {
-      const int64_t t = c0 + tid;
+      const int64_t t = c0 + lane;
       int4 r = make_int4(0, 0, 0, -1);
-      if (t < kp.total_vis) {
+      if (t < end) {
         int j = 0;
         int64_t n = t;
         if (kp.njobs > 1) {
@@ -146,11 +155,11 @@ __global__ void __launch_bounds__(kScatterThreads)
       }
       rec[tid] = r;
     }
-    __syncthreads();
+    __syncwarp();
     // Lane l takes the taps l, l + 32, ... of a visibility: their places in
     // the footprint are the same for all, and so are the table offsets.  The
     // job's fields stay in registers while the job does.
-    for (int q = warp; q < NT; q += NT / 32) {
+    for (int q = tid - lane; q < tid - lane + 32; ++q) {
       const int4 r = rec[q];
       if (r.w < 0) continue;
       if (r.w >> 1 != job) {
@@ -212,7 +221,7 @@ __global__ void __launch_bounds__(kScatterThreads)
           // FP64 products bind: a tap without an imaginary part takes one per
           // component instead of two (unless 0 * v matters), decided for the
           // whole warp, as a choice per tap would compute both.
-          constexpr int PARTS = (S * S * 2 + 31) / 32, U = PARTS < 8 ? PARTS : 8;
+          constexpr int PARTS = (S * S * 2 + 31) / 32, U = PARTS < 4 ? PARTS : 4;
           constexpr int PROWS = S < 16 ? 16 / S : 1;  // rows between a lane's parts
           const int px = (lane >> 1) % S, py = (lane >> 1) / S, im = lane & 1;
           // component = a * re(g) + b * im(g)
@@ -307,7 +316,7 @@ static cudaError_t scatter_launch(const KParams &kp, int sm_count, cudaStream_t 
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kScatterThreads, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  int64_t chunks = (kp.total_vis + kScatterThreads - 1) / kScatterThreads;
+  const int64_t chunks = (kp.total_vis + 31) / 32;  // at least four a warp
   int64_t grid = (int64_t)sm_count * per_sm;
   if (grid > chunks) grid = chunks;
   if (grid < 1) return cudaSuccess;

@@ -76,6 +76,20 @@ def test_supports_edges_and_tables(ctx, S, N, P, kind, f64):
 
 
 @pytest.mark.parametrize("f64", [True, False])
+@pytest.mark.parametrize("n", [1, 31, 33, 1217, 19457, 40001])
+def test_shares_of_the_warps(ctx, n, f64):
+    """fewer visibilities than warps, shares of one or two groups of 32, uneven ones"""
+    S, N, P = 8, 60, 1
+    uv, vals, gcf = case(S, N, n, "real", f64, P)
+    d = device(uv, vals, gcf, P * N * N)
+    o = gg.Options(mode=gg.MODE_SCATTER, layout=gg.LAYOUT_INTERLEAVED, polarizations=P)
+    ctx.grid(o, d[3], *d[:3], N, S)
+    torch.cuda.synchronize()
+    assert ctx.read_flags() == [0, 0, 0, 0]
+    check(d[3], uv, vals, gcf, N, S, P)
+
+
+@pytest.mark.parametrize("f64", [True, False])
 def test_jobs_change_within_a_block(ctx, f64):
     sets = [case(8, N, n, kind, f64, seed=k)
             for k, (N, n, kind) in enumerate([(20, 30, "real"), (64, 5, "complex"),
