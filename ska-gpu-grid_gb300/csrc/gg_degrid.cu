@@ -24,8 +24,9 @@
 //    the real, the other with the imaginary parts, which halves its shuffles.
 //
 // 4.19 M visibilities of support 8 from a 4096^2 grid: 658 us at 131 warp
-// instructions a visibility before, 333 us at 65 now (304 without the test for sums
-// that are not finite).
+// instructions a visibility before, 328 us at 65 now (25 less without the test
+// for sums that are not finite).  With the table in shared memory (one CTA of
+// 1024 threads): 6 % less above 1.5 M visibilities, more below: not taken.
 #include <type_traits>
 
 #include "gg_kernels.cuh"
@@ -93,11 +94,20 @@ __global__ void __launch_bounds__(256, kDegridCtas) degrid_kernel(const __grid_c
   const size_t NN = (size_t)d.N * d.N;
   const int N = d.N, GG = d.G * d.G;
   const VT2 *const tabs = reinterpret_cast<const VT2 *>(d.gcf) + sl;
-  for (int64_t base = warp * 32; base < d.npts; base += nwarps * 32) {
+  // Few visibilities: every warp an equal share, in steps of VPW (160 k of
+  // support 8: 20.4 -> 17.9 us, 10 k of support 16 24 -> 9.8).  From four groups
+  // of 32 a warp on, the groups go round the warps: neighbouring ones share
+  // cells (1 M: the same; 4.19 M: 344 us, in shares 387).
+  const bool shares = d.npts < nwarps * 32 * 4;
+  const int64_t steps = (d.npts + VPW - 1) / VPW;
+  const int64_t end = shares ? min(d.npts, steps * (warp + 1) / nwarps * VPW) : d.npts;
+  const int64_t stride = shares ? 32 : nwarps * 32;
+  for (int64_t base = shares ? steps * warp / nwarps * VPW : warp * 32; base < end;
+       base += stride) {
     // one visibility per lane: first cell of its footprint and sub-kernel (of
     // all tables; -1: dropped)
     int fx = 0, fy = 0, sub = -1;
-    if (base + lane < d.npts) {
+    if (base + lane < end) {
       int sx, sy, mx, my, tab = 0;
       bool ok = uv_step(d.uv, d.uv_f64, base + lane, d.G, mx, sx, my, sy) &&
                 (unsigned)sx < (unsigned)d.G && (unsigned)sy < (unsigned)d.G;
@@ -114,7 +124,7 @@ __global__ void __launch_bounds__(256, kDegridCtas) degrid_kernel(const __grid_c
       }
     }
 #pragma unroll 1
-    for (int it = 0; it < S && base + it * VPW < d.npts; ++it) {
+    for (int it = 0; it < S && base + it * VPW < end; ++it) {
       const int src = it * VPW + sv;
       const int x0 = __shfl_sync(0xffffffffu, fx, src), y0 = __shfl_sync(0xffffffffu, fy, src);
       const int k = __shfl_sync(0xffffffffu, sub, src);
@@ -236,7 +246,7 @@ __global__ void __launch_bounds__(256, kDegridCtas) degrid_kernel(const __grid_c
         t.merge(oh, ol);
 #pragma unroll
         for (int o = 2; o < S; o <<= 1) t.merge_lane(o);
-        if (sl < 2 && base + src < d.npts)
+        if (sl < 2 && base + src < end)
           reinterpret_cast<VT *>(d.vals)[2 * ((size_t)(base + src) * d.P + p) + sl] = t.value();
       }
     }
@@ -270,7 +280,8 @@ cudaError_t degrid_types(const DegridLaunch &d, unsigned blocks, cudaStream_t s)
 
 cudaError_t launch_degrid(const DegridLaunch &d, cudaStream_t s) {
   if (d.npts <= 0) return cudaSuccess;
-  const int64_t b = (d.npts + 255) / 256;
+  // a step for every warp, until the resident CTAs are reached
+  const int64_t steps = (d.npts + 32 / d.S - 1) / (32 / d.S), b = (steps + 7) / 8;
   const int64_t cap = (int64_t)d.sm_count * kDegridCtas;
   const unsigned blocks = (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
   switch (d.S) {

@@ -78,3 +78,18 @@ def test_grid_that_is_not_finite(ctx):
     assert hit.any() and not hit.all()
     assert np.isnan(got.real[hit]).all() and not np.isfinite(got.imag[hit]).any()
     assert np.isfinite(got[~hit]).all()
+
+
+@pytest.mark.parametrize("S,n", [(4, 1), (4, 640_001), (8, 5), (8, 4_999), (8, 622_592 + 3),
+                                 (16, 9_731), (16, 40_003), (32, 4_865), (32, 1_217)])
+def test_shares_of_the_warps(ctx, S, n):
+    """a step or less for a warp, shares of several groups of 32, and groups dealt out"""
+    N, rng = 70, np.random.default_rng(n)
+    uv = synth.fr(rng.uniform(0, N, size=(n, 2)))
+    tab = synth.gcf_table(synth.gaussian_gcf_1d(S)).astype(np.complex64)
+    grid = (rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))).astype(np.complex64)
+    got = degrid(ctx, uv, grid, tab, N, S)
+    planar = np.stack([grid.real, grid.imag]).astype(np.float64).reshape(2, 1, N, N)
+    ref = np.asarray(O.degrid_pz(uv, planar, pairs(tab), N, S, nthreads=8)).reshape(n, -1)
+    ref = ref[:, 0] + 1j * ref[:, 1] if ref.shape[1] == 2 else ref.reshape(-1)
+    assert np.abs(got - ref).max() <= 1e-6 * np.abs(ref).max()
