@@ -708,7 +708,8 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
   pl.o_tileb = take(sizeof(int) * (njobs + 1));
   pl.o_class = take(sizeof(int) * njobs);
   pl.table_bytes = off;
-  pl.vstride = vis + 8;
+  // even: the planes of 8-byte values are copied in bulk from 16-byte boundaries
+  pl.vstride = (vis + 9) & ~(int64_t)1;
   int64_t full_items = vis / pl.chunk;
   for (const auto &kv : cfgs)
     if (kv.second.auto_chunk)
