@@ -39,6 +39,10 @@ constexpr int kScatterThreads = 256;
 // resident on an SM (FP64 values, support 16, the case below: 2 CTAs 362 us of
 // the whole call, 3 324, 4 305, 5 310)
 constexpr int kScatterCtas = 4;
+// compensated sums wait for the previous value of every tap (support 16, 1 M
+// and 4.19 M visibilities: 4 CTAs 1.00 and 4.30 ms, 5 0.95 and 4.04, 6 0.92
+// and 3.62, 8, which spill, 1.15 and 4.12; 973 and 3838 us before)
+constexpr int kScatterCtasComp = 6;
 
 __device__ __forceinline__ int find_job_v(const int64_t *base, int njobs,
                                           int64_t g) {
@@ -56,7 +60,8 @@ __device__ __forceinline__ bool finite_bits(double x) {
 }
 
 template <int S, class ACC, int GK>
-__global__ void __launch_bounds__(kScatterThreads, kScatterCtas)
+__global__ void __launch_bounds__(kScatterThreads, std::is_same<ACC, AccComp>::value
+                                                       ? kScatterCtasComp : kScatterCtas)
     scatter_kernel(KParams kp) {
   constexpr bool GAUSS = GK == 1, WPHASE = GK == 2;
   using VT = typename ACC::VT;
