@@ -25,6 +25,10 @@
 //    added into (hi, lo) by TwoSum.
 //  * Few blocks (small grids): the warps of a CTA share a block and add their
 //    (hi, lo) sums by TwoSum in shared memory.
+//
+// Bound by instruction issue (77 % of active cycles; 62 % of the shared-memory
+// wavefronts).  1.05 M visibilities of support 8 on 4096^2, whole call: 858 us
+// by 32-cell tiles, 227 now; 4.19 M, this kernel, 2.09 -> 0.56 ms.
 #include <algorithm>
 
 #include "gg_kernels.cuh"

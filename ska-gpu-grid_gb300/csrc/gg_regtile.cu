@@ -49,14 +49,14 @@
 // records of 4 planes and 32 tables of support 16 on 2048^2, whole call:
 // window_kernel 880 us, planes out of step 808, in step 746.
 //
-// Bound by instruction issue (60-63 % of active cycles issue; 42 and 87 warp
+// Bound by instruction issue (60-64 % of active cycles issue; 39 and 79 warp
 // instructions a record for supports 8 and 16 on the batched tracks, about
 // half of them sorting, TwoSum and flushes of small tiles).  Measured against
 // window_kernel on the same jobs: 4.19 M support-8 records of a 4096^2
-// observation 435 -> 253 us; 256 mixed jobs, 24.4 M support-8 records 1366 ->
-// 1337 us, 20.9 M support-16 records 3189 -> 2228 us; 10 k support-8 records
+// observation 435 -> 247 us; 256 mixed jobs, 24.4 M support-8 records 1366 ->
+// 1311 us, 20.9 M support-16 records 3189 -> 2141 us; 10 k support-8 records
 // on 256^2 36 -> 13 us; 100 k support-16 records on 777^2, whole call, 135 ->
-// 73 us.
+// 68 us.
 #include <algorithm>
 
 #include "gg_kernels.cuh"
