@@ -39,10 +39,12 @@ constexpr int kScatterThreads = 256;
 // resident on an SM (FP64 values, support 16, the case below: 2 CTAs 362 us of
 // the whole call, 3 324, 4 305, 5 310)
 constexpr int kScatterCtas = 4;
-// compensated sums wait for the previous value of every tap (support 16, 1 M
-// and 4.19 M visibilities: 4 CTAs 1.00 and 4.30 ms, 5 0.95 and 4.04, 6 0.92
-// and 3.62, 8, which spill, 1.15 and 4.12; 973 and 3838 us before)
-constexpr int kScatterCtasComp = 6;
+// Compensated sums wait for the previous value of every tap: more warps hide
+// it, until those on the same cells get in each other's way.  Support 16, on
+// tracks, us: 262 k visibilities 286 / 275 / 325 with 4 / 5 / 6 CTAs, 1 M 995 /
+// 942 / 934 (sorted by tile 983 / 956 / 966), 4.19 M 4270 / 4012 / 3613.
+constexpr int kScatterCtasComp = 5, kScatterCtasLarge = 6;
+constexpr int64_t kScatterLarge = 1 << 21;  // visibilities
 
 __device__ __forceinline__ int find_job_v(const int64_t *base, int njobs,
                                           int64_t g) {
@@ -59,9 +61,8 @@ __device__ __forceinline__ bool finite_bits(double x) {
   return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
 }
 
-template <int S, class ACC, int GK>
-__global__ void __launch_bounds__(kScatterThreads, std::is_same<ACC, AccComp>::value
-                                                       ? kScatterCtasComp : kScatterCtas)
+template <int S, class ACC, int GK, int CTAS>
+__global__ void __launch_bounds__(kScatterThreads, CTAS)
     scatter_kernel(KParams kp) {
   constexpr bool GAUSS = GK == 1, WPHASE = GK == 2;
   using VT = typename ACC::VT;
@@ -307,13 +308,13 @@ __global__ void __launch_bounds__(kScatterThreads, std::is_same<ACC, AccComp>::v
   }
 }
 
-template <int S, class ACC, int GK>
+template <int S, class ACC, int GK, int CTAS>
 static cudaError_t scatter_launch(const KParams &kp, int sm_count, cudaStream_t s) {
   using VT2 = typename vec2_of<typename ACC::VT>::type;
   size_t smem = kScatterThreads * sizeof(int4) +
                 (size_t)kScatterThreads * kp.P * sizeof(VT2) + 64 * S * 4 +
                 (GK == 2 ? kScatterThreads * sizeof(float2) : 0);
-  auto kern = scatter_kernel<S, ACC, GK>;
+  auto kern = scatter_kernel<S, ACC, GK, CTAS>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
@@ -335,13 +336,16 @@ static cudaError_t scatter_dispatch(const GridLaunch &g, const KParams &kp,
                                     cudaStream_t s) {
   // GCF source: 0 table, 1 Gaussian on the fly, 2 COMPUTE_GCF phase factor
   const int gk = g.wphase ? 2 : (g.gauss ? 1 : 0);
-#define GG_SC(ACCT)                                                      \
-  return gk == 2 ? scatter_launch<S, ACCT, 2>(kp, g.sm_count, s)         \
-                 : (gk == 1 ? scatter_launch<S, ACCT, 1>(kp, g.sm_count, s) \
-                            : scatter_launch<S, ACCT, 0>(kp, g.sm_count, s))
-  if (g.vals_f64) GG_SC(AccF64);
-  if (g.accum == GG_ACC_COMPENSATED) GG_SC(AccComp);
-  GG_SC(AccF32);
+#define GG_SC(ACCT, CTAS)                                                      \
+  return gk == 2 ? scatter_launch<S, ACCT, 2, CTAS>(kp, g.sm_count, s)         \
+                 : (gk == 1 ? scatter_launch<S, ACCT, 1, CTAS>(kp, g.sm_count, s) \
+                            : scatter_launch<S, ACCT, 0, CTAS>(kp, g.sm_count, s))
+  if (g.vals_f64) GG_SC(AccF64, kScatterCtas);
+  if (g.accum == GG_ACC_COMPENSATED) {
+    if (g.total_vis >= kScatterLarge) GG_SC(AccComp, kScatterCtasLarge);
+    GG_SC(AccComp, kScatterCtasComp);
+  }
+  GG_SC(AccF32, kScatterCtas);
 #undef GG_SC
 }
 

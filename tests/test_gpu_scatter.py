@@ -119,3 +119,17 @@ def test_fp64_values_that_are_not_finite(ctx):
     inside[y0:y0 + S, x0:x0 + S] = True
     assert np.isnan(got.real[inside]).all() and not np.isfinite(got.imag[inside]).any()
     assert np.isfinite(got.real[~inside]).all() and np.isfinite(got.imag[~inside]).all()
+
+
+@pytest.mark.parametrize("n", [3_001, (1 << 21) - 1, 1 << 21])
+def test_compensated_on_both_sides_of_the_large_calls(ctx, n):
+    S, N, P = 4, 300, 1
+    uv, vals, gcf = case(S, N, n, "real", False, P)
+    d = device(uv, vals, gcf, N * N)
+    o = gg.Options(mode=gg.MODE_SCATTER, accum=gg.ACC_COMPENSATED,
+                   layout=gg.LAYOUT_INTERLEAVED)
+    ctx.grid(o, d[3], *d[:3], N, S)
+    torch.cuda.synchronize()
+    got = planar_from_grid(torch.view_as_real(d[3]).reshape(-1).cpu().numpy(), P, N, False)
+    ref = O.grid_pz(uv, pairs(vals), pairs(gcf), N, S, nthreads=8)
+    assert rel_err(got, ref) <= 1e-6
