@@ -213,6 +213,16 @@ __global__ void __launch_bounds__(kScatterThreads, CTAS)
         gi = g.y;
         return true;
       };
+      // the Gaussian's factor is real: an infinite component of a value stays
+      // in its own component of the grid
+      auto product = [&](const VT2 v, VT gr, VT gi, VT &tr, VT &ti) {
+        if constexpr (GAUSS) {
+          tr = v.x * gr;
+          ti = v.y * gr;
+        } else {
+          cmul<VT>(v.x, v.y, gr, gi, tr, ti);
+        }
+      };
       // from a lane's first part to its part k, in doubles
       auto part_step = [&](int k) -> int64_t {
         if constexpr (S == 32) return 2 * ((int64_t)(k >> 1) * N + 16 * (k & 1));
@@ -238,7 +248,7 @@ __global__ void __launch_bounds__(kScatterThreads, CTAS)
           for (int k0 = 0; k0 < PARTS; k0 += U) {
             double2 g[U];
             bool on[U];
-            bool full = !finite_bits(va) || !finite_bits(vb);
+            bool full = !GAUSS && (!finite_bits(va) || !finite_bits(vb));
 #pragma unroll
             for (int k = 0; k < U; ++k) {
               // S = 32: two parts per row
@@ -267,7 +277,7 @@ __global__ void __launch_bounds__(kScatterThreads, CTAS)
           for (int k = 0; k < TAPS; ++k) {
             VT gr, gi, tr, ti;
             if (!factor(k, gr, gi)) continue;
-            cmul<VT>(v.x, v.y, gr, gi, tr, ti);
+            product(v, gr, gi, tr, ti);
             red_add_v2(cell + 2 * (int64_t)(k * step), (float)tr, (float)ti);
           }
           continue;
@@ -276,7 +286,7 @@ __global__ void __launch_bounds__(kScatterThreads, CTAS)
         for (int k = 0; k < TAPS; ++k) {
           VT gr, gi, tr, ti;
           if (!factor(k, gr, gi)) continue;
-          cmul<VT>(v.x, v.y, gr, gi, tr, ti);
+          product(v, gr, gi, tr, ti);
           const size_t c = p * NN + (size_t)(cell0 + k * step);
           if constexpr (std::is_same<ACC, AccComp>::value) {
             if (!f64) {
