@@ -29,7 +29,7 @@ __device__ __forceinline__ int find_job64(const int64_t *base, int njobs,
   int lo = 0, hi = njobs - 1;
   while (lo < hi) {
     int mid = (lo + hi + 1) >> 1;
-    if (__ldg(base + mid) <= g) lo = mid; else hi = mid - 1;
+    if (base[mid] <= g) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
@@ -37,7 +37,7 @@ __device__ __forceinline__ int find_job32(const int *base, int njobs, int g) {
   int lo = 0, hi = njobs - 1;
   while (lo < hi) {
     int mid = (lo + hi + 1) >> 1;
-    if (__ldg(base + mid) <= g) lo = mid; else hi = mid - 1;
+    if (base[mid] <= g) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
@@ -72,7 +72,7 @@ __device__ __forceinline__ void for_jobs(const BinBuffers &b, const WarpSlice &w
   }
   int j = find_job64(b.vis_base, b.njobs, ws.w0);
   for (int64_t s = ws.w0; s < ws.w1; ++j) {
-    const int64_t e = min(ws.w1, __ldg(b.vis_base + j + 1));
+    const int64_t e = min(ws.w1, b.vis_base[j + 1]);
     if (e <= s) continue;  // an empty job
     const BinJob J = b.jobs[j];
     f(J, s, e);
@@ -225,7 +225,7 @@ __device__ __forceinline__ void bin_scatter_job(const BinBuffers &b, const BinJo
   // the next visibility's coordinates, rank and value are loaded meanwhile
   const bool on = s + lane < e;
   T2 c = load_or_zero(uv + s + lane, on);
-  int rank = on ? __ldg(b.rank + s + lane) : -1;
+  int rank = on ? b.rank[s + lane] : -1;
   float2 v8 = load_or_zero(vals + (s + lane) * b.P, on && v32);
   for (int64_t g = s + lane; g < e; g += 32) {
     const bool more = g + 32 < e;
@@ -233,7 +233,7 @@ __device__ __forceinline__ void bin_scatter_job(const BinBuffers &b, const BinJo
     const int rank0 = rank;
     const float2 v0 = v8;
     c = load_or_zero(uv + g + 32, more);
-    rank = more ? __ldg(b.rank + g + 32) : -1;
+    rank = more ? b.rank[g + 32] : -1;
     v8 = load_or_zero(vals + (g + 32) * b.P, more && v32);
     if (rank0 < 0) continue;
     int mx, sx, my, sy;

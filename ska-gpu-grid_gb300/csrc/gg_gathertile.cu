@@ -107,10 +107,10 @@ __device__ __forceinline__ void gt_store(const JobDesc &J, int gx, int gy, int p
 __device__ __forceinline__ void gt_record(const GatherTileLaunch &p, int k, int plane, int2 &q,
                                           float2 &v) {
   if (p.vals) {
-    q = __ldg(p.idx + k);
-    v = __ldg(p.vals + plane * p.vstride + k);
+    q = p.idx[k];
+    v = p.vals[plane * p.vstride + k];
   } else {
-    const float4 t = __ldg(reinterpret_cast<const float4 *>(p.idx) + k);
+    const float4 t = reinterpret_cast<const float4 *>(p.idx)[k];
     q = make_int2(__float_as_int(t.x), __float_as_int(t.y));
     v = make_float2(t.z, t.w);
   }
@@ -200,8 +200,8 @@ __device__ __forceinline__ void gt_blocks(const GatherTileLaunch &p, unsigned ch
     int beg = 0, end = 0;
     if (lane < 4 && by + lane < J.ntx) {
       const int *const bm = J.bookmarks + (by + lane) * J.ntx;
-      beg = __ldg(bm + bx);
-      end = __ldg(bm + min(bx + 4, J.ntx));
+      beg = bm[bx];
+      end = bm[min(bx + 4, J.ntx)];
     }
     // the ranges as one list: record t of it is record t + shift[r] of the
     // sorted ones, r the last range with start[r] <= t

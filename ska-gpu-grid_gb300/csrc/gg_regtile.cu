@@ -112,10 +112,10 @@ template <int I, int N, class F> __device__ __forceinline__ void rt_for(F &&f) {
 __device__ __forceinline__ void rt_record(const RegTileLaunch &p, int k, int plane, int2 &q,
                                           float2 &v) {
   if (p.vals) {
-    q = __ldg(p.idx + k);
-    v = __ldg(p.vals + plane * p.vstride + k);
+    q = p.idx[k];
+    v = p.vals[plane * p.vstride + k];
   } else {
-    const float4 t = __ldg(reinterpret_cast<const float4 *>(p.idx) + k);
+    const float4 t = reinterpret_cast<const float4 *>(p.idx)[k];
     q = make_int2(__float_as_int(t.x), __float_as_int(t.y));
     v = make_float2(t.z, t.w);
   }
@@ -222,7 +222,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
     return c;
   };
   auto range = [&](int it) {
-    return it < total ? __ldg(reinterpret_cast<const int4 *>(p.items + (P == 1 ? it : it / P)))
+    return it < total ? *reinterpret_cast<const int4 *>(p.items + (P == 1 ? it : it / P))
                       : make_int4(0, 0, 0, 0);
   };
   constexpr int PER = kRtBlock / 32;
@@ -247,7 +247,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
     claim = claim_one();
     const int4 nxt2 = range(next2);
     const int item = P == 1 ? unit : unit / P, plane = unit - item * P;
-    const int4 tail = __ldg(reinterpret_cast<const int4 *>(p.items + item) + 1);  // {slot, ox, oy}
+    const int4 tail = reinterpret_cast<const int4 *>(p.items + item)[1];  // {slot, ox, oy}
     const JobDesc &J = p.jobs[cur.x];
     const int N = J.N;
     const bool other = J.out_f64 || J.planar;
