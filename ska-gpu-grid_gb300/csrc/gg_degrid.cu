@@ -17,16 +17,19 @@
 //  * Rows are taken four at a time: their cells and factors are loaded, then
 //    summed.  Factors without imaginary parts, as a warp sees them, take one
 //    packed multiply-add per tap instead of two.
-//  * FP32 values with GG_ACC_COMPENSATED: runs of four taps are summed plainly
-//    and added into a two-sum (hi, lo) pair, which the reduction over the
+//  * FP32 values with GG_ACC_COMPENSATED: every tap by a table with imaginary
+//    parts, and every two taps by one without together with what their own sum
+//    lost, are added into a two-sum (hi, lo) pair, which the reduction over the
 //    lanes carries; else plain FP32 sums.  FP64 values: FP64 sums.
 //  * The reduction splits the components first: one lane of a pair goes on with
 //    the real, the other with the imaginary parts, which halves its shuffles.
 //
-// 4.19 M visibilities of support 8 from a 4096^2 grid: 658 us at 131 warp
-// instructions a visibility before, 328 us at 65 now (25 less without the test
-// for sums that are not finite).  With the table in shared memory (one CTA of
-// 1024 threads): 6 % less above 1.5 M visibilities, more below: not taken.
+// 4.19 M visibilities of support 8 from a 4096^2 grid: 664 us with a two-sum for
+// every tap and the index step in every lane, 372 now.  Errors against 64 bits
+// of that case: 3.6e-8 and 3.1e-8 (rms, relative).  Runs of four taps summed
+// plainly take 328 us, but 4.7e-8: not taken.  With the table in shared memory
+// (one CTA of 1024 threads): 6 % less above 1.5 M visibilities, more below: not
+// taken.
 #include <type_traits>
 
 #include "gg_kernels.cuh"
@@ -94,6 +97,7 @@ __global__ void __launch_bounds__(256, kDegridCtas) degrid_kernel(const __grid_c
   const size_t NN = (size_t)d.N * d.N;
   const int N = d.N, GG = d.G * d.G;
   const VT2 *const tabs = reinterpret_cast<const VT2 *>(d.gcf) + sl;
+  const u64 minus_one = pk2(-1.f, -1.f);
   // Few visibilities: every warp an equal share, in steps of VPW (160 k of
   // support 8: 20.4 -> 17.9 us, 10 k of support 16 24 -> 9.8).  From four groups
   // of 32 a warp on, the groups go round the warps: neighbouring ones share
@@ -137,7 +141,12 @@ __global__ void __launch_bounds__(256, kDegridCtas) degrid_kernel(const __grid_c
       const int sy = GK == 1 ? (k < 0 ? 0 : k / d.G) : 0;
       const float gx = GK == 1 ? g1[(k < 0 ? 0 : k - sy * d.G) * S + sl] : 0.f;
       for (int p = 0; p < d.P; ++p) {
-        u64 run = 0ull, hi = 0ull, lo = 0ull;  // FP32
+        u64 run = 0ull, hi = 0ull, lo = 0ull;  // FP32: plain, or (hi, lo)
+        auto put = [&](u64 t) {
+          u64 e;
+          hi = two_sum2(hi, t, e);
+          lo = add2(lo, e);
+        };
         VT re = 0, im = 0;                     // FP64
         bool force = false;
         rows:
@@ -189,14 +198,21 @@ __global__ void __launch_bounds__(256, kDegridCtas) degrid_kernel(const __grid_c
             for (int b = 0; b < R; ++b) {
               // grid * conj(w)
               if constexpr (F32) {
-                run = fma2(pk2(c[b].x, c[b].y), pk2(w[b].x, w[b].x), run);
-                if constexpr (!decltype(real)::value)
-                  run = fma2(pk2(c[b].y, -c[b].x), pk2(w[b].y, w[b].y), run);
-                if (COMP && (b & 3) == 3) {
-                  u64 e;
-                  hi = two_sum2(hi, run, e);
-                  lo = add2(lo, e);
-                  run = 0ull;
+                const u64 c1 = pk2(c[b].x, c[b].y), g1 = pk2(w[b].x, w[b].x);
+                if constexpr (!COMP) {
+                  run = fma2(c1, g1, run);
+                  if constexpr (!decltype(real)::value)
+                    run = fma2(pk2(c[b].y, -c[b].x), pk2(w[b].y, w[b].y), run);
+                } else if constexpr (decltype(real)::value) {
+                  if (b & 1) continue;
+                  // two taps t, and what their sum lost: of -t + c1 g1 + c2 g2 only
+                  // the first addition rounds to the size of a tap
+                  const u64 c2 = pk2(c[b + 1].x, c[b + 1].y), g2 = pk2(w[b + 1].x, w[b + 1].x);
+                  const u64 t = fma2(c2, g2, mul2(c1, g1));
+                  put(t);
+                  lo = add2(lo, fma2(c2, g2, fma2(c1, g1, mul2(t, minus_one))));
+                } else {
+                  put(fma2(pk2(c[b].y, -c[b].x), pk2(w[b].y, w[b].y), mul2(c1, g1)));
                 }
               } else {
                 re += c[b].x * w[b].x;
