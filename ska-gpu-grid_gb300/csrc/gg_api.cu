@@ -219,6 +219,7 @@ struct Plan {
     int T, W, chunk; // tile, warps per sub-grid group (0: by support), records per item
     ClassKind kind;
     int blocks;      // output blocks (kSep) or pieces to clear, see JobDesc::blk0
+    int64_t tables;  // whose largest magnitudes are wanted (kTab)
   };
   std::vector<ClassRange> classes;
   std::vector<JobDesc> hjobs;
@@ -248,9 +249,10 @@ struct Plan {
   size_t o_merge[kMaxClasses] = {}, o_mdesc[kMaxClasses] = {};
   int merge_cap[kMaxClasses] = {}, merge_cells[kMaxClasses] = {};
   // workspace carve (offsets into the device workspace)
-  size_t o_jobs, o_bin, o_visb, o_tileb, o_class, o_rank, o_cnt, o_bm, o_scan, o_sidx, o_svals, o_order, o_items, o_kept, o_lo,
-      o_count_vals, o_count_gcf, ws_bytes;
+  size_t o_jobs, o_bin, o_visb, o_tileb, o_class, o_rank, o_cnt, o_bm, o_scan, o_sidx, o_svals,
+      o_order, o_items, o_kept, o_lo, o_gcf_max, o_count_vals, o_count_gcf, ws_bytes;
   int64_t vstride = 0, class_cap = 0;
+  size_t gcf_max_n = 0;    // tables whose largest magnitudes are wanted
   size_t table_bytes = 0;  // bytes uploaded from staging (jobs..class)
   char *ws = nullptr;      // workspace the addresses are bound to
 };
@@ -457,7 +459,7 @@ static ClassKind regtile_class(const gg_options *o, const gg_job *jobs, int njob
 // one: 10 k records on 256^2 41.2 us, with 128 42.6) and 128 for support 16
 // (every item of a cut tile adds 529 cells into its merge slot: 100 k records
 // on 777^2 72 us, with 64 97).
-constexpr int kRegChunkMax = 512, kRegItemsPerSm = 16 * 4;
+constexpr int kRegChunkMax = 512, kRegChunkLimit = 4096, kRegItemsPerSm = 16 * 4;
 static int regtile_chunk_min(int S) { return S == 8 ? 64 : 128; }
 static int regtile_chunk(int64_t vis, int S, int sm_count) {
   const int64_t c = vis / ((int64_t)sm_count * kRegItemsPerSm);
@@ -594,6 +596,8 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
         cf.auto_chunk = true;
       }
       if (cf.chunk == 0) cf.chunk = 2048;
+      // the remainders of a register tile's sums grow with the item's length
+      if (cf.kind == kReg || cf.kind == kTab) cf.chunk = std::min(cf.chunk, kRegChunkLimit);
       cfgs[S] = cf;
     }
     pl.T = cfgs.begin()->second.T;
@@ -769,6 +773,23 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     }
     pl.o_gcf_flags = take(sizeof(int) * (pl.gcf_copies.size() + 1));
   }
+  // register tiles that read several tables, compensated: a float per table,
+  // once for jobs that share them (k -> first table, owner)
+  std::vector<std::pair<size_t, bool>> gcf_max(njobs, {SIZE_MAX, false});
+  pl.gcf_max_n = 0;
+  if (pl.accum == GG_ACC_COMPENSATED) {
+    std::map<std::tuple<const void *, int, int>, size_t> seen;
+    for (int k = 0; k < njobs; ++k) {
+      const gg_job &J = jobs[order[k]];
+      if (cfgs[(int)J.gcf_dim].kind != kTab) continue;
+      const int ntab = J.gcf_index ? (int)J.n_gcf : 1;
+      const auto it = seen.emplace(std::make_tuple((const void *)J.gcf, (int)J.gcf_dim, ntab),
+                                   pl.gcf_max_n);
+      gcf_max[k] = {it.first->second, it.second};
+      if (it.second) pl.gcf_max_n += ntab;
+    }
+  }
+  pl.o_gcf_max = pl.gcf_max_n ? take(sizeof(float) * pl.gcf_max_n) : 0;
   // merge slots: classes in ascending support, like cfgs
   if (mode == GG_MODE_WINDOW && pl.accum == GG_ACC_COMPENSATED && !pl.vals_f64) {
     int ci = 0;
@@ -818,7 +839,7 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
         pl.classes.back().t1 = tb;
       }
       const ClassCfg &cf = cfgs[S];
-      pl.classes.push_back({S, k, k, vb, vb, tb, tb, cf.T, cf.W, cf.chunk, cf.kind, 0});
+      pl.classes.push_back({S, k, k, vb, vb, tb, tb, cf.T, cf.W, cf.chunk, cf.kind, 0, 0});
     }
     const int T = pl.classes.back().T;
     const int N = (int)J.img_dim;
@@ -855,6 +876,12 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     D.sigma = pl.sigma;
     D.gcf_index = J.gcf_index;
     D.n_gcf = J.gcf_index ? (int)J.n_gcf : 1;
+    if (gcf_max[k].first != SIZE_MAX) {
+      // an offset until the workspace base is known (plan_bind)
+      D.gcf_max = reinterpret_cast<float *>(gcf_max[k].first * sizeof(float) + 1);
+      D.gcf_max_owner = gcf_max[k].second;
+      if (D.gcf_max_owner) pl.classes.back().tables += D.n_gcf;
+    }
     BinJob &B = pl.hbin[k];
     memset(&B, 0, sizeof B);
     B.uv = J.uv;
@@ -918,6 +945,7 @@ static void plan_bind(const gg_options *opt, Plan &pl, char *ws, char *host) {
   for (int k = 0; k < pl.njobs; ++k) {
     JobDesc &D = pl.hjobs[k];
     if (pl.comp_lo && D.lo) D.lo = (float *)(ws + pl.o_lo + ((size_t)D.lo - 1));
+    if (D.gcf_max) D.gcf_max = (float *)(ws + pl.o_gcf_max + ((size_t)D.gcf_max - 1));
     if (opt->gcf_kind == GG_GCF_COUNT) {
       void *cv = ws + pl.o_count_vals +
                  vbytes * (size_t)reinterpret_cast<intptr_t>(pl.count_fill[k].first);
@@ -1005,6 +1033,7 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
   // [16, 20)
   if (binned) zero.add(flags + 8, 12 * sizeof(int));
   if (!pl.gcf_copies.empty()) zero.add(ws + pl.o_gcf_flags, sizeof(int) * pl.gcf_copies.size());
+  if (pl.gcf_max_n) zero.add(ws + pl.o_gcf_max, sizeof(float) * pl.gcf_max_n);
   const bool small_out = pl.zero_ranges.size() == 1 && pl.zero_ranges[0].second <= (4u << 20);
   if (small_out) zero.add(pl.zero_ranges[0].first, pl.zero_ranges[0].second);
   GG_CUDA(launch_setup(ws, upload, upload ? pl.table_bytes : 0, zero, s));
@@ -1065,6 +1094,10 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
   g.P = pl.P;
   g.flags = flags;
   g.sm_count = sm_count;
+
+  for (const auto &cl : pl.classes)
+    if (cl.tables)
+      GG_CUDA(launch_table_max(djobs + cl.j0, cl.j1 - cl.j0, cl.S, pl.G, cl.tables, s));
 
   ItemBuffers it{};
   if (binned) {

@@ -310,13 +310,13 @@ __device__ __forceinline__ void after_predecessor() {
 }
 
 template <class... P, class... A>
-cudaError_t launch_overlapped(void (*kern)(P...), unsigned blocks, unsigned threads, size_t smem,
+cudaError_t launch_overlapped(void (*kern)(P...), dim3 blocks, unsigned threads, size_t smem,
                               cudaStream_t s, bool overlap, const A &...args) {
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(blocks);
+  cfg.gridDim = blocks;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;

@@ -150,7 +150,7 @@ cudaError_t launch_merge_finalize(const MergeSlots &m, const int *heavy_counter,
 // injection behind gg_debug_inject_device_flags.
 cudaError_t launch_inject_flags(int *flags, int bits, cudaStream_t s);
 // Up to kMaxZero ranges of device memory (4-byte aligned) to clear.
-constexpr int kMaxZero = 7;
+constexpr int kMaxZero = 8;
 struct ZeroRanges {
   void *p[kMaxZero];
   size_t bytes[kMaxZero];
@@ -263,6 +263,10 @@ struct RegTileLaunch {
   int overlap;             // table fill while the binning ends (launch_overlapped)
 };
 cudaError_t launch_regtile(const RegTileLaunch &g, cudaStream_t s);
+// Largest magnitudes of the tables of a class's jobs (of `tables` in all) into
+// JobDesc::gcf_max, zeroed before.
+cudaError_t launch_table_max(const JobDesc *jobs, int njobs, int S, int G, int64_t tables,
+                             cudaStream_t s);
 // Support 32 with the on-the-fly Gaussian, FP32 values (gg_septile.cu): one
 // launch over the 16x16 output blocks of all jobs of a class.
 struct SepTileLaunch {

@@ -16,8 +16,9 @@
 //    of each pair (j, j + S/LY), j < 8/LY, the first when fy <= LY j + ly and
 //    the second otherwise.  The records of a block are therefore put in order
 //    of fy (a counting sort of up to kRtBlock records in shared memory): while
-//    fy stays the same a lane adds to one cell of each pair in a running sum,
-//    which goes to the right cell when fy changes.
+//    fy stays the same a lane adds to one cell of each pair, and the two change
+//    places when fy passes their row (plain sums: a running sum goes to the
+//    right cell when fy changes).
 //  * Columns.  Support 8: table rows sit behind eight zeros in shared memory,
 //    so the four columns of a lane are read at fixed offsets and those outside
 //    the footprint read zero.  Support 16, whose table reads would bind: of
@@ -29,8 +30,14 @@
 //    NaN in cells its footprint does not cover.  A sub-grid that is not finite
 //    at the end of its item is therefore summed again cell by cell, only
 //    inside footprints.
-//  * Compensated sums: a run of at most kRtRun records is summed plainly,
-//    then added into the cell's (hi, lo) pair by TwoSum.
+//  * Compensated sums: every cell's sum starts at a power of two and a half so
+//    large that the item's terms do not lead out of its binade, which makes
+//    what an addition rounds off exact to work out (rt_add2): three packed
+//    operations a term, taken two at a time, where a TwoSum of each takes eight.
+//    No term is ever added to another plainly.  Runs of 16 summed plainly
+//    between TwoSums, as it was, take one and a half, but made the error of
+//    the sums larger than window_kernel's (in the listed sizes below up to 1.3
+//    times; now 0.54 to 0.87 times).
 //  * The records of a block are fetched while the previous block (also of the
 //    previous plane or item) is summed.
 //  * Real and imaginary parts of the table are kept apart; an item of a table
@@ -42,21 +49,22 @@
 // regtile_tables_kernel, complex entries as the caller keeps them.  There the
 // planes of an item are units of their own, next to each other, and the warps
 // that sum them keep in step (where their number divides the CTA's warps), so
-// that all but the first find a record's sub-kernel (2 KB for support 16) in
-// L1: 80 % of the sectors, 42 % without.  Bound by the latency of the rest,
-// which one record of lookahead does not cover (48 % of cycles issue; fetching
-// the lines of the next 8 to 32 records into L1 cost more than it hid).  524 k
-// records of 4 planes and 32 tables of support 16 on 2048^2, whole call:
-// window_kernel 880 us, planes out of step 808, in step 746.
+// that all but the first find a record's sub-kernel (2 KB for support 16) in L1.
+// 524 k records of 4 planes and 32 tables of support 16 on 2048^2, whole call,
+// and error against 64 bits: window_kernel 878 us, 9.2e-8; plain runs of 16 735,
+// 1.2e-7; now 825, 8.0e-8 (with 12 warps a CTA instead of 8, whose registers
+// spill, 910; two records at once 850).
 //
-// Bound by instruction issue (60-64 % of active cycles issue; 39 and 79 warp
-// instructions a record for supports 8 and 16 on the batched tracks, about
-// half of them sorting, TwoSum and flushes of small tiles).  Measured against
-// window_kernel on the same jobs: 4.19 M support-8 records of a 4096^2
-// observation 435 -> 247 us; 256 mixed jobs, 24.4 M support-8 records 1366 ->
-// 1311 us, 20.9 M support-16 records 3189 -> 2141 us; 10 k support-8 records
-// on 256^2 36 -> 13 us; 100 k support-16 records on 777^2, whole call, 135 ->
-// 68 us.
+// Bound by the FMA pipe and its latency: support 16, 2.1 M records of tracks, 62 %
+// of the heavy half's cycles, 61 % of the issue slots, 113 warp instructions a
+// record with 12 warps an SM (8 warps without spills: the same for large jobs, 93
+// instead of 78 us for 100 k records on 777^2).  Whole calls against
+// window_kernel, us, and errors against 64 bits:
+//   4.19 M records of support 8 on 4096^2     590 -> 383   5.4e-8 -> 4.6e-8
+//   10 k of support 8 on 256^2                 86 -> 32    8.0e-8 -> 4.3e-8
+//   100 k of support 16 on 777^2              124 -> 78    7.3e-8 -> 5.3e-8
+//   256 mixed jobs, 45 M records             6481 -> 5476  7.8e-8 -> 5.6e-8
+// (plain runs of 16: 356, 32, 68 and 4429 us with 7.1e-8, 7.5e-8, 9.1e-8, 9.0e-8).
 #include <algorithm>
 
 #include "gg_kernels.cuh"
@@ -65,6 +73,8 @@ namespace gg {
 
 namespace {
 
+// records between barriers of the warps that keep in step, and the most that
+// are summed in a plain run (GG_ACC_PLAIN)
 constexpr int kRtRun = 16;
 // records sorted together: four per lane
 constexpr int kRtBlock = 128;
@@ -82,7 +92,7 @@ template <int S, bool GT> struct RtCfg {
   // and last column, which are complementary
   static constexpr bool PADX = S == 8 && !GT;
   static constexpr int NL = PADX ? NX : NX - 1;  // loads per row
-  static constexpr int WARPS = S == 8 ? 16 : 12;
+  static constexpr int WARPS = S == 8 ? 16 : GT ? 8 : 12;
   static constexpr int ENTRY = GT ? 8 : 4;    // bytes of a table entry
   static constexpr int ROW = GT ? 8 * S : regtile_row(S);  // of a table row
   static constexpr int PAD = GT ? 0 : regtile_pad(S);      // before its first tap
@@ -127,6 +137,32 @@ template <int S> __device__ __forceinline__ const float2 *rt_table(const JobDesc
          (size_t)(J.n_gcf > 1 ? bin % J.n_gcf : 0) * J.G * J.G * S * S;
 }
 
+// Compensated sums.  A cell's sum starts at `base`, a number so large that no
+// sum of the item's terms leads out of its binade: every addition then rounds
+// to the same unit, and what it rounded off is exact to work out.  Two terms
+// va ga + vb gb go into the sum A and what A lost of them into l; of their
+// remainders only one intermediate rounds, to the size of vb gb.  Six packed
+// operations for two terms, where a two-sum of each takes 16.
+__device__ __forceinline__ void rt_add2(u64 &A, u64 &l, u64 va, u64 ga, u64 vb, u64 gb) {
+  const u64 n = fma2(vb, gb, fma2(va, ga, A));
+  l = add2(l, fma2(vb, gb, fma2(va, ga, sub2(A, n))));
+  A = n;
+}
+
+// finite magnitude as ordered bits, 0 for an infinity or NaN (those end up in
+// the sums all the same)
+__device__ __forceinline__ unsigned rt_magnitude(float x) {
+  const unsigned b = __float_as_uint(x) & 0x7fffffffu;
+  return b < 0x7f800000u ? b : 0u;
+}
+
+// 1.5 * 2^k, 2^k at least `need` (not finite if need is too large: the sums then
+// are not either, and are worked out again cell by cell)
+__device__ __forceinline__ float rt_base(float need) {
+  const unsigned b = __float_as_uint(fminf(fmaxf(need, 0x1p-124f), 0x1p127f));
+  return __uint_as_float((b & 0x7f800000u) + 0x00c00000u);
+}
+
 // The sub-grid of an item whose packed sums are not finite, cell by cell and
 // only from the records whose footprints cover the cell.
 template <int S, bool COMP, bool GT>
@@ -142,13 +178,11 @@ __device__ __noinline__ void rt_redo(const RegTileLaunch &p, const WorkItem &w, 
     const int gx = w.ox + x, gy = w.oy + y;
     if ((unsigned)gx >= (unsigned)J.N || (unsigned)gy >= (unsigned)J.N) continue;
     u64 run = 0ull, hi = 0ull, lo = 0ull;
-    int since = 0;
     auto merge = [&]() {
       u64 e;
       hi = two_sum2(hi, run, e);
       lo = add2(lo, e);
       run = 0ull;
-      since = 0;
     };
     for (int k = w.start; k < w.end; ++k) {
       int2 q;
@@ -163,9 +197,8 @@ __device__ __noinline__ void rt_redo(const RegTileLaunch &p, const WorkItem &w, 
       else g = make_float2(tr[at], cplx ? ti[at] : 0.f);
       run = fma2(pk2(v.x, v.y), pk2(g.x, g.x), run);
       if (cplx) run = fma2(pk2(-v.y, v.x), pk2(g.y, g.y), run);
-      if (COMP && ++since == kRtRun) merge();
+      if (COMP) merge();
     }
-    if (COMP) merge();
     const float2 h = upk2(COMP ? hi : run), l = upk2(lo);
     if (slot) {
       red_add(&slot[c].x, (double)h.x + (double)l.x);
@@ -184,7 +217,7 @@ __device__ __noinline__ void rt_redo(const RegTileLaunch &p, const WorkItem &w, 
 // of an item next to each other (they read the same records and table rows).
 template <int S, bool COMP, bool GT>
 __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr, float4 *stage,
-                                         bool cplx) {
+                                         bool cplx, float gmax) {
   using C = RtCfg<S, GT>;
   constexpr int LX = C::LX, LY = C::LY, NX = C::NX, NY = C::NY, R = C::R, Q = C::Q,
                 PAIRS = C::PAIRS;
@@ -253,40 +286,85 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
     const bool other = J.out_f64 || J.planar;
     float2 *const out = static_cast<float2 *>(J.out);
     const char *gt = nullptr;  // this lane's entry under the sub-grid's first cell
-    if constexpr (GT)
+    float factor_max = gmax;
+    if constexpr (GT) {
       gt = reinterpret_cast<const char *>(rt_table<S>(J, cur.y)) + lx * 8 + ly * C::ROW;
+      if constexpr (COMP) factor_max = J.gcf_max[J.n_gcf > 1 ? cur.y % J.n_gcf : 0];
+    }
     do {  // once; `break` ends the unit
-      // cells: (hi, lo) pairs, or plain sums in hi; run: the running sums of
-      // the rows that the current fy selects
-      u64 run[NX][Q], hi[NX][NY], lo[COMP ? NX : 1][COMP ? NY : 1];
+      // Cells.  Compensated: sums in hi from `base` on and their remainders in
+      // lo; of a pair, the cell that the current fy selects at j, the other at
+      // j + Q.  Plain: sums in hi, and in run the running sums of the rows that
+      // the current fy selects or every footprint covers.
+      u64 hi[NX][NY], lo[COMP ? NX : 1][COMP ? NY : 1], run[COMP ? 1 : NX][COMP ? 1 : Q];
+      u64 base = 0ull;
+      float room = 0.f;  // bound on the item's sums that `base` is good for
+      auto clear = [&]() {
 #pragma unroll
-      for (int i = 0; i < NX; ++i) {
+        for (int i = 0; i < NX; ++i) {
 #pragma unroll
-        for (int j = 0; j < NY; ++j) {
-          hi[i][j] = 0ull;
-          if constexpr (COMP) lo[i][j] = 0ull;
-        }
+          for (int j = 0; j < NY; ++j) {
+            hi[i][j] = base;
+            if constexpr (COMP) lo[i][j] = 0ull;
+          }
+          if constexpr (!COMP) {
 #pragma unroll
-        for (int j = 0; j < Q; ++j) run[i][j] = 0ull;
-      }
-      auto put = [&](int i, int j, u64 r) {
-        if constexpr (COMP) {
-          u64 e;
-          hi[i][j] = two_sum2(hi[i][j], r, e);
-          lo[i][j] = add2(lo[i][j], e);
-        } else {
-          hi[i][j] = add2(hi[i][j], r);
+            for (int j = 0; j < Q; ++j) run[i][j] = 0ull;
+          }
         }
       };
-      // the running sums of the alternating rows into the cells of fy = f
+      if constexpr (!COMP) clear();
+      // a base for the terms of a block: room for twice what the item would take
+      // if all its values were this large, and the sums moved when a later
+      // block needs more
+      auto rebase = [&](float need) {
+        const float b = rt_base(2.f * need);
+        const u64 old = base;
+        base = pk2(b, b);
+        if (room == 0.f) {
+          clear();
+        } else {
+#pragma unroll
+          for (int i = 0; i < NX; ++i)
+#pragma unroll
+            for (int j = 0; j < NY; ++j) {
+              const u64 t = sub2(hi[i][j], old), n = add2(t, base);
+              lo[i][j] = add2(lo[i][j], sub2(t, sub2(n, base)));
+              hi[i][j] = n;
+            }
+        }
+        room = b * (1.f / 1.5f);
+      };
+      // compensated: the cells of fy = f to the first place of their pairs (the
+      // second of a pair is selected once fy > LY j + ly)
+      int at_fy = 0;
+      auto select = [&](int f) {
+#pragma unroll
+        for (int j = 0; j < PAIRS; ++j) {
+          if (min(at_fy, f) >= LY * (j + 1) || max(at_fy, f) <= LY * j) continue;
+          const bool change = (LY * j + ly < at_fy) != (LY * j + ly < f);
+          auto exchange = [&](u64 &a, u64 &b) {
+            const u64 t = change ? b : a;
+            b = change ? a : b;
+            a = t;
+          };
+#pragma unroll
+          for (int i = 0; i < NX; ++i) {
+            exchange(hi[i][j], hi[i][j + Q]);
+            exchange(lo[i][j], lo[i][j + Q]);
+          }
+        }
+        at_fy = f;
+      };
+      // plain: the running sums of the alternating rows into the cells of fy = f
       auto merge_pairs = [&](int f) {
 #pragma unroll
         for (int j = 0; j < PAIRS; ++j) {
           const bool low = f <= LY * j + ly;
 #pragma unroll
           for (int i = 0; i < NX; ++i) {
-            put(i, j, low ? run[i][j] : 0ull);
-            put(i, j + Q, low ? 0ull : run[i][j]);
+            hi[i][j] = add2(hi[i][j], low ? run[i][j] : 0ull);
+            hi[i][j + Q] = add2(hi[i][j + Q], low ? 0ull : run[i][j]);
             run[i][j] = 0ull;
           }
         }
@@ -297,7 +375,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
         for (int j = PAIRS; j < Q; ++j)
 #pragma unroll
           for (int i = 0; i < NX; ++i) {
-            put(i, j, run[i][j]);
+            hi[i][j] = add2(hi[i][j], run[i][j]);
             run[i][j] = 0ull;
           }
       };
@@ -307,35 +385,27 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
         float vr, vi;
         bool left;  // the first column, not the last, is in the footprint
       };
-      auto load = [&](Taps &t, const float4 q, auto cx) {
+      // the factors of one of a lane's rows
+      auto load_row = [&](Taps &t, const float4 q, auto cx, auto JJ) {
+        constexpr int j = decltype(JJ)::value;
         const int at = __float_as_int(q.y);
         const int fy = C::PADX ? at : at & 0xff;
-        t.vr = q.z;
-        t.vi = q.w;
-        t.left = at < (lx + 1) << 8;
+        const bool left = at < (lx + 1) << 8;
         if constexpr (GT) {
-          const char *const b = gt + __float_as_int(q.x);
-          const int side = t.left ? 0 : C::ROW;
-          rt_for<0, Q>([&](auto JJ) {
-            constexpr int j = decltype(JJ)::value;
-            const char *a = b;
-            if (j < PAIRS && fy > ly + LY * j) a = b + C::SUB;
-            rt_for<0, C::NL>([&](auto II) {
-              constexpr int i = decltype(II)::value;
-              const float2 w = __ldg(reinterpret_cast<const float2 *>(
-                  (i == 0 ? a + side : a) + (j * LY * C::ROW + i * LX * 8)));
-              t.g[j][i] = w.x;
-              t.h[j][i] = w.y;
-            });
+          const char *a = gt + __float_as_int(q.x);
+          if (j < PAIRS && fy > ly + LY * j) a += C::SUB;
+          const int side = left ? 0 : C::ROW;
+          rt_for<0, C::NL>([&](auto II) {
+            constexpr int i = decltype(II)::value;
+            const float2 w = __ldg(reinterpret_cast<const float2 *>(
+                (i == 0 ? a + side : a) + (j * LY * C::ROW + i * LX * 8)));
+            t.g[j][i] = w.x;
+            t.h[j][i] = w.y;
           });
-          return;
-        }
-        const uint32_t b = tab + (uint32_t)__float_as_int(q.x);
-        const uint32_t side = C::PADX || t.left ? 0 : 64;
-        rt_for<0, Q>([&](auto JJ) {
-          constexpr int j = decltype(JJ)::value;
-          uint32_t a = b;
-          if (j < PAIRS && fy > ly + LY * j) a = b + C::SUB;
+        } else {
+          uint32_t a = tab + (uint32_t)__float_as_int(q.x);
+          if (j < PAIRS && fy > ly + LY * j) a += C::SUB;
+          const uint32_t side = C::PADX || left ? 0 : 64;
           rt_for<0, C::NL>([&](auto II) {
             constexpr int i = decltype(II)::value;
             constexpr int OFF = j * LY * C::ROW + i * LX * 4;
@@ -343,27 +413,78 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
             t.g[j][i] = lds<OFF>(ai);
             if constexpr (decltype(cx)::value) t.h[j][i] = lds<OFF>(ai + im_off);
           });
-        });
+        }
+      };
+      auto load_value = [&](Taps &t, const float4 q) {
+        t.vr = q.z;
+        t.vi = q.w;
+        t.left = __float_as_int(q.y) < (lx + 1) << 8;
+      };
+      auto load = [&](Taps &t, const float4 q, auto cx) {
+        load_value(t, q);
+        rt_for<0, Q>([&](auto JJ) { load_row(t, q, cx, JJ); });
+      };
+      // a value in the outer columns, of which the footprint covers one
+      auto at_column = [&](u64 v, bool left, auto II) {
+        constexpr int i = decltype(II)::value;
+        if constexpr (C::PADX || (i > 0 && i < NX - 1)) return v;
+        else return (i == 0) == left ? v : 0ull;
+      };
+      // terms va ga + vb gb into the sums of row j, column i
+      auto add_two = [&](auto JJ, auto II, u64 va, u64 ga, u64 vb, u64 gb) {
+        constexpr int j = decltype(JJ)::value, i = decltype(II)::value;
+        if constexpr (COMP) rt_add2(hi[i][j], lo[i][j], va, ga, vb, gb);
+        else run[i][j] = fma2(vb, gb, fma2(va, ga, run[i][j]));
       };
       auto add = [&](const Taps &t, auto cx) {
-        auto columns = [&](u64 v, const float(&g)[Q][C::NL]) {
-          const u64 v0 = C::PADX || t.left ? v : 0ull, v2 = t.left ? 0ull : v;
-          rt_for<0, Q>([&](auto JJ) {
-            constexpr int j = decltype(JJ)::value;
-            rt_for<0, NX>([&](auto II) {
-              constexpr int i = decltype(II)::value;
-              constexpr bool outer = !C::PADX && (i == 0 || i == NX - 1);
-              constexpr int l = outer ? 0 : i;
-              run[i][j] = fma2(!outer ? v : (i == 0 ? v0 : v2), pk2(g[j][l], g[j][l]), run[i][j]);
-            });
+        const u64 v = pk2(t.vr, t.vi), w = pk2(-t.vi, t.vr);
+        rt_for<0, Q>([&](auto JJ) {
+          constexpr int j = decltype(JJ)::value;
+          rt_for<0, NX>([&](auto II) {
+            constexpr int i = decltype(II)::value, l = C::PADX || (i > 0 && i < NX - 1) ? i : 0;
+            const u64 vi = at_column(v, t.left, II), g2 = pk2(t.g[j][l], t.g[j][l]);
+            if constexpr (decltype(cx)::value)
+              add_two(JJ, II, vi, g2, at_column(w, t.left, II), pk2(t.h[j][l], t.h[j][l]));
+            else run[i][j] = fma2(vi, g2, run[i][j]);
           });
-        };
-        columns(pk2(t.vr, t.vi), t.g);
-        if constexpr (decltype(cx)::value) columns(pk2(-t.vi, t.vr), t.h);
+        });
       };
       // the staged records of a block in order of fy, cnt[f] of them (bytes;
-      // even numbers) for each, the table entries of one loaded while the
-      // previous one is added
+      // even numbers) for each.  Compensated, two at a time by tables without
+      // imaginary parts: a row's factors of the next two are loaded once it has
+      // been added.
+      auto add_block_by_two = [&](u64 cnt, auto cx) {
+        Taps a, b;
+        load(a, stage[0], cx);
+        load(b, stage[1], cx);
+        const float4 *st = stage + 2;
+#pragma unroll 1
+        for (int f = 0; f < 8; ++f) {
+          const float4 *const end = st + ((int)(cnt >> (8 * f)) & 0xff);
+          if (st == end) continue;
+          select(f);
+#pragma unroll 1
+          do {
+            const float4 qa = st[0], qb = st[1];
+            const u64 va = pk2(a.vr, a.vi), vb = pk2(b.vr, b.vi);
+            rt_for<0, Q>([&](auto JJ) {
+              constexpr int j = decltype(JJ)::value;
+              rt_for<0, NX>([&](auto II) {
+                constexpr int i = decltype(II)::value, l = C::PADX || (i > 0 && i < NX - 1) ? i : 0;
+                add_two(JJ, II, at_column(va, a.left, II), pk2(a.g[j][l], a.g[j][l]),
+                        at_column(vb, b.left, II), pk2(b.g[j][l], b.g[j][l]));
+              });
+              load_row(a, qa, cx, JJ);
+              load_row(b, qb, cx, JJ);
+            });
+            load_value(a, qa);
+            load_value(b, qb);
+            st += 2;
+          } while (st != end);
+        }
+      };
+      // The others one at a time, the table entries of one loaded while the
+      // previous one is added.
       auto add_block = [&](u64 cnt, auto cx) {
         Taps a, b;
         load(a, stage[0], cx);
@@ -373,6 +494,8 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
 #pragma unroll 1
         for (int f = 0; f < 8; ++f) {
           int left = (int)(cnt >> (8 * f)) & 0xff;
+          if constexpr (COMP)
+            if (left > 0) select(f);
 #pragma unroll 1
           while (left > 0) {
             const int m = min(left, kRtRun);
@@ -389,15 +512,17 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
               st += 2;
             }
             left -= m;
-            since += m;
-            merge_pairs(f);
-            if (PAIRS < Q && since >= kRtRun) {
-              merge_rest();
-              since = 0;
+            if constexpr (!COMP) {
+              merge_pairs(f);
+              since += m;
+              if (PAIRS < Q && since >= kRtRun) {
+                merge_rest();
+                since = 0;
+              }
             }
           }
         }
-        if (PAIRS < Q) merge_rest();
+        if constexpr (!COMP && PAIRS < Q) merge_rest();
       };
       for (int k0 = cur.z; k0 < cur.w; k0 += kRtBlock) {
         const int n = min(kRtBlock, cur.w - k0);
@@ -407,6 +532,17 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
 #pragma unroll
         for (int u = 0; u < PER; ++u)
           if (u * 32 + lane < n) mine += 1ull << (8 * (pk[u].y & 7));
+        if constexpr (COMP) {
+          unsigned top = 0;
+#pragma unroll
+          for (int u = 0; u < PER; ++u)
+            if (u * 32 + lane < n) top = max(top, max(rt_magnitude(pv[u].x), rt_magnitude(pv[u].y)));
+          top = __reduce_max_sync(0xffffffffu, top);
+          // twice the sum of the item's terms, were all of them as large
+          const float need = (GT || cplx ? 4.f : 2.f) * (float)(cur.w - cur.z + 8) *
+                             (__uint_as_float(top) * factor_max);
+          if (room == 0.f || !(need <= room)) rebase(need);
+        }
         u64 incl = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -439,17 +575,22 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
         else fetch(nxt.z, nxt.w, P == 1 ? 0 : next % P);
         __syncwarp();
         if (GT || cplx) add_block(even, std::true_type{});
-        else add_block(even, std::false_type{});
+        else if constexpr (!GT && COMP) add_block_by_two(even, std::false_type{});
+        else if constexpr (!GT) add_block(even, std::false_type{});
       }
       const int ox = tail.y, oy = tail.z;
       double2 *const slot = COMP && p.merge.base && tail.x >= 0
                                 ? p.merge.base + (size_t)tail.x * p.merge.cells + plane * R * R
                                 : nullptr;
+      if constexpr (COMP) select(0);
       u64 z = 0ull;
 #pragma unroll
       for (int i = 0; i < NX; ++i)
 #pragma unroll
-        for (int j = 0; j < NY; ++j) z = fma2(hi[i][j], 0ull, z);
+        for (int j = 0; j < NY; ++j) {
+          if constexpr (COMP) hi[i][j] = sub2(hi[i][j], base);
+          z = fma2(hi[i][j], 0ull, z);
+        }
       const float2 zf = upk2(z);
       if (__any_sync(0xffffffffu, !(zf.x == 0.f && zf.y == 0.f))) {
         rt_redo<S, COMP, GT>(p, p.items[item], plane, tr, GT || cplx, slot);
@@ -536,7 +677,8 @@ __global__ void __launch_bounds__(32 * RtCfg<S, true>::WARPS, 1)
   extern __shared__ __align__(16) unsigned char smem[];
   after_predecessor();
   rt_items<S, COMP, true>(p, nullptr,
-                          reinterpret_cast<float4 *>(smem) + (threadIdx.x >> 5) * kRtStage, true);
+                          reinterpret_cast<float4 *>(smem) + (threadIdx.x >> 5) * kRtStage, true,
+                          0.f);
 }
 
 template <int S, bool COMP>
@@ -553,6 +695,13 @@ __global__ void __launch_bounds__(32 * RtCfg<S, false>::WARPS, 1)
   // tables: from the caller's [G*G][S][S], or the Gaussian's factors (expf as
   // everywhere; their product rounds as the on-the-fly factor does)
   int imag = 0;
+  __shared__ unsigned s_top;  // largest magnitude in the table (the Gaussian's: at most 1)
+  unsigned top = __float_as_uint(1.f);
+  if (COMP && !p.gauss) {
+    top = 0;
+    if (tid == 0) s_top = 0;
+    __syncthreads();
+  }
   if (!p.overlap) after_predecessor();
   if (p.gauss) {
     float *g1 = reinterpret_cast<float *>(smem + 8 * (size_t)nf);
@@ -576,24 +725,56 @@ __global__ void __launch_bounds__(32 * RtCfg<S, false>::WARPS, 1)
       tr[i] = v.x;
       ti[i] = v.y;
       imag |= v.y != 0.f;
+      if constexpr (COMP) top = max(top, max(rt_magnitude(v.x), rt_magnitude(v.y)));
+    }
+    if constexpr (COMP) {
+      top = __reduce_max_sync(0xffffffffu, top);
+      if ((tid & 31) == 0) atomicMax(&s_top, top);
     }
   }
   if (p.overlap) after_predecessor();
-  rt_items<S, COMP, false>(p, tr, stage, __syncthreads_or(imag));
+  const bool cplx = __syncthreads_or(imag);
+  if (COMP && !p.gauss) top = s_top;
+  rt_items<S, COMP, false>(p, tr, stage, cplx, __uint_as_float(top));
+}
+
+// Largest finite magnitude of every table of a class (blockIdx.y: jobs, those
+// that share a stack of tables once), zeroed by the caller: what the compensated
+// sums of regtile_tables_kernel choose their base by.
+__global__ void __launch_bounds__(256)
+    table_max_kernel(const JobDesc *jobs, int njobs, int entries) {
+  after_predecessor();
+  const int chunk = min(entries, 4096);
+  for (int j = blockIdx.y; j < njobs; j += gridDim.y) {
+    const JobDesc &J = jobs[j];
+    if (!J.gcf_max_owner) continue;
+    const int64_t chunks = (int64_t)J.n_gcf * (entries / chunk);
+    for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
+      const float2 *const t = static_cast<const float2 *>(J.gcf) + c * chunk;
+      unsigned top = 0;
+#pragma unroll 4
+      for (int i = threadIdx.x; i < chunk; i += 256) {
+        const float2 v = __ldg(t + i);
+        top = max(top, max(rt_magnitude(v.x), rt_magnitude(v.y)));
+      }
+      top = __reduce_max_sync(0xffffffffu, top);
+      if ((threadIdx.x & 31) == 0)
+        atomicMax(reinterpret_cast<unsigned *>(J.gcf_max + c / (entries / chunk)), top);
+    }
+  }
 }
 
 template <int S, bool COMP> cudaError_t rt_launch(const RegTileLaunch &g, cudaStream_t s) {
-  using C = RtCfg<S, false>;
-  static_assert(C::WARPS == RtCfg<S, true>::WARPS, "one launch shape");
+  const int warps = g.tables ? RtCfg<S, true>::WARPS : RtCfg<S, false>::WARPS;
   const size_t smem =
-      g.tables ? C::WARPS * kRtStage * sizeof(float4) : regtile_smem_bytes(S, g.G);
+      g.tables ? warps * kRtStage * sizeof(float4) : regtile_smem_bytes(S, g.G);
   auto kern = g.tables ? regtile_tables_kernel<S, COMP> : regtile_kernel<S, COMP>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
   const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(g.sm_count, g.max_items * g.P));
   count_launch();
-  return launch_overlapped(kern, (unsigned)blocks, 32 * C::WARPS, smem, s, g.overlap, g);
+  return launch_overlapped(kern, (unsigned)blocks, 32 * warps, smem, s, g.overlap, g);
 }
 
 }  // namespace
@@ -601,6 +782,15 @@ template <int S, bool COMP> cudaError_t rt_launch(const RegTileLaunch &g, cudaSt
 size_t regtile_smem_bytes(int S, int G) {
   const int warps = S == 8 ? RtCfg<8, false>::WARPS : RtCfg<16, false>::WARPS;
   return 8 * (size_t)rt_table_floats(S, G) + (size_t)warps * kRtStage * sizeof(float4);
+}
+
+cudaError_t launch_table_max(const JobDesc *jobs, int njobs, int S, int G, int64_t tables,
+                             cudaStream_t s) {
+  const int entries = G * G * S * S;
+  const int64_t chunks = tables * ((entries + 4095) / 4096);
+  const int y = std::min(njobs, 1024), x = (int)std::min<int64_t>(chunks, std::max(1, 2048 / y));
+  count_launch();
+  return launch_overlapped(table_max_kernel, dim3(x, y), 256, 0, s, true, jobs, njobs, entries);
 }
 
 cudaError_t launch_regtile(const RegTileLaunch &g, cudaStream_t s) {

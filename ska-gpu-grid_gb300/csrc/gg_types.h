@@ -52,6 +52,10 @@ struct JobDesc {
   // flag that is nonzero when any imaginary part is (null: not available)
   const float *gcf_real;
   const int *gcf_imag;
+  // largest magnitudes of its tables (register tiles that read several tables,
+  // compensated sums), and whether this job's launch block finds them
+  float *gcf_max;
+  int gcf_max_owner;
 };
 
 // A slice of one uv tile's sorted visibilities: the unit of the device work
