@@ -219,7 +219,7 @@ struct Plan {
     int T, W, chunk; // tile, warps per sub-grid group (0: by support), records per item
     ClassKind kind;
     int blocks;      // output blocks (kSep) or pieces to clear, see JobDesc::blk0
-    int64_t tables;  // whose largest magnitudes are wanted (kTab)
+    int64_t tables;  // whose TableInfo is wanted (kTab)
   };
   std::vector<ClassRange> classes;
   std::vector<JobDesc> hjobs;
@@ -250,9 +250,9 @@ struct Plan {
   int merge_cap[kMaxClasses] = {}, merge_cells[kMaxClasses] = {};
   // workspace carve (offsets into the device workspace)
   size_t o_jobs, o_bin, o_visb, o_tileb, o_class, o_rank, o_cnt, o_bm, o_scan, o_sidx, o_svals,
-      o_order, o_items, o_kept, o_lo, o_gcf_max, o_count_vals, o_count_gcf, ws_bytes;
+      o_order, o_items, o_kept, o_lo, o_gcf_info, o_count_vals, o_count_gcf, ws_bytes;
   int64_t vstride = 0, class_cap = 0;
-  size_t gcf_max_n = 0;    // tables whose largest magnitudes are wanted
+  size_t gcf_info_n = 0;   // tables whose TableInfo is wanted
   size_t table_bytes = 0;  // bytes uploaded from staging (jobs..class)
   char *ws = nullptr;      // workspace the addresses are bound to
 };
@@ -773,23 +773,24 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     }
     pl.o_gcf_flags = take(sizeof(int) * (pl.gcf_copies.size() + 1));
   }
-  // register tiles that read several tables, compensated: a float per table,
-  // once for jobs that share them (k -> first table, owner)
-  std::vector<std::pair<size_t, bool>> gcf_max(njobs, {SIZE_MAX, false});
-  pl.gcf_max_n = 0;
-  if (pl.accum == GG_ACC_COMPENSATED) {
+  // register tiles that read several tables: what is known of each, once for
+  // jobs that share them (k -> first table, owner)
+  std::vector<std::pair<size_t, bool>> gcf_info(njobs, {SIZE_MAX, false});
+  pl.gcf_info_n = 0;
+  {
     std::map<std::tuple<const void *, int, int>, size_t> seen;
     for (int k = 0; k < njobs; ++k) {
       const gg_job &J = jobs[order[k]];
       if (cfgs[(int)J.gcf_dim].kind != kTab) continue;
       const int ntab = J.gcf_index ? (int)J.n_gcf : 1;
       const auto it = seen.emplace(std::make_tuple((const void *)J.gcf, (int)J.gcf_dim, ntab),
-                                   pl.gcf_max_n);
-      gcf_max[k] = {it.first->second, it.second};
-      if (it.second) pl.gcf_max_n += ntab;
+                                   pl.gcf_info_n);
+      gcf_info[k] = {it.first->second, it.second};
+      if (it.second) pl.gcf_info_n += ntab;
     }
   }
-  pl.o_gcf_max = pl.gcf_max_n ? take(sizeof(float) * pl.gcf_max_n) : 0;
+  // behind them a flag for every class
+  pl.o_gcf_info = pl.gcf_info_n ? take(sizeof(TableInfo) * (pl.gcf_info_n + kMaxClasses)) : 0;
   // merge slots: classes in ascending support, like cfgs
   if (mode == GG_MODE_WINDOW && pl.accum == GG_ACC_COMPENSATED && !pl.vals_f64) {
     int ci = 0;
@@ -876,11 +877,11 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     D.sigma = pl.sigma;
     D.gcf_index = J.gcf_index;
     D.n_gcf = J.gcf_index ? (int)J.n_gcf : 1;
-    if (gcf_max[k].first != SIZE_MAX) {
+    if (gcf_info[k].first != SIZE_MAX) {
       // an offset until the workspace base is known (plan_bind)
-      D.gcf_max = reinterpret_cast<float *>(gcf_max[k].first * sizeof(float) + 1);
-      D.gcf_max_owner = gcf_max[k].second;
-      if (D.gcf_max_owner) pl.classes.back().tables += D.n_gcf;
+      D.gcf_info = reinterpret_cast<TableInfo *>(gcf_info[k].first * sizeof(TableInfo) + 1);
+      D.gcf_info_owner = gcf_info[k].second;
+      if (D.gcf_info_owner) pl.classes.back().tables += D.n_gcf;
     }
     BinJob &B = pl.hbin[k];
     memset(&B, 0, sizeof B);
@@ -945,7 +946,7 @@ static void plan_bind(const gg_options *opt, Plan &pl, char *ws, char *host) {
   for (int k = 0; k < pl.njobs; ++k) {
     JobDesc &D = pl.hjobs[k];
     if (pl.comp_lo && D.lo) D.lo = (float *)(ws + pl.o_lo + ((size_t)D.lo - 1));
-    if (D.gcf_max) D.gcf_max = (float *)(ws + pl.o_gcf_max + ((size_t)D.gcf_max - 1));
+    if (D.gcf_info) D.gcf_info = (TableInfo *)(ws + pl.o_gcf_info + ((size_t)D.gcf_info - 1));
     if (opt->gcf_kind == GG_GCF_COUNT) {
       void *cv = ws + pl.o_count_vals +
                  vbytes * (size_t)reinterpret_cast<intptr_t>(pl.count_fill[k].first);
@@ -1033,7 +1034,7 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
   // [16, 20)
   if (binned) zero.add(flags + 8, 12 * sizeof(int));
   if (!pl.gcf_copies.empty()) zero.add(ws + pl.o_gcf_flags, sizeof(int) * pl.gcf_copies.size());
-  if (pl.gcf_max_n) zero.add(ws + pl.o_gcf_max, sizeof(float) * pl.gcf_max_n);
+  if (pl.gcf_info_n) zero.add(ws + pl.o_gcf_info, sizeof(TableInfo) * (pl.gcf_info_n + kMaxClasses));
   const bool small_out = pl.zero_ranges.size() == 1 && pl.zero_ranges[0].second <= (4u << 20);
   if (small_out) zero.add(pl.zero_ranges[0].first, pl.zero_ranges[0].second);
   GG_CUDA(launch_setup(ws, upload, upload ? pl.table_bytes : 0, zero, s));
@@ -1095,9 +1096,15 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
   g.flags = flags;
   g.sm_count = sm_count;
 
-  for (const auto &cl : pl.classes)
+  auto any_imag = [&](size_t ci) {
+    return &((TableInfo *)(ws + pl.o_gcf_info))[pl.gcf_info_n + ci].imag;
+  };
+  for (size_t ci = 0; ci < pl.classes.size(); ++ci) {
+    const auto &cl = pl.classes[ci];
     if (cl.tables)
-      GG_CUDA(launch_table_max(djobs + cl.j0, cl.j1 - cl.j0, cl.S, pl.G, cl.tables, s));
+      GG_CUDA(launch_table_info(djobs + cl.j0, cl.j1 - cl.j0, cl.S, pl.G, cl.tables,
+                                any_imag(ci), s));
+  }
 
   ItemBuffers it{};
   if (binned) {
@@ -1172,6 +1179,7 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
       } else if (cl.kind == kReg || cl.kind == kTab) {
         RegTileLaunch r{};
         r.tables = cl.kind == kTab;
+        r.any_imag = r.tables ? any_imag(ci) : nullptr;
         r.jobs = djobs;
         r.items = g.items;
         r.nitems = g.nitems;

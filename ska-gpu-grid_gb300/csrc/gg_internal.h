@@ -252,6 +252,7 @@ struct RegTileLaunch {
   const float2 *vals;      // sorted values, P planes of vstride
   int64_t vstride;
   int tables;              // tables read per item from the jobs' (gcf ignored)
+  const unsigned *any_imag;  // whether any of those has imaginary parts
   const float2 *gcf;       // [G*G][S][S]
   int S, G, P;
   int compensated;
@@ -263,10 +264,10 @@ struct RegTileLaunch {
   int overlap;             // table fill while the binning ends (launch_overlapped)
 };
 cudaError_t launch_regtile(const RegTileLaunch &g, cudaStream_t s);
-// Largest magnitudes of the tables of a class's jobs (of `tables` in all) into
-// JobDesc::gcf_max, zeroed before.
-cudaError_t launch_table_max(const JobDesc *jobs, int njobs, int S, int G, int64_t tables,
-                             cudaStream_t s);
+// JobDesc::gcf_info of the tables of a class's jobs (`tables` in all), and whether
+// any of them has imaginary parts; both zeroed before.
+cudaError_t launch_table_info(const JobDesc *jobs, int njobs, int S, int G, int64_t tables,
+                              unsigned *any_imag, cudaStream_t s);
 // Support 32 with the on-the-fly Gaussian, FP32 values (gg_septile.cu): one
 // launch over the 16x16 output blocks of all jobs of a class.
 struct SepTileLaunch {

@@ -46,7 +46,10 @@
 // The whole table lives in each CTA's shared memory (2 x 98 KB for support 16
 // at oversampling 8), hence one CTA per SM and one table per launch.  Several
 // tables, or one that does not fit, are read from global memory by
-// regtile_tables_kernel, complex entries as the caller keeps them.  There the
+// regtile_tables_kernel, complex entries as the caller keeps them, their
+// imaginary parts only if any table of the class has some (1.05 M records of
+// support 16 and 16 real tables on 2048^2: 372 us, as complex ones 421,
+// window_kernel 420; what the tables are like costs 5 us to find out).  There the
 // planes of an item are units of their own, next to each other, and the warps
 // that sum them keep in step (where their number divides the CTA's warps), so
 // that all but the first find a record's sub-kernel (2 KB for support 16) in L1.
@@ -163,6 +166,10 @@ __device__ __forceinline__ float rt_base(float need) {
   return __uint_as_float((b & 0x7f800000u) + 0x00c00000u);
 }
 
+__device__ __forceinline__ TableInfo rt_info(const JobDesc &J, int bin) {
+  return J.gcf_info[J.n_gcf > 1 ? bin % J.n_gcf : 0];
+}
+
 // The sub-grid of an item whose packed sums are not finite, cell by cell and
 // only from the records whose footprints cover the cell.
 template <int S, bool COMP, bool GT>
@@ -215,7 +222,10 @@ __device__ __noinline__ void rt_redo(const RegTileLaunch &p, const WorkItem &w, 
 
 // A warp's share of the launch's units: one plane of an item each, the planes
 // of an item next to each other (they read the same records and table rows).
-template <int S, bool COMP, bool GT>
+// GT: CX says whether any table of the class has imaginary parts (the products of
+// a table without them are then complex too, with the same finite sums: a choice
+// for every item cost 4 to 13 %).  cplx: whether the launch's table has, or CX.
+template <int S, bool COMP, bool GT, bool CX>
 __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr, float4 *stage,
                                          bool cplx, float gmax) {
   using C = RtCfg<S, GT>;
@@ -289,7 +299,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
     float factor_max = gmax;
     if constexpr (GT) {
       gt = reinterpret_cast<const char *>(rt_table<S>(J, cur.y)) + lx * 8 + ly * C::ROW;
-      if constexpr (COMP) factor_max = J.gcf_max[J.n_gcf > 1 ? cur.y % J.n_gcf : 0];
+      if constexpr (COMP) factor_max = __uint_as_float(rt_info(J, cur.y).top);
     }
     do {  // once; `break` ends the unit
       // Cells.  Compensated: sums in hi from `base` on and their remainders in
@@ -397,10 +407,14 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
           const int side = left ? 0 : C::ROW;
           rt_for<0, C::NL>([&](auto II) {
             constexpr int i = decltype(II)::value;
-            const float2 w = __ldg(reinterpret_cast<const float2 *>(
-                (i == 0 ? a + side : a) + (j * LY * C::ROW + i * LX * 8)));
-            t.g[j][i] = w.x;
-            t.h[j][i] = w.y;
+            const char *const e = (i == 0 ? a + side : a) + (j * LY * C::ROW + i * LX * 8);
+            if constexpr (decltype(cx)::value) {
+              const float2 w = __ldg(reinterpret_cast<const float2 *>(e));
+              t.g[j][i] = w.x;
+              t.h[j][i] = w.y;
+            } else {
+              t.g[j][i] = __ldg(reinterpret_cast<const float *>(e));
+            }
           });
         } else {
           uint32_t a = tab + (uint32_t)__float_as_int(q.x);
@@ -460,27 +474,34 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
         const float4 *st = stage + 2;
 #pragma unroll 1
         for (int f = 0; f < 8; ++f) {
-          const float4 *const end = st + ((int)(cnt >> (8 * f)) & 0xff);
-          if (st == end) continue;
+          int left = (int)(cnt >> (8 * f)) & 0xff;
+          if (left == 0) continue;
           select(f);
 #pragma unroll 1
           do {
-            const float4 qa = st[0], qb = st[1];
-            const u64 va = pk2(a.vr, a.vi), vb = pk2(b.vr, b.vi);
-            rt_for<0, Q>([&](auto JJ) {
-              constexpr int j = decltype(JJ)::value;
-              rt_for<0, NX>([&](auto II) {
-                constexpr int i = decltype(II)::value, l = C::PADX || (i > 0 && i < NX - 1) ? i : 0;
-                add_two(JJ, II, at_column(va, a.left, II), pk2(a.g[j][l], a.g[j][l]),
-                        at_column(vb, b.left, II), pk2(b.g[j][l], b.g[j][l]));
+            const int m = GT ? min(left, kRtRun) : left;
+            const float4 *const end = st + m;
+            left -= m;
+            in_step();
+#pragma unroll 1
+            do {
+              const float4 qa = st[0], qb = st[1];
+              const u64 va = pk2(a.vr, a.vi), vb = pk2(b.vr, b.vi);
+              rt_for<0, Q>([&](auto JJ) {
+                constexpr int j = decltype(JJ)::value;
+                rt_for<0, NX>([&](auto II) {
+                  constexpr int i = decltype(II)::value, l = C::PADX || (i > 0 && i < NX - 1) ? i : 0;
+                  add_two(JJ, II, at_column(va, a.left, II), pk2(a.g[j][l], a.g[j][l]),
+                          at_column(vb, b.left, II), pk2(b.g[j][l], b.g[j][l]));
+                });
+                load_row(a, qa, cx, JJ);
+                load_row(b, qb, cx, JJ);
               });
-              load_row(a, qa, cx, JJ);
-              load_row(b, qb, cx, JJ);
-            });
-            load_value(a, qa);
-            load_value(b, qb);
-            st += 2;
-          } while (st != end);
+              load_value(a, qa);
+              load_value(b, qb);
+              st += 2;
+            } while (st != end);
+          } while (left > 0);
         }
       };
       // The others one at a time, the table entries of one loaded while the
@@ -539,7 +560,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
             if (u * 32 + lane < n) top = max(top, max(rt_magnitude(pv[u].x), rt_magnitude(pv[u].y)));
           top = __reduce_max_sync(0xffffffffu, top);
           // twice the sum of the item's terms, were all of them as large
-          const float need = (GT || cplx ? 4.f : 2.f) * (float)(cur.w - cur.z + 8) *
+          const float need = (cplx ? 4.f : 2.f) * (float)(cur.w - cur.z + 8) *
                              (__uint_as_float(top) * factor_max);
           if (room == 0.f || !(need <= room)) rebase(need);
         }
@@ -574,9 +595,10 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
         if (k0 + kRtBlock < cur.w) fetch(k0 + kRtBlock, cur.w, plane);
         else fetch(nxt.z, nxt.w, P == 1 ? 0 : next % P);
         __syncwarp();
-        if (GT || cplx) add_block(even, std::true_type{});
-        else if constexpr (!GT && COMP) add_block_by_two(even, std::false_type{});
-        else if constexpr (!GT) add_block(even, std::false_type{});
+        if constexpr (GT && CX) add_block(even, std::true_type{});
+        else if (!GT && cplx) add_block(even, std::true_type{});
+        else if constexpr (COMP) add_block_by_two(even, std::false_type{});
+        else add_block(even, std::false_type{});
       }
       const int ox = tail.y, oy = tail.z;
       double2 *const slot = COMP && p.merge.base && tail.x >= 0
@@ -593,7 +615,8 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
         }
       const float2 zf = upk2(z);
       if (__any_sync(0xffffffffu, !(zf.x == 0.f && zf.y == 0.f))) {
-        rt_redo<S, COMP, GT>(p, p.items[item], plane, tr, GT || cplx, slot);
+        rt_redo<S, COMP, GT>(p, p.items[item], plane, tr, GT ? rt_info(J, cur.y).imag : cplx,
+                             slot);
         break;
       }
       if (!slot && !other) {
@@ -670,15 +693,16 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
   }
 }
 
-// tables read from global memory: any number of them, complex or not
-template <int S, bool COMP>
+// tables read from global memory, any number of them.  Both forms are launched
+// (the flag is on the device) and one of them returns at once: as two branches
+// of one kernel, the complex form of support 8 took 15 % longer.
+template <int S, bool COMP, bool CX>
 __global__ void __launch_bounds__(32 * RtCfg<S, true>::WARPS, 1)
     regtile_tables_kernel(const __grid_constant__ RegTileLaunch p) {
   extern __shared__ __align__(16) unsigned char smem[];
   after_predecessor();
-  rt_items<S, COMP, true>(p, nullptr,
-                          reinterpret_cast<float4 *>(smem) + (threadIdx.x >> 5) * kRtStage, true,
-                          0.f);
+  float4 *const stage = reinterpret_cast<float4 *>(smem) + (threadIdx.x >> 5) * kRtStage;
+  if ((*p.any_imag != 0) == CX) rt_items<S, COMP, true, CX>(p, nullptr, stage, CX, 0.f);
 }
 
 template <int S, bool COMP>
@@ -735,46 +759,63 @@ __global__ void __launch_bounds__(32 * RtCfg<S, false>::WARPS, 1)
   if (p.overlap) after_predecessor();
   const bool cplx = __syncthreads_or(imag);
   if (COMP && !p.gauss) top = s_top;
-  rt_items<S, COMP, false>(p, tr, stage, cplx, __uint_as_float(top));
+  rt_items<S, COMP, false, true>(p, tr, stage, cplx, __uint_as_float(top));
 }
 
-// Largest finite magnitude of every table of a class (blockIdx.y: jobs, those
-// that share a stack of tables once), zeroed by the caller: what the compensated
-// sums of regtile_tables_kernel choose their base by.
+constexpr int kInfoChunk = 1024;  // entries of a table that a block looks at
+
+// What regtile_tables_kernel needs to know of every table of a class (blockIdx.y:
+// jobs, those that share a stack of tables once): compensated sums choose their
+// base by the largest magnitude, and a class of tables without imaginary parts
+// takes half the products.
 __global__ void __launch_bounds__(256)
-    table_max_kernel(const JobDesc *jobs, int njobs, int entries) {
+    table_info_kernel(const JobDesc *jobs, int njobs, int entries, unsigned *any_imag) {
   after_predecessor();
-  const int chunk = min(entries, 4096);
+  const int chunk = min(entries, kInfoChunk);
   for (int j = blockIdx.y; j < njobs; j += gridDim.y) {
     const JobDesc &J = jobs[j];
-    if (!J.gcf_max_owner) continue;
+    if (!J.gcf_info_owner) continue;
     const int64_t chunks = (int64_t)J.n_gcf * (entries / chunk);
     for (int64_t c = blockIdx.x; c < chunks; c += gridDim.x) {
       const float2 *const t = static_cast<const float2 *>(J.gcf) + c * chunk;
       unsigned top = 0;
+      bool imag = false;
 #pragma unroll 4
       for (int i = threadIdx.x; i < chunk; i += 256) {
         const float2 v = __ldg(t + i);
+        imag = imag || v.y != 0.f;
         top = max(top, max(rt_magnitude(v.x), rt_magnitude(v.y)));
       }
       top = __reduce_max_sync(0xffffffffu, top);
-      if ((threadIdx.x & 31) == 0)
-        atomicMax(reinterpret_cast<unsigned *>(J.gcf_max + c / (entries / chunk)), top);
+      imag = __any_sync(0xffffffffu, imag);
+      if ((threadIdx.x & 31) == 0) {
+        TableInfo *const info = J.gcf_info + c / (entries / chunk);
+        atomicMax(&info->top, top);
+        if (imag) {
+          atomicOr(&info->imag, 1u);
+          atomicOr(any_imag, 1u);
+        }
+      }
     }
   }
 }
 
-template <int S, bool COMP> cudaError_t rt_launch(const RegTileLaunch &g, cudaStream_t s) {
-  const int warps = g.tables ? RtCfg<S, true>::WARPS : RtCfg<S, false>::WARPS;
-  const size_t smem =
-      g.tables ? warps * kRtStage * sizeof(float4) : regtile_smem_bytes(S, g.G);
-  auto kern = g.tables ? regtile_tables_kernel<S, COMP> : regtile_kernel<S, COMP>;
+template <int S, bool GT>
+cudaError_t rt_launch(void (*kern)(RegTileLaunch), const RegTileLaunch &g, cudaStream_t s) {
+  constexpr int warps = RtCfg<S, GT>::WARPS;
+  const size_t smem = GT ? warps * kRtStage * sizeof(float4) : regtile_smem_bytes(S, g.G);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
   const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(g.sm_count, g.max_items * g.P));
   count_launch();
   return launch_overlapped(kern, (unsigned)blocks, 32 * warps, smem, s, g.overlap, g);
+}
+
+template <int S, bool COMP> cudaError_t rt_launches(const RegTileLaunch &g, cudaStream_t s) {
+  if (!g.tables) return rt_launch<S, false>(regtile_kernel<S, COMP>, g, s);
+  const cudaError_t e = rt_launch<S, true>(regtile_tables_kernel<S, COMP, false>, g, s);
+  return e != cudaSuccess ? e : rt_launch<S, true>(regtile_tables_kernel<S, COMP, true>, g, s);
 }
 
 }  // namespace
@@ -784,19 +825,20 @@ size_t regtile_smem_bytes(int S, int G) {
   return 8 * (size_t)rt_table_floats(S, G) + (size_t)warps * kRtStage * sizeof(float4);
 }
 
-cudaError_t launch_table_max(const JobDesc *jobs, int njobs, int S, int G, int64_t tables,
-                             cudaStream_t s) {
+cudaError_t launch_table_info(const JobDesc *jobs, int njobs, int S, int G, int64_t tables,
+                              unsigned *any_imag, cudaStream_t s) {
   const int entries = G * G * S * S;
-  const int64_t chunks = tables * ((entries + 4095) / 4096);
+  const int64_t chunks = tables * ((entries + kInfoChunk - 1) / kInfoChunk);
   const int y = std::min(njobs, 1024), x = (int)std::min<int64_t>(chunks, std::max(1, 2048 / y));
   count_launch();
-  return launch_overlapped(table_max_kernel, dim3(x, y), 256, 0, s, true, jobs, njobs, entries);
+  return launch_overlapped(table_info_kernel, dim3(x, y), 256, 0, s, true, jobs, njobs, entries,
+                           any_imag);
 }
 
 cudaError_t launch_regtile(const RegTileLaunch &g, cudaStream_t s) {
   switch (g.S) {
-    case 8: return g.compensated ? rt_launch<8, true>(g, s) : rt_launch<8, false>(g, s);
-    case 16: return g.compensated ? rt_launch<16, true>(g, s) : rt_launch<16, false>(g, s);
+    case 8: return g.compensated ? rt_launches<8, true>(g, s) : rt_launches<8, false>(g, s);
+    case 16: return g.compensated ? rt_launches<16, true>(g, s) : rt_launches<16, false>(g, s);
   }
   return cudaErrorInvalidValue;
 }

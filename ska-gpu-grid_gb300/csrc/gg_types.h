@@ -24,6 +24,12 @@ constexpr int kSepTile = 8, kSepOff = 16, kSepBlock = 16;
 // register tiles; block side in cells.
 constexpr int kGatBlock = 16;
 
+// A complex64 table: the bits of its largest finite magnitude (of either part),
+// and whether it has any imaginary part.
+struct TableInfo {
+  unsigned top, imag;
+};
+
 // One gridding job as the kernels see it.  For the binned methods `idx` and
 // `vals` are the tile-sorted copies made by the binning pass: idx[k] is the
 // packed (main*G+sub) pair of sorted visibility k and vals holds P planes of
@@ -52,10 +58,10 @@ struct JobDesc {
   // flag that is nonzero when any imaginary part is (null: not available)
   const float *gcf_real;
   const int *gcf_imag;
-  // largest magnitudes of its tables (register tiles that read several tables,
-  // compensated sums), and whether this job's launch block finds them
-  float *gcf_max;
-  int gcf_max_owner;
+  // register tiles that read several tables: what is known of each, and whether
+  // this job's blocks find it out (one of those that share the tables)
+  TableInfo *gcf_info;
+  int gcf_info_owner;
 };
 
 // A slice of one uv tile's sorted visibilities: the unit of the device work
