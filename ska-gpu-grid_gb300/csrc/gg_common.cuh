@@ -136,6 +136,32 @@ __device__ __forceinline__ u64 two_sum2(u64 a, u64 b, u64 &e) {
   return s;
 }
 
+// Compensated sums of products.  A cell's sum starts at a number (sum_base) so
+// large that no sum of its terms leads out of its binade: every addition then
+// rounds to the same unit, and what it rounded off is exact to work out.  Two
+// terms va ga + vb gb go into the sum A and what A lost of them into l; of their
+// remainders only one intermediate rounds, to the size of vb gb.  Six packed
+// operations for two terms, where a two-sum of each takes 16.
+__device__ __forceinline__ void exact_add2(u64 &A, u64 &l, u64 va, u64 ga, u64 vb, u64 gb) {
+  const u64 n = fma2(vb, gb, fma2(va, ga, A));
+  l = add2(l, fma2(vb, gb, fma2(va, ga, sub2(A, n))));
+  A = n;
+}
+
+// finite magnitude as ordered bits, 0 for an infinity or NaN (those end up in
+// the sums all the same)
+__device__ __forceinline__ unsigned finite_magnitude(float x) {
+  const unsigned b = __float_as_uint(x) & 0x7fffffffu;
+  return b < 0x7f800000u ? b : 0u;
+}
+
+// 1.5 * 2^k, 2^k at least `need` (not finite if need is too large: the sums then
+// are not either, and are worked out again cell by cell)
+__device__ __forceinline__ float sum_base(float need) {
+  const unsigned b = __float_as_uint(fminf(fmaxf(need, 0x1p-124f), 0x1p127f));
+  return __uint_as_float((b & 0x7f800000u) + 0x00c00000u);
+}
+
 // ---------------------------------------------------------------------------
 // accumulators: one complex running sum per thread and cell
 // ---------------------------------------------------------------------------

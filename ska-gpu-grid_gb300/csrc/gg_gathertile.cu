@@ -28,7 +28,7 @@
 //
 // Bound by instruction issue (77 % of active cycles; 62 % of the shared-memory
 // wavefronts).  1.05 M visibilities of support 8 on 4096^2, whole call: 858 us
-// by 32-cell tiles, 227 now; 4.19 M, this kernel, 2.09 -> 0.56 ms.
+// by 32-cell tiles, 251 now.
 #include <algorithm>
 
 #include "gg_kernels.cuh"
@@ -39,7 +39,11 @@ namespace {
 
 constexpr int kGtB = kGatBlock;  // block side
 constexpr int kGtWarps = 16;
-constexpr int kGtRun = 16;
+// records summed plainly.  Errors against 64 bits with 16 / 8 / 4, where gather_kernel
+// has 5.7e-8, 6.0e-8 and 7.3e-8: 1 M random ones of support 8 on 800^2 6.2e-8 /
+// 5.0e-8 / 4.3e-8, on 200^2 6.4e-8 / 5.1e-8 / 4.3e-8, 1.05 M of tracks on 4096^2
+// 6.4e-8 / 5.4e-8 / 4.6e-8 (whole calls of that 221 / 251 / 318 us).
+constexpr int kGtRun = 8;
 constexpr int kGtStage = 36;  // a group of 32 and zeros for the read-ahead
 
 template <int S> struct GtCfg {

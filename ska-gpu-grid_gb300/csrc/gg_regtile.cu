@@ -32,7 +32,7 @@
 //    inside footprints.
 //  * Compensated sums: every cell's sum starts at a power of two and a half so
 //    large that the item's terms do not lead out of its binade, which makes
-//    what an addition rounds off exact to work out (rt_add2): three packed
+//    what an addition rounds off exact to work out (exact_add2): three packed
 //    operations a term, taken two at a time, where a TwoSum of each takes eight.
 //    No term is ever added to another plainly.  Runs of 16 summed plainly
 //    between TwoSums, as it was, take one and a half, but made the error of
@@ -138,32 +138,6 @@ __device__ __forceinline__ void rt_record(const RegTileLaunch &p, int k, int pla
 template <int S> __device__ __forceinline__ const float2 *rt_table(const JobDesc &J, int bin) {
   return reinterpret_cast<const float2 *>(J.gcf) +
          (size_t)(J.n_gcf > 1 ? bin % J.n_gcf : 0) * J.G * J.G * S * S;
-}
-
-// Compensated sums.  A cell's sum starts at `base`, a number so large that no
-// sum of the item's terms leads out of its binade: every addition then rounds
-// to the same unit, and what it rounded off is exact to work out.  Two terms
-// va ga + vb gb go into the sum A and what A lost of them into l; of their
-// remainders only one intermediate rounds, to the size of vb gb.  Six packed
-// operations for two terms, where a two-sum of each takes 16.
-__device__ __forceinline__ void rt_add2(u64 &A, u64 &l, u64 va, u64 ga, u64 vb, u64 gb) {
-  const u64 n = fma2(vb, gb, fma2(va, ga, A));
-  l = add2(l, fma2(vb, gb, fma2(va, ga, sub2(A, n))));
-  A = n;
-}
-
-// finite magnitude as ordered bits, 0 for an infinity or NaN (those end up in
-// the sums all the same)
-__device__ __forceinline__ unsigned rt_magnitude(float x) {
-  const unsigned b = __float_as_uint(x) & 0x7fffffffu;
-  return b < 0x7f800000u ? b : 0u;
-}
-
-// 1.5 * 2^k, 2^k at least `need` (not finite if need is too large: the sums then
-// are not either, and are worked out again cell by cell)
-__device__ __forceinline__ float rt_base(float need) {
-  const unsigned b = __float_as_uint(fminf(fmaxf(need, 0x1p-124f), 0x1p127f));
-  return __uint_as_float((b & 0x7f800000u) + 0x00c00000u);
 }
 
 __device__ __forceinline__ TableInfo rt_info(const JobDesc &J, int bin) {
@@ -328,7 +302,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
       // if all its values were this large, and the sums moved when a later
       // block needs more
       auto rebase = [&](float need) {
-        const float b = rt_base(2.f * need);
+        const float b = sum_base(2.f * need);
         const u64 old = base;
         base = pk2(b, b);
         if (room == 0.f) {
@@ -447,7 +421,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
       // terms va ga + vb gb into the sums of row j, column i
       auto add_two = [&](auto JJ, auto II, u64 va, u64 ga, u64 vb, u64 gb) {
         constexpr int j = decltype(JJ)::value, i = decltype(II)::value;
-        if constexpr (COMP) rt_add2(hi[i][j], lo[i][j], va, ga, vb, gb);
+        if constexpr (COMP) exact_add2(hi[i][j], lo[i][j], va, ga, vb, gb);
         else run[i][j] = fma2(vb, gb, fma2(va, ga, run[i][j]));
       };
       auto add = [&](const Taps &t, auto cx) {
@@ -557,7 +531,7 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
           unsigned top = 0;
 #pragma unroll
           for (int u = 0; u < PER; ++u)
-            if (u * 32 + lane < n) top = max(top, max(rt_magnitude(pv[u].x), rt_magnitude(pv[u].y)));
+            if (u * 32 + lane < n) top = max(top, max(finite_magnitude(pv[u].x), finite_magnitude(pv[u].y)));
           top = __reduce_max_sync(0xffffffffu, top);
           // twice the sum of the item's terms, were all of them as large
           const float need = (cplx ? 4.f : 2.f) * (float)(cur.w - cur.z + 8) *
@@ -749,7 +723,7 @@ __global__ void __launch_bounds__(32 * RtCfg<S, false>::WARPS, 1)
       tr[i] = v.x;
       ti[i] = v.y;
       imag |= v.y != 0.f;
-      if constexpr (COMP) top = max(top, max(rt_magnitude(v.x), rt_magnitude(v.y)));
+      if constexpr (COMP) top = max(top, max(finite_magnitude(v.x), finite_magnitude(v.y)));
     }
     if constexpr (COMP) {
       top = __reduce_max_sync(0xffffffffu, top);
@@ -784,7 +758,7 @@ __global__ void __launch_bounds__(256)
       for (int i = threadIdx.x; i < chunk; i += 256) {
         const float2 v = __ldg(t + i);
         imag = imag || v.y != 0.f;
-        top = max(top, max(rt_magnitude(v.x), rt_magnitude(v.y)));
+        top = max(top, max(finite_magnitude(v.x), finite_magnitude(v.y)));
       }
       top = __reduce_max_sync(0xffffffffu, top);
       imag = __any_sync(0xffffffffu, imag);
