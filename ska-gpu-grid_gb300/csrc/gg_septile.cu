@@ -25,21 +25,23 @@
 // A value that is not finite would reach cells outside its footprint through
 // the zeros: a block whose sums are not finite is summed again cell by cell.
 //
-// Compensated sums: runs of 16 records are summed plainly (about half of them
-// cover a given cell), then added into (hi, lo) by TwoSum.
+// Compensated sums: every cell's sum starts at a number so large that no term leads
+// out of its binade, which makes what an addition rounds off exact to work out
+// (exact_add2), two records at once; the sums are moved to a larger one when they
+// come to need it.
 //
 // Few blocks (small grids), compensated sums: the warps of a CTA share a
 // block, every warp takes every WARPS-th group of 32 records, and the partial
 // (hi, lo) sums are added by TwoSum in shared memory.  Plain sums stay one
 // sequence of additions.
 //
-// Bound by the FMA pipe (about 70 % of its cycles).  Measured on 16.8 M
-// visibilities of a uniform disk on 8192^2, whole call: the moving window's
-// shared-memory sub-grid 25.3 ms; this kernel 6.25 ms with all 8 multiply-adds
-// for every record, 5.52 with 4 where a range reaches half the rows, 4.95 with
-// half groups unrolled (two CTAs per SM: with three, which spill, 5.31).  Runs
-// of 32 records take another 0.6 off, with 1.3 times the error against 64
-// bits: not taken.
+// Bound by the FMA pipe.  16.8 M visibilities of a uniform disk on 8192^2, whole
+// call, and error against 64 bits: the moving window's shared-memory sub-grid 25.3
+// ms, 7.3e-8; this kernel 7.87 ms, 6.1e-8 (8 groups of two unrolled; 4 8.1, 16
+// 9.5; three CTAs per SM, which spill, 8.25; one record at once 9.8).  Four records
+// at once take 7.1 ms, but in random order into a complex128 grid have 6.3e-8 where
+// the moving window has 5.9e-8; runs of 16 summed plainly 4.95 ms with 9.3e-8 and
+// 9.2e-8: not taken.
 #include <algorithm>
 #include <type_traits>
 
@@ -53,9 +55,8 @@ constexpr int kSepS = 32, kSepB = kSepBlock;  // support, block side
 constexpr int kSepWarps = 8;
 constexpr int kSepRow = 64;  // floats of a padded factor row: tap 0 at 16
 
-constexpr int kSepRun = 16;  // records summed plainly: half a group
-// staged records of a warp: a group of 32 and zeros for the read-ahead
-constexpr int kSepStage = 36;
+constexpr int kSepAt = 2;  // records added at once
+constexpr int kSepStage = 32;  // staged records of a warp: a group
 
 // shared memory: factors [G][2][64] (copy c holds the row from its entry c
 // on), a staging block per warp, and the partial sums of a shared block
@@ -133,13 +134,11 @@ __device__ __noinline__ void sep_redo(const SepTileLaunch &p, const JobDesc &J, 
   for (int c = tid; c < kSepB * kSepB; c += nt) {
     const int x = x0 + c % kSepB, y = y0 + c / kSepB;
     u64 run = 0ull, hi = 0ull, lo = 0ull;
-    int since = 0;
     auto merge = [&]() {
       u64 e;
       hi = two_sum2(hi, run, e);
       lo = add2(lo, e);
       run = 0ull;
-      since = 0;
     };
     const int bx = x0 / kSepTile, by = y0 / kSepTile;
     for (int r = 0; r < 6; ++r) {
@@ -155,10 +154,9 @@ __device__ __noinline__ void sep_redo(const SepTileLaunch &p, const JobDesc &J, 
         if ((unsigned)a >= (unsigned)kSepS || (unsigned)b >= (unsigned)kSepS) continue;
         const float gx = gt[sx * 2 * kSepRow + 16 + a], gy = gt[sy * 2 * kSepRow + 16 + b];
         run = fma2(mul2(pk2(v.x, v.y), pk2(gx, gx)), pk2(gy, gy), run);
-        if (COMP && ++since == kSepRun) merge();
+        if (COMP) merge();
       }
     }
-    if (COMP) merge();
     sep_store<COMP>(J, x, y, plane, p.P, p.accumulate, upk2(COMP ? hi : run), upk2(lo));
   }
 }
@@ -170,14 +168,10 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 2 : 4)
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float *const gt = reinterpret_cast<float *>(smem);
-  // factor offsets and values of a group, and the zeros behind it
+  // factor offsets and values of a group
   float4 *const rec = reinterpret_cast<float4 *>(gt + sep_factor_floats(p.G)) + warp * kSepStage;
   float4 *const part = reinterpret_cast<float4 *>(gt + sep_factor_floats(p.G)) +
                        kSepWarps * kSepStage;
-  if (lane < kSepStage - 32) {
-    rec[32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-
   // padded factors: entry i of a row is tap i - 16, zero outside
   const float inv = 1.0f / (2.0f * p.sigma * p.sigma);
   for (int i = tid; i < p.G * 2 * kSepRow; i += NT) {
@@ -230,22 +224,39 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 2 : 4)
     const int first_end = __shfl_sync(0xffffffffu, sum, 0);
     const int last_beg = __shfl_sync(0xffffffffu, start, 5);
     for (int plane = 0; plane < p.P; ++plane) {
-      // cell k: column 2c + (k & 1), row 2h + (k >> 1 & 1) + 8 (k >> 2)
-      u64 run[8], hi[COMP ? 8 : 1], lo[COMP ? 8 : 1];
+      // cell k: column 2c + (k & 1), row 2h + (k >> 1 & 1) + 8 (k >> 2).  Plain
+      // sums, or sums from `base` on and their remainders.
+      u64 sum[8], lo[COMP ? 8 : 1];
+      u64 base = 0ull;
+      float room = 0.f, bound = 0.f;  // that `base` is good for, and of the sums
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        run[k] = 0ull;
-        if constexpr (COMP) hi[k] = lo[k] = 0ull;
+        sum[k] = 0ull;
+        if constexpr (COMP) lo[k] = 0ull;
       }
-      // the records of a half group, into the cells [K0, K1)
-      auto merge = [&](auto k0, auto k1) {
+      // the next terms add up to `more` at most: bound the sums by what they are
+      // (sums of random signs stay far below those of magnitudes), and if they
+      // and the terms need it move them to a larger base
+      auto make_room = [&](float more) {
         if constexpr (COMP) {
+          unsigned top = 0;
 #pragma unroll
-          for (int k = decltype(k0)::value; k < decltype(k1)::value; ++k) {
-            u64 e;
-            hi[k] = two_sum2(hi[k], run[k], e);
-            lo[k] = add2(lo[k], e);
+          for (int k = 0; k < 8; ++k) {
+            const float2 t = upk2(sub2(sum[k], base));
+            top = max(top, max(finite_magnitude(t.x), finite_magnitude(t.y)));
           }
+          bound = __uint_as_float(__reduce_max_sync(0xffffffffu, top)) + more;
+          if (room > 0.f && 4.f * bound <= room) return;
+          const float b = sum_base(16.f * bound);
+          const u64 b2 = pk2(b, b);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const u64 t = sub2(sum[k], base), n = add2(t, b2);
+            lo[k] = add2(lo[k], sub2(t, sub2(n, b2)));
+            sum[k] = n;
+          }
+          base = b2;
+          room = b * (1.f / 1.5f);
         }
       };
       // the list in groups of 32
@@ -282,69 +293,56 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 2 : 4)
           v = make_float2(0.f, 0.f);
         }
         rec[lane] = make_float4(__int_as_float(at.x), __int_as_float(at.y), v.x, v.y);
+        if constexpr (COMP) {
+          const unsigned top = __reduce_max_sync(
+              0xffffffffu, max(finite_magnitude(v.x), finite_magnitude(v.y)));
+          const float more = (float)m * __uint_as_float(top);  // factors are at most 1
+          bound += more;
+          if (!(2.f * bound <= room)) make_room(more);
+        }
         g += SHARE ? kSepWarps : 1;
         fetch(g);
         __syncwarp();
-        // the factors of a record are loaded while the previous one is added
+        // kSepAt records at once into the cells [K0, K1)
         auto group = [&](auto k0, auto k1) {
-          constexpr bool LOW = decltype(k0)::value == 0, HIGH = decltype(k1)::value == 8;
-          struct Taps {
-            float2 v, gx, g0, g1;
-          } a, b;
-          auto load = [&](Taps &t, const float4 o) {
-            t.gx = lds64(ax + __float_as_uint(o.x));
-            if constexpr (LOW) t.g0 = lds64(ay + __float_as_uint(o.y));
-            if constexpr (HIGH) t.g1 = lds64(ay + __float_as_uint(o.y) + 32);
-            t.v = make_float2(o.z, o.w);
-          };
-          // fresh: the first of a run, whose sums are zero
-          auto add = [&](const Taps &t, bool fresh) {
-            const u64 vv = pk2(t.v.x, t.v.y);
-            const u64 w0 = mul2(vv, pk2(t.gx.x, t.gx.x)), w1 = mul2(vv, pk2(t.gx.y, t.gx.y));
-            auto cell = [&](int k, u64 w, float g) {
-              run[k] = fresh ? mul2(w, pk2(g, g)) : fma2(w, pk2(g, g), run[k]);
-            };
-            if constexpr (LOW) {
-              cell(0, w0, t.g0.x);
-              cell(1, w1, t.g0.x);
-              cell(2, w0, t.g0.y);
-              cell(3, w1, t.g0.y);
-            }
-            if constexpr (HIGH) {
-              cell(4, w0, t.g1.x);
-              cell(5, w1, t.g1.x);
-              cell(6, w0, t.g1.y);
-              cell(7, w1, t.g1.y);
-            }
-          };
-          load(a, rec[0]);
-          float4 o = rec[1];
-          for (int i0 = 0; i0 < m; i0 += kSepRun) {
-            if (m - i0 >= kSepRun) {
+          constexpr int K0 = decltype(k0)::value, K1 = decltype(k1)::value;
+          constexpr bool LOW = K0 == 0, HIGH = K1 == 8;
+          auto add = [&](const float4 *o) {
+            u64 w[2][kSepAt];
+            float2 g0[kSepAt], g1[kSepAt];
 #pragma unroll
-              for (int i = 0; i < kSepRun; i += 2) {
-                load(b, o);
-                o = rec[i0 + i + 2];
-                add(a, COMP && i == 0);
-                load(a, o);
-                o = rec[i0 + i + 3];
-                add(b, false);
-              }
-            } else {
-              if constexpr (COMP)
+            for (int r = 0; r < kSepAt; ++r) {
+              const float4 t = o[r];
+              const float2 gx = lds64(ax + __float_as_uint(t.x));
+              if constexpr (LOW) g0[r] = lds64(ay + __float_as_uint(t.y));
+              if constexpr (HIGH) g1[r] = lds64(ay + __float_as_uint(t.y) + 32);
+              const u64 vv = pk2(t.z, t.w);
+              w[0][r] = mul2(vv, pk2(gx.x, gx.x));
+              w[1][r] = mul2(vv, pk2(gx.y, gx.y));
+            }
 #pragma unroll
-                for (int k = 0; k < 8; ++k) run[k] = 0ull;
+            for (int k = K0; k < K1; ++k) {
+              auto terms = [&](u64 a) {
+#pragma unroll
+                for (int r = 0; r < kSepAt; ++r) {
+                  const float2 gy = k < 4 ? g0[r] : g1[r];
+                  const float g = k & 2 ? gy.y : gy.x;
+                  a = fma2(w[k & 1][r], pk2(g, g), a);
+                }
+                return a;
+              };
+              const u64 n = terms(sum[k]);
+              // what the sum lost of them, see exact_add2
+              if constexpr (COMP) lo[k] = add2(lo[k], terms(sub2(sum[k], n)));
+              sum[k] = n;
+            }
+          };
+          if (m == 32) {
+#pragma unroll 8
+            for (int i = 0; i < 32; i += kSepAt) add(rec + i);
+          } else {
 #pragma unroll 1
-              for (int i = i0; i < m; i += 2) {
-                load(b, o);
-                o = rec[i + 2];
-                add(a, false);
-                load(a, o);
-                o = rec[i + 3];
-                add(b, false);
-              }
-            }
-            merge(k0, k1);
+            for (int i = 0; i < m; i += kSepAt) add(rec + i);
           }
         };
         using std::integral_constant;
@@ -355,13 +353,17 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 2 : 4)
         else
           group(integral_constant<int, 0>(), integral_constant<int, 8>());
       }
+      if constexpr (COMP) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) sum[k] = sub2(sum[k], base);
+      }
       bool bad = false;
       if constexpr (SHARE) {
         // cell (x, y) of warp w at part[w][16 y + x]
         __syncthreads();  // the previous block's partial sums were read
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const float2 a = upk2(COMP ? hi[k] : run[k]);
+          const float2 a = upk2(sum[k]);
           float2 l = make_float2(0.f, 0.f);
           if constexpr (COMP) l = upk2(lo[k]);
           part[warp * 256 + row(k) * 16 + 2 * c + (k & 1)] = make_float4(a.x, a.y, l.x, l.y);
@@ -387,10 +389,7 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 2 : 4)
       } else {
         u64 z = 0ull;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          if constexpr (COMP) z = fma2(hi[k], 0ull, z);
-          else z = fma2(run[k], 0ull, z);
-        }
+        for (int k = 0; k < 8; ++k) z = fma2(sum[k], 0ull, z);
         const float2 zf = upk2(z);
         bad = __any_sync(0xffffffffu, !(zf.x == 0.f && zf.y == 0.f));
         if (!bad) {
@@ -399,7 +398,7 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 2 : 4)
             float2 l = make_float2(0.f, 0.f);
             if constexpr (COMP) l = upk2(lo[k]);
             sep_store<COMP>(J, x0 + 2 * c + (k & 1), y0 + row(k), plane, p.P, p.accumulate,
-                            upk2(COMP ? hi[k] : run[k]), l);
+                            upk2(sum[k]), l);
           }
         } else {
           sep_redo<COMP>(p, J, x0, y0, plane, gt, lane, 32);
