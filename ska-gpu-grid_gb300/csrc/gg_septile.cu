@@ -82,6 +82,8 @@ template <bool COMP>
 __device__ __forceinline__ void sep_store(const JobDesc &J, int gx, int gy, int plane, int P,
                                           bool accumulate, const float2 h, const float2 l) {
   if (gx >= J.N || gy >= J.N) return;
+  // a grid that is added into: its other cells stay as they are
+  if (accumulate && h.x == 0.f && h.y == 0.f && l.x == 0.f && l.y == 0.f) return;
   const size_t cell = (size_t)gy * J.N + gx, NN = (size_t)J.N * J.N;
   // FP64 sums only for a complex128 grid: the FP64 pipe is narrow
   if (J.out_f64) {
@@ -223,7 +225,9 @@ __global__ void __launch_bounds__(32 * kSepWarps, COMP ? 2 : 4)
     const int records = __shfl_sync(0xffffffffu, sum, 5);
     const int first_end = __shfl_sync(0xffffffffu, sum, 0);
     const int last_beg = __shfl_sync(0xffffffffu, start, 5);
-    for (int plane = 0; plane < p.P; ++plane) {
+    // nothing to add: no cell is touched
+    const int planes = p.accumulate && records == 0 ? 0 : p.P;
+    for (int plane = 0; plane < planes; ++plane) {
       // cell k: column 2c + (k & 1), row 2h + (k >> 1 & 1) + 8 (k >> 2).  Plain
       // sums, or sums from `base` on and their remainders.
       u64 sum[8], lo[COMP ? 8 : 1];
