@@ -250,9 +250,11 @@ struct Plan {
   int merge_cap[kMaxClasses] = {}, merge_cells[kMaxClasses] = {};
   // workspace carve (offsets into the device workspace)
   size_t o_jobs, o_bin, o_visb, o_tileb, o_class, o_rank, o_cnt, o_bm, o_scan, o_sidx, o_svals,
-      o_order, o_items, o_kept, o_lo, o_gcf_info, o_count_vals, o_count_gcf, ws_bytes;
+      o_order, o_items, o_kept, o_lo, o_gcf_info, o_sep_mask, o_sep_dense, o_sep_slots,
+      o_count_vals, o_count_gcf, ws_bytes;
   int64_t vstride = 0, class_cap = 0;
   size_t gcf_info_n = 0;   // tables whose TableInfo is wanted
+  int64_t sep_dense_cap = 0;
   size_t table_bytes = 0;  // bytes uploaded from staging (jobs..class)
   char *ws = nullptr;      // workspace the addresses are bound to
 };
@@ -773,6 +775,16 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     }
     pl.o_gcf_flags = take(sizeof(int) * (pl.gcf_copies.size() + 1));
   }
+  // support 32 by output blocks: which are reached, the dense ones and their
+  // merge slots
+  if (mode == GG_MODE_WINDOW && cfgs.begin()->second.kind == kSep) {
+    int64_t blocks = 0;
+    for (int j = 0; j < njobs; ++j) blocks += septile_blocks(jobs[j].img_dim);
+    pl.sep_dense_cap = septile_dense_cap(vis, blocks, c->sm_count);
+    pl.o_sep_mask = take((blocks + 31) / 32 * sizeof(unsigned));
+    pl.o_sep_dense = take(sizeof(int4) * pl.sep_dense_cap);
+    pl.o_sep_slots = take(sizeof(double2) * kSepBlock * kSepBlock * pl.P * pl.sep_dense_cap);
+  }
   // register tiles that read several tables: what is known of each, once for
   // jobs that share them (k -> first table, owner)
   std::vector<std::pair<size_t, bool>> gcf_info(njobs, {SIZE_MAX, false});
@@ -1175,6 +1187,14 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
         q.accumulate = opt->accumulate;
         q.sigma = pl.sigma;
         q.sm_count = sm_count;
+        q.vis = cl.v1 - cl.v0;
+        q.overlap = !prof;
+        q.mask = (unsigned *)(ws + pl.o_sep_mask);
+        q.dense = (int4 *)(ws + pl.o_sep_dense);
+        q.slots = (double2 *)(ws + pl.o_sep_slots);
+        q.dense_cap = (int)pl.sep_dense_cap;
+        // two of the item counters, which this class has no use for
+        q.dense_count = (unsigned long long *)(flags + 8);
         GG_CUDA(launch_septile(q, s));
       } else if (cl.kind == kReg || cl.kind == kTab) {
         RegTileLaunch r{};

@@ -284,7 +284,31 @@ struct SepTileLaunch {
   int accumulate;          // add into the grid instead of storing
   float sigma;
   int sm_count;
+  int64_t vis;             // visibilities of the class
+  int overlap;             // follow each other by launch_overlapped
+  // what sep_plan_kernel finds: a bit for every block that is summed as a whole,
+  // and the dense ones {block, first unit, units, units done} with a merge slot
+  // of P * 256 sums each; dense_count (slots taken << 32 | units) zeroed by the
+  // caller
+  unsigned *mask;
+  int4 *dense;
+  double2 *slots;
+  unsigned long long *dense_count;
+  int dense_cap;           // septile_dense_cap
+  int dense_min, dense_unit, chunk;  // set by launch_septile
 };
+// More records than this make a block of support 32 dense: half a resident
+// warp's share of all the visits that records pay to blocks (9 a record), so that
+// no block keeps one warp much longer than the others; from 1024 records on.
+inline int septile_dense_min(int64_t vis, int sm_count) {
+  const int64_t half = 9 * vis / ((int64_t)sm_count * 32);
+  return (int)(half > 1024 ? half : 1024);
+}
+// Dense blocks that there can be.
+inline int64_t septile_dense_cap(int64_t vis, int64_t blocks, int sm_count) {
+  const int64_t most = 9 * vis / septile_dense_min(vis, sm_count) + 1;
+  return most < blocks ? most : blocks;
+}
 cudaError_t launch_septile(const SepTileLaunch &g, cudaStream_t s);
 // Gather by output block (gg_gathertile.cu): FP32 values, support 8 or 16, one
 // GCF table per launch.
