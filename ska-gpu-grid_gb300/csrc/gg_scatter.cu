@@ -37,14 +37,19 @@ namespace gg {
 
 constexpr int kScatterThreads = 256;
 // resident on an SM (FP64 values, support 16, the case below: 2 CTAs 362 us of
-// the whole call, 3 324, 4 305, 5 310)
-constexpr int kScatterCtas = 4;
+// the whole call, 3 324, 4 305, 5 310).  FP32 values, plain sums, several planes,
+// 524 k visibilities of support 8 on 1024^2: two 160 us with 4, 152 with 5 and
+// 159 with 6, four 290, 278 and 272; one 90, 95 and 98.
+constexpr int kScatterCtas = 4, kScatterCtasPlanes = 5;
 // Compensated sums wait for the previous value of every tap: more warps hide
-// it, until those on the same cells get in each other's way.  Support 16, on
-// tracks, us: 262 k visibilities 286 / 275 / 325 with 4 / 5 / 6 CTAs, 1 M 995 /
-// 942 / 934 (sorted by tile 983 / 956 / 966), 4.19 M 4270 / 4012 / 3613.
+// it, until those on the same cells get in each other's way, which takes longer
+// on small footprints.  us with 4 / 5 / 6 CTAs, on tracks: support 4, 1 M
+// visibilities 212 / 198 / 179, 4 M 715 / 657 / 574; support 8, 100 k 58 / 60 / 57,
+// 1 M 317 / 300 / 298, 3 M 855 / 799 / 809; support 16, 262 k 286 / 275 / 325, 1 M
+// 995 / 942 / 934, 4.19 M 4270 / 4012 / 3613; support 32, 300 k 1264 / 1088 /
+// 1193, 2 M 8515 / 7301 / 6634.
 constexpr int kScatterCtasComp = 5, kScatterCtasLarge = 6;
-constexpr int64_t kScatterLarge = 1 << 21;  // visibilities
+constexpr int64_t kScatterLarge = 1 << 21;  // visibilities, supports 16 and 32
 
 __device__ __forceinline__ int find_job_v(const int64_t *base, int njobs,
                                           int64_t g) {
@@ -352,9 +357,14 @@ static cudaError_t scatter_dispatch(const GridLaunch &g, const KParams &kp,
                             : scatter_launch<S, ACCT, 0, CTAS>(kp, g.sm_count, s))
   if (g.vals_f64) GG_SC(AccF64, kScatterCtas);
   if (g.accum == GG_ACC_COMPENSATED) {
-    if (g.total_vis >= kScatterLarge) GG_SC(AccComp, kScatterCtasLarge);
-    GG_SC(AccComp, kScatterCtasComp);
+    if constexpr (S <= 8) {
+      GG_SC(AccComp, kScatterCtasLarge);
+    } else {
+      if (g.total_vis >= kScatterLarge) GG_SC(AccComp, kScatterCtasLarge);
+      GG_SC(AccComp, kScatterCtasComp);
+    }
   }
+  if (g.P > 1) GG_SC(AccF32, kScatterCtasPlanes);
   GG_SC(AccF32, kScatterCtas);
 #undef GG_SC
 }
