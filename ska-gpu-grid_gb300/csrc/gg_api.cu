@@ -538,10 +538,11 @@ static int64_t tile_side(int64_t N, int S, const ClassCfg &cf) {
 // Build the plan for a batch: validate, resolve, order jobs by support class,
 // lay out the workspace.  No device work.  `force` fixes the configuration of
 // support classes (autotuner trials); `bin_only`: the caller wants the tiles
-// of set_bookmarks (gg_bin), nothing is gridded.
+// of set_bookmarks (gg_bin), nothing is gridded; `general`: the methods' general
+// kernels only.
 static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
                       int njobs, Plan &pl, const ClassCfgs *force = nullptr,
-                      bool bin_only = false) {
+                      bool bin_only = false, bool general = false) {
   int st = check_options(opt);
   if (st) return st;
   if (njobs < 1) return fail(GG_ERR_ARG, "no jobs");
@@ -578,10 +579,12 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
           if (e) cf = e->cfg;
         }
       }
-      if (m0 == GG_MODE_GATHER && !bin_only && gathertile_class(opt, jobs, njobs, S)) {
+      if (bin_only || general) {
+        cf.kind = kOwn;
+      } else if (m0 == GG_MODE_GATHER && gathertile_class(opt, jobs, njobs, S)) {
         cf.kind = kGat;
         cf.T = kRegTile;
-      } else if (m0 == GG_MODE_WINDOW && !bin_only) {
+      } else if (m0 == GG_MODE_WINDOW) {
         if (septile_class(opt, jobs, njobs, S)) {
           cf.kind = kSep;
           cf.T = kSepTile;
@@ -680,7 +683,14 @@ static int plan_build(gg_context *c, const gg_options *opt, const gg_job *jobs,
     tiles += (int64_t)ntx * ntx * (J.gcf_index ? J.n_gcf : 1);
   }
   if (vis >= (1ll << 31) - 1024) return fail(GG_ERR_ARG, "batch has >= 2^31 visibilities");
-  if (tiles >= (1ll << 30)) return fail(GG_ERR_ARG, "batch has too many uv tiles");
+  if (tiles >= (1ll << 30)) {
+    // the tile kernels' uv tiles are smaller and start before the grid: a batch
+    // may have too many of them, but not of the general kernels'
+    if (!general && !bin_only) {
+      return plan_build(c, opt, jobs, njobs, pl, force, false, true);
+    }
+    return fail(GG_ERR_ARG, "batch has too many uv tiles");
+  }
   pl.mode = mode;
   if (mode == GG_MODE_WINDOW) {
     for (int j = 0; j < njobs; ++j) {
