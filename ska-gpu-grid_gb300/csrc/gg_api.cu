@@ -1569,14 +1569,18 @@ int gg_reserve(gg_context *ctx, const gg_options *opt, int64_t max_npts,
   int st = plan_build(ctx, opt, &j, 1, pl);
   if (st) return st;
   size_t ws = pl.ws_bytes, tables = pl.table_bytes;
-  // smaller supports can take another kernel with more workspace
-  for (const int S : {4, 8, 16}) {
-    if (S >= max_gcf_dim) break;
-    Plan small;
+  // smaller supports can take another kernel with more workspace, and so can
+  // grids aligned to one float
+  for (const int S : {4, 8, 16, 32}) {
+    if (S > max_gcf_dim) break;
     j.gcf_dim = S;
-    if (plan_build(ctx, opt, &j, 1, small)) continue;
-    ws = std::max(ws, small.ws_bytes);
-    tables = std::max(tables, small.table_bytes);
+    for (const uintptr_t out : {16, 4}) {
+      Plan other;
+      j.out = (void *)out;
+      if (plan_build(ctx, opt, &j, 1, other)) continue;
+      ws = std::max(ws, other.ws_bytes);
+      tables = std::max(tables, other.table_bytes);
+    }
   }
   g_last_error.clear();
   GG_CUDA(cudaEventSynchronize(ctx->exec_done));
