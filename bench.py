@@ -258,6 +258,16 @@ def red_peaks(dev):
     return _RED
 
 
+def kernel_name(method, support, w):
+    """the gridding kernel that a single job's call takes"""
+    if w["vals"] == "c64":
+        if method == "window" and support == 32 and w.get("gcf") == "gauss":
+            return "septile_kernel"
+        if method in ("window", "gather") and support in (8, 16):
+            return {"window": "regtile_kernel", "gather": "gathertile_kernel"}[method]
+    return f"{method}_kernel"
+
+
 def roofline(kernel, alg_bytes, kern_ms, tag, taps=None, dev=0):
     hbm, kind = peaks()
     achieved = alg_bytes / (kern_ms / 1e3) / 1e9
@@ -1109,7 +1119,7 @@ def run_single(args, rank, world, local_rank, dist):
         "phase_ms": {"setup_and_binning": round(statistics.mean(bin_ms), 4),
                      "gridding_kernel": round(mean_kern, 4)},
         "accuracy": err, "flags": flags,
-        "roofline": roofline(f"{mode_name}_kernel", alg, mean_kern,
+        "roofline": roofline(kernel_name(mode_name, S, w), alg, mean_kern,
                              f"{mode_name}_{args.workload}", n * S * S, local_rank),
         "cpu_baseline": cpu_baseline(w, rank),
         "e2e": e2e, "gpu_launches": int(launches),

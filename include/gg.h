@@ -62,7 +62,10 @@ extern "C" {
 
 /* ---- accumulation ------------------------------------------------------ */
 #define GG_ACC_PLAIN 0       /* arithmetic in the values' precision         */
-#define GG_ACC_COMPENSATED 1 /* FP32 two-sum hi/lo per cell (FP32 values)    */
+#define GG_ACC_COMPENSATED 1 /* FP32 values: FP32 sums with their rounding
+                                errors kept beside them; gather adds runs of
+                                up to 8 visibilities plainly (32 by its general
+                                kernel, as does the general moving window)    */
 
 /* ---- GCF source -------------------------------------------------------- */
 #define GG_GCF_TABLE 0    /* tabulated [G*G][S][S] complex (init_gcf layout)  */
@@ -232,7 +235,7 @@ int gg_grid_device(gg_context *ctx, const gg_options *opt, const gg_job *job,
  * the table (or Gaussian) and gcf_index/n_gcf select the kernel as for
  * gridding.  Visibilities with an oversample or table index out of range get
  * zero and are counted (gg_read_flags()[0]).  FP32 values: plain FP32 sums,
- * or two-sum compensated ones with GG_ACC_COMPENSATED; FP64 values: FP64.
+ * or compensated ones with GG_ACC_COMPENSATED; FP64 values: FP64.
  * Asynchronous on `stream`; no workspace, no allocation. */
 int gg_degrid_device(gg_context *ctx, const gg_options *opt, const gg_job *job,
                      void *stream);

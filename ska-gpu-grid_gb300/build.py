@@ -27,8 +27,9 @@ PROBE_SRC = "gg_probe.cu"
 PROBE_LIB = os.path.join(HERE, "libgg_probe.so")
 INCLUDE = os.path.join(ROOT, "include")
 
-SOURCES = ["gg_api.cu", "gg_bin.cu", "gg_scatter.cu", "gg_window.cu", "gg_regtile.cu", "gg_septile.cu", "gg_gathertile.cu",
-           "gg_gather.cu", "gg_noalloc.cu", "gg_server.cu", "gg_degrid.cu", "gg_image.cu"]
+SOURCES = ["gg_api.cu", "gg_bin.cu", "gg_scatter.cu", "gg_window.cu", "gg_regtile.cu",
+           "gg_septile.cu", "gg_gathertile.cu", "gg_gather.cu", "gg_noalloc.cu", "gg_server.cu",
+           "gg_degrid.cu", "gg_image.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

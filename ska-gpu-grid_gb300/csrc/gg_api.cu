@@ -195,7 +195,8 @@ static int check_options(const gg_options *o) {
 // context and plan
 // ---------------------------------------------------------------------------
 // Kernel of a class: the method's own; the register-tile form of the moving
-// window with one table in shared memory, or with tables in global memory; the output-block forms of support 32 with the Gaussian and of gather
+// window with one table in shared memory, or with tables in global memory; the
+// output-block forms of support 32 with the Gaussian and of gather
 enum ClassKind { kOwn = 0, kReg, kTab, kSep, kGat };
 
 struct Plan {
@@ -1045,7 +1046,8 @@ static int plan_enqueue(const gg_options *opt, const Plan &pl, int *flags, int s
 
   // One launch writes the tables and clears what starts at zero: the binning's
   // counters and, of a single job, an output small enough (4 MB: 2 us) not to
-  // be worth a stream of its own.
+  // be worth a stream of its own.  (A larger one's tile kernel then waits for
+  // that stream, and does not fill its table while the binning ends.)
   ZeroRanges zero{};
   if (binned) {
     zero.add(ws + pl.o_cnt, ((size_t)(pl.total_tiles + 1) * sizeof(int) + 15) & ~(size_t)15);

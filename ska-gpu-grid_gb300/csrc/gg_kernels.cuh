@@ -31,7 +31,7 @@ struct KParams {
 };
 
 // GCF value of tap (a', b') of sub-kernel (sx, sy); KIND 0 table, 1 Gaussian
-// computed on the fly, 2 the reference's per-visibility COMPUTE_GCF factor
+// computed on the fly
 template <int S, int KIND, typename VT>
 struct GcfSrc;
 
@@ -62,18 +62,8 @@ struct GcfSrc<S, 1, VT> {
 };
 
 // COMPUTE_GCF as the reference's scatter kernel evaluates it: one factor per
-// visibility (set by the caller from wphase_factor), the same for every tap
-template <int S, typename VT>
-struct GcfSrc<S, 2, VT> {
-  float fr, fi;
-  __device__ __forceinline__ void value(int, int, int, int, VT &gr, VT &gi) const {
-    gr = (VT)fr;
-    gi = (VT)fi;
-  }
-};
-
-// The factor of GcfSrc<S, 2>: (T, w) = the centre-offset table entry; dx, dy
-// in double then float, the rest in float, each step rounded as written
+// visibility, the same for every tap.  (T, w) = the centre-offset table entry;
+// dx, dy in double then float, the rest in float, each step rounded as written
 // (no contraction), sine and cosine from the device library.
 __device__ __forceinline__ float2 wphase_factor(double u, double v, int mx, int sx, int my,
                                                 int sy, int G, double T, double w) {

@@ -11,7 +11,6 @@ namespace gg {
 enum { FLAG_INDEX = 0, FLAG_TIMEOUT = 1, FLAG_UNSORTED = 2, FLAG_BOUNDS = 3 };
 
 constexpr int kMaxPols = 8;
-constexpr int kBinThreads = 256;
 
 // Register-tile classes (gg_regtile.cu): uv tiles of 8 cells whose numbering
 // starts kRegOff cells before the grid, so that every visibility that can
