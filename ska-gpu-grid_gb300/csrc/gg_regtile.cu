@@ -58,15 +58,16 @@
 // 1.2e-7; now 825, 8.0e-8 (with 12 warps a CTA instead of 8, whose registers
 // spill, 910; two records at once 850).
 //
-// Bound by the FMA pipe and its latency: support 16, 2.1 M records of tracks, 62 %
-// of the heavy half's cycles, 61 % of the issue slots, 113 warp instructions a
-// record with 12 warps an SM (8 warps without spills: the same for large jobs, 93
-// instead of 78 us for 100 k records on 777^2).  Whole calls against
-// window_kernel, us, and errors against 64 bits:
-//   4.19 M records of support 8 on 4096^2     590 -> 383   5.4e-8 -> 4.6e-8
-//   10 k of support 8 on 256^2                 86 -> 32    8.0e-8 -> 4.3e-8
-//   100 k of support 16 on 777^2              124 -> 78    7.3e-8 -> 5.3e-8
-//   256 mixed jobs, 45 M records             6481 -> 5476  7.8e-8 -> 5.6e-8
+// Bound by the FMA pipe, its latency and issue: 256 mixed jobs, support 8 / 16, 54 % of
+// the pipe's cycles and 65 / 61 % of the issue slots, with 12 warps an SM for
+// support 16 (8 warps without spills: the same for large jobs, 93 instead of 78 us
+// for 100 k records on 777^2; 16 of 128 registers: 5 % slower; four records at once:
+// 3.5 % faster, but in random order less exact than window_kernel).  Whole calls
+// against window_kernel, us, and errors against 64 bits:
+//   4.19 M records of support 8 on 4096^2     576 -> 369   5.4e-8 -> 4.6e-8
+//   10 k of support 8 on 256^2                 86 -> 32    8.0e-8 -> 4.2e-8
+//   100 k of support 16 on 777^2              125 -> 79    7.3e-8 -> 5.3e-8
+//   256 mixed jobs, 45 M records             6491 -> 5327  7.8e-8 -> 5.6e-8
 // (plain runs of 16: 356, 32, 68 and 4429 us with 7.1e-8, 7.5e-8, 9.1e-8, 9.0e-8).
 #include <algorithm>
 
@@ -441,7 +442,8 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
       // even numbers) for each.  Compensated, two at a time by tables without
       // imaginary parts: a row's factors of the next two are loaded once it has
       // been added.
-      auto add_block_by_two = [&](u64 cnt, auto cx) {
+      auto add_block_by_two = [&](u64 cnt) {
+        constexpr std::false_type cx{};
         Taps a, b;
         load(a, stage[0], cx);
         load(b, stage[1], cx);
@@ -476,6 +478,70 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
               st += 2;
             } while (st != end);
           } while (left > 0);
+        }
+      };
+      // Compensated, a table in shared memory: two at a time without imaginary parts,
+      // else one, and nothing loaded ahead, so that the rows that fy selects are the
+      // same for a whole share and registers suffice.  For support 16 without
+      // imaginary parts add_block_by_two takes 1 % less time.  add_block for complex
+      // tables, 6 % faster for them, made the real ones 2 to 5 % slower (386 instead
+      // of 369 us for 4.19 M records of support 8).
+      auto add_share = [&](const float4 *st, const float4 *end, int f, auto cx) {
+        constexpr bool CXR = decltype(cx)::value;
+        constexpr int N2 = CXR ? 1 : 2;
+        uint32_t at[PAIRS];
+#pragma unroll
+        for (int j = 0; j < PAIRS; ++j) at[j] = tab + (f > ly + LY * j ? C::SUB : 0);
+        const int left_below = (lx + 1) << 8;
+#pragma unroll 1
+        do {
+          float4 q[N2];
+          uint32_t side[N2];
+          bool left[N2];
+#pragma unroll
+          for (int r = 0; r < N2; ++r) {
+            q[r] = st[r];
+            left[r] = __float_as_int(q[r].y) < left_below;
+            side[r] = __float_as_uint(q[r].x) + (C::PADX || left[r] ? 0 : 64);
+          }
+          rt_for<0, Q>([&](auto JJ) {
+            constexpr int j = decltype(JJ)::value;
+            const uint32_t row = j < PAIRS ? at[j < PAIRS ? j : 0] : tab;
+            float g[N2][C::NL], h[N2][C::NL];
+#pragma unroll
+            for (int r = 0; r < N2; ++r)
+              rt_for<0, C::NL>([&](auto II) {
+                constexpr int i = decltype(II)::value;
+                constexpr int OFF = j * LY * C::ROW + i * LX * 4;
+                const uint32_t a =
+                    row + (!C::PADX && i == 0 ? side[r] : __float_as_uint(q[r].x));
+                g[r][i] = lds<OFF>(a);
+                if constexpr (CXR) h[r][i] = lds<OFF>(a + im_off);
+              });
+            rt_for<0, NX>([&](auto II) {
+              constexpr int i = decltype(II)::value, l = C::PADX || (i > 0 && i < NX - 1) ? i : 0;
+              const u64 va = at_column(pk2(q[0].z, q[0].w), left[0], II);
+              const u64 ga = pk2(g[0][l], g[0][l]);
+              if constexpr (CXR)
+                add_two(JJ, II, va, ga, at_column(pk2(-q[0].w, q[0].z), left[0], II),
+                        pk2(h[0][l], h[0][l]));
+              else
+                add_two(JJ, II, va, ga, at_column(pk2(q[1].z, q[1].w), left[1], II),
+                        pk2(g[1][l], g[1][l]));
+            });
+          });
+          st += N2;
+        } while (st != end);
+      };
+      auto add_shares = [&](u64 cnt, auto cx) {
+        const float4 *st = stage;
+#pragma unroll 1
+        for (int f = 0; f < 8; ++f) {
+          const float4 *const end = st + ((int)(cnt >> (8 * f)) & 0xff);
+          if (st == end) continue;
+          select(f);
+          add_share(st, end, f, cx);
+          st = end;
         }
       };
       // The others one at a time, the table entries of one loaded while the
@@ -569,10 +635,18 @@ __device__ __forceinline__ void rt_items(const RegTileLaunch &p, const float *tr
         if (k0 + kRtBlock < cur.w) fetch(k0 + kRtBlock, cur.w, plane);
         else fetch(nxt.z, nxt.w, P == 1 ? 0 : next % P);
         __syncwarp();
-        if constexpr (GT && CX) add_block(even, std::true_type{});
-        else if (!GT && cplx) add_block(even, std::true_type{});
-        else if constexpr (COMP) add_block_by_two(even, std::false_type{});
-        else add_block(even, std::false_type{});
+        if constexpr (!COMP) {
+          if (cplx) add_block(even, std::true_type{});
+          else add_block(even, std::false_type{});
+        } else if constexpr (GT) {
+          if constexpr (CX) add_block(even, std::true_type{});
+          else add_block_by_two(even);
+        } else if (cplx) {
+          add_shares(even, std::true_type{});
+        } else {
+          if constexpr (S == 8) add_shares(even, std::false_type{});
+          else add_block_by_two(even);
+        }
       }
       const int ox = tail.y, oy = tail.z;
       double2 *const slot = COMP && p.merge.base && tail.x >= 0
