@@ -26,8 +26,8 @@
 //  * Few blocks (small grids): the warps of a CTA share a block and add their
 //    (hi, lo) sums by TwoSum in shared memory.
 //
-// Bound by instruction issue (77 % of active cycles; 62 % of the shared-memory
-// wavefronts).  1.05 M visibilities of support 8 on 4096^2, whole call: 858 us
+// Bound by instruction issue (76 % of active cycles; 54 % of the FMA pipe's and of
+// the shared-memory wavefronts).  1.05 M visibilities of support 8 on 4096^2, whole call: 858 us
 // by 32-cell tiles, 251 now.
 #include <algorithm>
 
